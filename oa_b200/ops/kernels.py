@@ -991,9 +991,12 @@ def rnn_scan_bwd(gates_i, w_hh, b_hh, hprev, dout, gates: int):
             dgh[:, t] = gh_g
         dh0.copy_(carry)
         return dgi, dgh, dh0
-    _launch(N.require().oa_rnn_scan_bwd(dt(gates_i), gates, gates_i.contiguous().data_ptr(), w_hh.contiguous().data_ptr(), N.ptr(b_hh),
-                                        hprev.data_ptr(), dout.contiguous().data_ptr(), dgi.data_ptr(), dgh.data_ptr(), dh0.data_ptr(),
-                                        B, S, H, N.stream()), "oa_rnn_scan_bwd")
+    lib = N.require()
+    n = lib.oa_rnn_scan_bwd_scratch_floats(gates, B, S, H)
+    sc = torch.empty(n, dtype=torch.float32, device=gates_i.device) if n else None
+    _launch(lib.oa_rnn_scan_bwd(dt(gates_i), gates, gates_i.contiguous().data_ptr(), w_hh.contiguous().data_ptr(), N.ptr(b_hh),
+                                hprev.data_ptr(), dout.contiguous().data_ptr(), dgi.data_ptr(), dgh.data_ptr(), dh0.data_ptr(), N.ptr(sc),
+                                B, S, H, N.stream()), "oa_rnn_scan_bwd", 2 if n else 1)
     return dgi, dgh, dh0
 
 

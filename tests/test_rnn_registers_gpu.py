@@ -1,0 +1,29 @@
+"""Recurrent scans with the weights in registers: hidden widths at the edges of the 16-wide pieces, odd batches, initial state."""
+import pytest
+import torch
+
+from oa_b200.ops import kernels as K
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("gates", [1, 3])
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, 2e-5), (torch.bfloat16, 4e-2)])
+@pytest.mark.parametrize("B,S,H", [(1, 1, 8), (3, 2, 24), (2, 5, 32), (5, 9, 40), (2, 33, 64), (3, 6, 72), (2, 17, 128), (150, 4, 128), (2, 4, 136), (2, 4, 20)])
+def test_scan(gates, dtype, tol, B, S, H):
+    g = torch.Generator().manual_seed(B * 1009 + S * 31 + H)
+    r = lambda *s, k=1.0: (k * torch.randn(*s, generator=g)).to(dtype)
+    gi, w, b, h0, do = r(B, S, gates * H), r(gates * H, H, k=H ** -0.5), r(gates * H, k=0.1), r(B, H, k=0.5), r(B, S, H)
+    c = lambda t: t.float()
+    for bias in (b, None):
+        cb = c(bias) if bias is not None else None
+        gb = bias.cuda() if bias is not None else None
+        out, hp = K.rnn_scan_fwd(gi.cuda(), w.cuda(), gb, gates, h0=h0.cuda())
+        outr, hpr = K.rnn_scan_fwd(c(gi), c(w), cb, gates, h0=c(h0))
+        assert (out.float().cpu() - outr).abs().max().item() <= tol
+        assert (hp.float().cpu() - hpr).abs().max().item() <= tol
+        got = K.rnn_scan_bwd(gi.cuda(), w.cuda(), gb, hpr.to(dtype).cuda(), do.cuda(), gates)
+        ref = K.rnn_scan_bwd(c(gi), c(w), cb, hpr.to(dtype).float(), c(do), gates)
+        for a, e, nm in zip(got, ref, ("dgi", "dgh", "dh0")):
+            assert (a.float().cpu() - e).abs().max().item() <= tol * max(1.0, e.abs().max().item()), nm
+    torch.cuda.synchronize()
