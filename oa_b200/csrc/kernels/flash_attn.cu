@@ -13,7 +13,7 @@
 // products are issue bound), an MUFU exponential occupies its pipe for 8 cycles per warp (1024 cycles per 128 x 128
 // tile), and a warp that waits for the tensor pipe between key blocks idles the SFU.  Hence: score tiles are copied
 // to registers and released at once so the next score product is issued under this block's exponentials, products are
-// issued by two or three warps, and every kernel but the head_dim 128 forward is persistent (one CTA per SM walks its
+// issued by two or three warps, and every kernel is persistent (one CTA per SM walks its
 // work items in snake order, heaviest causal items first), so TMEM, barriers and the operand rings live across items.
 //
 // Backward is two kernels, both deterministic (single writer per output element, like the reference's
@@ -28,7 +28,6 @@ namespace oa {
 constexpr int FA_BM = 128;   // queries per tile
 constexpr int FA_BN = 128;   // keys per tile
 constexpr float LOG2E = 1.4426950408889634f;
-constexpr int FA_THREADS = 320;   // head_dim 128 forward: 8 softmax warps + MMA warp + TMA warp
 
 // 64-thread named barrier shared by the two warps that own the same 32 query rows.
 __device__ __forceinline__ void pair_sync(int quad) {
@@ -45,293 +44,22 @@ struct FlashParams {
   int* status;
 };
 
-// ===================================================================================== forward, S double-buffered in TMEM
-// One CTA owns one 128-query tile of one (batch, head).  S = Q K_j^T alternates between two TMEM buffers, and the MMA warp
-// always runs two key blocks ahead of the softmax (Q K_{j+2}^T is issued right after P_j V_j), so the softmax warps never
-// wait for the tensor pipe: they go from block j straight to block j+1 and the SFU stays busy.
-//   warps 0-7  softmax: two threads per query row (warp w: TMEM lane quadrant w % 4, key columns [64 * (w / 4), +64)), the
-//              64 scores of a thread are read from TMEM once, the row maximum is exchanged with the partner thread through
-//              a parity-double-buffered slot, probabilities go back to TMEM as packed bf16 over the columns of S_j;
-//   warp 8     MMA issuer: P is the A operand straight from TMEM, V the B operand from shared memory, O accumulates in
-//              TMEM over all key blocks and is read once at the end;
-//   warp 9     TMA producer (Q once, K / V rings).
-// The running maximum is updated lazily: while the new row maximum exceeds the one in use by less than 2^8 the old one is
-// kept (probabilities then stay below 256), so O in TMEM is rescaled only in the rare iterations where some row of a warp
-// jumps by more than that; the final 1/l uses the same maxima, so the result is the exact softmax.
-// TMEM: S0 | S1 | O = 128 + 128 + head_dim columns.
-template <int HD>
-struct Fwd2Cfg {
-  static constexpr int NSK = 3;                            // K ring depth (K runs two blocks ahead of V)
-  static constexpr int NSV = (HD == 64) ? 3 : 2;           // V ring depth
-  static constexpr int Q_BYTES = FA_BM * HD * 2;
-  static constexpr int KV_BYTES = FA_BN * HD * 2;
-  static constexpr int OFF_Q = 0;
-  static constexpr int OFF_K = OFF_Q + Q_BYTES;
-  static constexpr int OFF_V = OFF_K + NSK * KV_BYTES;
-  static constexpr int OFF_X = OFF_V + NSV * KV_BYTES;     // float[2 parities][2 halves][128 rows]: row-maximum exchange
-  static constexpr int OFF_BAR = OFF_X + 2 * 2 * FA_BM * 4;
-  static constexpr int SMEM_BYTES = OFF_BAR + 256;
-  static constexpr int TMEM_COLS = 512;
-  static constexpr int TM_S = 0;                           // + 128 * (j & 1)
-  static constexpr int TM_O = 256;
-};
-
 constexpr float FA_RESCALE_THRESHOLD = 8.f;                // log2 units
 
-
-template <int HD>
-__global__ void __launch_bounds__(FA_THREADS, 1)
-flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                  const __grid_constant__ CUtensorMap tmV, const FlashParams p) {
-  using Cfg = Fwd2Cfg<HD>;
-  constexpr int NSK = Cfg::NSK, NSV = Cfg::NSV;
-  extern __shared__ __align__(1024) uint8_t smem[];
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::OFF_BAR);
-  uint64_t* q_full = bars + 0;
-  uint64_t* k_full = bars + 1;                 // [NSK]
-  uint64_t* k_empty = k_full + NSK;            // [NSK]
-  uint64_t* v_full = k_empty + NSK;            // [NSV]
-  uint64_t* v_empty = v_full + NSV;            // [NSV]
-  uint64_t* s_full = v_empty + NSV;            // [2]  S buffer holds Q K_j^T
-  uint64_t* p_full = s_full + 2;               // [2]  P_j written over S buffer (and O rescaled if needed)
-  uint64_t* o_done = s_full + 4;               //      O += P_j V_j finished
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(s_full + 5);
-  float* xch = reinterpret_cast<float*>(smem + Cfg::OFF_X);
-
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nblk = (p.seq + FA_BM - 1) / FA_BM;
-  const int qb = nblk - 1 - blockIdx.x;        // heaviest causal tiles first
-  const int h = blockIdx.y, b = blockIdx.z;
-  const int n_kv = p.causal ? (qb + 1) : nblk;
-  const int row0 = b * p.seq;
-
-  if ((smem_u32(smem) & 1023u) != 0) {
-    if (threadIdx.x == 0) report_error(p.status, OA_KERR_BAD_ARG);
-    return;
-  }
-  if (threadIdx.x == 0) {
-    tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV);
-    mbar_init(q_full, 1);
-    for (int s = 0; s < NSK; ++s) { mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1); }
-    for (int s = 0; s < NSV; ++s) { mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1); }
-    for (int t = 0; t < 2; ++t) { mbar_init(&s_full[t], 1); mbar_init(&p_full[t], 8); }
-    mbar_init(o_done, 1);
-    mbar_fence_init();
-  }
-  if (warp == 8) { tmem_alloc<Cfg::TMEM_COLS>(tmem_slot); tmem_relinquish(); }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
-  pdl_wait();                            // the prologue above ran under the previous kernel's tail; global memory from here on
-
-  if (warp == 9) {
-    // ------------- producer: the whole warp walks the loop and waits together; one lane issues the copies.  K block i is
-    // loaded two iterations before V block i - 2... both rings are simply filled in order, K first.
-    if (lane == 0) {
-      mbar_expect_tx(q_full, Cfg::Q_BYTES);
-#pragma unroll
-      for (int x = 0; x < HD / 64; ++x)
-        tma_load_2d(smem + Cfg::OFF_Q + x * (FA_BM * 128), &tmQ, q_full, h * HD + x * 64, row0 + qb * FA_BM);
-    }
-    for (int i = 0; i < n_kv + 2; ++i) {
-      if (i < n_kv) {
-        const int st = i % NSK;
-        if (!warp_wait(&k_empty[st], ((i / NSK) & 1) ^ 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_EMPTY); break; }
-        if (lane == 0) {
-          mbar_expect_tx(&k_full[st], Cfg::KV_BYTES);
-#pragma unroll
-          for (int x = 0; x < HD / 64; ++x)
-            tma_load_2d(smem + Cfg::OFF_K + st * Cfg::KV_BYTES + x * (FA_BN * 128), &tmK, &k_full[st], h * HD + x * 64, row0 + i * FA_BN);
-        }
-      }
-      const int jv = i - 2;                    // V lags K by two blocks, like its consumer
-      if (jv >= 0) {
-        const int st = jv % NSV;
-        if (!warp_wait(&v_empty[st], ((jv / NSV) & 1) ^ 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_EMPTY); break; }
-        if (lane == 0) {
-          mbar_expect_tx(&v_full[st], Cfg::KV_BYTES);
-#pragma unroll
-          for (int x = 0; x < HD / 64; ++x)
-            tma_load_2d(smem + Cfg::OFF_V + st * Cfg::KV_BYTES + x * (FA_BN * 128), &tmV, &v_full[st], h * HD + x * 64, row0 + jv * FA_BN);
-        }
-      }
-      __syncwarp();
-    }
-  } else if (warp == 8) {
-    // ------------- MMA issuer (warp-uniform waits, lane 0 issues)
-    constexpr uint32_t idesc_qk = umma_idesc_bf16(FA_BM, FA_BN, 0, 0);
-    constexpr uint32_t idesc_pv = umma_idesc_bf16(FA_BM, HD, 0, 1);
-    const uint32_t q_addr = smem_u32(smem + Cfg::OFF_Q);
-    auto issue_qk = [&](int i) -> bool {       // S[i & 1] = Q K_i^T
-      const int st = i % NSK;
-      if (!warp_wait(&k_full[st], (i / NSK) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_FULL); return false; }
-      tc_fence_after();
-      if (lane == 0) {
-        const uint32_t k_addr = smem_u32(smem + Cfg::OFF_K + st * Cfg::KV_BYTES);
-#pragma unroll
-        for (int ks = 0; ks < HD / 16; ++ks) {
-          const uint32_t off = (ks >> 2) * (FA_BM * 128) + (ks & 3) * 32;
-          umma_f16(tmem_base + Cfg::TM_S + (i & 1) * FA_BN, umma_smem_desc_sw128(q_addr + off, 16, 1024),
-                   umma_smem_desc_sw128(k_addr + off, 16, 1024), idesc_qk, ks > 0 ? 1u : 0u);
-        }
-        umma_commit(&k_empty[st]);
-        umma_commit(&s_full[i & 1]);
-      }
-      __syncwarp();
-      return true;
-    };
-    bool ok = warp_wait(q_full, 0);
-    if (!ok && lane == 0) report_error(p.status, OA_KERR_WAIT_FULL);
-    if (ok) ok = issue_qk(0);
-    if (ok && n_kv > 1) ok = issue_qk(1);
-    for (int j = 0; j < n_kv && ok; ++j) {
-      const int st = j % NSV;
-      if (!warp_wait(&v_full[st], (j / NSV) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_FULL); break; }
-      if (!warp_wait(&p_full[j & 1], (j >> 1) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_SOFTMAX); break; }
-      tc_fence_after();
-      if (lane == 0) {
-        const uint32_t v_addr = smem_u32(smem + Cfg::OFF_V + st * Cfg::KV_BYTES);
-#pragma unroll
-        for (int ks = 0; ks < FA_BN / 16; ++ks)
-          umma_f16_ts(tmem_base + Cfg::TM_O, tmem_base + Cfg::TM_S + (j & 1) * FA_BN + ks * 8,
-                      umma_smem_desc_sw128(v_addr + ks * 2048, FA_BN * 128, 1024), idesc_pv, (j > 0 || ks > 0) ? 1u : 0u);
-        umma_commit(&v_empty[st]);
-        umma_commit(o_done);
-      }
-      __syncwarp();
-      if (j + 2 < n_kv) ok = issue_qk(j + 2);  // overwrites S[j & 1] = P_j: ordered after P_j V_j by the pipe
-    }
-  } else {
-    // ------------- softmax + output: two threads per query row (key columns split in halves)
-    constexpr int OC = HD / 2;                   // output columns owned by this thread
-    const int quad = warp & 3;
-    const int half = warp >> 2;
-    const int r = quad * 32 + lane;
-    const int qi = qb * FA_BM + r;               // query index inside the sequence
-    const uint32_t t_lane = (uint32_t)(quad * 32) << 16;
-    const uint32_t o_addr = tmem_base + t_lane + Cfg::TM_O + half * OC;
-    const float sl2 = p.scale * LOG2E;
-    float m_run = -INFINITY, l_run = 0.f;
-    bool ok = true;
-    for (int j = 0; j < n_kv; ++j) {
-      ok = warp_wait(&s_full[j & 1], (j >> 1) & 1);
-      if (!ok) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_TMEM_FULL); break; }
-      tc_fence_after();
-      const uint32_t s_addr = tmem_base + t_lane + Cfg::TM_S + (j & 1) * FA_BN;
-      uint32_t sv[64];
-      tmem_ld32(s_addr + half * 64, sv);
-      tmem_ld32(s_addr + half * 64 + 32, sv + 32);
-      tmem_ld_wait();
-      const bool need_mask = (p.causal && j == qb) || (j * FA_BN + FA_BN > p.seq);
-      if (need_mask) {
-        const int lim = min(p.causal ? qi : 0x7fffffff, p.seq - 1) - j * FA_BN - half * 64;   // columns i <= lim are alive
-#pragma unroll
-        for (int i = 0; i < 64; ++i) sv[i] = (i <= lim) ? sv[i] : 0xff800000u;                 // -inf
-      }
-      float m0 = __uint_as_float(sv[0]), m1 = __uint_as_float(sv[1]), m2 = __uint_as_float(sv[2]), m3 = __uint_as_float(sv[3]);
-#pragma unroll
-      for (int i = 4; i < 64; i += 4) {
-        m0 = fmaxf(m0, __uint_as_float(sv[i])); m1 = fmaxf(m1, __uint_as_float(sv[i + 1]));
-        m2 = fmaxf(m2, __uint_as_float(sv[i + 2])); m3 = fmaxf(m3, __uint_as_float(sv[i + 3]));
-      }
-      float mx = fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
-      // Exchange with the partner thread of this row.  Both threads now hold their scores in registers, so after this
-      // barrier the S buffer may be overwritten by either of them.
-      float* slots = xch + (j & 1) * (2 * FA_BM);
-      slots[(half ^ 1) * FA_BM + r] = mx;
-      pair_sync(quad);
-      mx = fmaxf(mx, slots[half * FA_BM + r]) * sl2;
-      const float m_new = fmaxf(m_run, mx);
-      const bool grow = (m_new - m_run) > FA_RESCALE_THRESHOLD;           // first block: m_run = -inf -> true
-      const float m_cand = grow ? m_new : m_run;
-      const float m_use = (m_cand == -INFINITY) ? 0.f : m_cand;           // row fully masked so far
-      const float alpha = grow ? fast_exp2(m_run - m_use) : 1.f;           // m_run = -inf -> 0
-      const float neg_m = -m_use;
-      float l0 = 0.f, l1 = 0.f, l2 = 0.f, l3 = 0.f;
-      uint32_t pk[32];
-#pragma unroll
-      for (int i = 0; i < 64; i += 4) {
-        const float e0 = fast_exp2(fmaf(__uint_as_float(sv[i]), sl2, neg_m));
-        const float e1 = fast_exp2(fmaf(__uint_as_float(sv[i + 1]), sl2, neg_m));
-        const float e2 = fast_exp2(fmaf(__uint_as_float(sv[i + 2]), sl2, neg_m));
-        const float e3 = fast_exp2(fmaf(__uint_as_float(sv[i + 3]), sl2, neg_m));
-        l0 += e0; l1 += e1; l2 += e2; l3 += e3;
-        pk[i >> 1] = pack_bf16x2(e0, e1);
-        pk[(i >> 1) + 1] = pack_bf16x2(e2, e3);
-      }
-      tmem_st32(s_addr + half * 32, pk);          // P over the first 64 columns of S (two keys per column)
-      l_run = l_run * alpha + ((l0 + l1) + (l2 + l3));
-      m_run = m_cand;
-      if (j > 0 && __any_sync(0xffffffffu, grow)) {
-        // some row of this warp moved its maximum: rescale O (needs the previous P*V finished)
-        ok = warp_wait(o_done, (j - 1) & 1);
-        if (!ok) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_TMEM_FULL); break; }
-        tc_fence_after();
-#pragma unroll
-        for (int c = 0; c < OC / 32; ++c) {
-          uint32_t o[32];
-          tmem_ld32(o_addr + c * 32, o);
-          tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-          tmem_st32(o_addr + c * 32, o);
-        }
-      }
-      tmem_st_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&p_full[j & 1]);
-    }
-    // combine the two partial row sums (parity slot of an iteration that is two behind any reader)
-    {
-      float* slots = xch + (n_kv & 1) * (2 * FA_BM);
-      slots[(half ^ 1) * FA_BM + r] = l_run;
-      pair_sync(quad);
-      l_run += slots[half * FA_BM + r];
-    }
-    if (ok) {
-      ok = warp_wait(o_done, (n_kv - 1) & 1);
-      if (!ok && lane == 0) report_error(p.status, OA_KERR_WAIT_TMEM_FULL);
-    }
-    if (ok) {
-      tc_fence_after();
-      const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
-      __nv_bfloat16* op = p.o + (long long)(row0 + qi) * p.o_stride + h * HD + half * OC;
-#pragma unroll
-      for (int c = 0; c < OC / 32; ++c) {
-        uint32_t o[32];
-        tmem_ld32(o_addr + c * 32, o);
-        tmem_ld_wait();
-        if (qi < p.seq) {
-#pragma unroll
-          for (int g = 0; g < 4; ++g)
-            *reinterpret_cast<uint4*>(op + c * 32 + g * 8) = make_uint4(
-                pack_bf16x2(__uint_as_float(o[g * 8]) * inv, __uint_as_float(o[g * 8 + 1]) * inv),
-                pack_bf16x2(__uint_as_float(o[g * 8 + 2]) * inv, __uint_as_float(o[g * 8 + 3]) * inv),
-                pack_bf16x2(__uint_as_float(o[g * 8 + 4]) * inv, __uint_as_float(o[g * 8 + 5]) * inv),
-                pack_bf16x2(__uint_as_float(o[g * 8 + 6]) * inv, __uint_as_float(o[g * 8 + 7]) * inv));
-        }
-      }
-      if (p.lse && half == 0 && qi < p.seq) p.lse[((long long)b * p.heads + h) * p.seq + qi] = (m_run + log2f(l_run)) / LOG2E;
-    }
-  }
-  pdl_launch_dependents();
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 8) { tc_fence_after(); tmem_dealloc<Cfg::TMEM_COLS>(tmem_base); }
-}
-
-// ===================================================================================== forward, head_dim 64: two tiles per CTA
+// ===================================================================================== forward: two tiles per CTA
 // Two adjacent 128-query tiles of one (batch, head) share a CTA and the K / V rings but are otherwise independent pipelines
 // (softmax warps 0-3 + MMA warp 8 for tile 0, warps 4-7 + MMA warp 9 for tile 1), so their phases drift apart and the
 // exponentials of one tile cover the TMEM traffic, row maxima and barrier hand-offs of the other.  One thread owns one query
 // row (all 128 key columns: no partner exchange).  The score tile is copied to registers and RELEASED at once, so
 // Q K_{j+1}^T is issued while the exponentials of block j run; probabilities have their own TMEM columns:
 // S0 | S1 | P0 | P1 | O0 | O1 = 128 + 128 + 64 + 64 + 64 + 64.
+// Head dim 128: O takes the columns of P, so P_t overwrites the first half of S_t (S0 | S1 | O0 | O1 = 4 x 128 columns).  Then
+// Q K_{j+1}^T is issued behind P V_j by the same thread, and it is the other tile's products and exponentials that fill the gap.
+template <int HD_>
 struct FwdPairCfg {
-  static constexpr int HD = 64;
-  static constexpr int NS = 3;
+  static constexpr int HD = HD_;
+  static constexpr bool ALIAS = HD == 128;
+  static constexpr int NS = ALIAS ? 2 : 3;
   static constexpr int Q_BYTES = FA_BM * HD * 2;
   static constexpr int KV_BYTES = FA_BN * HD * 2;
   static constexpr int OFF_Q = 0;
@@ -340,7 +68,7 @@ struct FwdPairCfg {
   static constexpr int OFF_BAR = OFF_V + NS * KV_BYTES;
   static constexpr int SMEM_BYTES = OFF_BAR + 256;
   static constexpr int TMEM_COLS = 512;
-  static constexpr int TM_S = 0, TM_P = 256, TM_O = 384;   // + 128 / 64 / 64 * tile
+  static constexpr int TM_S = 0, TM_P = ALIAS ? 0 : 256, P_STEP = ALIAS ? FA_BN : 64, TM_O = ALIAS ? 256 : 384;   // S: + 128 * tile, O: + HD * tile
   static constexpr int THREADS = 352;                        // 8 softmax warps, 2 MMA warps, 1 TMA warp
 };
 
@@ -354,11 +82,13 @@ __device__ __forceinline__ float fmax3(float a, float b, float c) {
 // dealt in snake order (round r: CTA c takes item r G + c, or r G + G-1-c when r is odd; within 3 % of the greedy optimum), so TMEM, barriers and the K / V rings live across items, the producer and the MMA warps run ahead
 // into the next item while the softmax warps write the previous output, and no SM pays a CTA launch per item.  Every
 // barrier phase is derived from a running count kept identically by its producers and consumers.
-__global__ void __launch_bounds__(FwdPairCfg::THREADS, 1)
+template <int HD>
+__global__ void __launch_bounds__(FwdPairCfg<HD>::THREADS, 1)
 flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                       const __grid_constant__ CUtensorMap tmV, const FlashParams p) {
-  using Cfg = FwdPairCfg;
-  constexpr int NS = Cfg::NS, HD = Cfg::HD;
+  using Cfg = FwdPairCfg<HD>;
+  constexpr int NS = Cfg::NS;
+  constexpr bool ALIAS = Cfg::ALIAS;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::OFF_BAR);
   uint64_t* q_full = bars + 0;
@@ -427,7 +157,9 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         const int tiles = nkv1 > 0 ? 2 : 1;
         mbar_expect_tx(q_full, tiles * Cfg::Q_BYTES);
         for (int t = 0; t < tiles; ++t)
-          tma_load_2d(smem + Cfg::OFF_Q + t * Cfg::Q_BYTES, &tmQ, q_full, h * HD, row0 + (2 * pr + t) * FA_BM);
+#pragma unroll
+          for (int x = 0; x < HD / 64; ++x)
+            tma_load_2d(smem + Cfg::OFF_Q + t * Cfg::Q_BYTES + x * (FA_BM * 128), &tmQ, q_full, h * HD + x * 64, row0 + (2 * pr + t) * FA_BM);
       }
       for (int j = 0; j < n_it; ++j, ++blk) {
         const int st = blk % NS;
@@ -435,12 +167,16 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         if (!warp_wait(&k_empty[st], ph ^ 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_EMPTY); ok = false; break; }
         if (lane == 0) {
           mbar_expect_tx(&k_full[st], Cfg::KV_BYTES);
-          tma_load_2d(smem + Cfg::OFF_K + st * Cfg::KV_BYTES, &tmK, &k_full[st], h * HD, row0 + j * FA_BN);
+#pragma unroll
+          for (int x = 0; x < HD / 64; ++x)
+            tma_load_2d(smem + Cfg::OFF_K + st * Cfg::KV_BYTES + x * (FA_BN * 128), &tmK, &k_full[st], h * HD + x * 64, row0 + j * FA_BN);
         }
         if (!warp_wait(&v_empty[st], ph ^ 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_EMPTY); ok = false; break; }
         if (lane == 0) {
           mbar_expect_tx(&v_full[st], Cfg::KV_BYTES);
-          tma_load_2d(smem + Cfg::OFF_V + st * Cfg::KV_BYTES, &tmV, &v_full[st], h * HD, row0 + j * FA_BN);
+#pragma unroll
+          for (int x = 0; x < HD / 64; ++x)
+            tma_load_2d(smem + Cfg::OFF_V + st * Cfg::KV_BYTES + x * (FA_BN * 128), &tmV, &v_full[st], h * HD + x * 64, row0 + j * FA_BN);
         }
         __syncwarp();
       }
@@ -452,20 +188,22 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     constexpr uint32_t idesc_qk = umma_idesc_bf16(FA_BM, FA_BN, 0, 0);
     constexpr uint32_t idesc_pv = umma_idesc_bf16(FA_BM, HD, 0, 1);
     const uint32_t q_addr = smem_u32(smem + Cfg::OFF_Q + t * Cfg::Q_BYTES);
-    const uint32_t s_tm = tmem_base + Cfg::TM_S + t * FA_BN, p_tm = tmem_base + Cfg::TM_P + t * 64, o_tm = tmem_base + Cfg::TM_O + t * HD;
+    const uint32_t s_tm = tmem_base + Cfg::TM_S + t * FA_BN, p_tm = tmem_base + Cfg::TM_P + t * Cfg::P_STEP, o_tm = tmem_base + Cfg::TM_O + t * HD;
     uint32_t base = 0, itc = 0, sc = 0, pc = 0;   // K / V blocks before this item, items, S products and P V products of this tile so far
     bool ok = true;
     auto issue_qk = [&](uint32_t blk, bool last) -> bool {       // S_t = Q_t K^T of ring block `blk`
       const int st = blk % NS;
       if (!warp_wait(&k_full[st], (blk / NS) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_FULL); return false; }
-      if (sc > 0 && !warp_wait(&s_empty[t], (sc - 1) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_TMEM_EMPTY); return false; }
+      if (!ALIAS && sc > 0 && !warp_wait(&s_empty[t], (sc - 1) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_TMEM_EMPTY); return false; }
       tc_fence_after();
       if (lane == 0) {
         const uint32_t k_addr = smem_u32(smem + Cfg::OFF_K + st * Cfg::KV_BYTES);
 #pragma unroll
-        for (int ks = 0; ks < HD / 16; ++ks)
-          umma_f16(s_tm, umma_smem_desc_sw128(q_addr + ks * 32, 16, 1024), umma_smem_desc_sw128(k_addr + ks * 32, 16, 1024),
+        for (int ks = 0; ks < HD / 16; ++ks) {
+          const uint32_t off = (ks >> 2) * (FA_BM * 128) + (ks & 3) * 32;
+          umma_f16(s_tm, umma_smem_desc_sw128(q_addr + off, 16, 1024), umma_smem_desc_sw128(k_addr + off, 16, 1024),
                    idesc_qk, ks > 0 ? 1u : 0u);
+        }
         umma_commit(&k_empty[st]);
         umma_commit(&s_full[t]);
         if (last) umma_commit(q_empty);
@@ -484,7 +222,7 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       if (!warp_wait(q_full, itc & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_FULL); break; }
       if (n > 0) ok = issue_qk(base, n == 1);
       for (int j = 0; j < n && ok; ++j) {
-        if (j + 1 < n) { ok = issue_qk(base + j + 1, j + 2 == n); if (!ok) break; }
+        if (!ALIAS && j + 1 < n) { ok = issue_qk(base + j + 1, j + 2 == n); if (!ok) break; }
         const int st = (base + j) % NS;
         if (!warp_wait(&v_full[st], ((base + j) / NS) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_FULL); ok = false; break; }
         if (!warp_wait(&p_full[t], pc & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_SOFTMAX); ok = false; break; }
@@ -495,10 +233,11 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           for (int ks = 0; ks < FA_BN / 16; ++ks)
             umma_f16_ts(o_tm, p_tm + ks * 8, umma_smem_desc_sw128(v_addr + ks * 2048, FA_BN * 128, 1024), idesc_pv, (j > 0 || ks > 0) ? 1u : 0u);
           umma_commit(&v_empty[st]);
-          umma_commit(&o_done[t]);
+          if (!ALIAS || j + 1 == n) umma_commit(&o_done[t]);
         }
         __syncwarp();
         ++pc;
+        if (ALIAS && j + 1 < n) { ok = issue_qk(base + j + 1, j + 2 == n); if (!ok) break; }   // overwrites P_j: ordered after P_j V_j by the pipe
       }
       // blocks of this item that this tile does not use (the last one of the pair's shorter tile, or all of an absent tile):
       // the rings still expect one arrival per MMA warp, given once the block has landed
@@ -523,7 +262,7 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     const int r = quad * 32 + lane;
     const uint32_t t_lane = (uint32_t)(quad * 32) << 16;
     const uint32_t s_addr = tmem_base + t_lane + Cfg::TM_S + t * FA_BN;
-    const uint32_t p_addr = tmem_base + t_lane + Cfg::TM_P + t * 64;
+    const uint32_t p_addr = tmem_base + t_lane + Cfg::TM_P + t * Cfg::P_STEP;
     const uint32_t o_addr = tmem_base + t_lane + Cfg::TM_O + t * HD;
     const float sl2 = p.scale * LOG2E;
     uint32_t sc = 0, pc = 0;     // score tiles consumed and P V completions awaited so far
@@ -547,9 +286,11 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 #pragma unroll
         for (int c = 0; c < FA_BN / 32; ++c) tmem_ld32(s_addr + c * 32, sv + c * 32);
         tmem_ld_wait();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&s_empty[t]);   // the next block's scores may overwrite S_t now
+        if (!ALIAS) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&s_empty[t]);   // the next block's scores may overwrite S_t now
+        }
         const bool need_mask = (p.causal && j == qbt) || (j * FA_BN + FA_BN > p.seq);
         if (need_mask) {
           const int lim = min(p.causal ? qi : 0x7fffffff, p.seq - 1) - j * FA_BN;   // columns i <= lim are alive
@@ -569,7 +310,9 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         const float m_use = (m_cand == -INFINITY) ? 0.f : m_cand;           // row fully masked so far
         const float alpha = grow ? fast_exp2(m_run - m_use) : 1.f;           // m_run = -inf -> 0
         const float neg_m = -m_use;
-        if (j > 0) {                               // P_t is free and O_t is complete once the previous P V has finished
+        // P_t is free and O_t is complete once the previous P V has finished (head dim 128: s_full already says so, the scores were
+        // issued behind it)
+        if (!ALIAS && j > 0) {
           ok = warp_wait(&o_done[t], pc & 1);
           if (!ok) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_TMEM_FULL); break; }
           ++pc;
@@ -643,13 +386,18 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 }
 
 template <int HD>
-static int launch_fwd2(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FlashParams& p, dim3 grid, cudaStream_t st) {
-  static bool set = false;
-  if (!set) {
-    if (cudaFuncSetAttribute(flash_fwd2_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, Fwd2Cfg<HD>::SMEM_BYTES) != cudaSuccess) return OA_ERR_LAUNCH;
-    set = true;
+static int launch_fwd_pair(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FlashParams& p, cudaStream_t st) {
+  static int sms = 0;
+  if (sms == 0) {
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return OA_ERR_DRIVER;
+    if (cudaFuncSetAttribute(flash_fwd_pair_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdPairCfg<HD>::SMEM_BYTES) != cudaSuccess) return OA_ERR_LAUNCH;
+    sms = n;
   }
-  launch_pdl(flash_fwd2_kernel<HD>, grid, dim3(FA_THREADS), Fwd2Cfg<HD>::SMEM_BYTES, st, tq, tk, tv, p);
+  const int nblk = (p.seq + FA_BM - 1) / FA_BM;
+  const long long items = (long long)((nblk + 1) / 2) * p.heads * p.batch;
+  const int ctas = (int)(items < sms ? items : sms);
+  launch_pdl(flash_fwd_pair_kernel<HD>, dim3(ctas), dim3(FwdPairCfg<HD>::THREADS), FwdPairCfg<HD>::SMEM_BYTES, st, tq, tk, tv, p);
   return cudaGetLastError() == cudaSuccess ? OA_OK : OA_ERR_LAUNCH;
 }
 
@@ -1326,21 +1074,7 @@ extern "C" int oa_flash_fwd(const void* q, const void* k, const void* v, void* o
   p.batch = batch; p.heads = heads; p.seq = seq; p.head_dim = head_dim; p.scale = scale; p.causal = causal;
   p.o = (__nv_bfloat16*)o; p.o_stride = o_row_stride; p.lse = lse; p.status = status;
   cudaStream_t st = (cudaStream_t)stream;
-  if (head_dim == 64) {
-    // persistent kernel, two query tiles per work item
-    static int sms = 0;
-    if (sms == 0) {
-      int dev = 0;
-      if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return OA_ERR_DRIVER;
-      if (cudaFuncSetAttribute(flash_fwd_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdPairCfg::SMEM_BYTES) != cudaSuccess) return OA_ERR_LAUNCH;
-    }
-    const int nblk = (seq + FA_BM - 1) / FA_BM;
-    const long long items = (long long)((nblk + 1) / 2) * heads * batch;
-    const int ctas = (int)(items < sms ? items : sms);
-    launch_pdl(flash_fwd_pair_kernel, dim3(ctas), dim3(FwdPairCfg::THREADS), FwdPairCfg::SMEM_BYTES, st, tq, tk, tv, p);
-    return cudaGetLastError() == cudaSuccess ? OA_OK : OA_ERR_LAUNCH;
-  }
-  return launch_fwd2<128>(tq, tk, tv, p, dim3((seq + FA_BM - 1) / FA_BM, heads, batch), st);
+  return head_dim == 64 ? launch_fwd_pair<64>(tq, tk, tv, p, st) : launch_fwd_pair<128>(tq, tk, tv, p, st);
 }
 
 // scratch: float[B*H*S] for delta
