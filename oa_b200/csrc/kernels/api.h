@@ -307,7 +307,7 @@ int oa_ssd_state_bwd(const void* T, const void* cum, const void* Hin, void* dHou
 int oa_ssd_out_fwd(const void* Y, const void* z, long long ldz, void* y, void* yraw, long long ldy, int B, int L, int H, int P,
                    void* stream);
 int oa_ssd_dy_prep(const void* dy, const void* yraw, long long ldy, const void* z, long long ldz, void* dz, long long lddz, void* dY,
-                   int B, int L, int H, int P, void* stream);
+                   const void* cum, void* dYe, int B, int L, int H, int P, void* stream);
 int oa_ssd_mask_bwd(const void* dM, const void* Gm, const void* cum, const void* scale, void* dG, void* row_mm, void* col_mm,
                     void* col_ge, void* diag, int G, void* stream);
 int oa_ssd_prep_bwd(const void* dCt, const void* dBt, const void* dCe, const void* Ct, const void* Bt, const void* cum, const void* dqk,
@@ -333,6 +333,15 @@ int oa_ssd_tail(const void* dw, const void* w, const void* col_ge, const void* r
                 const void* diag, const void* qk, const void* cum, const void* dcumQ, const void* dt, const void* trap,
                 const void* ddt_theta, void* dadt, void* ddt, void* dtrap, void* dD, void* scratch, int B, int L, int H,
                 void* stream);
+
+// ---- chunk products of the Mamba-3 scan (mamba3_ssd_tc.cu): state width 128, head width 64
+int oa_ssd_chunk_fwd(const void* C, const void* Bt, const void* X, const void* Hin, const void* cum, const void* scale, const void* gamma,
+                     const void* qk, const void* D, const void* z, long long ldz, void* y, void* yraw, long long ldy, int B, int L, int H,
+                     void* status, void* stream);
+int oa_ssd_chunk_bwd(const void* C, const void* Bt, const void* X, const void* Xw, const void* dY, const void* Hin, const void* dH,
+                     const void* cum, const void* scale, const void* gamma, const void* qk, const void* w, const void* D, void* dC, void* dB,
+                     void* row_mm, void* col_mm, void* col_ge, void* diag, void* dcum_ce, void* dw, void* dx, long long lddx, int B, int L,
+                     int H, void* status, void* stream);
 
 // ---- audio DSP (audio.cu)
 int oa_audio_stft_frame(const void* x, void* frames, int channels, long long samples, int n_frames, int fft, int hop, int win, int kind,

@@ -8,7 +8,7 @@
 //   ssd_mask_fwd    G (fp32) -> M (bf16): decayed strict lower triangle + exact diagonal
 //   ssd_state_fwd   recurrence over the chunk states, emits the state entering every chunk
 //   ssd_out_fwd     Y (fp32 chunk layout) -> y (token layout) with the silu(z) gate
-//   ssd_dy_prep     dy -> dY (bf16 chunk layout) through the gate, dz
+//   ssd_dy_prep     dy -> dY (bf16 chunk layout) through the gate, dz; optionally dY e^cum too
 //   ssd_state_bwd   reverse recurrence: gradient w.r.t. every chunk's outgoing state and w.r.t. cumQ
 //   ssd_mask_bwd    dM, G -> dG (bf16) + row / column sums that carry d cum, d scale, d gamma, d D
 //   ssd_prep_bwd    dC~, dB~, d(C~e^cum) -> un-rotate, d theta, dCn / dBn (summed over heads), dCb / dBb
@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(256) ssd_prep_fwd_kernel(SsdPrepFwd a) {
       const long long o = og * d.N + n4 * 4;
       *reinterpret_cast<uint2*>(a.Ct + o) = make_uint2(pack_bf16x2(cv.x, cv.y), pack_bf16x2(cv.z, cv.w));
       *reinterpret_cast<uint2*>(a.Bt + o) = make_uint2(pack_bf16x2(bv.x, bv.y), pack_bf16x2(bv.z, bv.w));
-      *reinterpret_cast<uint2*>(a.Ce + o) = make_uint2(pack_bf16x2(cv.x * e, cv.y * e), pack_bf16x2(cv.z * e, cv.w * e));
+      if (a.Ce) *reinterpret_cast<uint2*>(a.Ce + o) = make_uint2(pack_bf16x2(cv.x * e, cv.y * e), pack_bf16x2(cv.z * e, cv.w * e));
     }
     qk = warp_sum(qk);
     if (lane == 0) a.qk[og] = qk;
@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(256) ssd_out_fwd_kernel(const float* __restric
 __global__ void __launch_bounds__(256) ssd_dy_prep_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ yraw,
                                                           long long ldy, const __nv_bfloat16* __restrict__ z, long long ldz,
                                                           __nv_bfloat16* __restrict__ dz, long long lddz, __nv_bfloat16* __restrict__ dY,
-                                                          SsdDims d) {
+                                                          const float* __restrict__ cum, __nv_bfloat16* __restrict__ dYe, SsdDims d) {
   const int P2 = d.P >> 1;
   const long long total = (long long)d.B * d.H * d.nC * SQ * P2;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -240,6 +240,10 @@ __global__ void __launch_bounds__(256) ssd_dy_prep_kernel(const __nv_bfloat16* _
       g.x *= zf.x * s0; g.y *= zf.y * s1;
     }
     *reinterpret_cast<unsigned*>(dY + i * 2) = pack_bf16x2(g.x, g.y);
+    if (dYe) {
+      const float e = __expf(cum[i / P2]);                     // i / P2 = g * SQ + t
+      *reinterpret_cast<unsigned*>(dYe + i * 2) = pack_bf16x2(g.x * e, g.y * e);
+    }
   }
 }
 
@@ -302,7 +306,7 @@ __global__ void __launch_bounds__(256) ssd_mask_bwd_kernel(const float* __restri
 
 // ------------------------------------------------------------------------------------------------------ prep backward
 struct SsdPrepBwd {
-  const float *dCt, *dBt, *dCe;                  // [G, Q, N] fp32 (GEMM outputs)
+  const float *dCt, *dBt, *dCe;                  // [G, Q, N] fp32; dCe null: dCt and dBt already hold every term
   const __nv_bfloat16 *Ct, *Bt;                  // saved rotated operands
   const float *cum, *dqk;                        // [G, Q]
   const float* theta;                            // [B*L, H, A]
@@ -335,22 +339,24 @@ __global__ void __launch_bounds__(256) ssd_prep_bwd_kernel(SsdPrepBwd a) {
     for (int i = 0; i < 4; ++i) {
       const int t = q4 * 32 + warp + 8 * i;
       const long long r = row0 + t, og = g * SQ + t;
-      const float ecum = __expf(a.cum[og]), dqk = a.dqk[og];
+      const float ecum = a.dCe ? __expf(a.cum[og]) : 0.f, dqk = a.dCe ? a.dqk[og] : 0.f;
       float dce = 0.f;
       if (live) {
         const long long o = og * d.N + lane * 4;
         const float4 dc = *reinterpret_cast<const float4*>(a.dCt + o), db = *reinterpret_cast<const float4*>(a.dBt + o);
-        const float4 de = *reinterpret_cast<const float4*>(a.dCe + o);
+        const float4 de = a.dCe ? *reinterpret_cast<const float4*>(a.dCe + o) : make_float4(0.f, 0.f, 0.f, 0.f);
         const uint2 cu = *reinterpret_cast<const uint2*>(a.Ct + o), bu = *reinterpret_cast<const uint2*>(a.Bt + o);
         const float2 c01 = unpack_bf16x2(cu.x), c23 = unpack_bf16x2(cu.y), b01 = unpack_bf16x2(bu.x), b23 = unpack_bf16x2(bu.y);
         const float cv[4] = {c01.x, c01.y, c23.x, c23.y}, bv[4] = {b01.x, b01.y, b23.x, b23.y};
         const float dev[4] = {de.x, de.y, de.z, de.w};
         float gc[4] = {dc.x, dc.y, dc.z, dc.w}, gb[4] = {db.x, db.y, db.z, db.w};
+        if (a.dCe) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          dce += dev[j] * cv[j];
-          gc[j] += dev[j] * ecum + dqk * bv[j];
-          gb[j] += dqk * cv[j];
+          for (int j = 0; j < 4; ++j) {
+            dce += dev[j] * cv[j];
+            gc[j] += dev[j] * ecum + dqk * bv[j];
+            gb[j] += dqk * cv[j];
+          }
         }
         const int k0 = lane * 2;
         if (k0 < d.A) {
@@ -371,8 +377,10 @@ __global__ void __launch_bounds__(256) ssd_prep_bwd_kernel(SsdPrepBwd a) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) { accC[i][j] += gc[j]; accB[i][j] += gb[j]; pc[j] += gc[j]; pb[j] += gb[j]; }
       }
-      dce = warp_sum(dce);
-      if (lane == 0) a.dcum_ce[og] = dce * ecum;
+      if (a.dCe) {
+        dce = warp_sum(dce);
+        if (lane == 0) a.dcum_ce[og] = dce * ecum;
+      }
     }
     if (live) {
 #pragma unroll
@@ -619,13 +627,13 @@ int oa_ssd_out_fwd(const void* Y, const void* z, long long ldz, void* y, void* y
 }
 
 int oa_ssd_dy_prep(const void* dy, const void* yraw, long long ldy, const void* z, long long ldz, void* dz, long long lddz, void* dY,
-                   int B, int L, int H, int P, void* stream) {
+                   const void* cum, void* dYe, int B, int L, int H, int P, void* stream) {
   SsdDims d{B, L, H, P, 4, 0, L / SQ};
-  if (!ssd_dims_ok(d) || (z && (!yraw || !dz))) return OA_ERR_ARG;
+  if (!ssd_dims_ok(d) || (z && (!yraw || !dz)) || (dYe && !cum)) return OA_ERR_ARG;
   const long long total = (long long)B * L * H * (P / 2);
   ssd_dy_prep_kernel<<<(int)((total + 255) / 256 > 148 * 32 ? 148 * 32 : (total + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
       (const __nv_bfloat16*)dy, (const __nv_bfloat16*)yraw, ldy, (const __nv_bfloat16*)z, ldz, (__nv_bfloat16*)dz, lddz,
-      (__nv_bfloat16*)dY, d);
+      (__nv_bfloat16*)dY, (const float*)cum, (__nv_bfloat16*)dYe, d);
   return ssd_status();
 }
 

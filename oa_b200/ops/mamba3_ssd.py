@@ -269,27 +269,38 @@ def ssd_fwd_cuda(proj: torch.Tensor, Bn, Cn, dt, adt, trap, angle, Bb, Cb, D, d:
         theta, tot = f32(B, L, H, A), f32(B, nC, H, A)
         K._launch(lib.oa_ssd_theta_fwd(angle.data_ptr(), angle.shape[-1], dt.data_ptr(), tot.data_ptr(), theta.data_ptr(), B, L, H, A, st),
                   "oa_ssd_theta_fwd", 2)
-    Ct, Bt, Ce, X, Xw = bf(G, Q, Nn), bf(G, Q, Nn), bf(G, Q, Nn), bf(G, Q, P), bf(G, Q, P)
+    # State width 128 and head width 64 run everything between the chunk states and y in one kernel (and likewise in the
+    # backward pass), which needs neither C~ e^cum nor the mask in memory; other widths run the GEMMs one by one.
+    fused = P == 64 and Nn == 128
+    Ct, Bt, X, Xw = bf(G, Q, Nn), bf(G, Q, Nn), bf(G, Q, P), bf(G, Q, P)
+    Ce = None if fused else bf(G, Q, Nn)
     cum, gamma, scale, w, qk = f32(G, Q), f32(G, Q), f32(G, Q), f32(G, Q), f32(G, Q)
     K._launch(lib.oa_ssd_prep_fwd(proj.data_ptr() + o[1] * es, d.d_in_proj, Bn.data_ptr(), Cn.data_ptr(), Bb.data_ptr(), Cb.data_ptr(),
-                                  dt.data_ptr(), adt.data_ptr(), trap.data_ptr(), N.ptr(theta), Ct.data_ptr(), Bt.data_ptr(), Ce.data_ptr(),
+                                  dt.data_ptr(), adt.data_ptr(), trap.data_ptr(), N.ptr(theta), Ct.data_ptr(), Bt.data_ptr(), N.ptr(Ce),
                                   X.data_ptr(), Xw.data_ptr(), cum.data_ptr(), gamma.data_ptr(), scale.data_ptr(), w.data_ptr(),
                                   qk.data_ptr(), B, L, H, P, Nn, A, st), "oa_ssd_prep_fwd")
-    Gm = K.bgemm(Ct, Bt, out_dtype=torch.float32)
-    M = bf(G, Q, Q)
-    K._launch(lib.oa_ssd_mask_fwd(Gm.data_ptr(), cum.data_ptr(), scale.data_ptr(), gamma.data_ptr(), qk.data_ptr(), N.ptr(D), M.data_ptr(),
-                                  G, H, nC, st), "oa_ssd_mask_fwd")
-    del Gm
-    Y = K.bgemm(M, X, b_mn=True, out_dtype=torch.float32)
+    M = Y = None
+    if not fused:
+        Gm = K.bgemm(Ct, Bt, out_dtype=torch.float32)
+        M = bf(G, Q, Q)
+        K._launch(lib.oa_ssd_mask_fwd(Gm.data_ptr(), cum.data_ptr(), scale.data_ptr(), gamma.data_ptr(), qk.data_ptr(), N.ptr(D), M.data_ptr(),
+                                      G, H, nC, st), "oa_ssd_mask_fwd")
+        del Gm
+        Y = K.bgemm(M, X, b_mn=True, out_dtype=torch.float32)
     S = K.bgemm(Xw, Bt, a_mn=True, b_mn=True, out_dtype=torch.float32)
     Hin = bf(G, P, Nn)
     K._launch(lib.oa_ssd_state_fwd(S.data_ptr(), cum.data_ptr(), Hin.data_ptr(), B * H, nC, P * Nn, st), "oa_ssd_state_fwd")
     del S
-    K.bgemm(Ce, Hin, out=Y, accumulate=True)
     y = bf(rows, d.d_inner)
     yraw = bf(rows, d.d_inner) if d.has_z else None
-    K._launch(lib.oa_ssd_out_fwd(Y.data_ptr(), proj.data_ptr() + o[0] * es if d.has_z else None, d.d_in_proj, y.data_ptr(), N.ptr(yraw),
-                                 d.d_inner, B, L, H, P, st), "oa_ssd_out_fwd")
+    z_ptr = proj.data_ptr() + o[0] * es if d.has_z else None
+    if fused:
+        K._launch(lib.oa_ssd_chunk_fwd(Ct.data_ptr(), Bt.data_ptr(), X.data_ptr(), Hin.data_ptr(), cum.data_ptr(), scale.data_ptr(),
+                                       gamma.data_ptr(), qk.data_ptr(), N.ptr(D), z_ptr, d.d_in_proj, y.data_ptr(), N.ptr(yraw), d.d_inner,
+                                       B, L, H, K.status_word(dev).data_ptr(), st), "oa_ssd_chunk_fwd")
+    else:
+        K.bgemm(Ce, Hin, out=Y, accumulate=True)
+        K._launch(lib.oa_ssd_out_fwd(Y.data_ptr(), z_ptr, d.d_in_proj, y.data_ptr(), N.ptr(yraw), d.d_inner, B, L, H, P, st), "oa_ssd_out_fwd")
     if not save:
         return y, None
     s = SsdSavedCuda()
@@ -314,38 +325,50 @@ def ssd_bwd_cuda(s: SsdSavedCuda, proj: torch.Tensor, dy: torch.Tensor, dproj: t
     f32 = lambda *sh: torch.empty(sh, dtype=torch.float32, device=dev)
     z32 = lambda *sh: torch.zeros(sh, dtype=torch.float32, device=dev)
     dy = dy.contiguous()
+    fused = s.M is None
     dY = bf(G, Q, P)
+    dYe = bf(G, Q, P) if fused else None
     K._launch(lib.oa_ssd_dy_prep(dy.data_ptr(), N.ptr(s.yraw), d.d_inner, proj.data_ptr() + o[0] * es if d.has_z else None, d.d_in_proj,
-                                 dproj.data_ptr() + o[0] * es if d.has_z else None, d.d_in_proj, dY.data_ptr(), B, L, H, P, st),
-              "oa_ssd_dy_prep")
-    dM = K.bgemm(dY, s.X, out_dtype=torch.float32)
-    dX = K.bgemm(s.M, dY, a_mn=True, b_mn=True, out_dtype=torch.float32)
-    dCe = K.bgemm(dY, s.Hin, b_mn=True, out_dtype=torch.float32)
-    T = K.bgemm(dY, s.Ce, a_mn=True, b_mn=True, out_dtype=torch.float32)
+                                 dproj.data_ptr() + o[0] * es if d.has_z else None, d.d_in_proj, dY.data_ptr(),
+                                 s.cum.data_ptr() if fused else None, N.ptr(dYe), B, L, H, P, st), "oa_ssd_dy_prep")
+    # gradient of the chunk states through y: T = dY^T (C~ e^cum)
+    T = K.bgemm(dYe, s.Ct, a_mn=True, b_mn=True, out_dtype=torch.float32) if fused else \
+        K.bgemm(dY, s.Ce, a_mn=True, b_mn=True, out_dtype=torch.float32)
     dHout, dcumQ = bf(G, P, Nn), z32(G)
     K._launch(lib.oa_ssd_state_bwd(T.data_ptr(), s.cum.data_ptr(), s.Hin.data_ptr(), dHout.data_ptr(), dcumQ.data_ptr(), B * H, nC, P * Nn, st),
               "oa_ssd_state_bwd")
-    del T
-    dXw = K.bgemm(s.Bt, dHout, out_dtype=torch.float32)
-    dBt = K.bgemm(s.Xw, dHout, b_mn=True, out_dtype=torch.float32)
-    Gm = K.bgemm(s.Ct, s.Bt, out_dtype=torch.float32)
-    dG, row_mm, col_mm, col_ge, diag = bf(G, Q, Q), f32(G, Q), f32(G, Q), f32(G, Q), f32(G, Q)
-    K._launch(lib.oa_ssd_mask_bwd(dM.data_ptr(), Gm.data_ptr(), s.cum.data_ptr(), s.scale.data_ptr(), dG.data_ptr(), row_mm.data_ptr(),
-                                  col_mm.data_ptr(), col_ge.data_ptr(), diag.data_ptr(), G, st), "oa_ssd_mask_bwd")
-    del dM, Gm
-    dCt = K.bgemm(dG, s.Bt, b_mn=True, out_dtype=torch.float32)
-    K.bgemm(dG, s.Ct, a_mn=True, b_mn=True, out=dBt, accumulate=True)
-    dqk = K.binary("mul", diag, s.gamma)
+    del T, dYe
+    row_mm, col_mm, col_ge, diag, dcum_ce, dw = (f32(G, Q) for _ in range(6))
+    dqk = dCe = None
+    if fused:
+        dCt, dBt = f32(G, Q, Nn), f32(G, Q, Nn)
+        K._launch(lib.oa_ssd_chunk_bwd(s.Ct.data_ptr(), s.Bt.data_ptr(), s.X.data_ptr(), s.Xw.data_ptr(), dY.data_ptr(), s.Hin.data_ptr(),
+                                       dHout.data_ptr(), s.cum.data_ptr(), s.scale.data_ptr(), s.gamma.data_ptr(), s.qk.data_ptr(), s.w.data_ptr(),
+                                       N.ptr(s.Dh), dCt.data_ptr(), dBt.data_ptr(), row_mm.data_ptr(), col_mm.data_ptr(), col_ge.data_ptr(),
+                                       diag.data_ptr(), dcum_ce.data_ptr(), dw.data_ptr(), dproj.data_ptr() + o[1] * es, d.d_in_proj, B, L, H,
+                                       K.status_word(dev).data_ptr(), st), "oa_ssd_chunk_bwd")
+    else:
+        dM = K.bgemm(dY, s.X, out_dtype=torch.float32)
+        dX = K.bgemm(s.M, dY, a_mn=True, b_mn=True, out_dtype=torch.float32)
+        dCe = K.bgemm(dY, s.Hin, b_mn=True, out_dtype=torch.float32)
+        dXw = K.bgemm(s.Bt, dHout, out_dtype=torch.float32)
+        dBt = K.bgemm(s.Xw, dHout, b_mn=True, out_dtype=torch.float32)
+        Gm = K.bgemm(s.Ct, s.Bt, out_dtype=torch.float32)
+        dG = bf(G, Q, Q)
+        K._launch(lib.oa_ssd_mask_bwd(dM.data_ptr(), Gm.data_ptr(), s.cum.data_ptr(), s.scale.data_ptr(), dG.data_ptr(), row_mm.data_ptr(),
+                                      col_mm.data_ptr(), col_ge.data_ptr(), diag.data_ptr(), G, st), "oa_ssd_mask_bwd")
+        del dM, Gm
+        dCt = K.bgemm(dG, s.Bt, b_mn=True, out_dtype=torch.float32)
+        K.bgemm(dG, s.Ct, a_mn=True, b_mn=True, out=dBt, accumulate=True)
+        dqk = K.binary("mul", diag, s.gamma)
+        K._launch(lib.oa_ssd_dx_out(dX.data_ptr(), dXw.data_ptr(), s.X.data_ptr(), s.w.data_ptr(), dproj.data_ptr() + o[1] * es, d.d_in_proj,
+                                    dw.data_ptr(), B, L, H, P, st), "oa_ssd_dx_out")
     dCn, dBn, dCb, dBb = f32(rows, Nn), f32(rows, Nn), z32(H, Nn), z32(H, Nn)
     dtheta = f32(B, L, H, A) if A else None
-    dcum_ce = f32(G, Q)
-    K._launch(lib.oa_ssd_prep_bwd(dCt.data_ptr(), dBt.data_ptr(), dCe.data_ptr(), s.Ct.data_ptr(), s.Bt.data_ptr(), s.cum.data_ptr(),
-                                  dqk.data_ptr(), N.ptr(s.theta), dCn.data_ptr(), dBn.data_ptr(), dCb.data_ptr(), dBb.data_ptr(),
+    K._launch(lib.oa_ssd_prep_bwd(dCt.data_ptr(), dBt.data_ptr(), N.ptr(dCe), s.Ct.data_ptr(), s.Bt.data_ptr(), s.cum.data_ptr(),
+                                  N.ptr(dqk), N.ptr(s.theta), dCn.data_ptr(), dBn.data_ptr(), dCb.data_ptr(), dBb.data_ptr(),
                                   N.ptr(dtheta), dcum_ce.data_ptr(), B, L, H, Nn, A, st), "oa_ssd_prep_bwd")
     del dCt, dBt, dCe
-    dw = f32(G, Q)
-    K._launch(lib.oa_ssd_dx_out(dX.data_ptr(), dXw.data_ptr(), s.X.data_ptr(), s.w.data_ptr(), dproj.data_ptr() + o[1] * es, d.d_in_proj,
-                                dw.data_ptr(), B, L, H, P, st), "oa_ssd_dx_out")
     # ---- per-token scalar tail ([G, Q] / [B, L, H] sized tensors): three small kernels
     out = {"Bn": dBn, "Cn": dCn, "Bb": dBb, "Cb": dCb}
     ddt_theta = None
