@@ -36,19 +36,6 @@ class OaKvCache:
         self.Length = 0
 
 
-def _skinny_linear(x: OaMatrix, w: OaMatrix, residual: Optional[OaMatrix] = None) -> OaMatrix:
-    """x [m, K] @ W[N, K]^T for a handful of rows: computed as (W @ x^T)^T so that the weight rows fill the 128-row MMA
-    tile and the few tokens sit on the narrow N side, with split-K spreading the weight stream over all SMs."""
-    tx, tw = x.Tensor(), w.Tensor()
-    if not tx.is_cuda or tx.dtype != torch.bfloat16 or tx.shape[0] > 64 or tx.shape[0] % 8:
-        return F.Linear(x, w, None, residual=residual)
-    yt = K.gemm(tw, tx)                                    # [N, m]
-    y = K.contiguous(yt.t())
-    if residual is not None:
-        y = K.binary("add", y, residual.Tensor(), out=y)
-    return OaMatrix(y)
-
-
 class _GraphedStep:
     """One decode step captured in a CUDA graph.  The position lives on the device (`pos`, int32 [1]): RoPE, the cache
     append and the attention length read it inside their kernels and the graph's last node adds one, so replaying needs no
@@ -92,16 +79,7 @@ class OaGptDecoder:
         if pd is not None:
             pos0 = 0                                  # the device-resident position carries the offset
         h = b.LnAttn.Forward(x)
-        qw, kw, vw = a.QProj.Weight.Tensor(), a.KProj.Weight.Tensor(), a.VProj.Weight.Tensor()
-        step = D * D * qw.element_size()
-        adjacent = kw.data_ptr() == qw.data_ptr() + step and vw.data_ptr() == kw.data_ptr() + step
-        if s_new == 1 and a.QProj.Bias is None and h.Tensor().is_cuda and adjacent:
-            packed = qw
-            base = packed.untyped_storage()
-            wqkv = torch.empty(0, dtype=packed.dtype, device=packed.device).set_(base, packed.storage_offset(), (3 * D, D), (D, 1))
-            qkv = _skinny_linear(h, OaMatrix(wqkv))            # q, k, v weights are row slices of one packed tensor
-        else:
-            qkv = a.ProjectQkv(h)
+        qkv = a.ProjectQkv(h)
         t = qkv.Tensor()
         if s_new > 1:
             # prompt: tiled attention over the new tokens (rotates q and k in place), then cache the rotated k and v
@@ -114,22 +92,18 @@ class OaGptDecoder:
             K.kv_append(t[:, D:2 * D], t[:, 2 * D:], self.Cache.K[i], self.Cache.V[i], batch, 1, pos0, pos_dev=pd)
             attn = OaMatrix(K.decode_attn(t[:, :D], self.Cache.K[i], self.Cache.V[i], pos0 + 1, pos_dev=pd))
         o = a.OutProj
-        if s_new == 1 and o.Bias is None:
-            x = _skinny_linear(attn, o.Weight.Data, residual=x)
-        else:
-            x = F.Linear(attn, o.Weight.Data, o.Bias.Data if o.Bias else None, residual=x)
+        x = F.Linear(attn, o.Weight.Data, o.Bias.Data if o.Bias else None, residual=x)
         if b.Moe is not None:
             return b.Moe.Forward(x)
         if b.FfnKind == "gelu":
             hh = b.LnFfn.Forward(x)
             return FF.FfnGelu(hh, b.Ffn1.Weight.Data, b.Ffn1.Bias.Data if b.Ffn1.Bias else None, b.Ffn2.Weight.Data,
                               b.Ffn2.Bias.Data if b.Ffn2.Bias else None, residual=x)
-        if s_new == 1:
-            f = b.Ffn
-            hh = f.Norm.Forward(x)
-            gate, up = _skinny_linear(hh, f.Gate.Weight.Data), _skinny_linear(hh, f.Up.Weight.Data)
-            return _skinny_linear(F.SiluMul(gate, up), f.Down.Weight.Data, residual=x)
-        return b.Ffn.Forward(x)
+        f = b.Ffn
+        if s_new == 1 and FF.packed_view([f.Gate.Weight.Tensor(), f.Up.Weight.Tensor()]) is None:
+            hh = f.Norm.Forward(x)                    # weights that do not lie side by side: two products rather than a joined copy
+            return F.Linear(F.SiluMul(F.Linear(hh, f.Gate.Weight.Data), F.Linear(hh, f.Up.Weight.Data)), f.Down.Weight.Data, None, residual=x)
+        return f.Forward(x)
 
     def _forward(self, ids: torch.Tensor) -> torch.Tensor:
         """ids [B, s_new] int32 -> logits of the last new position [B, vocab]; the cache grows by s_new."""

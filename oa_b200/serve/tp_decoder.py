@@ -22,7 +22,7 @@ from ..ml import autograd as AG
 from ..ops import kernels as K
 from ..parallel.mesh import OaDeviceMesh
 from ..parallel.tp_model import OaTpGptModel
-from .decoder import OaKvCache, _GraphedStep, _skinny_linear
+from .decoder import OaKvCache, _GraphedStep
 
 
 class OaOneShotAllReduce:
@@ -81,7 +81,7 @@ class OaTpGptDecoder:
         if pd is not None:
             pos0 = 0
         small = s_new == 1
-        lin = _skinny_linear if small else (lambda a, w_: F.Linear(a, w_, None))
+        lin = lambda a, w_: F.Linear(a, w_, None)
         h = b.LnAttn.Forward(x)
         qkv = lin(h, b.Qkv.Data)                                   # [rows, 3 * Dl]: this rank's heads, q | k | v
         t = qkv.Tensor()
@@ -124,7 +124,7 @@ class OaTpGptDecoder:
             self.Cache.Length += s_new
             last = x.Tensor().reshape(batch, s_new, -1)[:, -1].contiguous() if s_new > 1 else x.Tensor()
             h = m.LnFinal.Forward(OaMatrix(last))
-            return (_skinny_linear(h, m.Head.Data) if s_new == 1 else F.Linear(h, m.Head.Data, None)).Tensor().contiguous()
+            return F.Linear(h, m.Head.Data, None).Tensor().contiguous()
 
     def Prefill(self, prompt: torch.Tensor) -> torch.Tensor:
         self.Cache.Reset()
