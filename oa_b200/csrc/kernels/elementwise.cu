@@ -245,15 +245,17 @@ __global__ void rope_kernel(T* x, long long rows, int row_stride, int n_heads, i
 // them to every head of the row with 16-byte accesses (the angle depends on the position and on j only).
 __global__ void __launch_bounds__(256)
 rope_bf16_vec_kernel(__nv_bfloat16* x, long long rows, int row_stride, int n_heads, int hd, int seq_len, int pos_offset, float theta,
-                     int backward, const int* __restrict__ pos_dev) {
+                     int backward, const int* __restrict__ pos_dev, int heads_per) {
   pdl_launch_dependents();
   pdl_wait();
   if (pos_dev) pos_offset += *pos_dev;
   const int half = hd >> 1, jv = half >> 3;                 // 8-wide vectors per half head
-  const long long total = rows * jv;
+  const int groups = (n_heads + heads_per - 1) / heads_per;
+  const long long total = rows * groups * jv;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const int v = (int)(i % jv);
-    const long long r = i / jv;
+    const int h_lo = (int)((i / jv) % groups) * heads_per, h_hi = min(n_heads, h_lo + heads_per);
+    const long long r = i / jv / groups;
     const float pos = (float)((int)(r % seq_len) + pos_offset);
     float c[8], s[8];
 #pragma unroll
@@ -265,18 +267,18 @@ rope_bf16_vec_kernel(__nv_bfloat16* x, long long rows, int row_stride, int n_hea
     __nv_bfloat16* row = x + r * row_stride + v * 8;
     // four heads per round: their eight 16-byte loads are issued before the first use, so one thread keeps 128 bytes in flight
     constexpr int HB = 4;
-    for (int h0 = 0; h0 < n_heads; h0 += HB) {
+    for (int h0 = h_lo; h0 < h_hi; h0 += HB) {
       uint4 ua[HB], ub[HB];
 #pragma unroll
       for (int u = 0; u < HB; ++u) {
-        if (h0 + u < n_heads) {
+        if (h0 + u < h_hi) {
           ua[u] = *reinterpret_cast<const uint4*>(row + (h0 + u) * hd);
           ub[u] = *reinterpret_cast<const uint4*>(row + (h0 + u) * hd + half);
         }
       }
 #pragma unroll
       for (int u = 0; u < HB; ++u) {
-        if (h0 + u < n_heads) {
+        if (h0 + u < h_hi) {
           const uint32_t wa[4] = {ua[u].x, ua[u].y, ua[u].z, ua[u].w}, wb[4] = {ub[u].x, ub[u].y, ub[u].z, ub[u].w};
           uint32_t oa[4], ob[4];
 #pragma unroll
@@ -662,8 +664,14 @@ extern "C" int oa_rope(int dtype, void* x, long long rows, int row_stride, int n
                        int pos_offset, float theta, int backward, const int* pos_dev, void* stream) {
   if (head_dim % 2) return OA_ERR_ARG;
   if (dtype == OA_BF16 && head_dim % 16 == 0 && row_stride % 8 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
-    launch_pdl(rope_bf16_vec_kernel, dim3(grid_for(rows * (head_dim / 16), 256)), dim3(256), 0, ST, (__nv_bfloat16*)x, rows, row_stride, n_heads,
-               head_dim, seq_len, pos_offset, theta, backward, pos_dev);
+    // One thread turns all heads of a row (the angle is theirs in common) while there are rows enough to fill the machine; a
+    // decoding step has a handful of rows, where that loop was a chain of memory round trips, and spreads the heads,
+    // four to a thread: 32 rows x 64 heads of 128 go from 18 to 5 us.
+    const long long per_head_group = rows * (head_dim / 16);
+    int heads_per = n_heads;
+    while (heads_per > 4 && per_head_group * ((n_heads + heads_per - 1) / heads_per) < 148 * 256) heads_per = (heads_per + 1) / 2;
+    launch_pdl(rope_bf16_vec_kernel, dim3(grid_for(per_head_group * ((n_heads + heads_per - 1) / heads_per), 256)), dim3(256), 0, ST,
+               (__nv_bfloat16*)x, rows, row_stride, n_heads, head_dim, seq_len, pos_offset, theta, backward, pos_dev, heads_per);
     return CHECK_LAUNCH();
   }
   DISPATCH_T(dtype, rope_kernel<T><<<grid_for(rows * n_heads * head_dim / 2, 256), 256, 0, ST>>>(
