@@ -117,6 +117,121 @@ mamba3_conv_bwd_kernel(T* __restrict__ dy, long long ld, int col0, const T* __re
   for (int k = 0; k < Kw; ++k) dw_part[((long long)blockIdx.y * Kw + k) * C + c] = dwk[k];
 }
 
+// Width-4 convolution of bf16 columns in 16-byte pieces: a thread owns eight neighbouring columns.  The kernels above move two
+// bytes per lane and access and fetch every tap again: 2 x 4096 tokens x 3328 columns: forward 177 -> 76 us,
+// backward 306 -> 130 us.
+constexpr int MC_KW = 4;
+__device__ __forceinline__ void mc_ld8(const __nv_bfloat16* p, float (&v)[8]) {
+  const uint4 u = *reinterpret_cast<const uint4*>(p);
+  const float2 a = unpack_bf16x2(u.x), b = unpack_bf16x2(u.y), c = unpack_bf16x2(u.z), d = unpack_bf16x2(u.w);
+  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y; v[4] = c.x; v[5] = c.y; v[6] = d.x; v[7] = d.y;
+}
+__device__ __forceinline__ void mc_st8(__nv_bfloat16* p, const float (&v)[8]) {
+  *reinterpret_cast<uint4*>(p) = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
+}
+
+__global__ void __launch_bounds__(256)
+mamba3_cols_copy_vec_kernel(const __nv_bfloat16* __restrict__ x, long long ld, int col0, __nv_bfloat16* __restrict__ out, long long rows, int C) {
+  const int c8 = C >> 3;
+  const long long total = rows * c8, stride = (long long)gridDim.x * blockDim.x;
+#pragma unroll 4
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
+    const long long r = i / c8;
+    *reinterpret_cast<uint4*>(out + i * 8) = *reinterpret_cast<const uint4*>(x + r * ld + col0 + (i - r * c8) * 8);
+  }
+}
+
+// MODE 0: y = silu(conv) over x;  1: g = dy silu'(pre) into gbuf;  2: dx from g over dy, and the weight-gradient partials.
+// Grid as above with 128 x 8 columns per block; MODE 2 walks a window of g forwards and of the inputs backwards.
+template <int MODE>
+__global__ void __launch_bounds__(128)
+mamba3_conv4_vec_kernel(__nv_bfloat16* __restrict__ x, long long ld, int col0, const __nv_bfloat16* __restrict__ saved, const float* __restrict__ w,
+                        __nv_bfloat16* __restrict__ gbuf, float* __restrict__ dw_part, int L, int C, int tb) {
+  const int c = (blockIdx.x * 128 + threadIdx.x) * 8;
+  if (c >= C) return;
+  const int nb = (L + tb - 1) / tb;
+  const int b = blockIdx.y / nb, t0 = (blockIdx.y % nb) * tb, t1 = min(L, t0 + tb);
+  const long long base = (long long)b * L;
+  float wk[MC_KW][8], win[MC_KW - 1][8];                     // win[k] = input at t - 1 - k
+#pragma unroll
+  for (int k = 0; k < MC_KW; ++k)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) wk[k][j] = w[(long long)k * C + c + j];
+#pragma unroll
+  for (int k = 0; k < MC_KW - 1; ++k) {
+    if (t0 - 1 - k >= 0) mc_ld8(saved + (base + t0 - 1 - k) * C + c, win[k]);
+    else
+#pragma unroll
+      for (int j = 0; j < 8; ++j) win[k][j] = 0.f;
+  }
+  if (MODE != 2) {
+#pragma unroll 4
+    for (int t = t0; t < t1; ++t) {
+      const long long row = base + t;
+      float xt[8], d[8], o[8];
+      mc_ld8(saved + row * C + c, xt);
+      if (MODE == 1) mc_ld8(x + row * ld + col0 + c, d);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        float pre = wk[0][j] * xt[j];
+        pre = fmaf(wk[1][j], win[0][j], pre);
+        pre = fmaf(wk[2][j], win[1][j], pre);
+        pre = fmaf(wk[3][j], win[2][j], pre);
+        win[2][j] = win[1][j]; win[1][j] = win[0][j]; win[0][j] = xt[j];
+        if (MODE == 0) o[j] = silu_f(pre);
+        else {
+          const float sg = sigmoid_f(pre);
+          o[j] = d[j] * sg * (1.f + pre * (1.f - sg));
+        }
+      }
+      if (MODE == 0) mc_st8(x + row * ld + col0 + c, o);
+      else mc_st8(gbuf + row * C + c, o);
+    }
+  } else {
+    float dwk[MC_KW][8], g[MC_KW][8];                        // g[k] = g[t + k]
+#pragma unroll
+    for (int k = 0; k < MC_KW; ++k)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) dwk[k][j] = g[k][j] = 0.f;
+#pragma unroll
+    for (int k = 0; k < MC_KW - 1; ++k)
+      if (t0 + k < L) mc_ld8(gbuf + (base + t0 + k) * C + c, g[k]);
+#pragma unroll 2
+    for (int t = t0; t < t1; ++t) {
+      const long long row = base + t;
+      float xt[8], o[8];
+      mc_ld8(saved + row * C + c, xt);
+      if (t + MC_KW - 1 < L) mc_ld8(gbuf + (row + MC_KW - 1) * C + c, g[MC_KW - 1]);
+      else
+#pragma unroll
+        for (int j = 0; j < 8; ++j) g[MC_KW - 1][j] = 0.f;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        float dx = wk[0][j] * g[0][j];
+        dx = fmaf(wk[1][j], g[1][j], dx);
+        dx = fmaf(wk[2][j], g[2][j], dx);
+        o[j] = fmaf(wk[3][j], g[3][j], dx);
+        dwk[0][j] = fmaf(g[0][j], xt[j], dwk[0][j]);
+        dwk[1][j] = fmaf(g[0][j], win[0][j], dwk[1][j]);
+        dwk[2][j] = fmaf(g[0][j], win[1][j], dwk[2][j]);
+        dwk[3][j] = fmaf(g[0][j], win[2][j], dwk[3][j]);
+        win[2][j] = win[1][j]; win[1][j] = win[0][j]; win[0][j] = xt[j];
+        g[0][j] = g[1][j]; g[1][j] = g[2][j]; g[2][j] = g[3][j];
+      }
+      mc_st8(x + row * ld + col0 + c, o);
+    }
+#pragma unroll
+    for (int k = 0; k < MC_KW; ++k)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) dw_part[((long long)blockIdx.y * MC_KW + k) * C + c + j] = dwk[k][j];
+  }
+}
+
+inline bool mc_vec_ok(int dtype, int C, int Kw, long long ld, int col0, const void* a, const void* b, const void* c) {
+  return dtype == OA_BF16 && Kw == MC_KW && (C & 7) == 0 && (ld & 7) == 0 && (col0 & 7) == 0 &&
+         ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15) == 0;
+}
+
 // x[row, col0 + h] = exp(a_log[h]) - 1
 template <typename T>
 __global__ void mamba3_alog_fill_kernel(T* __restrict__ x, long long ld, int col0, const float* __restrict__ a_log, long long rows, int H) {
@@ -145,6 +260,13 @@ extern "C" int oa_mamba3_conv_fwd(int dtype, void* x, long long ld, int col0, vo
   if (Kw < 1 || Kw > MC_MAXK || B <= 0 || L <= 0 || C <= 0) return OA_ERR_ARG;
   const long long rows = (long long)B * L;
   dim3 grid((C + 127) / 128, B * ((L + MC_TB - 1) / MC_TB));
+  const int tb = 16; // short blocks: three halo rows each, but enough of them to fill the SMs
+  if (mc_vec_ok(dtype, C, Kw, ld, col0, x, saved, nullptr) && (long long)B * ((L + tb - 1) / tb) <= 65535) {
+    mamba3_cols_copy_vec_kernel<<<mc_grid(rows * (C / 8)), 256, 0, ST>>>((const __nv_bfloat16*)x, ld, col0, (__nv_bfloat16*)saved, rows, C);
+    mamba3_conv4_vec_kernel<0><<<dim3((C / 8 + 127) / 128, B * ((L + tb - 1) / tb)), 128, 0, ST>>>((__nv_bfloat16*)x, ld, col0,
+        (const __nv_bfloat16*)saved, w, nullptr, nullptr, L, C, tb);
+    return CHECK_LAUNCH();
+  }
   if (dtype == OA_F32) {
     mamba3_cols_copy_kernel<float><<<mc_grid(rows * C), 256, 0, ST>>>((const float*)x, ld, col0, (float*)saved, rows, C);
     mamba3_conv_fwd_kernel<float><<<grid, 128, 0, ST>>>((float*)x, ld, col0, (float*)saved, w, B, L, C, Kw);
@@ -160,6 +282,14 @@ extern "C" int oa_mamba3_conv_bwd(int dtype, void* dy, long long ld, int col0, c
                                   void* gbuf, int B, int L, int C, int Kw, void* stream) {
   if (Kw < 1 || Kw > MC_MAXK || B <= 0 || L <= 0 || C <= 0) return OA_ERR_ARG;
   dim3 grid((C + 127) / 128, B * ((L + MC_TB - 1) / MC_TB));
+  const int tb = 16;
+  if (mc_vec_ok(dtype, C, Kw, ld, col0, dy, saved, gbuf) && (long long)B * ((L + tb - 1) / tb) <= 65535) {
+    mamba3_conv4_vec_kernel<1><<<dim3((C / 8 + 127) / 128, B * ((L + tb - 1) / tb)), 128, 0, ST>>>((__nv_bfloat16*)dy, ld, col0,
+        (const __nv_bfloat16*)saved, w, (__nv_bfloat16*)gbuf, nullptr, L, C, tb);
+    mamba3_conv4_vec_kernel<2><<<dim3((C / 8 + 127) / 128, B * ((L + MC_TB - 1) / MC_TB)), 128, 0, ST>>>((__nv_bfloat16*)dy, ld, col0,
+        (const __nv_bfloat16*)saved, w, (__nv_bfloat16*)gbuf, dw_part, L, C, MC_TB);
+    return CHECK_LAUNCH();
+  }
   if (dtype == OA_F32) {
     mamba3_conv_bwd_kernel<float><<<grid, 128, 0, ST>>>((float*)dy, ld, col0, (const float*)saved, w, nullptr, (float*)gbuf, B, L, C, Kw);
     mamba3_conv_bwd_kernel<float><<<grid, 128, 0, ST>>>((float*)dy, ld, col0, (const float*)saved, w, dw_part, (float*)gbuf, B, L, C, Kw);
