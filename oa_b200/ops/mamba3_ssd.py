@@ -269,9 +269,9 @@ def ssd_fwd_cuda(proj: torch.Tensor, Bn, Cn, dt, adt, trap, angle, Bb, Cb, D, d:
         theta, tot = f32(B, L, H, A), f32(B, nC, H, A)
         K._launch(lib.oa_ssd_theta_fwd(angle.data_ptr(), angle.shape[-1], dt.data_ptr(), tot.data_ptr(), theta.data_ptr(), B, L, H, A, st),
                   "oa_ssd_theta_fwd", 2)
-    # State width 128 and head width 64 run everything between the chunk states and y in one kernel (and likewise in the
+    # State width 128 and head width 64 (projected rows on 16-byte boundaries) run everything between the chunk states and y in one kernel (and likewise in the
     # backward pass), which needs neither C~ e^cum nor the mask in memory; other widths run the GEMMs one by one.
-    fused = P == 64 and Nn == 128
+    fused = P == 64 and Nn == 128 and d.d_in_proj % 8 == 0 and proj.data_ptr() % 16 == 0
     Ct, Bt, X, Xw = bf(G, Q, Nn), bf(G, Q, Nn), bf(G, Q, P), bf(G, Q, P)
     Ce = None if fused else bf(G, Q, Nn)
     cum, gamma, scale, w, qk = f32(G, Q), f32(G, Q), f32(G, Q), f32(G, Q), f32(G, Q)
