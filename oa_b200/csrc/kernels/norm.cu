@@ -39,7 +39,7 @@ constexpr int NORM_WARPS = NORM_THREADS / 32;
 
 // Rows of up to 32 * VEC * NV columns: the row stays in registers (packed as it is stored) between the sum of squares and the
 // output, so memory is read once and all of a lane's loads are in flight together.  16384 x 1024 is at the copy rate either way
-// (10.8 us); 32 x 4096 (a decoding step) goes from 11.6 to 5.2 us, where two dependent passes were all latency.
+// (10.8 us); with few rows two dependent passes were all latency: 32 x 4096 went from 11.6 to 5.2 us.
 template <typename T, int NV>
 __global__ void __launch_bounds__(NORM_THREADS)
 rmsnorm_fwd_reg_kernel(const T* __restrict__ x, const T* __restrict__ w, T* __restrict__ y, float* __restrict__ rstd_out,
@@ -89,6 +89,70 @@ rmsnorm_fwd_reg_kernel(const T* __restrict__ x, const T* __restrict__ w, T* __re
 #pragma unroll
       for (int j = 0; j < V; ++j) v[j] = v[j] * rstd * g[j];
       NIO<T>::store(y + row * cols + (i * 32 + lane) * V, v);
+    }
+  }
+}
+
+// A block per row while there are fewer rows than SMs (decoding steps): a lane has at most two 16-byte pieces per operand instead of
+// sixteen, and the loads of the weight and of the row are one round trip.  32 x 4096: 5.2 us with a warp per
+// row, 2.2 us here.
+template <typename T>
+__global__ void __launch_bounds__(NORM_THREADS)
+rmsnorm_fwd_row_kernel(const T* __restrict__ x, const T* __restrict__ w, T* __restrict__ y, float* __restrict__ rstd_out, int cols, float eps,
+                       const T* __restrict__ res_in, T* __restrict__ res_out) {
+  pdl_launch_dependents();
+  pdl_wait();
+  constexpr int V = NIO<T>::VEC, NV = 2;                  // rows of up to NORM_THREADS * NV vectors
+  __shared__ float s_sum[NORM_WARPS];
+  const int nv = cols / V;
+  const long long base = (long long)blockIdx.x * cols;
+  uint4 xp[NV], wp[NV], rp[NV];
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int c = i * NORM_THREADS + threadIdx.x;
+    if (c < nv) {
+      xp[i] = *reinterpret_cast<const uint4*>(x + base + c * V);
+      wp[i] = *reinterpret_cast<const uint4*>(w + c * V);
+      if (res_in) rp[i] = *reinterpret_cast<const uint4*>(res_in + base + c * V);
+    }
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int c = i * NORM_THREADS + threadIdx.x;
+    if (c < nv) {
+      float v[V];
+      NIO<T>::load(reinterpret_cast<const T*>(&xp[i]), v);
+      if (res_in) {
+        float r[V];
+        NIO<T>::load(reinterpret_cast<const T*>(&rp[i]), r);
+#pragma unroll
+        for (int j = 0; j < V; ++j) v[j] += r[j];
+        NIO<T>::store(reinterpret_cast<T*>(&xp[i]), v);
+        *reinterpret_cast<uint4*>(res_out + base + c * V) = xp[i];
+      }
+#pragma unroll
+      for (int j = 0; j < V; ++j) ss += v[j] * v[j];
+    }
+  }
+  ss = warp_sum(ss);
+  if ((threadIdx.x & 31) == 0) s_sum[threadIdx.x >> 5] = ss;
+  __syncthreads();
+  ss = 0.f;
+#pragma unroll
+  for (int k = 0; k < NORM_WARPS; ++k) ss += s_sum[k];
+  const float rstd = rsqrtf(ss / (float)cols + eps);
+  if (threadIdx.x == 0 && rstd_out) rstd_out[blockIdx.x] = rstd;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int c = i * NORM_THREADS + threadIdx.x;
+    if (c < nv) {
+      float v[V], g[V];
+      NIO<T>::load(reinterpret_cast<const T*>(&xp[i]), v);
+      NIO<T>::load(reinterpret_cast<const T*>(&wp[i]), g);
+#pragma unroll
+      for (int j = 0; j < V; ++j) v[j] = v[j] * rstd * g[j];
+      NIO<T>::store(y + base + c * V, v);
     }
   }
 }
@@ -493,6 +557,15 @@ extern "C" int oa_rmsnorm_fwd(int dtype, const void* x, const void* w, void* y, 
   if (dtype != OA_F32 && dtype != OA_BF16) return OA_ERR_UNSUPPORTED;
   long long b = (rows + NORM_WARPS - 1) / NORM_WARPS;
   const int nv = (cols + 32 * vec - 1) / (32 * vec);
+  if ((at & 15) == 0 && rows <= 148 && nv > 2 && cols / vec <= 2 * NORM_THREADS) {
+    if (dtype == OA_F32)
+      launch_pdl(rmsnorm_fwd_row_kernel<float>, dim3((unsigned)rows), dim3(NORM_THREADS), 0, ST, (const float*)x, (const float*)w, (float*)y, rstd, cols, eps,
+                 (const float*)residual_in, (float*)residual_out);
+    else
+      launch_pdl(rmsnorm_fwd_row_kernel<__nv_bfloat16>, dim3((unsigned)rows), dim3(NORM_THREADS), 0, ST, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w,
+                 (__nv_bfloat16*)y, rstd, cols, eps, (const __nv_bfloat16*)residual_in, (__nv_bfloat16*)residual_out);
+    return CHECK_LAUNCH();
+  }
   if (nv <= 16 && (at & 15) == 0 && b < 0x7fffffffLL) {
 #define OA_RMS_FWD_REG(T, NV)                                                                                                   \
     launch_pdl(rmsnorm_fwd_reg_kernel<T, NV>, dim3((unsigned)b), dim3(NORM_THREADS), 0, ST, (const T*)x, (const T*)w, (T*)y, rstd, \
