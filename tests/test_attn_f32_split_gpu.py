@@ -1,0 +1,26 @@
+"""fp32 attention with eight head dimensions per thread, at widths and lengths off the tile grid."""
+import pytest
+import torch
+
+from oa_b200.ops import kernels as K
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("hd", [8, 30, 32, 48, 64])
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("batch,seq,heads", [(1, 1, 1), (2, 33, 2), (1, 128, 4), (2, 257, 1)])
+def test_attention(hd, causal, batch, seq, heads):
+    g = torch.Generator(device="cuda").manual_seed(hd + seq)
+    D = heads * hd
+    qkv, do = torch.randn(batch * seq, 3 * D, device="cuda", generator=g), torch.randn(batch * seq, D, device="cuda", generator=g)
+    q, k, v = qkv[:, :D], qkv[:, D:2 * D], qkv[:, 2 * D:]
+    o, lse = K.flash_fwd(q, k, v, batch, seq, heads, hd, causal=causal)
+    got = K.flash_bwd(q, k, v, o, do, lse, batch, seq, heads, hd, causal=causal)
+    leaves = [t.double().reshape(batch, seq, heads, hd).transpose(1, 2).requires_grad_(True) for t in (q, k, v)]
+    ref = torch.nn.functional.scaled_dot_product_attention(*leaves, is_causal=causal).transpose(1, 2).reshape(batch * seq, D)
+    grads = torch.autograd.grad(ref, leaves, do.double())
+    # __expf of arguments up to 2^4 carries 2^-20; sums of 257 products
+    for a, e in zip((o, *got), (ref, *[x.transpose(1, 2).reshape(batch * seq, D) for x in grads])):
+        # (a gradient that cancels to nothing, as with one key, is measured against the upstream gradient)
+        assert float((a.double() - e.detach()).norm() / torch.maximum(e.detach().norm(), do.double().norm())) <= 8e-6
