@@ -43,7 +43,8 @@ def test_cross_entropy_rows(dtype, tol, rows, vocab, ld, in_place):
             ref[tr] -= 0.25
         else:
             assert torch.isnan(loss[r])
-        assert float((d[r].double().cpu() - ref).norm() / ref.norm()) <= tol
+        # p - 1 cancels at a sure target, so the error is that of p itself
+        assert float((d[r].double().cpu() - ref).norm() / torch.maximum(ref.norm(), 0.25 * p[r].norm())) <= tol
     if not in_place and ld > vocab:
         pad = out.as_strided((rows, ld - vocab), (ld, 1), out.storage_offset() + vocab)
         assert bool((pad == 7.0).all())
