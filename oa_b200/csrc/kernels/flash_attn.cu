@@ -53,6 +53,11 @@ constexpr float FA_RESCALE_THRESHOLD = 8.f;                // log2 units
 // row (all 128 key columns: no partner exchange).  The score tile is copied to registers and RELEASED at once, so
 // Q K_{j+1}^T is issued while the exponentials of block j run; probabilities have their own TMEM columns:
 // S0 | S1 | P0 | P1 | O0 | O1 = 128 + 128 + 64 + 64 + 64 + 64.
+// The running maximum is updated lazily: while the new row maximum exceeds the one in use by less than 2^8 the old one is kept
+// (probabilities then stay below 256), so O in TMEM is rescaled only in the rare iterations where some row of a warp jumps by
+// more than that; the final 1/l uses the same maxima, so the result is the exact softmax.
+// Two threads per row (sixteen softmax warps, maxima exchanged through shared memory) measured 127.7 instead of 121.7 us at head
+// dim 64 (8 x 2048 x 16) and 193 instead of 188 us at head dim 128 (4096 x 32): the warps' chains are not what bounds it.
 // Head dim 128: O takes the columns of P, so P_t overwrites the first half of S_t (S0 | S1 | O0 | O1 = 4 x 128 columns).  Then
 // Q K_{j+1}^T is issued behind P V_j by the same thread, and it is the other tile's products and exponentials that fill the gap.
 template <int HD_>
