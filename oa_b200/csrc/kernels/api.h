@@ -64,6 +64,9 @@ int oa_gemm_bf16_tp(int mode, const void* A, const void* B, void* out, int M, in
 int oa_gemm_f32(const float* A, const float* B, float* C, int M, int N, int K, long long sam, long long sak,
                 long long sbn, long long sbk, int ldc, int batch, long long batch_a, long long batch_b,
                 long long batch_c, const float* bias, int act, int accumulate, float alpha, void* stream);
+int oa_gemm_f32_epi(const float* A, const float* B, float* C, int M, int N, int K, long long sam, long long sak, long long sbn,
+                    long long sbk, int ldc, const float* bias, const float* residual, int ldr, float* aux_out, const float* aux_in,
+                    int ldaux, int act, int accumulate, float alpha, void* stream);
 
 // ---- elementwise (elementwise.cu)
 int oa_unary(int op, int dtype, const void* x, void* y, long long n, float s0, float s1, void* stream);

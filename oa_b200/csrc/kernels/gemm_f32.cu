@@ -2,7 +2,10 @@
 // epilogues.  It backs the engine's FP32 precision mode (the reference's only fully exercised
 // precision) and the finite-difference gradient checks, where TF32/bf16 rounding is not acceptable.
 // The bf16 path uses gemm_tcgen05.cu instead.
-//   C[b][m,n] = act(alpha * sum_k A[b][m*sam + k*sak] * B[b][n*sbn + k*sbk] + bias[n]) (+ C)
+//   v = alpha * sum_k A[b][m*sam + k*sak] * B[b][n*sbn + k*sbk] + bias[n];  aux_out = v;  v = act(v) or v * act'(aux_in);
+//   C[b][m,n] = v + residual (+ C)
+// The epilogue carries what the bf16 kernel's does, so that a Transformer layer in fp32 launches no pass of its own for the saved
+// pre-activation, the activation's gradient or the residual sum.
 // 64x64x16 tiles, 256 threads, 4x4 outputs per thread with 16-byte shared-memory reads and the next
 // K tile prefetched into registers (the reference's GemmTiled,
 // Source/Private/Oa/Core/Shader/Compute/Blas/Gemm/GemmTiled.slang:1-110, is the same tiling class), here
@@ -14,11 +17,38 @@ namespace oa {
 
 constexpr int FT = 64, FK = 16;
 
+struct F32Epi {
+  const float *bias, *residual, *aux_in;
+  float* aux_out;
+  int ldr, ldaux, act, accumulate;
+  float alpha;
+};
+
+// Not inlined: sixteen copies of tanhf and its gradient made the epilogue some tens of kilobytes of code, and a launch of a few
+// microseconds waited for the instruction fetches of the copies it jumped over.
+__device__ __noinline__ float f32_activation(int act, float v, float z) {
+  if (act == OA_ACT_GELU) return gelu_tanh(v);
+  if (act == OA_ACT_RELU) return fmaxf(v, 0.f);
+  if (act == OA_ACT_SILU) return silu_f(v);
+  if (act == OA_ACT_GELU_BWD) return v * gelu_tanh_grad(z);
+  if (act == OA_ACT_RELU_BWD) return z > 0.f ? v : 0.f;
+  return v;
+}
+
+__device__ __forceinline__ float f32_epilogue(const F32Epi& e, float acc, int m, int n, float* c) {
+  float v = acc * e.alpha;
+  if (e.bias) v += e.bias[n];
+  if (e.aux_out) e.aux_out[(long long)m * e.ldaux + n] = v;
+  if (e.act != OA_ACT_NONE) v = f32_activation(e.act, v, e.aux_in ? e.aux_in[(long long)m * e.ldaux + n] : 0.f);
+  if (e.residual) v += e.residual[(long long)m * e.ldr + n];
+  if (e.accumulate) v += *c;
+  return v;
+}
+
 __global__ void __launch_bounds__(256)
 gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ B, float* __restrict__ C, int M, int N, int K,
                 long long sam, long long sak, long long sbn, long long sbk, int ldc, long long batch_a,
-                long long batch_b, long long batch_c, const float* __restrict__ bias, int act, int accumulate,
-                float alpha, int k_chunk) {
+                long long batch_b, long long batch_c, const F32Epi epi, int k_chunk) {
   __shared__ __align__(16) float sA[FK][FT + 4];
   __shared__ __align__(16) float sB[FK][FT + 4];
   const int b = blockIdx.z;
@@ -81,16 +111,145 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ B, float*
     for (int j = 0; j < 4; ++j) {
       int gn = n0 + tx * 4 + j;
       if (gn >= N) continue;
-      float v = acc[i][j] * alpha;
-      if (bias) v += bias[gn];
-      if (act == OA_ACT_GELU) v = gelu_tanh(v);
-      else if (act == OA_ACT_RELU) v = fmaxf(v, 0.f);
-      else if (act == OA_ACT_SILU) v = silu_f(v);
       float* c = C + (long long)gm * ldc + gn;
-      if (accumulate) v += *c;
-      *c = v;
+      *c = f32_epilogue(epi, acc[i][j], gm, gn, c);
     }
   }
+}
+
+// Operands with one contiguous direction and 16-byte rows: the tile arrives through a ring of three 16-byte cp.async stages and
+// the fourth is multiplied, so that a block waits for memory once instead of once per 16 columns.  An operand keeps the layout it
+// has in memory ([row][k] with a pitch of 20 floats, or [k][row]); the columns a thread owns follow it, which leaves its 16-byte
+// reads free of bank conflicts.  TM x 4 outputs per thread: 32-row tiles while 64-row tiles would leave SMs without a block.  What
+// bounds it at these sizes: the ramp of a launch and the shared-memory reads.  The 51 products of a character-model step (2048
+// rows, widths 128 to 512): 852 us before, 650 us now.  128 threads with twice the outputs each measured 760 us.
+constexpr int F_THREADS = 256, F_TM = FT * 16 / F_THREADS, FS = 4, FP_K = FK + 4, FP_MN = FT + 4, F_STAGE = FT * FP_K;
+__device__ __forceinline__ void f32_cp16(float* dst, const float* src, int bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
+}
+// the 16-byte pieces of a [ROWS x 16] tile; `ld` is the pitch of the direction that is not contiguous
+template <int MN, int ROWS>
+__device__ __forceinline__ void f32_fetch(float* sm, const float* __restrict__ g, long long ld, int r0, int k0, int rows, int k_hi) {
+#pragma unroll
+  for (int i = threadIdx.x; i < ROWS * 4; i += F_THREADS) {
+    if (MN) {
+      constexpr int PER = ROWS / 4;
+      const int k = i / PER, r = (i % PER) * 4, left = rows - (r0 + r);
+      const int bytes = k0 + k < k_hi ? max(0, min(4, left)) * 4 : 0;
+      f32_cp16(sm + k * FP_MN + r, bytes ? g + (long long)(k0 + k) * ld + r0 + r : g, bytes);
+    } else {
+      const int r = i >> 2, k = (i & 3) * 4, left = k_hi - (k0 + k);
+      const int bytes = r0 + r < rows ? max(0, min(4, left)) * 4 : 0;
+      f32_cp16(sm + r * FP_K + k, bytes ? g + (long long)(r0 + r) * ld + k0 + k : g, bytes);
+    }
+  }
+}
+
+template <int A_MN, int B_MN, int TM>
+__global__ void __launch_bounds__(F_THREADS)
+gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ B, float* __restrict__ C, int M, int N, int K, long long lda,
+                     long long ldb, int ldc, long long batch_a, long long batch_b, long long batch_c, const F32Epi epi, int k_chunk) {
+  constexpr int TY = F_THREADS / 16, ROWS = TY * TM;
+  __shared__ __align__(16) float sA[FS][F_STAGE], sB[FS][F_STAGE];
+  const int b = blockIdx.z;
+  const int k_lo = k_chunk > 0 ? b * k_chunk : 0, k_hi = k_chunk > 0 ? min(K, k_lo + k_chunk) : K;
+  if (k_chunk == 0) { A += (long long)b * batch_a; B += (long long)b * batch_b; }
+  C += (long long)b * batch_c;
+  const int m0 = blockIdx.y * ROWS, n0 = blockIdx.x * FT;
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const int steps = (k_hi - k_lo + FK - 1) / FK;
+  auto load = [&](int i) {
+    if (i < steps) {
+      f32_fetch<A_MN, ROWS>(sA[i % FS], A, lda, m0, k_lo + i * FK, M, k_hi);
+      f32_fetch<B_MN, FT>(sB[i % FS], B, ldb, n0, k_lo + i * FK, N, k_hi);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int i = 0; i < FS - 1; ++i) load(i);
+  float acc[TM][4] = {};
+  for (int i = 0; i < steps; ++i) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(FS - 2) : "memory");
+    __syncthreads();                                  // stage i has landed everywhere, stage i - 1 has been read
+    load(i + FS - 1);
+    const float *pa = sA[i % FS], *pb = sB[i % FS];
+#pragma unroll
+    for (int kk = 0; kk < FK; kk += 4) {
+      float a[4][TM], bb[4][4];                       // [k][row], [k][column]
+      if (A_MN) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+#pragma unroll
+          for (int r = 0; r < TM; r += 2) {
+            const float2 v = *reinterpret_cast<const float2*>(pa + (kk + k) * FP_MN + ty * TM + r);
+            a[k][r] = v.x; a[k][r + 1] = v.y;
+          }
+        }
+      } else {
+#pragma unroll
+        for (int r = 0; r < TM; ++r) {
+          const float4 v = *reinterpret_cast<const float4*>(pa + (ty + TY * r) * FP_K + kk);
+          a[0][r] = v.x; a[1][r] = v.y; a[2][r] = v.z; a[3][r] = v.w;
+        }
+      }
+      if (B_MN) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const float4 v = *reinterpret_cast<const float4*>(pb + (kk + k) * FP_MN + tx * 4);
+          bb[k][0] = v.x; bb[k][1] = v.y; bb[k][2] = v.z; bb[k][3] = v.w;
+        }
+      } else {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const float4 v = *reinterpret_cast<const float4*>(pb + (tx + 16 * c) * FP_K + kk);
+          bb[0][c] = v.x; bb[1][c] = v.y; bb[2][c] = v.z; bb[3][c] = v.w;
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int r = 0; r < TM; ++r)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) acc[r][c] = fmaf(a[k][r], bb[k][c], acc[r][c]);
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < TM; ++r) {
+    const int gm = m0 + (A_MN ? ty * TM + r : ty + TY * r);
+    if (gm >= M) continue;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int gn = n0 + (B_MN ? tx * 4 + c : tx + 16 * c);
+      if (gn >= N) continue;
+      float* o = C + (long long)gm * ldc + gn;
+      *o = f32_epilogue(epi, acc[r][c], gm, gn, o);
+    }
+  }
+}
+
+// false: the operands do not fit the tile kernel
+static bool gemm_f32_tiles(const float* A, const float* B, float* C, int M, int N, int K, long long sam, long long sak, long long sbn, long long sbk,
+                           int ldc, int batch, long long batch_a, long long batch_b, long long batch_c, const F32Epi& epi, int k_chunk, int slices,
+                           cudaStream_t st) {
+  const bool a_k = sak == 1, b_k = sbk == 1;
+  const long long lda = a_k ? sam : sak, ldb = b_k ? sbn : sbk;
+  if ((!a_k && sam != 1) || (!b_k && sbn != 1) || ((lda | ldb | batch_a | batch_b) & 3) || lda < 0 || ldb < 0 || K <= 0 ||
+      ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B)) & 15))
+    return false;
+  const int z = k_chunk > 0 ? slices : batch;
+  const long long tiles = (long long)((N + FT - 1) / FT) * ((M + FT - 1) / FT) * z;
+  const int rows = tiles >= 148 ? 64 : 32;
+  const dim3 grid((N + FT - 1) / FT, (M + rows - 1) / rows, z);
+  if (grid.y > 65535) return false;
+#define OA_F32_TILE(AM, BMN)                                                                                                                  \
+  if (rows == 64) gemm_f32_tile_kernel<AM, BMN, F_TM><<<grid, F_THREADS, 0, st>>>(A, B, C, M, N, K, lda, ldb, ldc, batch_a, batch_b, batch_c, epi, k_chunk); \
+  else gemm_f32_tile_kernel<AM, BMN, F_TM / 2><<<grid, F_THREADS, 0, st>>>(A, B, C, M, N, K, lda, ldb, ldc, batch_a, batch_b, batch_c, epi, k_chunk)
+  if (a_k && b_k) { OA_F32_TILE(0, 0); }
+  else if (a_k) { OA_F32_TILE(0, 1); }
+  else if (b_k) { OA_F32_TILE(1, 0); }
+  else { OA_F32_TILE(1, 1); }
+#undef OA_F32_TILE
+  return true;
 }
 
 // C[m,n] = alpha * sum_s part[s][m,n] (+ C): fixed slice order, so the split-K result is reproducible
@@ -125,16 +284,17 @@ static float* splitk_scratch(size_t bytes, cudaStream_t st) {
 
 }  // namespace oa
 
-extern "C" int oa_gemm_f32(const float* A, const float* B, float* C, int M, int N, int K, long long sam, long long sak,
-                           long long sbn, long long sbk, int ldc, int batch, long long batch_a, long long batch_b,
-                           long long batch_c, const float* bias, int act, int accumulate, float alpha, void* stream) {
+static int gemm_f32(const float* A, const float* B, float* C, int M, int N, int K, long long sam, long long sak, long long sbn, long long sbk,
+                    int ldc, int batch, long long batch_a, long long batch_b, long long batch_c, const oa::F32Epi& epi, void* stream) {
   if (M <= 0 || N <= 0 || batch <= 0) return OA_OK;
   if (K < 0 || batch > 65535) return OA_ERR_ARG;
+  const oa::F32Epi part_epi{nullptr, nullptr, nullptr, nullptr, 0, 0, OA_ACT_NONE, 0, 1.0f};
+  const bool plain = !epi.bias && epi.act == OA_ACT_NONE && !epi.residual && !epi.aux_out;
   dim3 grid((N + oa::FT - 1) / oa::FT, (M + oa::FT - 1) / oa::FT, batch);
   cudaStream_t st = (cudaStream_t)stream;
   // Few output tiles and a long reduction (weight gradients of small models): slice K over more CTAs, then reduce the slices
   const int tiles = (int)(grid.x * grid.y);
-  if (batch == 1 && !bias && act == OA_ACT_NONE && tiles < 64 && K >= 512) {
+  if (batch == 1 && plain && tiles < 64 && K >= 512) {
     int splits = (256 + tiles - 1) / tiles;
     if (splits > K / 128) splits = K / 128;
     if (splits > 64) splits = 64;
@@ -144,15 +304,32 @@ extern "C" int oa_gemm_f32(const float* A, const float* B, float* C, int M, int 
       float* part = oa::splitk_scratch((size_t)splits * M * N * sizeof(float), st);
       if (part && splits >= 2) {
         grid.z = splits;
-        oa::gemm_f32_kernel<<<grid, 256, 0, st>>>(A, B, part, M, N, K, sam, sak, sbn, sbk, N, 0, 0, (long long)M * N, nullptr,
-                                                  OA_ACT_NONE, 0, 1.0f, k_chunk);
+        if (!oa::gemm_f32_tiles(A, B, part, M, N, K, sam, sak, sbn, sbk, N, 1, 0, 0, (long long)M * N, part_epi, k_chunk, splits, st))
+          oa::gemm_f32_kernel<<<grid, 256, 0, st>>>(A, B, part, M, N, K, sam, sak, sbn, sbk, N, 0, 0, (long long)M * N, part_epi,
+                                                  k_chunk);
         const long long n = (long long)M * N;
-        oa::gemm_f32_splitk_reduce_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(part, C, M, N, ldc, splits, accumulate, alpha);
+        oa::gemm_f32_splitk_reduce_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(part, C, M, N, ldc, splits, epi.accumulate, epi.alpha);
         return cudaGetLastError() == cudaSuccess ? OA_OK : OA_ERR_LAUNCH;
       }
     }
   }
-  oa::gemm_f32_kernel<<<grid, 256, 0, st>>>(A, B, C, M, N, K, sam, sak, sbn, sbk, ldc, batch_a, batch_b, batch_c, bias, act,
-                                            accumulate, alpha, 0);
+  if (!oa::gemm_f32_tiles(A, B, C, M, N, K, sam, sak, sbn, sbk, ldc, batch, batch_a, batch_b, batch_c, epi, 0, 0, st))
+    oa::gemm_f32_kernel<<<grid, 256, 0, st>>>(A, B, C, M, N, K, sam, sak, sbn, sbk, ldc, batch_a, batch_b, batch_c, epi, 0);
   return cudaGetLastError() == cudaSuccess ? OA_OK : OA_ERR_LAUNCH;
+}
+
+extern "C" int oa_gemm_f32(const float* A, const float* B, float* C, int M, int N, int K, long long sam, long long sak,
+                           long long sbn, long long sbk, int ldc, int batch, long long batch_a, long long batch_b,
+                           long long batch_c, const float* bias, int act, int accumulate, float alpha, void* stream) {
+  if (act == OA_ACT_GELU_BWD || act == OA_ACT_RELU_BWD) return OA_ERR_UNSUPPORTED;
+  return gemm_f32(A, B, C, M, N, K, sam, sak, sbn, sbk, ldc, batch, batch_a, batch_b, batch_c,
+                  oa::F32Epi{bias, nullptr, nullptr, nullptr, 0, 0, act, accumulate, alpha}, stream);
+}
+
+extern "C" int oa_gemm_f32_epi(const float* A, const float* B, float* C, int M, int N, int K, long long sam, long long sak, long long sbn,
+                               long long sbk, int ldc, const float* bias, const float* residual, int ldr, float* aux_out, const float* aux_in,
+                               int ldaux, int act, int accumulate, float alpha, void* stream) {
+  if ((act == OA_ACT_GELU_BWD || act == OA_ACT_RELU_BWD) && !aux_in) return OA_ERR_ARG;
+  return gemm_f32(A, B, C, M, N, K, sam, sak, sbn, sbk, ldc, 1, 0, 0, 0, oa::F32Epi{bias, residual, aux_in, aux_out, ldr, ldaux, act, accumulate, alpha},
+                  stream);
 }

@@ -241,12 +241,17 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         return out
     if a.dtype == torch.float32:
         assert b.dtype == torch.float32 and out.dtype == torch.float32
-        if (_f32_tensor_terms and 2.0 * M * Nn * K >= _F32_TENSOR_MIN_FLOPS and a.is_contiguous() and b.is_contiguous() and out.is_contiguous()
-                and M % 8 == 0 and Nn % 8 == 0 and K % 8 == 0 and act == ACT_NONE and bias is None and residual is None and aux_out is None
-                and aux_in is None):
+        tensor = bool(_f32_tensor_terms and 2.0 * M * Nn * K >= _F32_TENSOR_MIN_FLOPS and a.is_contiguous() and b.is_contiguous()
+                      and out.is_contiguous() and M % 8 == 0 and Nn % 8 == 0 and K % 8 == 0 and bias is None)
+        if tensor and act == ACT_NONE and residual is None and aux_out is None and aux_in is None:
             return _gemm_f32_tensor(a, b, a_mn, b_mn, out, accumulate, alpha, _f32_tensor_terms)
-        if act in (ACT_GELU_BWD, ACT_RELU_BWD) or residual is not None or aux_out is not None:
-            # composed from the plain product for the exact-fp32 path
+        sam, sak = (a.stride(1), a.stride(0)) if a_mn else (a.stride(0), a.stride(1))
+        sbn, sbk = (b.stride(1), b.stride(0)) if b_mn else (b.stride(0), b.stride(1))
+        aux = aux_out if aux_out is not None else (aux_in if act in (ACT_GELU_BWD, ACT_RELU_BWD) else None)
+        unit = lambda t: t is None or (t.dtype == torch.float32 and t.stride(1) == 1)
+        epilogue = residual is not None or aux_out is not None or act in (ACT_GELU_BWD, ACT_RELU_BWD)
+        if epilogue and (tensor or (aux_out is not None and act in (ACT_GELU_BWD, ACT_RELU_BWD)) or not (unit(residual) and unit(aux) and unit(out))):
+            # products on the tensor cores, and operands the kernel's epilogue does not take: composed from the plain product
             v = gemm(a, b, a_mn=a_mn, b_mn=b_mn, bias=bias, alpha=alpha)
             if aux_out is not None:
                 aux_out.copy_(v)
@@ -262,11 +267,11 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
                 v = binary("add", v, out)
             out.copy_(v)
             return out
-        sam, sak = (a.stride(1), a.stride(0)) if a_mn else (a.stride(0), a.stride(1))
-        sbn, sbk = (b.stride(1), b.stride(0)) if b_mn else (b.stride(0), b.stride(1))
-        rc = lib.oa_gemm_f32(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, Nn, K, sam, sak, sbn, sbk, out.stride(0),
-                             1, 0, 0, 0, N.ptr(bias), act, int(accumulate), float(alpha), st)
-        _launch(rc, "oa_gemm_f32")
+        rc = lib.oa_gemm_f32_epi(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, Nn, K, sam, sak, sbn, sbk, out.stride(0), N.ptr(bias),
+                                 N.ptr(residual), residual.stride(0) if residual is not None else 0, N.ptr(aux_out),
+                                 N.ptr(aux_in) if aux_out is None else None, aux.stride(0) if aux is not None else 0, act, int(accumulate),
+                                 float(alpha), st)
+        _launch(rc, "oa_gemm_f32_epi")
         return out
     raise N.OaKernelError(f"gemm: unsupported dtype {a.dtype}")
 

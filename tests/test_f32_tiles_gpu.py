@@ -1,0 +1,45 @@
+"""fp32 products through the tile kernel and its epilogue."""
+import pytest
+import torch
+
+from oa_b200.ops import kernels as K
+
+pytestmark = pytest.mark.gpu
+
+
+def _gelu(z):
+    return torch.nn.functional.gelu(z, approximate="tanh")
+
+
+# fp32 sums of up to 2048 products of unit variance in any order: a few 2^-24 sqrt(K), below 2e-6 of the result's norm
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, False), (True, True)])
+@pytest.mark.parametrize("m,n,k", [(1, 1, 1), (4, 4, 4), (65, 36, 20), (64, 64, 16), (132, 68, 100), (2048, 384, 128), (128, 512, 2048), (96, 200, 516), (33, 65, 17)])
+def test_products(m, n, k, a_mn, b_mn):
+    g = torch.Generator(device="cuda").manual_seed(m * 7 + n * 3 + k)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    a, b = r(k, m) if a_mn else r(m, k), r(k, n) if b_mn else r(n, k)
+    v = (a.t() if a_mn else a).double() @ (b if b_mn else b.t()).double()
+    bias, res, z, old = r(n), r(m, n), r(m, n), r(m, n)
+    rel = lambda got, ref: float((got.double() - ref).norm() / ref.norm().clamp_min(1e-30))
+    kw = dict(a_mn=a_mn, b_mn=b_mn)
+    assert rel(K.gemm(a, b, **kw), v) <= 2e-6
+    assert rel(K.gemm(a, b, alpha=0.5, out=old.clone(), accumulate=True, **kw), 0.5 * v + old.double()) <= 2e-6
+    assert rel(K.gemm(a, b, bias=bias, residual=res, **kw), v + bias.double() + res.double()) <= 2e-6
+    aux = torch.empty(m, n, device="cuda")
+    h = K.gemm(a, b, bias=bias, act=K.ACT_GELU, aux_out=aux, **kw)
+    assert rel(aux, v + bias.double()) <= 2e-6 and rel(h, _gelu(v + bias.double())) <= 4e-6
+    zz = z.double().requires_grad_(True)
+    (dg,) = torch.autograd.grad(_gelu(zz).sum(), zz)
+    assert rel(K.gemm(a, b, act=K.ACT_GELU_BWD, aux_in=z, **kw), v * dg) <= 4e-6
+    assert rel(K.gemm(a, b, act=K.ACT_RELU_BWD, aux_in=z, residual=res, **kw), v * (z > 0) + res.double()) <= 4e-6
+    strided = torch.full((m, n + 3), 5.0, device="cuda")
+    K.gemm(a, b, out=strided[:, :n], residual=res, **kw)
+    assert rel(strided[:, :n], v + res.double()) <= 2e-6 and bool((strided[:, n:] == 5.0).all())
+
+
+def test_unaligned_operands():
+    g = torch.Generator(device="cuda").manual_seed(1)
+    buf = torch.randn(40 * 33 + 1, device="cuda", generator=g)
+    a, b = buf[1:1 + 40 * 32].reshape(40, 32), torch.randn(24, 33, device="cuda", generator=g)[:, 1:]
+    ref = a.double() @ b.double().t()
+    assert float((K.gemm(a, b).double() - ref).norm() / ref.norm()) <= 2e-6
