@@ -829,8 +829,8 @@ gated_norm_bwd_kernel(const T* __restrict__ y, const T* __restrict__ z, long lon
 }
 
 // bf16 heads of 8, 16, 32, 64 or 128 columns: a lane owns eight neighbouring columns (one 16-byte access per operand), P / 8
-// lanes share a head.  The kernels above move one element per lane and access: at 8192 x 48 heads of 64 columns 142 us forward
-// and 172 us backward, where the bytes take 25 and 40 us.
+// lanes share a head.  The kernels above move one element per lane and access: 8192 x 48 heads of 64 columns take 142 us forward
+// and 172 us backward there, 42 and 82 us here (the bytes: 25 and 40).
 __device__ __forceinline__ void gn_load8(const __nv_bfloat16* p, float (&v)[8]) {
   const uint4 u = *reinterpret_cast<const uint4*>(p);
   const float2 a = unpack_bf16x2(u.x), b = unpack_bf16x2(u.y), c = unpack_bf16x2(u.z), d = unpack_bf16x2(u.w);
