@@ -172,15 +172,15 @@ __global__ void fill_vec_kernel(uint4* y, long long n16, uint4 pattern) {
 
 // Swiglu on a packed [rows, 2F] tensor: out = silu(A[:, :F]) * A[:, F:]
 // (Source/Private/Oa/Core/FnMatrix/.../FnMatrixActivation.gen.h:47-60).
-template <typename T>
+// I: 32-bit indices unless there are 2^31 vectors; the 64-bit division by the row length was most of the instructions.
+template <typename T, typename I>
 __global__ void swiglu_fwd_kernel(const T* __restrict__ gu, T* __restrict__ out, long long rows, int F) {
   constexpr int V = IO<T>::VEC;
-  long long per_row = F / V;
-  long long total = rows * per_row;
-  long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-    long long r = i / per_row;
-    int c = (int)(i % per_row) * V;
+  const I per_row = F / V, total = (I)rows * per_row, stride = (I)gridDim.x * blockDim.x;
+  for (I i = (I)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
+    const I row = i / per_row;
+    const long long r = row;
+    const int c = (int)(i - row * per_row) * V;
     float g[V], u[V];
     IO<T>::load(gu + r * 2 * F + c, g);
     IO<T>::load(gu + r * 2 * F + F + c, u);
@@ -189,16 +189,15 @@ __global__ void swiglu_fwd_kernel(const T* __restrict__ gu, T* __restrict__ out,
     IO<T>::store(out + r * F + c, g);
   }
 }
-template <typename T>
+template <typename T, typename I>
 __global__ void swiglu_bwd_kernel(const T* __restrict__ gu, const T* __restrict__ dout, T* __restrict__ dgu,
                                   long long rows, int F) {
   constexpr int V = IO<T>::VEC;
-  long long per_row = F / V;
-  long long total = rows * per_row;
-  long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-    long long r = i / per_row;
-    int c = (int)(i % per_row) * V;
+  const I per_row = F / V, total = (I)rows * per_row, stride = (I)gridDim.x * blockDim.x;
+  for (I i = (I)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
+    const I row = i / per_row;
+    const long long r = row;
+    const int c = (int)(i - row * per_row) * V;
     float g[V], u[V], d[V], dg[V], du[V];
     IO<T>::load(gu + r * 2 * F + c, g);
     IO<T>::load(gu + r * 2 * F + F + c, u);
@@ -652,12 +651,20 @@ extern "C" int oa_fill(int dtype, void* y, long long n, float value, void* strea
 }
 extern "C" int oa_swiglu_fwd(int dtype, const void* gu, void* out, long long rows, int F, void* stream) {
   if (F % 8) return OA_ERR_ALIGN;
-  DISPATCH_T(dtype, swiglu_fwd_kernel<T><<<grid_for(rows * F / IO<T>::VEC, 256), 256, 0, ST>>>((const T*)gu, (T*)out, rows, F));
+  if (rows * F / 4 < 0x70000000LL) {
+    DISPATCH_T(dtype, swiglu_fwd_kernel<T, unsigned><<<grid_for(rows * F / IO<T>::VEC, 256), 256, 0, ST>>>((const T*)gu, (T*)out, rows, F));
+  } else {
+    DISPATCH_T(dtype, swiglu_fwd_kernel<T, long long><<<grid_for(rows * F / IO<T>::VEC, 256), 256, 0, ST>>>((const T*)gu, (T*)out, rows, F));
+  }
   return CHECK_LAUNCH();
 }
 extern "C" int oa_swiglu_bwd(int dtype, const void* gu, const void* dout, void* dgu, long long rows, int F, void* stream) {
   if (F % 8) return OA_ERR_ALIGN;
-  DISPATCH_T(dtype, swiglu_bwd_kernel<T><<<grid_for(rows * F / IO<T>::VEC, 256), 256, 0, ST>>>((const T*)gu, (const T*)dout, (T*)dgu, rows, F));
+  if (rows * F / 4 < 0x70000000LL) {
+    DISPATCH_T(dtype, swiglu_bwd_kernel<T, unsigned><<<grid_for(rows * F / IO<T>::VEC, 256), 256, 0, ST>>>((const T*)gu, (const T*)dout, (T*)dgu, rows, F));
+  } else {
+    DISPATCH_T(dtype, swiglu_bwd_kernel<T, long long><<<grid_for(rows * F / IO<T>::VEC, 256), 256, 0, ST>>>((const T*)gu, (const T*)dout, (T*)dgu, rows, F));
+  }
   return CHECK_LAUNCH();
 }
 extern "C" int oa_rope(int dtype, void* x, long long rows, int row_stride, int n_heads, int head_dim, int seq_len,

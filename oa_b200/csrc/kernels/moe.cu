@@ -204,17 +204,17 @@ __global__ void moe_plan_place_kernel(const int* __restrict__ topk_idx, long lon
 }
 
 // packed[r,:] = x[packed_token[r],:]  (zero rows for padding, packed_token[r] < 0)
-template <typename T>
+// I: 32-bit indices unless there are 2^31 vectors (the 64-bit division by the row length was most of the instructions)
+template <typename T, typename I>
 __global__ void moe_gather_kernel(const T* __restrict__ x, const int* __restrict__ packed_token, T* __restrict__ packed,
                                   const int* __restrict__ offsets, int E, int dim, long long max_rows) {
   const long long rows = max_rows;   // rows past the last segment are padding too (packed_token = -1): keep them zero
   (void)offsets; (void)E;
   const int vec = dim / 8;
-  long long total = rows * vec;
-  long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-    long long r = i / vec;
-    int c = (int)(i % vec) * 8;
+  const I total = (I)(rows * vec), stride = (I)gridDim.x * blockDim.x;
+  for (I i = (I)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
+    const long long r = i / (I)vec;
+    const int c = (int)(i % (I)vec) * 8;
     int t = packed_token[r];
     uint4 v = make_uint4(0, 0, 0, 0);
     if (t >= 0) v = *reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(x) + (long long)t * dim + c);
@@ -223,15 +223,15 @@ __global__ void moe_gather_kernel(const T* __restrict__ x, const int* __restrict
 }
 
 // out[t,:] = (base ? base[t,:] : 0) + sum_k gate[t,k] * packed[inverse[t,k],:]      (bf16, 8 columns per thread)
+template <typename I>
 __global__ void moe_combine_kernel(const __nv_bfloat16* __restrict__ packed, const float* __restrict__ gate,
                                    const int* __restrict__ inverse, const __nv_bfloat16* __restrict__ base,
                                    __nv_bfloat16* __restrict__ out, long long tokens, int Kk, int dim) {
   const int vec = dim / 8;
-  long long total = tokens * vec;
-  long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-    long long t = i / vec;
-    int c = (int)(i % vec) * 8;
+  const I total = (I)(tokens * vec), stride = (I)gridDim.x * blockDim.x;
+  for (I i = (I)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
+    const long long t = i / (I)vec;
+    const int c = (int)(i % (I)vec) * 8;
     float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     if (base) {
       uint4 b = *reinterpret_cast<const uint4*>(base + t * dim + c);
@@ -289,15 +289,15 @@ __global__ void moe_combine_bwd_kernel(const __nv_bfloat16* __restrict__ packed,
 }
 
 // Backward of gather: dx[t,:] = (base ? base[t,:] : 0) + sum_k dpacked[inverse[t,k],:]  (single writer per token)
+template <typename I>
 __global__ void moe_gather_bwd_kernel(const __nv_bfloat16* __restrict__ dpacked, const int* __restrict__ inverse,
                                       const __nv_bfloat16* __restrict__ base, __nv_bfloat16* __restrict__ dx, long long tokens,
                                       int Kk, int dim) {
   const int vec = dim / 8;
-  long long total = tokens * vec;
-  long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-    long long t = i / vec;
-    int c = (int)(i % vec) * 8;
+  const I total = (I)(tokens * vec), stride = (I)gridDim.x * blockDim.x;
+  for (I i = (I)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
+    const long long t = i / (I)vec;
+    const int c = (int)(i % (I)vec) * 8;
     float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     if (base) {
       uint4 b = *reinterpret_cast<const uint4*>(base + t * dim + c);
@@ -378,13 +378,15 @@ extern "C" int oa_moe_plan(const int* topk_idx, long long tokens, int K, int E, 
 extern "C" int oa_moe_gather(const void* x, const int* packed_token, void* packed, const int* offsets, int E, int dim,
                              long long max_rows, void* stream) {
   if (dim % 8) return OA_ERR_ALIGN;
-  moe_gather_kernel<__nv_bfloat16><<<mgrid(max_rows * (dim / 8)), 256, 0, ST>>>((const __nv_bfloat16*)x, packed_token, (__nv_bfloat16*)packed, offsets, E, dim, max_rows);
+  if (max_rows * (dim / 8) < 0x70000000LL) moe_gather_kernel<__nv_bfloat16, unsigned><<<mgrid(max_rows * (dim / 8)), 256, 0, ST>>>((const __nv_bfloat16*)x, packed_token, (__nv_bfloat16*)packed, offsets, E, dim, max_rows);
+  else moe_gather_kernel<__nv_bfloat16, long long><<<mgrid(max_rows * (dim / 8)), 256, 0, ST>>>((const __nv_bfloat16*)x, packed_token, (__nv_bfloat16*)packed, offsets, E, dim, max_rows);
   return CHECK_LAUNCH();
 }
 extern "C" int oa_moe_combine(const void* packed, const float* gate, const int* inverse, const void* base, void* out,
                               long long tokens, int K, int dim, void* stream) {
   if (dim % 8) return OA_ERR_ALIGN;
-  moe_combine_kernel<<<mgrid(tokens * (dim / 8)), 256, 0, ST>>>((const __nv_bfloat16*)packed, gate, inverse, (const __nv_bfloat16*)base, (__nv_bfloat16*)out, tokens, K, dim);
+  if (tokens * (dim / 8) < 0x70000000LL) moe_combine_kernel<unsigned><<<mgrid(tokens * (dim / 8)), 256, 0, ST>>>((const __nv_bfloat16*)packed, gate, inverse, (const __nv_bfloat16*)base, (__nv_bfloat16*)out, tokens, K, dim);
+  else moe_combine_kernel<long long><<<mgrid(tokens * (dim / 8)), 256, 0, ST>>>((const __nv_bfloat16*)packed, gate, inverse, (const __nv_bfloat16*)base, (__nv_bfloat16*)out, tokens, K, dim);
   return CHECK_LAUNCH();
 }
 extern "C" int oa_moe_combine_bwd(const void* packed, const float* gate, const int* inverse, const int* packed_token,
@@ -398,7 +400,8 @@ extern "C" int oa_moe_combine_bwd(const void* packed, const float* gate, const i
 extern "C" int oa_moe_gather_bwd(const void* dpacked, const int* inverse, const void* base, void* dx, long long tokens, int K,
                                  int dim, void* stream) {
   if (dim % 8) return OA_ERR_ALIGN;
-  moe_gather_bwd_kernel<<<mgrid(tokens * (dim / 8)), 256, 0, ST>>>((const __nv_bfloat16*)dpacked, inverse, (const __nv_bfloat16*)base, (__nv_bfloat16*)dx, tokens, K, dim);
+  if (tokens * (dim / 8) < 0x70000000LL) moe_gather_bwd_kernel<unsigned><<<mgrid(tokens * (dim / 8)), 256, 0, ST>>>((const __nv_bfloat16*)dpacked, inverse, (const __nv_bfloat16*)base, (__nv_bfloat16*)dx, tokens, K, dim);
+  else moe_gather_bwd_kernel<long long><<<mgrid(tokens * (dim / 8)), 256, 0, ST>>>((const __nv_bfloat16*)dpacked, inverse, (const __nv_bfloat16*)base, (__nv_bfloat16*)dx, tokens, K, dim);
   return CHECK_LAUNCH();
 }
 
