@@ -590,9 +590,9 @@ __global__ void __launch_bounds__(256) ssd_theta_fwd_kernel(const float* __restr
   }
 }
 
-__global__ void __launch_bounds__(256) ssd_theta_bwd_kernel(const float* __restrict__ dtheta, const float* __restrict__ angle, int lda,
+__global__ void __launch_bounds__(256) ssd_theta_bwd_kernel(float* __restrict__ dtheta, const float* __restrict__ angle, int lda,
                                                             const float* __restrict__ dt, float* __restrict__ tot,
-                                                            float* __restrict__ dangle, float* __restrict__ ddt, SsdDims d, int pass) {
+                                                            float* __restrict__ ddt, SsdDims d, int pass) {
   const int wid = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (wid >= d.B * d.nC * d.H) return;
   const int h = wid % d.H, c = (wid / d.H) % d.nC, b = wid / (d.H * d.nC);
@@ -605,7 +605,9 @@ __global__ void __launch_bounds__(256) ssd_theta_bwd_kernel(const float* __restr
     }
     return;
   }
-  // A <= 32 * 4 supported: each lane carries up to 4 running suffix sums
+  // A <= 32 * 4 supported: each lane carries up to 4 running suffix sums.  Four tokens are requested at a time; the share of this
+  // head in d angle replaces d theta, and ssd_angle_sum_kernel adds the heads up (as atomics on d angle it took 60 us of 108 at
+  // 2 x 4096 tokens, 48 heads).
   float run[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
@@ -613,21 +615,48 @@ __global__ void __launch_bounds__(256) ssd_theta_bwd_kernel(const float* __restr
     if (a < d.A)
       for (int cp = c + 1; cp < d.nC; ++cp) run[q] += tot[(((long long)b * d.nC + cp) * d.H + h) * d.A + a];
   }
-  for (int t = SQ - 1; t >= 0; --t) {
-    const long long r = row0 + t;
-    const float dtv = dt[r * d.H + h];
-    float acc = 0.f;
+  for (int t0 = SQ - 1; t0 >= 0; t0 -= 4) {
+    float dth[4][4], an[4][4], dtv[4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int a = lane + 32 * q;
-      if (a < d.A) {
-        run[q] += dtheta[(r * d.H + h) * d.A + a];
-        atomicAdd(dangle + r * lda + a, run[q] * dtv);
-        acc += run[q] * angle[r * lda + a];
+    for (int u = 0; u < 4; ++u) {
+      const long long r = row0 + t0 - u;
+      dtv[u] = dt[r * d.H + h];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int a = lane + 32 * q;
+        dth[u][q] = a < d.A ? dtheta[(r * d.H + h) * d.A + a] : 0.f;
+        an[u][q] = a < d.A ? angle[r * lda + a] : 0.f;
       }
     }
-    acc = warp_sum(acc);
-    if (lane == 0) ddt[r * d.H + h] = acc;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const long long r = row0 + t0 - u;
+      float acc = 0.f;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int a = lane + 32 * q;
+        if (a < d.A) {
+          run[q] += dth[u][q];
+          dtheta[(r * d.H + h) * d.A + a] = run[q] * dtv[u];
+          acc += run[q] * an[u][q];
+        }
+      }
+      acc = warp_sum(acc);
+      if (lane == 0) ddt[r * d.H + h] = acc;
+    }
+  }
+}
+
+// dangle[row, a] += sum over heads of the shares left in d theta, in head order.  One warp per row.
+__global__ void __launch_bounds__(256) ssd_angle_sum_kernel(const float* __restrict__ share, float* __restrict__ dangle, int lda, long long rows, int H,
+                                                            int A) {
+  const long long r = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (r >= rows) return;
+  for (int a = threadIdx.x & 31; a < A; a += 32) {
+    float s = 0.f;
+#pragma unroll 8
+    for (int h = 0; h < H; ++h) s += share[(r * H + h) * A + a];
+    dangle[r * lda + a] += s;
   }
 }
 
@@ -827,16 +856,18 @@ int oa_ssd_theta_fwd(const void* angle, int lda, const void* dt, void* tot, void
   return ssd_status();
 }
 
-// dangle [B*L, lda] (+=, zeroed by the caller) and ddt [B*L, H] (=) from dtheta; A <= 128
-int oa_ssd_theta_bwd(const void* dtheta, const void* angle, int lda, const void* dt, void* tot, void* dangle, void* ddt, int B, int L,
+// dangle [B*L, lda] (+=, zeroed by the caller) and ddt [B*L, H] (=) from dtheta, which is used up; A <= 128
+int oa_ssd_theta_bwd(void* dtheta, const void* angle, int lda, const void* dt, void* tot, void* dangle, void* ddt, int B, int L,
                      int H, int A, void* stream) {
   SsdDims d{B, L, H, 2, 2 * A > 4 ? ((2 * A + 3) / 4) * 4 : 4, A, L / SQ};
   if (!ssd_dims_ok(d) || A <= 0 || A > 128 || lda < A) return OA_ERR_ARG;
   const int warps = B * d.nC * H, grid = (warps + 7) / 8;
-  ssd_theta_bwd_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>((const float*)dtheta, (const float*)angle, lda, (const float*)dt,
-                                                              (float*)tot, (float*)dangle, (float*)ddt, d, 0);
-  ssd_theta_bwd_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>((const float*)dtheta, (const float*)angle, lda, (const float*)dt,
-                                                              (float*)tot, (float*)dangle, (float*)ddt, d, 1);
+  ssd_theta_bwd_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>((float*)dtheta, (const float*)angle, lda, (const float*)dt,
+                                                              (float*)tot, (float*)ddt, d, 0);
+  ssd_theta_bwd_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>((float*)dtheta, (const float*)angle, lda, (const float*)dt,
+                                                              (float*)tot, (float*)ddt, d, 1);
+  const long long rows = (long long)B * L;
+  ssd_angle_sum_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, (cudaStream_t)stream>>>((const float*)dtheta, (float*)dangle, lda, rows, H, A);
   return ssd_status();
 }
 

@@ -376,7 +376,7 @@ def ssd_bwd_cuda(s: SsdSavedCuda, proj: torch.Tensor, dy: torch.Tensor, dproj: t
         lda = s.angle.shape[-1]
         dangle, ddt_theta, tot = z32(rows, lda), f32(B, L, H), f32(B, nC, H, A)
         K._launch(lib.oa_ssd_theta_bwd(dtheta.data_ptr(), s.angle.data_ptr(), lda, s.dt.data_ptr(), tot.data_ptr(), dangle.data_ptr(),
-                                       ddt_theta.data_ptr(), B, L, H, A, st), "oa_ssd_theta_bwd", 2)
+                                       ddt_theta.data_ptr(), B, L, H, A, st), "oa_ssd_theta_bwd", 3)
         out["angle"] = dangle
     else:
         out["angle"] = z32(rows, 1)
