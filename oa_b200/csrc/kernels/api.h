@@ -310,7 +310,7 @@ int oa_ssd_state_bwd(const void* T, const void* cum, const void* Hin, void* dHou
 int oa_ssd_out_fwd(const void* Y, const void* z, long long ldz, void* y, void* yraw, long long ldy, int B, int L, int H, int P,
                    void* stream);
 int oa_ssd_dy_prep(const void* dy, const void* yraw, long long ldy, const void* z, long long ldz, void* dz, long long lddz, void* dY,
-                   const void* cum, void* dYe, int B, int L, int H, int P, void* stream);
+                   int B, int L, int H, int P, void* stream);
 int oa_ssd_mask_bwd(const void* dM, const void* Gm, const void* cum, const void* scale, void* dG, void* row_mm, void* col_mm,
                     void* col_ge, void* diag, int G, void* stream);
 int oa_ssd_prep_bwd(const void* dCt, const void* dBt, const void* dCe, const void* Ct, const void* Bt, const void* cum, const void* dqk,

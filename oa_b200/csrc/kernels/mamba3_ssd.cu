@@ -8,7 +8,7 @@
 //   ssd_mask_fwd    G (fp32) -> M (bf16): decayed strict lower triangle + exact diagonal
 //   ssd_state_fwd   recurrence over the chunk states, emits the state entering every chunk
 //   ssd_out_fwd     Y (fp32 chunk layout) -> y (token layout) with the silu(z) gate
-//   ssd_dy_prep     dy -> dY (bf16 chunk layout) through the gate, dz; optionally dY e^cum too
+//   ssd_dy_prep     dy -> dY (bf16 chunk layout) through the gate, dz
 //   ssd_state_bwd   reverse recurrence: gradient w.r.t. every chunk's outgoing state and w.r.t. cumQ
 //   ssd_mask_bwd    dM, G -> dG (bf16) + row / column sums that carry d cum, d scale, d gamma, d D
 //   ssd_prep_bwd    dC~, dB~, d(C~e^cum) -> un-rotate, d theta, dCn / dBn (summed over heads), dCb / dBb
@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(256) ssd_prep_fwd_kernel(SsdPrepFwd a) {
         const long long o = og * d.N + lane * 4;
         *reinterpret_cast<uint2*>(a.Ct + o) = make_uint2(pack_bf16x2(cv.x, cv.y), pack_bf16x2(cv.z, cv.w));
         *reinterpret_cast<uint2*>(a.Bt + o) = make_uint2(pack_bf16x2(bv.x, bv.y), pack_bf16x2(bv.z, bv.w));
-        if (a.Ce) *reinterpret_cast<uint2*>(a.Ce + o) = make_uint2(pack_bf16x2(cv.x * e, cv.y * e), pack_bf16x2(cv.z * e, cv.w * e));
+        *reinterpret_cast<uint2*>(a.Ce + o) = make_uint2(pack_bf16x2(cv.x * e, cv.y * e), pack_bf16x2(cv.z * e, cv.w * e));
       }
       if (lane == 0) a.qk[og] = qk;
       if (live_x) {
@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(256) ssd_prep_fwd_kernel(SsdPrepFwd a) {
       const long long o = og * d.N + n4 * 4;
       *reinterpret_cast<uint2*>(a.Ct + o) = make_uint2(pack_bf16x2(cv.x, cv.y), pack_bf16x2(cv.z, cv.w));
       *reinterpret_cast<uint2*>(a.Bt + o) = make_uint2(pack_bf16x2(bv.x, bv.y), pack_bf16x2(bv.z, bv.w));
-      if (a.Ce) *reinterpret_cast<uint2*>(a.Ce + o) = make_uint2(pack_bf16x2(cv.x * e, cv.y * e), pack_bf16x2(cv.z * e, cv.w * e));
+      *reinterpret_cast<uint2*>(a.Ce + o) = make_uint2(pack_bf16x2(cv.x * e, cv.y * e), pack_bf16x2(cv.z * e, cv.w * e));
     }
     qk = warp_sum(qk);
     if (lane == 0) a.qk[og] = qk;
@@ -320,7 +320,7 @@ __global__ void __launch_bounds__(256) ssd_out_fwd_kernel(const float* __restric
 __global__ void __launch_bounds__(256) ssd_dy_prep_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ yraw,
                                                           long long ldy, const __nv_bfloat16* __restrict__ z, long long ldz,
                                                           __nv_bfloat16* __restrict__ dz, long long lddz, __nv_bfloat16* __restrict__ dY,
-                                                          const float* __restrict__ cum, __nv_bfloat16* __restrict__ dYe, SsdDims d) {
+                                                          SsdDims d) {
   const int P2 = d.P >> 1;
   const long long total = (long long)d.B * d.H * d.nC * SQ * P2;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -341,28 +341,18 @@ __global__ void __launch_bounds__(256) ssd_dy_prep_kernel(const __nv_bfloat16* _
       g.x *= zf.x * s0; g.y *= zf.y * s1;
     }
     *reinterpret_cast<unsigned*>(dY + i * 2) = pack_bf16x2(g.x, g.y);
-    if (dYe) {
-      const float e = __expf(cum[i / P2]);                     // i / P2 = g * SQ + t
-      *reinterpret_cast<unsigned*>(dYe + i * 2) = pack_bf16x2(g.x * e, g.y * e);
-    }
   }
 }
 
 // The same without the gate, eight columns per thread (P a multiple of 8, rows on 16-byte boundaries).
 __global__ void __launch_bounds__(256) ssd_dy_prep_vec_kernel(const __nv_bfloat16* __restrict__ dy, long long ldy, __nv_bfloat16* __restrict__ dY,
-                                                              const float* __restrict__ cum, __nv_bfloat16* __restrict__ dYe, SsdDims d) {
+                                                              SsdDims d) {
   const int P8 = d.P >> 3;
   const unsigned i = blockIdx.x * blockDim.x + threadIdx.x, total = (unsigned)d.B * d.H * d.nC * SQ * P8;
   if (i >= total) return;
   const unsigned gt = i / P8, p8 = i - gt * P8, g = gt / SQ, t = gt - g * SQ, bh = g / d.nC, c = g - bh * d.nC, b = bh / d.H, h = bh - b * d.H;
   const long long row = (long long)b * d.L + (long long)c * SQ + t;
-  const uint4 v = *reinterpret_cast<const uint4*>(dy + row * ldy + (long long)h * d.P + p8 * 8);
-  *reinterpret_cast<uint4*>(dY + (long long)i * 8) = v;
-  if (!dYe) return;
-  const float e = __expf(cum[gt]);
-  const float2 a0 = unpack_bf16x2(v.x), a1 = unpack_bf16x2(v.y), a2 = unpack_bf16x2(v.z), a3 = unpack_bf16x2(v.w);
-  *reinterpret_cast<uint4*>(dYe + (long long)i * 8) = make_uint4(pack_bf16x2(a0.x * e, a0.y * e), pack_bf16x2(a1.x * e, a1.y * e),
-                                                                 pack_bf16x2(a2.x * e, a2.y * e), pack_bf16x2(a3.x * e, a3.y * e));
+  *reinterpret_cast<uint4*>(dY + (long long)i * 8) = *reinterpret_cast<const uint4*>(dy + row * ldy + (long long)h * d.P + p8 * 8);
 }
 
 // ------------------------------------------------------------------------------------------------------ mask backward
@@ -799,20 +789,19 @@ int oa_ssd_out_fwd(const void* Y, const void* z, long long ldz, void* y, void* y
 }
 
 int oa_ssd_dy_prep(const void* dy, const void* yraw, long long ldy, const void* z, long long ldz, void* dz, long long lddz, void* dY,
-                   const void* cum, void* dYe, int B, int L, int H, int P, void* stream) {
+                   int B, int L, int H, int P, void* stream) {
   SsdDims d{B, L, H, P, 4, 0, L / SQ};
-  if (!ssd_dims_ok(d) || (z && (!yraw || !dz)) || (dYe && !cum)) return OA_ERR_ARG;
-  if (!z && P % 8 == 0 && ldy % 8 == 0 && ((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(dY) | reinterpret_cast<uintptr_t>(dYe)) & 15) == 0 &&
+  if (!ssd_dims_ok(d) || (z && (!yraw || !dz))) return OA_ERR_ARG;
+  if (!z && P % 8 == 0 && ldy % 8 == 0 && ((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(dY)) & 15) == 0 &&
       (long long)B * L * H * (P / 8) < 0x7fffff00LL) {
     const long long n = (long long)B * L * H * (P / 8);
-    ssd_dy_prep_vec_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)dy, ldy, (__nv_bfloat16*)dY,
-                                                                                        (const float*)cum, (__nv_bfloat16*)dYe, d);
+    ssd_dy_prep_vec_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)dy, ldy, (__nv_bfloat16*)dY, d);
     return ssd_status();
   }
   const long long total = (long long)B * L * H * (P / 2);
   ssd_dy_prep_kernel<<<(int)((total + 255) / 256 > 148 * 32 ? 148 * 32 : (total + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
       (const __nv_bfloat16*)dy, (const __nv_bfloat16*)yraw, ldy, (const __nv_bfloat16*)z, ldz, (__nv_bfloat16*)dz, lddz,
-      (__nv_bfloat16*)dY, (const float*)cum, (__nv_bfloat16*)dYe, d);
+      (__nv_bfloat16*)dY, d);
   return ssd_status();
 }
 

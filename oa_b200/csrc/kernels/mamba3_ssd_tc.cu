@@ -377,8 +377,8 @@ ssd_chunk_bwd_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_const
               const float e = k < lim ? __expf(ct - csv[j]) : 0.f;
               const float gg = __uint_as_float(gv[k]), dm = __uint_as_float(dv[k]);
               const float es = e * scv[j];
-              mv[j] = k == lim ? dval : gg * es;
-              gvv[j] = dm * es;
+              mv[j] = k < lim ? gg * es : (k == lim ? dval : 0.f);    // chosen, not multiplied by 0: a later token may hold an infinity
+              gvv[j] = k < lim ? dm * es : 0.f;
               ge[k] = k < lim ? dm * gg * e : 0.f;
               rsum += ge[k] * scv[j];
               if (k == lim) { p.diag[gi] = dm; s_dqk[t] = dm * gam; }

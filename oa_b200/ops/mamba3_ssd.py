@@ -269,14 +269,13 @@ def ssd_fwd_cuda(proj: torch.Tensor, Bn, Cn, dt, adt, trap, angle, Bb, Cb, D, d:
         theta, tot = f32(B, L, H, A), f32(B, nC, H, A)
         K._launch(lib.oa_ssd_theta_fwd(angle.data_ptr(), angle.shape[-1], dt.data_ptr(), tot.data_ptr(), theta.data_ptr(), B, L, H, A, st),
                   "oa_ssd_theta_fwd", 2)
-    # State width 128 and head width 64 (projected rows on 16-byte boundaries) run everything between the chunk states and y in one kernel (and likewise in the
-    # backward pass), which needs neither C~ e^cum nor the mask in memory; other widths run the GEMMs one by one.
+    # State width 128 and head width 64 (projected rows on 16-byte boundaries) run everything between the chunk states and y in
+    # one kernel (and likewise in the backward pass), which keeps the mask out of memory; other widths run the GEMMs one by one.
     fused = P == 64 and Nn == 128 and d.d_in_proj % 8 == 0 and proj.data_ptr() % 16 == 0
-    Ct, Bt, X, Xw = bf(G, Q, Nn), bf(G, Q, Nn), bf(G, Q, P), bf(G, Q, P)
-    Ce = None if fused else bf(G, Q, Nn)
+    Ct, Bt, Ce, X, Xw = bf(G, Q, Nn), bf(G, Q, Nn), bf(G, Q, Nn), bf(G, Q, P), bf(G, Q, P)
     cum, gamma, scale, w, qk = f32(G, Q), f32(G, Q), f32(G, Q), f32(G, Q), f32(G, Q)
     K._launch(lib.oa_ssd_prep_fwd(proj.data_ptr() + o[1] * es, d.d_in_proj, Bn.data_ptr(), Cn.data_ptr(), Bb.data_ptr(), Cb.data_ptr(),
-                                  dt.data_ptr(), adt.data_ptr(), trap.data_ptr(), N.ptr(theta), Ct.data_ptr(), Bt.data_ptr(), N.ptr(Ce),
+                                  dt.data_ptr(), adt.data_ptr(), trap.data_ptr(), N.ptr(theta), Ct.data_ptr(), Bt.data_ptr(), Ce.data_ptr(),
                                   X.data_ptr(), Xw.data_ptr(), cum.data_ptr(), gamma.data_ptr(), scale.data_ptr(), w.data_ptr(),
                                   qk.data_ptr(), B, L, H, P, Nn, A, st), "oa_ssd_prep_fwd")
     M = Y = None
@@ -327,17 +326,14 @@ def ssd_bwd_cuda(s: SsdSavedCuda, proj: torch.Tensor, dy: torch.Tensor, dproj: t
     dy = dy.contiguous()
     fused = s.M is None
     dY = bf(G, Q, P)
-    dYe = bf(G, Q, P) if fused else None
     K._launch(lib.oa_ssd_dy_prep(dy.data_ptr(), N.ptr(s.yraw), d.d_inner, proj.data_ptr() + o[0] * es if d.has_z else None, d.d_in_proj,
                                  dproj.data_ptr() + o[0] * es if d.has_z else None, d.d_in_proj, dY.data_ptr(),
-                                 s.cum.data_ptr() if fused else None, N.ptr(dYe), B, L, H, P, st), "oa_ssd_dy_prep")
-    # gradient of the chunk states through y: T = dY^T (C~ e^cum)
-    T = K.bgemm(dYe, s.Ct, a_mn=True, b_mn=True, out_dtype=torch.float32) if fused else \
-        K.bgemm(dY, s.Ce, a_mn=True, b_mn=True, out_dtype=torch.float32)
+                                 B, L, H, P, st), "oa_ssd_dy_prep")
+    T = K.bgemm(dY, s.Ce, a_mn=True, b_mn=True, out_dtype=torch.float32)    # gradient of the chunk states through y
     dHout, dcumQ = bf(G, P, Nn), z32(G)
     K._launch(lib.oa_ssd_state_bwd(T.data_ptr(), s.cum.data_ptr(), s.Hin.data_ptr(), dHout.data_ptr(), dcumQ.data_ptr(), B * H, nC, P * Nn, st),
               "oa_ssd_state_bwd")
-    del T, dYe
+    del T
     row_mm, col_mm, col_ge, diag, dcum_ce, dw = (f32(G, Q) for _ in range(6))
     dqk = dCe = None
     if fused:
