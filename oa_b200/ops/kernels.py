@@ -145,6 +145,11 @@ def split_bf16(x: torch.Tensor, terms: int) -> torch.Tensor:
     return out
 
 
+def _f32_epilogue_takes(t: Optional[torch.Tensor], m: int, n: int) -> bool:
+    """Whether the fp32 product's epilogue may address `t` as t[row * pitch + column]: it reads or writes all of [m, n]."""
+    return t is None or (t.dtype == torch.float32 and tuple(t.shape) == (m, n) and t.stride(1) == 1)
+
+
 def _gemm_f32_tensor(a, b, a_mn, b_mn, out, accumulate, alpha, terms) -> torch.Tensor:
     """out = alpha * A B^T in fp32 from bf16 products on the tensor cores: every pair of parts whose combined order is below
     `terms`, smallest contributions first, accumulated in the fp32 output."""
@@ -248,10 +253,11 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         sam, sak = (a.stride(1), a.stride(0)) if a_mn else (a.stride(0), a.stride(1))
         sbn, sbk = (b.stride(1), b.stride(0)) if b_mn else (b.stride(0), b.stride(1))
         aux = aux_out if aux_out is not None else (aux_in if act in (ACT_GELU_BWD, ACT_RELU_BWD) else None)
-        unit = lambda t: t is None or (t.dtype == torch.float32 and t.stride(1) == 1)
         epilogue = residual is not None or aux_out is not None or act in (ACT_GELU_BWD, ACT_RELU_BWD)
-        if epilogue and (tensor or (aux_out is not None and act in (ACT_GELU_BWD, ACT_RELU_BWD)) or not (unit(residual) and unit(aux) and unit(out))):
-            # products on the tensor cores, and operands the kernel's epilogue does not take: composed from the plain product
+        if epilogue and (tensor or (aux_out is not None and act in (ACT_GELU_BWD, ACT_RELU_BWD)) or
+                         not all(_f32_epilogue_takes(t, M, Nn) for t in (residual, aux, out))):
+            # products on the tensor cores, and operands the kernel's epilogue does not take (a row, a column or a scalar to be
+            # broadcast, or a shape to be refused): composed from the plain product
             v = gemm(a, b, a_mn=a_mn, b_mn=b_mn, bias=bias, alpha=alpha)
             if aux_out is not None:
                 aux_out.copy_(v)

@@ -43,3 +43,27 @@ def test_unaligned_operands():
     a, b = buf[1:1 + 40 * 32].reshape(40, 32), torch.randn(24, 33, device="cuda", generator=g)[:, 1:]
     ref = a.double() @ b.double().t()
     assert float((K.gemm(a, b).double() - ref).norm() / ref.norm()) <= 2e-6
+
+
+# A residual is [m, n], a row, a column or a scalar; the shapes beside them are refused, as are gradients of another shape.
+@pytest.mark.parametrize("m,n,k", [(40, 24, 32), (70, 65, 16), (5, 1, 8), (1, 7, 8)])
+def test_residual_shapes(m, n, k):
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    a, b, z = r(m, k), r(n, k), r(m, n)
+    v = a.double() @ b.double().t()
+    rel = lambda got, ref: float((got.double() - ref).norm() / ref.norm())
+    for res in (r(n), r(1, n), r(m, 1), r(1), r(1, n).expand(m, n), r(n, m).t()):
+        assert rel(K.gemm(a, b, residual=res), v + res.double()) <= 2e-6
+        assert rel(K.gemm(a, b, act=K.ACT_RELU_BWD, aux_in=z, residual=res), v * (z > 0) + res.double()) <= 4e-6
+    if m > 1 and n > 1:
+        for res in (r(m - 1, n), r(m + 1, n), r(m, n + 1), r(1, m, n), r(2)):
+            with pytest.raises(ValueError):
+                K.gemm(a, b, residual=res)
+        for aux in (r(m - 1, n), r(n), r(m, 1)):
+            with pytest.raises(ValueError):
+                K.gemm(a, b, act=K.ACT_GELU_BWD, aux_in=aux)
+        with pytest.raises(RuntimeError):
+            K.gemm(a, b, aux_out=torch.empty(m - 1, n, device="cuda"), act=K.ACT_GELU)
+        with pytest.raises(RuntimeError):
+            K.gemm(a, b, out=torch.empty(m - 1, n, device="cuda"), residual=z)
