@@ -55,18 +55,22 @@ int oa_gemm_bf16_grouped(int mode, const void* A, const void* B, void* out, int 
                          long long sc_batch, long long sbias_batch, int* status, void* stream);
 // fp32 SIMT GEMM with arbitrary element strides and a batch dimension:
 //   C[b][m,n] = act(alpha * sum_k A[b][m*sam + k*sak] * B[b][n*sbn + k*sbk] + bias[n]) (+ C if accumulate)
+// and, oa_gemm_f32_epi: v = alpha * sum + bias;  aux_out = v;  v = act(v) or v * act'(aux_in);  C = v + residual (+ C if accumulate).
+// residual and aux_* are [M, N] with unit column stride.  `scratch`: oa_gemm_f32_scratch_floats() floats of this call's own (plain: no
+// bias, activation, residual or auxiliary), or null: the reduction is not sliced.
+size_t oa_gemm_f32_scratch_floats(int M, int N, int K, int batch, int plain);
+int oa_gemm_f32(const float* A, const float* B, float* C, int M, int N, int K, long long sam, long long sak,
+                long long sbn, long long sbk, int ldc, int batch, long long batch_a, long long batch_b,
+                long long batch_c, const float* bias, int act, int accumulate, float alpha, float* scratch, void* stream);
+int oa_gemm_f32_epi(const float* A, const float* B, float* C, int M, int N, int K, long long sam, long long sak, long long sbn,
+                    long long sbk, int ldc, const float* bias, const float* residual, int ldr, float* aux_out, const float* aux_in,
+                    int ldaux, int act, int accumulate, float alpha, float* scratch, void* stream);
 // Tensor-parallel GEMM fused with its collective over peer memory: mode 1 all-gather(rows of A) -> GEMM, mode 2 GEMM ->
 // reduce-scatter(rows of out).  bufs / flags: host arrays of `world` device pointers; sync2: device u64[2] of the call site.
 int oa_gemm_bf16_tp(int mode, const void* A, const void* B, void* out, int M, int N, int K, int lda, int ldb, int ldc,
                     int b_mn, const void* residual, int ldr, int out_f32, float alpha, const void* src, int ld_src,
                     const void* const* bufs, const void* const* flags, void* sync2, int world, int rank,
                     int comm_ctas, int* status, void* stream);
-int oa_gemm_f32(const float* A, const float* B, float* C, int M, int N, int K, long long sam, long long sak,
-                long long sbn, long long sbk, int ldc, int batch, long long batch_a, long long batch_b,
-                long long batch_c, const float* bias, int act, int accumulate, float alpha, void* stream);
-int oa_gemm_f32_epi(const float* A, const float* B, float* C, int M, int N, int K, long long sam, long long sak, long long sbn,
-                    long long sbk, int ldc, const float* bias, const float* residual, int ldr, float* aux_out, const float* aux_in,
-                    int ldaux, int act, int accumulate, float alpha, void* stream);
 
 // ---- elementwise (elementwise.cu)
 int oa_unary(int op, int dtype, const void* x, void* y, long long n, float s0, float s1, void* stream);

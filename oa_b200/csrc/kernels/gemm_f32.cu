@@ -264,72 +264,65 @@ __global__ void gemm_f32_splitk_reduce_kernel(const float* __restrict__ part, fl
   *c = accumulate ? *c + s * alpha : s * alpha;
 }
 
-// Scratch for split-K partials: allocated outside stream capture only, sizes rounded up to a power of two, and an outgrown
-// buffer is kept (a captured graph may still hold its address), so at most 64 + 32 + ... MB are ever held.
-static float* g_splitk_buf = nullptr;
-static size_t g_splitk_bytes = 0;
-
-static float* splitk_scratch(size_t bytes, cudaStream_t st) {
-  if (bytes <= g_splitk_bytes) return g_splitk_buf;
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return nullptr;
-  if (bytes > (64u << 20)) return nullptr;
-  size_t cap = 1u << 20;
-  while (cap < bytes) cap <<= 1;
-  float* p = nullptr;
-  if (cudaMalloc(&p, cap) != cudaSuccess) { cudaGetLastError(); return nullptr; }
-  g_splitk_buf = p; g_splitk_bytes = cap;
-  return p;
+// Slices of K for a product with few output tiles and a long reduction (weight gradients of small models); 1: not sliced.  At most
+// 63 tiles and 64 slices: the partial sums take 64 MB at most.
+static int f32_splits(int M, int N, int K, int batch, int plain, int* k_chunk) {
+  const long long tiles = (long long)((N + FT - 1) / FT) * ((M + FT - 1) / FT);
+  if (batch != 1 || !plain || tiles >= 64 || K < 512) return 1;
+  int splits = (int)((256 + tiles - 1) / tiles);
+  if (splits > K / 128) splits = K / 128;
+  if (splits > 64) splits = 64;
+  if (splits < 2) return 1;
+  *k_chunk = (((K + splits - 1) / splits) + FK - 1) / FK * FK;
+  return (K + *k_chunk - 1) / *k_chunk;
 }
 
 }  // namespace oa
 
 static int gemm_f32(const float* A, const float* B, float* C, int M, int N, int K, long long sam, long long sak, long long sbn, long long sbk,
-                    int ldc, int batch, long long batch_a, long long batch_b, long long batch_c, const oa::F32Epi& epi, void* stream) {
+                    int ldc, int batch, long long batch_a, long long batch_b, long long batch_c, const oa::F32Epi& epi, float* scratch, void* stream) {
   if (M <= 0 || N <= 0 || batch <= 0) return OA_OK;
   if (K < 0 || batch > 65535) return OA_ERR_ARG;
   const oa::F32Epi part_epi{nullptr, nullptr, nullptr, nullptr, 0, 0, OA_ACT_NONE, 0, 1.0f};
   const bool plain = !epi.bias && epi.act == OA_ACT_NONE && !epi.residual && !epi.aux_out;
   dim3 grid((N + oa::FT - 1) / oa::FT, (M + oa::FT - 1) / oa::FT, batch);
   cudaStream_t st = (cudaStream_t)stream;
-  // Few output tiles and a long reduction (weight gradients of small models): slice K over more CTAs, then reduce the slices
-  const int tiles = (int)(grid.x * grid.y);
-  if (batch == 1 && plain && tiles < 64 && K >= 512) {
-    int splits = (256 + tiles - 1) / tiles;
-    if (splits > K / 128) splits = K / 128;
-    if (splits > 64) splits = 64;
-    if (splits >= 2) {
-      const int k_chunk = (((K + splits - 1) / splits) + oa::FK - 1) / oa::FK * oa::FK;
-      splits = (K + k_chunk - 1) / k_chunk;
-      float* part = oa::splitk_scratch((size_t)splits * M * N * sizeof(float), st);
-      if (part && splits >= 2) {
-        grid.z = splits;
-        if (!oa::gemm_f32_tiles(A, B, part, M, N, K, sam, sak, sbn, sbk, N, 1, 0, 0, (long long)M * N, part_epi, k_chunk, splits, st))
-          oa::gemm_f32_kernel<<<grid, 256, 0, st>>>(A, B, part, M, N, K, sam, sak, sbn, sbk, N, 0, 0, (long long)M * N, part_epi,
-                                                  k_chunk);
-        const long long n = (long long)M * N;
-        oa::gemm_f32_splitk_reduce_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(part, C, M, N, ldc, splits, epi.accumulate, epi.alpha);
-        return cudaGetLastError() == cudaSuccess ? OA_OK : OA_ERR_LAUNCH;
-      }
-    }
+  int k_chunk = 0;
+  const int splits = scratch ? oa::f32_splits(M, N, K, batch, plain, &k_chunk) : 1;
+  if (splits >= 2) {
+    grid.z = splits;
+    if (!oa::gemm_f32_tiles(A, B, scratch, M, N, K, sam, sak, sbn, sbk, N, 1, 0, 0, (long long)M * N, part_epi, k_chunk, splits, st))
+      oa::gemm_f32_kernel<<<grid, 256, 0, st>>>(A, B, scratch, M, N, K, sam, sak, sbn, sbk, N, 0, 0, (long long)M * N, part_epi, k_chunk);
+    const long long n = (long long)M * N;
+    oa::gemm_f32_splitk_reduce_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(scratch, C, M, N, ldc, splits, epi.accumulate, epi.alpha);
+    return cudaGetLastError() == cudaSuccess ? OA_OK : OA_ERR_LAUNCH;
   }
   if (!oa::gemm_f32_tiles(A, B, C, M, N, K, sam, sak, sbn, sbk, ldc, batch, batch_a, batch_b, batch_c, epi, 0, 0, st))
     oa::gemm_f32_kernel<<<grid, 256, 0, st>>>(A, B, C, M, N, K, sam, sak, sbn, sbk, ldc, batch_a, batch_b, batch_c, epi, 0);
   return cudaGetLastError() == cudaSuccess ? OA_OK : OA_ERR_LAUNCH;
 }
 
+// Floats of scratch with which the product's reduction is sliced (0: it is not); `plain`: no bias, activation, residual or auxiliary.
+// The caller owns the scratch, so products on several streams or devices never share partial sums.
+extern "C" size_t oa_gemm_f32_scratch_floats(int M, int N, int K, int batch, int plain) {
+  int k_chunk = 0;
+  if (M <= 0 || N <= 0) return 0;
+  const int splits = oa::f32_splits(M, N, K, batch, plain, &k_chunk);
+  return splits >= 2 ? (size_t)splits * M * N : 0;
+}
+
 extern "C" int oa_gemm_f32(const float* A, const float* B, float* C, int M, int N, int K, long long sam, long long sak,
                            long long sbn, long long sbk, int ldc, int batch, long long batch_a, long long batch_b,
-                           long long batch_c, const float* bias, int act, int accumulate, float alpha, void* stream) {
+                           long long batch_c, const float* bias, int act, int accumulate, float alpha, float* scratch, void* stream) {
   if (act == OA_ACT_GELU_BWD || act == OA_ACT_RELU_BWD) return OA_ERR_UNSUPPORTED;
   return gemm_f32(A, B, C, M, N, K, sam, sak, sbn, sbk, ldc, batch, batch_a, batch_b, batch_c,
-                  oa::F32Epi{bias, nullptr, nullptr, nullptr, 0, 0, act, accumulate, alpha}, stream);
+                  oa::F32Epi{bias, nullptr, nullptr, nullptr, 0, 0, act, accumulate, alpha}, scratch, stream);
 }
 
 extern "C" int oa_gemm_f32_epi(const float* A, const float* B, float* C, int M, int N, int K, long long sam, long long sak, long long sbn,
                                long long sbk, int ldc, const float* bias, const float* residual, int ldr, float* aux_out, const float* aux_in,
-                               int ldaux, int act, int accumulate, float alpha, void* stream) {
+                               int ldaux, int act, int accumulate, float alpha, float* scratch, void* stream) {
   if ((act == OA_ACT_GELU_BWD || act == OA_ACT_RELU_BWD) && !aux_in) return OA_ERR_ARG;
   return gemm_f32(A, B, C, M, N, K, sam, sak, sbn, sbk, ldc, 1, 0, 0, 0, oa::F32Epi{bias, residual, aux_in, aux_out, ldr, ldaux, act, accumulate, alpha},
-                  stream);
+                  scratch, stream);
 }

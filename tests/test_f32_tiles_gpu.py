@@ -67,3 +67,33 @@ def test_residual_shapes(m, n, k):
             K.gemm(a, b, aux_out=torch.empty(m - 1, n, device="cuda"), act=K.ACT_GELU)
         with pytest.raises(RuntimeError):
             K.gemm(a, b, out=torch.empty(m - 1, n, device="cuda"), residual=z)
+
+
+# Sliced reductions on two streams, and a captured one beside an eager one: each call's partial sums are its own.
+@pytest.mark.parametrize("captured", [False, True])
+def test_sliced_products_side_by_side(captured):
+    g = torch.Generator(device="cuda").manual_seed(3)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    pairs = [(r(128, 4096), r(192, 4096)), (r(192, 2048), r(128, 2048))]
+    alone = [K.gemm(*p) for p in pairs]                         # fixed order of slices: the same bits every time
+    for (a, b), y in zip(pairs, alone):
+        ref = a.double() @ b.double().t()
+        assert float((y.double() - ref).norm() / ref.norm()) <= 2e-6
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    outs = [[], []]
+    graph = torch.cuda.CUDAGraph()
+    if captured:
+        with torch.cuda.graph(graph):
+            replayed = K.gemm(*pairs[0])
+    torch.cuda.synchronize()
+    for _ in range(30):
+        for i, st in enumerate(streams):
+            with torch.cuda.stream(st):
+                if captured and i == 0:
+                    graph.replay()
+                    outs[0].append(replayed.clone())
+                else:
+                    outs[i].append(K.gemm(*pairs[i]))
+    torch.cuda.synchronize()
+    for i in (0, 1):
+        assert all(torch.equal(y, alone[i]) for y in outs[i])
