@@ -56,9 +56,9 @@ int oa_gemm_bf16_grouped(int mode, const void* A, const void* B, void* out, int 
 // fp32 SIMT GEMM with arbitrary element strides and a batch dimension:
 //   C[b][m,n] = act(alpha * sum_k A[b][m*sam + k*sak] * B[b][n*sbn + k*sbk] + bias[n]) (+ C if accumulate)
 // and, oa_gemm_f32_epi: v = alpha * sum + bias;  aux_out = v;  v = act(v) or v * act'(aux_in);  C = v + residual (+ C if accumulate).
-// residual and aux_* are [M, N] with unit column stride.  `scratch`: oa_gemm_f32_scratch_floats() floats of this call's own (plain: no
-// bias, activation, residual or auxiliary), or null: the reduction is not sliced.
-size_t oa_gemm_f32_scratch_floats(int M, int N, int K, int batch, int plain);
+// residual and aux_* are [M, N] with unit column stride.  `scratch`: oa_gemm_f32_scratch_floats() floats of this call's own, or null:
+// the reduction is not sliced.
+size_t oa_gemm_f32_scratch_floats(int M, int N, int K, int batch);
 int oa_gemm_f32(const float* A, const float* B, float* C, int M, int N, int K, long long sam, long long sak,
                 long long sbn, long long sbk, int ldc, int batch, long long batch_a, long long batch_b,
                 long long batch_c, const float* bias, int act, int accumulate, float alpha, float* scratch, void* stream);

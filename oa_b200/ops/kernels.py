@@ -150,9 +150,9 @@ def _f32_epilogue_takes(t: Optional[torch.Tensor], m: int, n: int) -> bool:
     return t is None or (t.dtype == torch.float32 and tuple(t.shape) == (m, n) and t.stride(1) == 1)
 
 
-def _f32_scratch(m: int, n: int, k: int, batch: int, plain: bool, device: torch.device) -> Optional[torch.Tensor]:
+def _f32_scratch(m: int, n: int, k: int, batch: int, device: torch.device) -> Optional[torch.Tensor]:
     """The partial sums of a product whose reduction is sliced, from the current stream's allocator; None when it is not sliced."""
-    floats = N.require().oa_gemm_f32_scratch_floats(m, n, k, batch, int(plain)) if plain and k >= 512 else 0
+    floats = N.require().oa_gemm_f32_scratch_floats(m, n, k, batch) if k >= 512 else 0
     return torch.empty(floats, dtype=torch.float32, device=device) if floats else None
 
 
@@ -279,8 +279,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
                 v = binary("add", v, out)
             out.copy_(v)
             return out
-        plain = not epilogue and bias is None and act == ACT_NONE
-        sc = _f32_scratch(M, Nn, K, 1, plain, a.device)
+        # a product with a bias, or with a forward activation alone, stays in one piece
+        sc = _f32_scratch(M, Nn, K, 1, a.device) if bias is None and (epilogue or act == ACT_NONE) else None
         rc = lib.oa_gemm_f32_epi(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, Nn, K, sam, sak, sbn, sbk, out.stride(0), N.ptr(bias),
                                  N.ptr(residual), residual.stride(0) if residual is not None else 0, N.ptr(aux_out),
                                  N.ptr(aux_in) if aux_out is None else None, aux.stride(0) if aux is not None else 0, act, int(accumulate),
@@ -339,7 +339,7 @@ def bmm_f32(a: torch.Tensor, b: torch.Tensor, *, b_mn: bool = False, alpha: floa
     b = b.contiguous()
     out = torch.empty((Bn, M, Nn), dtype=torch.float32, device=a.device)
     sbn, sbk = (1, b.stride(1)) if b_mn else (b.stride(1), 1)
-    sc = _f32_scratch(M, Nn, K, Bn, True, a.device)
+    sc = _f32_scratch(M, Nn, K, Bn, a.device)
     rc = N.require().oa_gemm_f32(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, Nn, K, a.stride(1), 1, sbn, sbk, Nn, Bn,
                                  a.stride(0), b.stride(0), out.stride(0), None, ACT_NONE, 0, float(alpha), N.ptr(sc), N.stream())
     _launch(rc, "oa_gemm_f32(batched)")

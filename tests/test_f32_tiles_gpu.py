@@ -97,3 +97,35 @@ def test_sliced_products_side_by_side(captured):
     torch.cuda.synchronize()
     for i in (0, 1):
         assert all(torch.equal(y, alone[i]) for y in outs[i])
+
+
+# A residual or an activation gradient on top of a sliced reduction, and the time it may take: in one slice 128 x 128 x 4096 took
+# eight times the plain product, with the epilogue in the kernel that adds the slices up it takes as long.
+def test_sliced_epilogue():
+    g = torch.Generator(device="cuda").manual_seed(5)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    rel = lambda got, ref: float((got.double() - ref).norm() / ref.norm())
+    a, b, z, res, old = r(130, 4096), r(126, 4096), r(130, 126), r(130, 126), r(130, 126)
+    v = a.double() @ b.double().t()
+    assert rel(K.gemm(a, b, residual=res, alpha=0.5), 0.5 * v + res.double()) <= 2e-6
+    assert rel(K.gemm(a, b, act=K.ACT_RELU_BWD, aux_in=z, residual=res), v * (z > 0) + res.double()) <= 4e-6
+    aux = torch.empty(130, 126, device="cuda")
+    y = K.gemm(a, b, act=K.ACT_GELU, aux_out=aux, out=old.clone(), accumulate=True)
+    assert rel(aux, v) <= 2e-6 and rel(y, _gelu(v) + old.double()) <= 4e-6
+
+    def us(fn):
+        for _ in range(3):
+            fn()
+        t0, t1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        best = 1e9
+        for _ in range(5):
+            t0.record()
+            for _ in range(20):
+                fn()
+            t1.record()
+            torch.cuda.synchronize()
+            best = min(best, t0.elapsed_time(t1) * 50)
+        return best
+
+    out = torch.empty(130, 126, device="cuda")
+    assert us(lambda: K.gemm(a, b, out=out, residual=res)) <= 2.5 * us(lambda: K.gemm(a, b, out=out))
