@@ -13,7 +13,7 @@
 // products are issue bound), an MUFU exponential occupies its pipe for 8 cycles per warp (1024 cycles per 128 x 128
 // tile), and a warp that waits for the tensor pipe between key blocks idles the SFU.  Hence: score tiles are copied
 // to registers and released at once so the next score product is issued under this block's exponentials, products are
-// issued by two or three warps, and every kernel is persistent (one CTA per SM walks its
+// issued by two or three warps, and every kernel but the single-tile forward is persistent (one CTA per SM walks its
 // work items in snake order, heaviest causal items first), so TMEM, barriers and the operand rings live across items.
 //
 // Backward is two kernels, both deterministic (single writer per output element, like the reference's
@@ -28,6 +28,7 @@ namespace oa {
 constexpr int FA_BM = 128;   // queries per tile
 constexpr int FA_BN = 128;   // keys per tile
 constexpr float LOG2E = 1.4426950408889634f;
+constexpr int FA_THREADS = 320;   // single-tile forward: 8 softmax warps + MMA warp + TMA warp
 
 // 64-thread named barrier shared by the two warps that own the same 32 query rows.
 __device__ __forceinline__ void pair_sync(int quad) {
@@ -44,7 +45,282 @@ struct FlashParams {
   int* status;
 };
 
+// ===================================================================================== forward, S double-buffered in TMEM
+// One CTA owns one 128-query tile of one (batch, head).  S = Q K_j^T alternates between two TMEM buffers, and the MMA warp
+// always runs two key blocks ahead of the softmax (Q K_{j+2}^T is issued right after P_j V_j), so the softmax warps never
+// wait for the tensor pipe: they go from block j straight to block j+1 and the SFU stays busy.
+//   warps 0-7  softmax: two threads per query row (warp w: TMEM lane quadrant w % 4, key columns [64 * (w / 4), +64)), the
+//              64 scores of a thread are read from TMEM once, the row maximum is exchanged with the partner thread through
+//              a parity-double-buffered slot, probabilities go back to TMEM as packed bf16 over the columns of S_j;
+//   warp 8     MMA issuer: P is the A operand straight from TMEM, V the B operand from shared memory, O accumulates in
+//              TMEM over all key blocks and is read once at the end;
+//   warp 9     TMA producer (Q once, K / V rings).
+// The running maximum is updated lazily: while the new row maximum exceeds the one in use by less than 2^8 the old one is
+// kept (probabilities then stay below 256), so O in TMEM is rescaled only in the rare iterations where some row of a warp
+// jumps by more than that; the final 1/l uses the same maxima, so the result is the exact softmax.
+// TMEM: S0 | S1 | O = 128 + 128 + head_dim columns.
+template <int HD>
+struct Fwd2Cfg {
+  static constexpr int NSK = 3;                            // K ring depth (K runs two blocks ahead of V)
+  static constexpr int NSV = (HD == 64) ? 3 : 2;           // V ring depth
+  static constexpr int Q_BYTES = FA_BM * HD * 2;
+  static constexpr int KV_BYTES = FA_BN * HD * 2;
+  static constexpr int OFF_Q = 0;
+  static constexpr int OFF_K = OFF_Q + Q_BYTES;
+  static constexpr int OFF_V = OFF_K + NSK * KV_BYTES;
+  static constexpr int OFF_X = OFF_V + NSV * KV_BYTES;     // float[2 parities][2 halves][128 rows]: row-maximum exchange
+  static constexpr int OFF_BAR = OFF_X + 2 * 2 * FA_BM * 4;
+  static constexpr int SMEM_BYTES = OFF_BAR + 256;
+  static constexpr int TMEM_COLS = 512;
+  static constexpr int TM_S = 0;                           // + 128 * (j & 1)
+  static constexpr int TM_O = 256;
+};
+
 constexpr float FA_RESCALE_THRESHOLD = 8.f;                // log2 units
+
+
+template <int HD>
+__global__ void __launch_bounds__(FA_THREADS, 1)
+flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
+                  const __grid_constant__ CUtensorMap tmV, const FlashParams p) {
+  using Cfg = Fwd2Cfg<HD>;
+  constexpr int NSK = Cfg::NSK, NSV = Cfg::NSV;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::OFF_BAR);
+  uint64_t* q_full = bars + 0;
+  uint64_t* k_full = bars + 1;                 // [NSK]
+  uint64_t* k_empty = k_full + NSK;            // [NSK]
+  uint64_t* v_full = k_empty + NSK;            // [NSV]
+  uint64_t* v_empty = v_full + NSV;            // [NSV]
+  uint64_t* s_full = v_empty + NSV;            // [2]  S buffer holds Q K_j^T
+  uint64_t* p_full = s_full + 2;               // [2]  P_j written over S buffer (and O rescaled if needed)
+  uint64_t* o_done = s_full + 4;               //      O += P_j V_j finished
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(s_full + 5);
+  float* xch = reinterpret_cast<float*>(smem + Cfg::OFF_X);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nblk = (p.seq + FA_BM - 1) / FA_BM;
+  const int qb = nblk - 1 - blockIdx.x;        // heaviest causal tiles first
+  const int h = blockIdx.y, b = blockIdx.z;
+  const int n_kv = p.causal ? (qb + 1) : nblk;
+  const int row0 = b * p.seq;
+
+  if ((smem_u32(smem) & 1023u) != 0) {
+    if (threadIdx.x == 0) report_error(p.status, OA_KERR_BAD_ARG);
+    return;
+  }
+  if (threadIdx.x == 0) {
+    tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV);
+    mbar_init(q_full, 1);
+    for (int s = 0; s < NSK; ++s) { mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1); }
+    for (int s = 0; s < NSV; ++s) { mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1); }
+    for (int t = 0; t < 2; ++t) { mbar_init(&s_full[t], 1); mbar_init(&p_full[t], 8); }
+    mbar_init(o_done, 1);
+    mbar_fence_init();
+  }
+  if (warp == 8) { tmem_alloc<Cfg::TMEM_COLS>(tmem_slot); tmem_relinquish(); }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();                            // the prologue above ran under the previous kernel's tail; global memory from here on
+
+  if (warp == 9) {
+    // ------------- producer: the whole warp walks the loop and waits together; one lane issues the copies.  K block i is
+    // loaded two iterations before V block i - 2... both rings are simply filled in order, K first.
+    if (lane == 0) {
+      mbar_expect_tx(q_full, Cfg::Q_BYTES);
+#pragma unroll
+      for (int x = 0; x < HD / 64; ++x)
+        tma_load_2d(smem + Cfg::OFF_Q + x * (FA_BM * 128), &tmQ, q_full, h * HD + x * 64, row0 + qb * FA_BM);
+    }
+    for (int i = 0; i < n_kv + 2; ++i) {
+      if (i < n_kv) {
+        const int st = i % NSK;
+        if (!warp_wait(&k_empty[st], ((i / NSK) & 1) ^ 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_EMPTY); break; }
+        if (lane == 0) {
+          mbar_expect_tx(&k_full[st], Cfg::KV_BYTES);
+#pragma unroll
+          for (int x = 0; x < HD / 64; ++x)
+            tma_load_2d(smem + Cfg::OFF_K + st * Cfg::KV_BYTES + x * (FA_BN * 128), &tmK, &k_full[st], h * HD + x * 64, row0 + i * FA_BN);
+        }
+      }
+      const int jv = i - 2;                    // V lags K by two blocks, like its consumer
+      if (jv >= 0) {
+        const int st = jv % NSV;
+        if (!warp_wait(&v_empty[st], ((jv / NSV) & 1) ^ 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_EMPTY); break; }
+        if (lane == 0) {
+          mbar_expect_tx(&v_full[st], Cfg::KV_BYTES);
+#pragma unroll
+          for (int x = 0; x < HD / 64; ++x)
+            tma_load_2d(smem + Cfg::OFF_V + st * Cfg::KV_BYTES + x * (FA_BN * 128), &tmV, &v_full[st], h * HD + x * 64, row0 + jv * FA_BN);
+        }
+      }
+      __syncwarp();
+    }
+  } else if (warp == 8) {
+    // ------------- MMA issuer (warp-uniform waits, lane 0 issues)
+    constexpr uint32_t idesc_qk = umma_idesc_bf16(FA_BM, FA_BN, 0, 0);
+    constexpr uint32_t idesc_pv = umma_idesc_bf16(FA_BM, HD, 0, 1);
+    const uint32_t q_addr = smem_u32(smem + Cfg::OFF_Q);
+    auto issue_qk = [&](int i) -> bool {       // S[i & 1] = Q K_i^T
+      const int st = i % NSK;
+      if (!warp_wait(&k_full[st], (i / NSK) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_FULL); return false; }
+      tc_fence_after();
+      if (lane == 0) {
+        const uint32_t k_addr = smem_u32(smem + Cfg::OFF_K + st * Cfg::KV_BYTES);
+#pragma unroll
+        for (int ks = 0; ks < HD / 16; ++ks) {
+          const uint32_t off = (ks >> 2) * (FA_BM * 128) + (ks & 3) * 32;
+          umma_f16(tmem_base + Cfg::TM_S + (i & 1) * FA_BN, umma_smem_desc_sw128(q_addr + off, 16, 1024),
+                   umma_smem_desc_sw128(k_addr + off, 16, 1024), idesc_qk, ks > 0 ? 1u : 0u);
+        }
+        umma_commit(&k_empty[st]);
+        umma_commit(&s_full[i & 1]);
+      }
+      __syncwarp();
+      return true;
+    };
+    bool ok = warp_wait(q_full, 0);
+    if (!ok && lane == 0) report_error(p.status, OA_KERR_WAIT_FULL);
+    if (ok) ok = issue_qk(0);
+    if (ok && n_kv > 1) ok = issue_qk(1);
+    for (int j = 0; j < n_kv && ok; ++j) {
+      const int st = j % NSV;
+      if (!warp_wait(&v_full[st], (j / NSV) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_FULL); break; }
+      if (!warp_wait(&p_full[j & 1], (j >> 1) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_SOFTMAX); break; }
+      tc_fence_after();
+      if (lane == 0) {
+        const uint32_t v_addr = smem_u32(smem + Cfg::OFF_V + st * Cfg::KV_BYTES);
+#pragma unroll
+        for (int ks = 0; ks < FA_BN / 16; ++ks)
+          umma_f16_ts(tmem_base + Cfg::TM_O, tmem_base + Cfg::TM_S + (j & 1) * FA_BN + ks * 8,
+                      umma_smem_desc_sw128(v_addr + ks * 2048, FA_BN * 128, 1024), idesc_pv, (j > 0 || ks > 0) ? 1u : 0u);
+        umma_commit(&v_empty[st]);
+        umma_commit(o_done);
+      }
+      __syncwarp();
+      if (j + 2 < n_kv) ok = issue_qk(j + 2);  // overwrites S[j & 1] = P_j: ordered after P_j V_j by the pipe
+    }
+  } else {
+    // ------------- softmax + output: two threads per query row (key columns split in halves)
+    constexpr int OC = HD / 2;                   // output columns owned by this thread
+    const int quad = warp & 3;
+    const int half = warp >> 2;
+    const int r = quad * 32 + lane;
+    const int qi = qb * FA_BM + r;               // query index inside the sequence
+    const uint32_t t_lane = (uint32_t)(quad * 32) << 16;
+    const uint32_t o_addr = tmem_base + t_lane + Cfg::TM_O + half * OC;
+    const float sl2 = p.scale * LOG2E;
+    float m_run = -INFINITY, l_run = 0.f;
+    bool ok = true;
+    for (int j = 0; j < n_kv; ++j) {
+      ok = warp_wait(&s_full[j & 1], (j >> 1) & 1);
+      if (!ok) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_TMEM_FULL); break; }
+      tc_fence_after();
+      const uint32_t s_addr = tmem_base + t_lane + Cfg::TM_S + (j & 1) * FA_BN;
+      uint32_t sv[64];
+      tmem_ld32(s_addr + half * 64, sv);
+      tmem_ld32(s_addr + half * 64 + 32, sv + 32);
+      tmem_ld_wait();
+      const bool need_mask = (p.causal && j == qb) || (j * FA_BN + FA_BN > p.seq);
+      if (need_mask) {
+        const int lim = min(p.causal ? qi : 0x7fffffff, p.seq - 1) - j * FA_BN - half * 64;   // columns i <= lim are alive
+#pragma unroll
+        for (int i = 0; i < 64; ++i) sv[i] = (i <= lim) ? sv[i] : 0xff800000u;                 // -inf
+      }
+      float m0 = __uint_as_float(sv[0]), m1 = __uint_as_float(sv[1]), m2 = __uint_as_float(sv[2]), m3 = __uint_as_float(sv[3]);
+#pragma unroll
+      for (int i = 4; i < 64; i += 4) {
+        m0 = fmaxf(m0, __uint_as_float(sv[i])); m1 = fmaxf(m1, __uint_as_float(sv[i + 1]));
+        m2 = fmaxf(m2, __uint_as_float(sv[i + 2])); m3 = fmaxf(m3, __uint_as_float(sv[i + 3]));
+      }
+      float mx = fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
+      // Exchange with the partner thread of this row.  Both threads now hold their scores in registers, so after this
+      // barrier the S buffer may be overwritten by either of them.
+      float* slots = xch + (j & 1) * (2 * FA_BM);
+      slots[(half ^ 1) * FA_BM + r] = mx;
+      pair_sync(quad);
+      mx = fmaxf(mx, slots[half * FA_BM + r]) * sl2;
+      const float m_new = fmaxf(m_run, mx);
+      const bool grow = (m_new - m_run) > FA_RESCALE_THRESHOLD;           // first block: m_run = -inf -> true
+      const float m_cand = grow ? m_new : m_run;
+      const float m_use = (m_cand == -INFINITY) ? 0.f : m_cand;           // row fully masked so far
+      const float alpha = grow ? fast_exp2(m_run - m_use) : 1.f;           // m_run = -inf -> 0
+      const float neg_m = -m_use;
+      float l0 = 0.f, l1 = 0.f, l2 = 0.f, l3 = 0.f;
+      uint32_t pk[32];
+#pragma unroll
+      for (int i = 0; i < 64; i += 4) {
+        const float e0 = fast_exp2(fmaf(__uint_as_float(sv[i]), sl2, neg_m));
+        const float e1 = fast_exp2(fmaf(__uint_as_float(sv[i + 1]), sl2, neg_m));
+        const float e2 = fast_exp2(fmaf(__uint_as_float(sv[i + 2]), sl2, neg_m));
+        const float e3 = fast_exp2(fmaf(__uint_as_float(sv[i + 3]), sl2, neg_m));
+        l0 += e0; l1 += e1; l2 += e2; l3 += e3;
+        pk[i >> 1] = pack_bf16x2(e0, e1);
+        pk[(i >> 1) + 1] = pack_bf16x2(e2, e3);
+      }
+      tmem_st32(s_addr + half * 32, pk);          // P over the first 64 columns of S (two keys per column)
+      l_run = l_run * alpha + ((l0 + l1) + (l2 + l3));
+      m_run = m_cand;
+      if (j > 0 && __any_sync(0xffffffffu, grow)) {
+        // some row of this warp moved its maximum: rescale O (needs the previous P*V finished)
+        ok = warp_wait(o_done, (j - 1) & 1);
+        if (!ok) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_TMEM_FULL); break; }
+        tc_fence_after();
+#pragma unroll
+        for (int c = 0; c < OC / 32; ++c) {
+          uint32_t o[32];
+          tmem_ld32(o_addr + c * 32, o);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+          tmem_st32(o_addr + c * 32, o);
+        }
+      }
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&p_full[j & 1]);
+    }
+    // combine the two partial row sums (parity slot of an iteration that is two behind any reader)
+    {
+      float* slots = xch + (n_kv & 1) * (2 * FA_BM);
+      slots[(half ^ 1) * FA_BM + r] = l_run;
+      pair_sync(quad);
+      l_run += slots[half * FA_BM + r];
+    }
+    if (ok) {
+      ok = warp_wait(o_done, (n_kv - 1) & 1);
+      if (!ok && lane == 0) report_error(p.status, OA_KERR_WAIT_TMEM_FULL);
+    }
+    if (ok) {
+      tc_fence_after();
+      const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
+      __nv_bfloat16* op = p.o + (long long)(row0 + qi) * p.o_stride + h * HD + half * OC;
+#pragma unroll
+      for (int c = 0; c < OC / 32; ++c) {
+        uint32_t o[32];
+        tmem_ld32(o_addr + c * 32, o);
+        tmem_ld_wait();
+        if (qi < p.seq) {
+#pragma unroll
+          for (int g = 0; g < 4; ++g)
+            *reinterpret_cast<uint4*>(op + c * 32 + g * 8) = make_uint4(
+                pack_bf16x2(__uint_as_float(o[g * 8]) * inv, __uint_as_float(o[g * 8 + 1]) * inv),
+                pack_bf16x2(__uint_as_float(o[g * 8 + 2]) * inv, __uint_as_float(o[g * 8 + 3]) * inv),
+                pack_bf16x2(__uint_as_float(o[g * 8 + 4]) * inv, __uint_as_float(o[g * 8 + 5]) * inv),
+                pack_bf16x2(__uint_as_float(o[g * 8 + 6]) * inv, __uint_as_float(o[g * 8 + 7]) * inv));
+        }
+      }
+      if (p.lse && half == 0 && qi < p.seq) p.lse[((long long)b * p.heads + h) * p.seq + qi] = (m_run + log2f(l_run)) / LOG2E;
+    }
+  }
+  pdl_launch_dependents();
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 8) { tc_fence_after(); tmem_dealloc<Cfg::TMEM_COLS>(tmem_base); }
+}
 
 // ===================================================================================== forward: two tiles per CTA
 // Two adjacent 128-query tiles of one (batch, head) share a CTA and the K / V rings but are otherwise independent pipelines
@@ -53,9 +329,7 @@ constexpr float FA_RESCALE_THRESHOLD = 8.f;                // log2 units
 // row (all 128 key columns: no partner exchange).  The score tile is copied to registers and RELEASED at once, so
 // Q K_{j+1}^T is issued while the exponentials of block j run; probabilities have their own TMEM columns:
 // S0 | S1 | P0 | P1 | O0 | O1 = 128 + 128 + 64 + 64 + 64 + 64.
-// The running maximum is updated lazily: while the new row maximum exceeds the one in use by less than 2^8 the old one is kept
-// (probabilities then stay below 256), so O in TMEM is rescaled only in the rare iterations where some row of a warp jumps by
-// more than that; the final 1/l uses the same maxima, so the result is the exact softmax.
+// The running maximum is updated lazily, as above.
 // Two threads per row (sixteen softmax warps, maxima exchanged through shared memory) measured 127.7 instead of 121.7 us at head
 // dim 64 (8 x 2048 x 16) and 193 instead of 188 us at head dim 128 (4096 x 32): the warps' chains are not what bounds it.
 // Head dim 128: O takes the columns of P, so P_t overwrites the first half of S_t (S0 | S1 | O0 | O1 = 4 x 128 columns).  Then
@@ -391,6 +665,30 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 }
 
 template <int HD>
+static int launch_fwd2(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FlashParams& p, dim3 grid, cudaStream_t st) {
+  static bool set = false;
+  if (!set) {
+    if (cudaFuncSetAttribute(flash_fwd2_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, Fwd2Cfg<HD>::SMEM_BYTES) != cudaSuccess) return OA_ERR_LAUNCH;
+    set = true;
+  }
+  launch_pdl(flash_fwd2_kernel<HD>, grid, dim3(FA_THREADS), Fwd2Cfg<HD>::SMEM_BYTES, st, tq, tk, tv, p);
+  return cudaGetLastError() == cudaSuccess ? OA_OK : OA_ERR_LAUNCH;
+}
+
+// Head dim 128: whether the pair kernel beats one tile per CTA.  Per key block it is the slower one (its P lies over S: 2.8 us for two
+// tiles, 1.1 us for one), and it puts two tiles where one SM each was free; it gains what a CTA costs to start and to drain, so it
+// wants enough items and short rows of key blocks.  Measured, single tile against pair: causal 32 x 256 x 16 heads 49 / 34 us,
+// 1 x 2048 x 32 59.5 / 50, 1 x 4096 x 32 178 / 175, 1 x 8192 x 16 312 / 332, and with few items 1 x 1024 x 8 13.8 / 25.8,
+// 1 x 4096 x 10 71 / 93, 2 x 2048 x 10 43 / 49; full 64 x 384 x 16 162 / 136, 4 x 1024 x 32 96 / 106, 1 x 4096 x 32 278 / 370.  The
+// lines lie where a sweep over 1 to 36 blocks and 150 to 1000 items changes sign (three blocks, 160 items: 15.9 / 18.3).
+static bool flash_pair_hd128(int nblk, long long heads, long long batch, int causal, int sms) {
+  if (heads > 65535 || batch > 65535) return true;       // beyond the single-tile kernel's grid
+  const long long items = (long long)((nblk + 1) / 2) * heads * batch;
+  if (!causal) return nblk == 1 ? items > sms : (nblk <= 3 ? items >= 2 * sms : nblk == 4 && items >= 4 * sms);
+  return nblk <= 8 && nblk != 3 ? items > sms : (nblk <= 32 && 2 * items >= 3 * sms);
+}
+
+template <int HD>
 static int launch_fwd_pair(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FlashParams& p, cudaStream_t st) {
   static int sms = 0;
   if (sms == 0) {
@@ -400,6 +698,8 @@ static int launch_fwd_pair(const CUtensorMap& tq, const CUtensorMap& tk, const C
     sms = n;
   }
   const int nblk = (p.seq + FA_BM - 1) / FA_BM;
+  if constexpr (HD == 128)
+    if (!flash_pair_hd128(nblk, p.heads, p.batch, p.causal, sms)) return launch_fwd2<HD>(tq, tk, tv, p, dim3(nblk, p.heads, p.batch), st);
   const long long items = (long long)((nblk + 1) / 2) * p.heads * p.batch;
   const int ctas = (int)(items < sms ? items : sms);
   launch_pdl(flash_fwd_pair_kernel<HD>, dim3(ctas), dim3(FwdPairCfg<HD>::THREADS), FwdPairCfg<HD>::SMEM_BYTES, st, tq, tk, tv, p);

@@ -1,4 +1,5 @@
-"""The two-tile forward kernel at both head dims: odd tile counts, sequences off the tile grid, full and causal, packed rows."""
+"""The two-tile forward kernel at both head dims and the single-tile one at head dim 128: odd tile counts, sequences off the tile grid,
+full and causal, packed rows, both sides of the line between them."""
 import pytest
 import torch
 
@@ -9,7 +10,8 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("hd", [64, 128])
 @pytest.mark.parametrize("causal", [True, False])
-@pytest.mark.parametrize("batch,seq,heads", [(1, 1, 1), (1, 100, 2), (2, 128, 1), (1, 129, 3), (2, 300, 2), (1, 513, 1), (3, 640, 25), (1, 1500, 4)])
+@pytest.mark.parametrize("batch,seq,heads", [(1, 1, 1), (1, 100, 2), (2, 128, 1), (1, 129, 3), (2, 300, 2), (1, 513, 1), (3, 640, 25), (1, 1500, 4), (149, 100, 1),
+                                             (37, 300, 4), (10, 1100, 5)])
 def test_forward(hd, causal, batch, seq, heads):
     g = torch.Generator(device="cuda").manual_seed(seq + heads)
     D = heads * hd
@@ -27,3 +29,29 @@ def test_forward(hd, causal, batch, seq, heads):
     assert (lse.double() - torch.logsumexp(s, -1)).abs().max().item() <= 1e-4
     torch.cuda.synchronize()
     K.check_status()
+
+
+# While there are fewer tiles than SMs each has one of its own: half the heads take about half the time, not the time of two tiles
+# that share an SM beside idle ones.
+@pytest.mark.parametrize("causal", [True, False])
+def test_few_tiles_take_an_sm_each(causal):
+    def us(heads, seq=1024, hd=128):
+        D = heads * hd
+        qkv = torch.randn(seq, 3 * D, device="cuda").bfloat16()
+        call = lambda: K.flash_fwd(qkv[:, :D], qkv[:, D:2 * D], qkv[:, 2 * D:], 1, seq, heads, hd, causal=causal)
+        call()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            for _ in range(10):
+                call()
+        t0, t1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        best = 1e9
+        for _ in range(6):
+            t0.record()
+            graph.replay()
+            t1.record()
+            torch.cuda.synchronize()
+            best = min(best, t0.elapsed_time(t1) * 100)
+        return best
+
+    assert us(18) <= 0.75 * us(36)
