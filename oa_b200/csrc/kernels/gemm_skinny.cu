@@ -6,9 +6,10 @@
 // tile's weights through a TMA ring into one TMEM accumulator, the partial tiles meet in distributed shared memory and every CTA
 // sums, in rank order, and writes its share of the rows.  No workspace, no second kernel, no transposed copy.
 //
-// Two CTAs of about 100 KB per SM keep some 160 KB of weights per SM on their way, and one wave holds the whole grid: CTAs get
-// equal shares of the bandwidth and of the bytes, whatever their number, so the cluster size only has to be large enough to have
-// enough bytes in flight.
+// Two CTAs of about 100 KB per SM keep some 160 KB of weights per SM on their way.  Up to 2 x 128 columns per SM (37,888) one wave
+// holds the whole grid: CTAs get equal shares of the bandwidth and of the bytes, whatever their number, so the cluster size only has
+// to be large enough to have enough bytes in flight.  Wider products run further waves, whose tiles do not overlap their epilogues
+// with the next tile's loads as the persistent tile kernel does; gemm_skinny_wins says where that costs more than it saves.
 //
 // What bounds it: the weights' bytes at about 70 % of the copy rate (128-byte pieces of 128 rows; the rest is the ramp of a launch).
 // One row against 12288 x 4096 / 4096 x 4096 / 32000 x 4096: 31 / 18 / 66 us, with the tile kernel 38 / 22 / 69; a decoding step of
@@ -184,6 +185,18 @@ static int launch_skinny(const CUtensorMap& tw, const CUtensorMap& tx, const Ski
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, gemm_skinny_kernel<MT>, tw, tx, p) == cudaSuccess && cudaGetLastError() == cudaSuccess ? OA_OK : OA_ERR_LAUNCH;
+}
+
+// Whether reading the weight this way beats the tile kernel: it depends on the weight's bytes against the output's, which a CTA writes
+// after its last product and under nothing else.  While the tiles leave half of the SMs free it always does.  Up to one full wave, tile
+// kernel against this one: 32 x 32000 x 512 12.8 / 12.1 us, 64 x 12288 x 512 9.0 / 10.7, 64 x 32000 x 1024 18.0 / 19.1, 48 x 18944 x 1024
+// 14.4 / 13.3, 64 x 32000 x 4096 70 / 50.  Further waves: 64 x 50264 x 1024 27 / 32, 32 x 128256 x 2048 90 / 96, 16 x 50264 x 512 17 / 18,
+// 48 x 50264 x 4096 80 / 79, 8 x 50264 x 1024 27 / 26.
+bool gemm_skinny_wins(int M, int N, int K) {
+  const long long tiles = (N + SK_BN - 1) / SK_BN, sms = num_sms();
+  if (2 * tiles < sms) return true;
+  if (tiles <= 2 * sms) return M <= 32 || K > 32 * M;
+  return K > 64 * M;
 }
 
 // Called by oa_gemm_bf16 for the shapes its dispatch names; the arguments have passed its checks.

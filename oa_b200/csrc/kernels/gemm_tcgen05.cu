@@ -1225,6 +1225,7 @@ static void try_store_map(GemmParams& p, void* out, uint64_t cols, uint64_t rows
 
 int gemm_skinny(const void* x, const void* w, void* out, int M, int N, int K, int ldx, int ldw, int ldc, const void* bias, const void* residual,
                 int ldr, int act, int out_f32, float alpha, int* status, cudaStream_t st);
+bool gemm_skinny_wins(int M, int N, int K);
 
 int num_sms() {
   static int n = 0;
@@ -1294,7 +1295,7 @@ extern "C" int oa_gemm_bf16_batched(const void* A, const void* B, void* out, int
   if ((ldc & (out_f32 ? 3 : 7)) || (residual && (ldr & 7)) || ((aux_out || aux_in) && (ldaux & 7))) return OA_ERR_ALIGN;
   if (batch > 1 && ((sc_batch & 7) || (sr_batch & 7) || (saux_batch & 7) || (sbias_batch & 7))) return OA_ERR_ALIGN;
   // A handful of rows against a large weight: the kernel that streams the weight (gemm_skinny.cu)
-  if (!force_bn && batch == 1 && !a_mn && !b_mn && M <= 64 && N >= 256 && K >= 512 && !accumulate && !aux_out && !aux_in)
+  if (!force_bn && batch == 1 && !a_mn && !b_mn && M <= 64 && N >= 256 && K >= 512 && !accumulate && !aux_out && !aux_in && gemm_skinny_wins(M, N, K))
     return gemm_skinny(A, B, out, M, N, K, lda, ldb, ldc, bias, residual, ldr, act, out_f32, alpha, status, (cudaStream_t)stream);
   int bn = force_bn ? force_bn : ((N >= 256) ? 256 : 128);
   int sms = num_sms();

@@ -1,4 +1,5 @@
-"""The product for a handful of rows against 64-bit sums: row counts at the padding edges, ragged widths, every cluster size."""
+"""The product for a handful of rows against 64-bit sums: row counts at the padding edges, ragged widths, cluster sizes 1, 2, 4 and 8 with
+even and uneven shares of K, several waves of tiles."""
 import pytest
 import torch
 
@@ -8,7 +9,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("m", [1, 3, 16, 17, 32, 40, 48, 49, 64, 65])
-@pytest.mark.parametrize("n,k", [(264, 512), (1024, 520), (4096, 4096), (11008, 1024), (32000, 576), (40008, 512)])
+@pytest.mark.parametrize("n,k", [(264, 512), (1024, 520), (4096, 4096), (11008, 1024), (32000, 576), (40008, 512),
+                                   (8192, 1096), (2048, 2120), (11008, 1096), (40008, 1032)])
 def test_few_rows(m, n, k):
     g = torch.Generator(device="cuda").manual_seed(m * 131 + n + k)
     x = torch.randn(m, k + 8, device="cuda", generator=g).bfloat16()[:, :k]      # a pitch that is not the width
@@ -26,3 +28,31 @@ def test_few_rows(m, n, k):
         assert float((got.double() - ref).norm() / ref.norm()) <= tol
     torch.cuda.synchronize()
     K.check_status()
+
+
+def _us(fns):
+    for f in fns:
+        f()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        for f in fns:
+            f()
+    t0, t1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    best = 1e9
+    for _ in range(8):
+        t0.record()
+        graph.replay()
+        t1.record()
+        torch.cuda.synchronize()
+        best = min(best, t0.elapsed_time(t1) * 1e3 / len(fns))
+    return best
+
+
+# The line between this kernel and the tile kernel lies where neither is much slower; weights come from memory (8 x 51 MB).
+@pytest.mark.parametrize("m,n,k", [(64, 50264, 512), (64, 38016, 1024), (48, 128256, 512), (16, 50264, 512), (1, 50264, 512), (64, 14336, 512),
+                                   (48, 12288, 768)])
+def test_not_slower_than_the_tile_kernel(m, n, k):
+    ws = [torch.randn(n, k, device="cuda").bfloat16() for _ in range(max(1, -(-400_000_000 // (n * k * 2))))]
+    x, out = torch.randn(m, k, device="cuda").bfloat16(), torch.empty(m, n, device="cuda", dtype=torch.bfloat16)
+    tiled = min(_us([lambda w=w, bn=bn: K.gemm(x, w, out=out, force_bn=bn) for w in ws]) for bn in (128, 256))
+    assert _us([lambda w=w: K.gemm(x, w, out=out) for w in ws]) <= 1.12 * tiled
