@@ -2,6 +2,7 @@
 import pytest
 import torch
 
+from device_time import graph_us
 from oa_b200.ops import kernels as K
 
 pytestmark = pytest.mark.gpu
@@ -113,19 +114,5 @@ def test_sliced_epilogue():
     y = K.gemm(a, b, act=K.ACT_GELU, aux_out=aux, out=old.clone(), accumulate=True)
     assert rel(aux, v) <= 2e-6 and rel(y, _gelu(v) + old.double()) <= 4e-6
 
-    def us(fn):
-        for _ in range(3):
-            fn()
-        t0, t1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-        best = 1e9
-        for _ in range(5):
-            t0.record()
-            for _ in range(20):
-                fn()
-            t1.record()
-            torch.cuda.synchronize()
-            best = min(best, t0.elapsed_time(t1) * 50)
-        return best
-
     out = torch.empty(130, 126, device="cuda")
-    assert us(lambda: K.gemm(a, b, out=out, residual=res)) <= 2.5 * us(lambda: K.gemm(a, b, out=out))
+    assert graph_us(*[lambda: K.gemm(a, b, out=out, residual=res)] * 10) <= 2.5 * graph_us(*[lambda: K.gemm(a, b, out=out)] * 10)

@@ -3,6 +3,7 @@ full and causal, packed rows, both sides of the line between them."""
 import pytest
 import torch
 
+from device_time import graph_us
 from oa_b200.ops import kernels as K
 
 pytestmark = pytest.mark.gpu
@@ -39,19 +40,6 @@ def test_few_tiles_take_an_sm_each(causal):
         D = heads * hd
         qkv = torch.randn(seq, 3 * D, device="cuda").bfloat16()
         call = lambda: K.flash_fwd(qkv[:, :D], qkv[:, D:2 * D], qkv[:, 2 * D:], 1, seq, heads, hd, causal=causal)
-        call()
-        graph = torch.cuda.CUDAGraph()
-        with torch.cuda.graph(graph):
-            for _ in range(10):
-                call()
-        t0, t1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-        best = 1e9
-        for _ in range(6):
-            t0.record()
-            graph.replay()
-            t1.record()
-            torch.cuda.synchronize()
-            best = min(best, t0.elapsed_time(t1) * 100)
-        return best
+        return graph_us(*[call] * 10)
 
     assert us(18) <= 0.75 * us(36)

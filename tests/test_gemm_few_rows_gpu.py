@@ -3,6 +3,7 @@ even and uneven shares of K, several waves of tiles."""
 import pytest
 import torch
 
+from device_time import graph_us
 from oa_b200.ops import kernels as K
 
 pytestmark = pytest.mark.gpu
@@ -29,30 +30,11 @@ def test_few_rows(m, n, k):
     torch.cuda.synchronize()
     K.check_status()
 
-
-def _us(fns):
-    for f in fns:
-        f()
-    graph = torch.cuda.CUDAGraph()
-    with torch.cuda.graph(graph):
-        for f in fns:
-            f()
-    t0, t1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-    best = 1e9
-    for _ in range(8):
-        t0.record()
-        graph.replay()
-        t1.record()
-        torch.cuda.synchronize()
-        best = min(best, t0.elapsed_time(t1) * 1e3 / len(fns))
-    return best
-
-
 # The line between this kernel and the tile kernel lies where neither is much slower; weights come from memory (8 x 51 MB).
 @pytest.mark.parametrize("m,n,k", [(64, 50264, 512), (64, 38016, 1024), (48, 128256, 512), (16, 50264, 512), (1, 50264, 512), (64, 14336, 512),
                                    (48, 12288, 768)])
 def test_not_slower_than_the_tile_kernel(m, n, k):
     ws = [torch.randn(n, k, device="cuda").bfloat16() for _ in range(max(1, -(-400_000_000 // (n * k * 2))))]
     x, out = torch.randn(m, k, device="cuda").bfloat16(), torch.empty(m, n, device="cuda", dtype=torch.bfloat16)
-    tiled = min(_us([lambda w=w, bn=bn: K.gemm(x, w, out=out, force_bn=bn) for w in ws]) for bn in (128, 256))
-    assert _us([lambda w=w: K.gemm(x, w, out=out) for w in ws]) <= 1.12 * tiled
+    tiled = min(graph_us(*[lambda w=w, bn=bn: K.gemm(x, w, out=out, force_bn=bn) for w in ws]) for bn in (128, 256))
+    assert graph_us(*[lambda w=w: K.gemm(x, w, out=out) for w in ws]) <= 1.12 * tiled
