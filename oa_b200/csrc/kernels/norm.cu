@@ -39,7 +39,9 @@ constexpr int NORM_WARPS = NORM_THREADS / 32;
 
 // Rows of up to 32 * VEC * NV columns: the row stays in registers (packed as it is stored) between the sum of squares and the
 // output, so memory is read once and all of a lane's loads are in flight together.  16384 x 1024 is at the copy rate either way
-// (10.8 us); with few rows two dependent passes were all latency: 32 x 4096 went from 11.6 to 5.2 us.
+// (9.5 and 9.0 us out of L2); with few rows two dependent passes were all latency: 149 x 4096 went from 6.8 to 4.4 us.  Where rows
+// are many and wide the registers leave too few warps (4736 x 2880: 9.4 us in two passes, 12.3 here), the more so with a residual,
+// whose loads wait behind the row's (33.6 and 54.3 us at 4736 x 4096): see rmsnorm_in_registers.
 template <typename T, int NV>
 __global__ void __launch_bounds__(NORM_THREADS)
 rmsnorm_fwd_reg_kernel(const T* __restrict__ x, const T* __restrict__ w, T* __restrict__ y, float* __restrict__ rstd_out,
@@ -547,6 +549,17 @@ extern "C" size_t oa_norm_bwd_scratch_bytes(long long rows, int cols) {
   return (size_t)2 * norm_bwd_blocks(rows) * cols * sizeof(float);
 }
 
+// Whether the row-in-registers kernel beats the two passes, by the 16-byte vectors per lane (nv) and the blocks of eight rows.  Up to
+// one block per SM it is latency that counts and registers win at any width.  Beyond, two passes against registers: 9472 x 1536 bf16
+// 9.1 / 9.7 us (nv 6), 16384 x 1024 fp32 24.2 / 20.2 (8), 2368 x 4096 bf16 7.4 / 8.2 (16); with a residual 16384 x 1024 23.1 / 24.5 (4), 4736 x 1536 7.4 / 8.2 (6),
+// 1200 x 2880 8.1 / 10.9 (12).
+static bool rmsnorm_in_registers(int nv, long long blocks, bool residual) {
+  if (nv <= 2) return true;
+  if (nv <= 4) return !residual || blocks <= 8 * 148;
+  if (nv <= 8) return residual ? blocks <= 2 * 148 : (nv > 6 || blocks <= 7 * 148);
+  return nv <= 16 && blocks <= 148;
+}
+
 extern "C" int oa_rmsnorm_fwd(int dtype, const void* x, const void* w, void* y, float* rstd, long long rows, int cols,
                               float eps, const void* residual_in, void* residual_out, void* stream) {
   if (rows <= 0) return OA_OK;
@@ -566,7 +579,7 @@ extern "C" int oa_rmsnorm_fwd(int dtype, const void* x, const void* w, void* y, 
                  (__nv_bfloat16*)y, rstd, cols, eps, (const __nv_bfloat16*)residual_in, (__nv_bfloat16*)residual_out);
     return CHECK_LAUNCH();
   }
-  if (nv <= 16 && (at & 15) == 0 && b < 0x7fffffffLL) {
+  if (rmsnorm_in_registers(nv, b, residual_in != nullptr) && (at & 15) == 0 && b < 0x7fffffffLL) {
 #define OA_RMS_FWD_REG(T, NV)                                                                                                   \
     launch_pdl(rmsnorm_fwd_reg_kernel<T, NV>, dim3((unsigned)b), dim3(NORM_THREADS), 0, ST, (const T*)x, (const T*)w, (T*)y, rstd, \
                rows, cols, eps, (const T*)residual_in, (T*)residual_out)
