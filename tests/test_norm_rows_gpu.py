@@ -16,7 +16,7 @@ def _rel(got, ref):
 # bf16 keeps 8 significant bits: one rounding changes a value by at most 2^-8 of it, and so the 2-norm
 @pytest.mark.parametrize("dtype,tol", [(torch.bfloat16, 2.0 ** -8), (torch.float32, 2e-6)])
 @pytest.mark.parametrize("rows,cols", [(1, 8), (7, 248), (33, 256), (5, 264), (300, 1024), (9, 1032), (1201, 1536), (17, 2048), (3, 2056), (130, 4096), (6, 4104),
-                                       (1185, 2056), (1185, 2880), (2369, 1032)])
+                                       (1185, 2056), (1185, 2880), (2369, 1032), (40, 512), (25, 768), (1300, 1024), (1184, 1024)])
 def test_rmsnorm_forward_and_backward(dtype, tol, rows, cols):
     g = torch.Generator().manual_seed(rows * 10007 + cols)
     x, dy, res, dres = (torch.randn(rows, cols, generator=g).to(dtype) for _ in range(4))
