@@ -4,6 +4,7 @@
 // equal to `ignore_index` gives loss 0 and a zero gradient row (masked cross-entropy).
 // Reference semantics: Source/Private/Oa/Ml/Shader/Compute/Nn/CrossEntropy/CrossEntropy.slang:58-75,
 // CrossEntropyBwd.slang:69-78 and the fused CrossEntropyLossGradBwd registry entry.
+#include <cfloat>
 #include "common.cuh"
 #include "api.h"
 
@@ -49,7 +50,7 @@ xent_kernel(const T* __restrict__ logits, const int* __restrict__ targets, float
   const bool oor = !ignored && (tgt < 0 || tgt >= vocab);
   // read before any thread can overwrite the logits with the gradient (dlogits may alias logits)
   const float tgt_logit = (threadIdx.x == 0 && !ignored && !oor) ? XIO<T>::ld1(p + tgt) : 0.f;
-  float m = -INFINITY, s = 0.f;
+  float m = -FLT_MAX, s = 0.f;                     // finite: a masked logit (-inf) adds exp(-inf) = 0 whatever came before it
   for (int i = threadIdx.x; i < nvec; i += XENT_THREADS) {
     float v[V];
     XIO<T>::load(p + i * V, v);
@@ -57,21 +58,20 @@ xent_kernel(const T* __restrict__ logits, const int* __restrict__ targets, float
 #pragma unroll
     for (int j = 1; j < V; ++j) mx = fmaxf(mx, v[j]);
     if (mx > m) { s *= __expf(m - mx); m = mx; }
-    if (m == -INFINITY) continue;                  // masked so far: nothing to add, and -inf - -inf is not a number
 #pragma unroll
     for (int j = 0; j < V; ++j) s += __expf(v[j] - m);
   }
   for (int c = nvec * V + threadIdx.x; c < vocab; c += XENT_THREADS) {
     float v = XIO<T>::ld1(p + c);
     if (v > m) { s *= __expf(m - v); m = v; }
-    if (m != -INFINITY) s += __expf(v - m);
+    s += __expf(v - m);
   }
   // block combine of (m, s)
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     float om = __shfl_xor_sync(0xffffffffu, m, o), os = __shfl_xor_sync(0xffffffffu, s, o);
     float nm = fmaxf(m, om);
-    s = (m == -INFINITY ? 0.f : s * __expf(m - nm)) + (om == -INFINITY ? 0.f : os * __expf(om - nm));
+    s = s * __expf(m - nm) + os * __expf(om - nm);
     m = nm;
   }
   if ((threadIdx.x & 31) == 0) { red_m[threadIdx.x >> 5] = m; red_s[threadIdx.x >> 5] = s; }
@@ -81,7 +81,7 @@ xent_kernel(const T* __restrict__ logits, const int* __restrict__ targets, float
   for (int w = 1; w < XENT_THREADS / 32; ++w) {
     float om = red_m[w], os = red_s[w];
     float nm = fmaxf(m, om);
-    s = (m == -INFINITY ? 0.f : s * __expf(m - nm)) + (om == -INFINITY ? 0.f : os * __expf(om - nm));
+    s = s * __expf(m - nm) + os * __expf(om - nm);
     m = nm;
   }
   const float lse = m + logf(s);
@@ -248,6 +248,16 @@ xent_warp_kernel(const T* __restrict__ logits, const int* __restrict__ targets, 
       xent_vec_grad<T>(reinterpret_cast<const T*>(&x[k]), d + (k * 32 + lane) * V, lse, gs, tgt - (k * 32 + lane) * V);
 }
 
+// Whether the row in shared memory beats the online kernel.  With the gradient it saves a read of the logits: always, except for 16-bit
+// rows of which only one fits an SM (2048 x 65536 139.6 us online, 143.6 on the chip).  The loss alone reads them once either way, and the
+// online kernel keeps more loads in flight when rows are long: 8192 x 16384 bf16 72.3 / 60.5 us, fp32 88.2 / 83.9; 2048 x 32000 bf16
+// 33.1 / 34.9, 2048 x 50264 46.7 / 55.2, 8192 x 20480 fp32 108 / 118, 8192 x 32000 162 / 247.  One wave of rows is latency, not
+// bandwidth: 148 x 50264 8.2 / 6.8.
+static bool xent_row_on_chip(size_t bytes, long long rows, bool grad, size_t elem) {
+  if (rows <= 148) return true;
+  return grad ? elem == 4 || bytes <= 112 * 1024 : bytes <= 16384 * elem;
+}
+
 template <typename T>
 static int launch_xent(const T* logits, const int* targets, float* row_loss, T* dlogits, long long rows, int vocab, int ld, float grad_scale,
                        int ignore_index, int vec_ok, cudaStream_t st) {
@@ -257,7 +267,7 @@ static int launch_xent(const T* logits, const int* targets, float* row_loss, T* 
   if (vec_ok && vocab % V == 0 && nvec <= XENT_WARP_VECS * 32) {
     const unsigned blocks = (unsigned)((rows + XENT_THREADS / 32 - 1) / (XENT_THREADS / 32));
     xent_warp_kernel<T><<<blocks, XENT_THREADS, 0, st>>>(logits, targets, row_loss, dlogits, rows, vocab, ld, grad_scale, ignore_index);
-  } else if (vec_ok && smem > 0 && smem <= XENT_SMEM_MAX) {
+  } else if (vec_ok && smem > 0 && smem <= XENT_SMEM_MAX && xent_row_on_chip(smem, rows, dlogits != nullptr, sizeof(T))) {
     // eight vectors or so per thread: fewer threads leave the copies of short rows in flight together with the next CTA's
     auto go = [&](auto kernel, int threads) -> int {
       if (smem > 40 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, XENT_SMEM_MAX) != cudaSuccess) return OA_ERR_LAUNCH;

@@ -2,6 +2,7 @@
 import pytest
 import torch
 
+from device_time import graph_us
 from oa_b200.ops import kernels as K
 
 pytestmark = pytest.mark.gpu
@@ -51,3 +52,38 @@ def test_cross_entropy_rows(dtype, tol, rows, vocab, ld, in_place):
     loss2, none = K.xent_fwd_bwd(full.cuda()[:, :vocab], t.cuda())
     assert none is None
     torch.testing.assert_close(loss2, loss, rtol=0, atol=0, equal_nan=True)
+
+
+# More rows than SMs, where the loss alone and the gradient may take different kernels; masks of -inf and of the type's lowest value.
+@pytest.mark.parametrize("dtype,tol", [(torch.bfloat16, 2.0 ** -8), (torch.float32, 4e-6)])
+@pytest.mark.parametrize("rows,vocab,ld", [(150, 16384, 16384), (151, 16392, 16392), (149, 57344, 57344), (149, 57352, 57352), (160, 999, 1001)])
+def test_many_rows(dtype, tol, rows, vocab, ld):
+    g = torch.Generator().manual_seed(vocab)
+    full = (3.0 * torch.randn(rows, ld, generator=g)).to(dtype)
+    low = torch.finfo(dtype).min
+    full[0, : vocab // 2] = float("-inf")
+    full[1, : vocab // 2] = low
+    full[2, : vocab - 1] = low
+    t = torch.randint(vocab // 2, vocab, (rows,), generator=g, dtype=torch.int32)
+    t[2] = vocab - 1
+    out = torch.empty(rows, ld, dtype=dtype, device="cuda")[:, :vocab]
+    loss, d = K.xent_fwd_bwd(full.cuda()[:, :vocab], t.cuda(), grad_scale=0.25, dlogits=out)
+    alone, _ = K.xent_fwd_bwd(full.cuda()[:, :vocab], t.cuda())
+    lf = full[:, :vocab].double()
+    lse = torch.logsumexp(lf, -1)
+    ref = lse - lf.gather(1, t.long()[:, None])[:, 0]
+    for got in (loss, alone):
+        assert bool(((got.double().cpu() - ref).abs() <= 4e-6 * lse.abs().clamp_min(1.0)).all())
+    p = torch.softmax(lf, -1) * 0.25
+    grad = p.clone()
+    grad.scatter_add_(1, t.long()[:, None], torch.full((rows, 1), -0.25, dtype=torch.float64))
+    err = (d.double().cpu() - grad).norm(dim=1) / torch.maximum(grad.norm(dim=1), p.norm(dim=1))
+    assert float(err.max()) <= tol
+
+
+def test_the_loss_alone_reads_as_fast_as_it_may():
+    x = torch.randn(4096, 32000, device="cuda")
+    t = torch.randint(0, 32000, (4096,), device="cuda", dtype=torch.int32)
+    d = torch.empty_like(x)
+    # it moves half the bytes of loss and gradient; with the row in shared memory it took 0.6 of their time
+    assert graph_us(*[lambda: K.xent_fwd_bwd(x, t)] * 4) <= 0.52 * graph_us(*[lambda: K.xent_fwd_bwd(x, t, grad_scale=1.0, dlogits=d)] * 4)
