@@ -748,7 +748,9 @@ def xent_fwd_bwd(logits: torch.Tensor, targets: torch.Tensor, *, grad_scale: Opt
     row_loss = torch.empty(rows, dtype=torch.float32, device=logits.device)
     want = grad_scale is not None
     if want and dlogits is None:
-        dlogits = torch.empty_like(logits)
+        # the kernel walks both with one pitch
+        ld = logits.stride(0)
+        dlogits = logits.new_empty((rows, ld))[:, :vocab] if logits.is_cuda and rows > 1 and ld > vocab else torch.empty_like(logits)
     if not logits.is_cuda:
         lf = logits.float()
         t = targets.reshape(-1).long()
@@ -770,6 +772,8 @@ def xent_fwd_bwd(logits: torch.Tensor, targets: torch.Tensor, *, grad_scale: Opt
             dlogits.copy_(g)
         return row_loss, dlogits
     assert logits.stride(1) == 1
+    if want and rows > 1 and dlogits.stride(0) != logits.stride(0):
+        raise ValueError(f"xent_fwd_bwd: the gradient's row pitch {dlogits.stride(0)} is not that of the logits, {logits.stride(0)}")
     tg = targets.reshape(-1).to(torch.int32).contiguous()
     _launch(N.require().oa_xent_fwd_bwd(dt(logits), logits.data_ptr(), tg.data_ptr(), row_loss.data_ptr(),
                                         dlogits.data_ptr() if want else None, rows, vocab, logits.stride(0),

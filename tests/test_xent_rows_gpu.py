@@ -87,3 +87,17 @@ def test_the_loss_alone_reads_as_fast_as_it_may():
     d = torch.empty_like(x)
     # it moves half the bytes of loss and gradient; with the row in shared memory it took 0.6 of their time
     assert graph_us(*[lambda: K.xent_fwd_bwd(x, t)] * 4) <= 0.52 * graph_us(*[lambda: K.xent_fwd_bwd(x, t, grad_scale=1.0, dlogits=d)] * 4)
+
+
+# Logits that are columns of a wider matrix: the gradient made for them has their pitch, one of another pitch is refused.
+def test_pitch():
+    full = torch.randn(6, 40, device="cuda")
+    t = torch.arange(6, device="cuda", dtype=torch.int32)
+    x = full[:, :33]
+    loss, d = K.xent_fwd_bwd(x, t, grad_scale=1.0)
+    ref = torch.softmax(x.double(), -1) - torch.nn.functional.one_hot(t.long(), 33)
+    assert d.shape == x.shape and float((d.double() - ref).norm() / ref.norm()) <= 4e-6
+    with pytest.raises(ValueError):
+        K.xent_fwd_bwd(x, t, grad_scale=1.0, dlogits=torch.empty(6, 33, device="cuda"))
+    loss1, d1 = K.xent_fwd_bwd(x[:1], t[:1], grad_scale=1.0, dlogits=torch.empty(1, 33, device="cuda"))
+    assert torch.equal(d1[0], d[0]) and torch.equal(loss1[0], loss[0])
