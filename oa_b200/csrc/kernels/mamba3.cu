@@ -917,6 +917,16 @@ gated_norm_bwd_vec_kernel(const __nv_bfloat16* __restrict__ y, const __nv_bfloat
     for (int j = 0; j < 8; ++j) atomicAdd(dw + c8 * 8 + j, acc[j]);
 }
 
+// Forward: a few thousand vectors are one short wave either way, and the kernel above starts sooner (128 x 8 x 64 2.35 / 2.59 us; 512 x 8
+// x 64, at 32768 vectors, 2.8 / 2.5).  Backward: a thread walks its GN_TOKENS tokens one after the other, so blocks have to be many and
+// their columns in use (128 x 8 x 64 3.6 / 33 us, 2048 x 32 x 64 27 / 37, 32768 x 4 x 64 50 / 127; 3000 x 48 x 64 60 / 48,
+// 8192 x 24 x 64 86 / 72, 8192 x 48 x 64 170 / 82).
+inline bool gn_vec_fwd_pays(long long rows, int H, int P) { return rows * H * (P >> 3) > 8192; }
+inline bool gn_vec_bwd_pays(long long rows, int H, int P) {
+  const long long cols8 = (long long)H * (P >> 3);
+  return cols8 >= 96 && cols8 * ((rows + GN_TOKENS - 1) / GN_TOKENS) > 32768;
+}
+
 // lanes of a head a power of two, every row and pointer on a 16-byte boundary
 inline bool gn_vec_ok(int dtype, int P, long long zs, const void* a, const void* b, const void* c, const void* d, const void* e, const void* w) {
   const uintptr_t at = reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c) |
@@ -935,7 +945,7 @@ extern "C" int oa_gated_norm_fwd(int dtype, const void* y, const void* z, long l
   long long warps = rows * H;
   int grid = (int)((warps + 7) / 8 < 148 * 8 ? (warps + 7) / 8 : 148 * 8);
   cudaStream_t st = (cudaStream_t)stream;
-  if (gn_vec_ok(dtype, P, zs, y, z, out, nullptr, nullptr, w) && (rows * H * (P / 8) + 255) / 256 < 0x7fffffffLL) {
+  if (gn_vec_ok(dtype, P, zs, y, z, out, nullptr, nullptr, w) && gn_vec_fwd_pays(rows, H, P) && (rows * H * (P / 8) + 255) / 256 < 0x7fffffffLL) {
     gated_norm_fwd_vec_kernel<<<(unsigned)((rows * H * (P / 8) + 255) / 256), 256, 0, st>>>((const __nv_bfloat16*)y, (const __nv_bfloat16*)z, zs, w,
                                                                                           (__nv_bfloat16*)out, rstd, rows, H, P, eps);
     return cudaGetLastError() == cudaSuccess ? OA_OK : OA_ERR_LAUNCH;
@@ -957,7 +967,7 @@ extern "C" int oa_gated_norm_bwd(int dtype, const void* y, const void* z, long l
   int grid = (int)((warps + 7) / 8 < 148 * 4 ? (warps + 7) / 8 : 148 * 4);
   cudaStream_t st = (cudaStream_t)stream;
   const size_t smem = (size_t)H * P * 4;
-  if (gn_vec_ok(dtype, P, zs | dzs, y, z, dout, dy, dz, w) && (rows + GN_TOKENS - 1) / GN_TOKENS <= 65535) {
+  if (gn_vec_ok(dtype, P, zs | dzs, y, z, dout, dy, dz, w) && gn_vec_bwd_pays(rows, H, P) && (rows + GN_TOKENS - 1) / GN_TOKENS <= 65535) {
     const dim3 vgrid((unsigned)((H * (P / 8) + 127) / 128), (unsigned)((rows + GN_TOKENS - 1) / GN_TOKENS));
     gated_norm_bwd_vec_kernel<<<vgrid, 128, 0, st>>>((const __nv_bfloat16*)y, (const __nv_bfloat16*)z, zs, w, rstd, (const __nv_bfloat16*)dout,
                                                      (__nv_bfloat16*)dy, (__nv_bfloat16*)dz, dzs, dw, rows, H, P);

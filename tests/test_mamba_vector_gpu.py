@@ -2,6 +2,7 @@
 import pytest
 import torch
 
+from device_time import graph_us
 from oa_b200 import _native as N
 from oa_b200.ops import kernels as K
 from oa_b200.ops import mamba3 as M3
@@ -42,7 +43,8 @@ def test_convolution(B, L, C, col0, tail, kw):
 
 
 @pytest.mark.parametrize("dtype,tol", [(torch.bfloat16, 2.0 ** -8), (torch.float32, 4e-6)])
-@pytest.mark.parametrize("rows,H,P,extra", [(1, 1, 8, 8), (33, 3, 64, 0), (70, 48, 64, 24), (40, 5, 128, 8), (37, 7, 24, 8), (9, 3, 16, 3)])
+@pytest.mark.parametrize("rows,H,P,extra", [(1, 1, 8, 8), (33, 3, 64, 0), (70, 48, 64, 24), (40, 5, 128, 8), (37, 7, 24, 8), (9, 3, 16, 3),
+                                            (2801, 48, 64, 8), (8201, 8, 128, 0), (2750, 96, 32, 16), (5470, 24, 64, 3)])
 def test_gated_norm(dtype, tol, rows, H, P, extra):
     g = torch.Generator(device="cuda").manual_seed(rows + P)
     d = M3.Mamba3Dims(H * P, H, P, 8, 0, has_z=False)
@@ -59,3 +61,13 @@ def test_gated_norm(dtype, tol, rows, H, P, extra):
     assert _rel(dy, gy) <= tol and _rel(dproj[:, :H * P], gz) <= tol
     assert _rel(dw, gw.reshape(-1)) <= 1e-5
     assert bool((dproj[:, H * P:] == 3.0).all())
+
+
+# A handful of tokens: the backward pass is a few microseconds like the forward pass, not a serial walk over 32 tokens.
+def test_gated_norm_few_tokens():
+    rows, H, P = 128, 8, 64
+    d = M3.Mamba3Dims(H * P, H, P, 8, 0, has_z=False)
+    y, proj, do, dproj = (torch.randn(rows, H * P, device="cuda").bfloat16() for _ in range(4))
+    w = torch.ones(H, P, device="cuda")
+    _, rstd = M3.gated_norm_fwd(y, proj, w, d)
+    assert graph_us(*[lambda: M3.gated_norm_bwd(y, proj, w, rstd, do, d, dproj)] * 10) <= 5 * graph_us(*[lambda: M3.gated_norm_fwd(y, proj, w, d)] * 10)
