@@ -227,6 +227,12 @@ mamba3_conv4_vec_kernel(__nv_bfloat16* __restrict__ x, long long ld, int col0, c
   }
 }
 
+// A step of the serial walk over tokens costs more with eight columns to a thread, which the better loads repay once there are many
+// threads, or tokens enough for the shorter blocks.  Scalar against vector, forward: 1 x 16 x 768 8.0 / 14 us, 1 x 32 x 3328 13.5 / 15.9,
+// 1 x 48 x 768 and 64 x 1 x 3328 the other way (6.9 / 5.5); backward: 1 x 16 x 768 15 / 19, 64 x 1 x 3328 8.8 / 11.1, 64 x 8 x 3328 22.5 / 19.6.
+inline bool mc_vec_fwd_pays(long long rows, int L, int C) { return L >= 48 || rows * (C >> 3) > 24576; }
+inline bool mc_vec_bwd_pays(long long rows, int L, int C) { return L >= 32 || rows * (C >> 3) > 131072; }
+
 inline bool mc_vec_ok(int dtype, int C, int Kw, long long ld, int col0, const void* a, const void* b, const void* c) {
   return dtype == OA_BF16 && Kw == MC_KW && (C & 7) == 0 && (ld & 7) == 0 && (col0 & 7) == 0 &&
          ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15) == 0;
@@ -261,7 +267,7 @@ extern "C" int oa_mamba3_conv_fwd(int dtype, void* x, long long ld, int col0, vo
   const long long rows = (long long)B * L;
   dim3 grid((C + 127) / 128, B * ((L + MC_TB - 1) / MC_TB));
   const int tb = 16; // short blocks: three halo rows each, but enough of them to fill the SMs
-  if (mc_vec_ok(dtype, C, Kw, ld, col0, x, saved, nullptr) && (long long)B * ((L + tb - 1) / tb) <= 65535) {
+  if (mc_vec_ok(dtype, C, Kw, ld, col0, x, saved, nullptr) && mc_vec_fwd_pays(rows, L, C) && (long long)B * ((L + tb - 1) / tb) <= 65535) {
     mamba3_cols_copy_vec_kernel<<<mc_grid(rows * (C / 8)), 256, 0, ST>>>((const __nv_bfloat16*)x, ld, col0, (__nv_bfloat16*)saved, rows, C);
     mamba3_conv4_vec_kernel<0><<<dim3((C / 8 + 127) / 128, B * ((L + tb - 1) / tb)), 128, 0, ST>>>((__nv_bfloat16*)x, ld, col0,
         (const __nv_bfloat16*)saved, w, nullptr, nullptr, L, C, tb);
@@ -283,7 +289,7 @@ extern "C" int oa_mamba3_conv_bwd(int dtype, void* dy, long long ld, int col0, c
   if (Kw < 1 || Kw > MC_MAXK || B <= 0 || L <= 0 || C <= 0) return OA_ERR_ARG;
   dim3 grid((C + 127) / 128, B * ((L + MC_TB - 1) / MC_TB));
   const int tb = 16;
-  if (mc_vec_ok(dtype, C, Kw, ld, col0, dy, saved, gbuf) && (long long)B * ((L + tb - 1) / tb) <= 65535) {
+  if (mc_vec_ok(dtype, C, Kw, ld, col0, dy, saved, gbuf) && mc_vec_bwd_pays((long long)B * L, L, C) && (long long)B * ((L + tb - 1) / tb) <= 65535) {
     mamba3_conv4_vec_kernel<1><<<dim3((C / 8 + 127) / 128, B * ((L + tb - 1) / tb)), 128, 0, ST>>>((__nv_bfloat16*)dy, ld, col0,
         (const __nv_bfloat16*)saved, w, (__nv_bfloat16*)gbuf, nullptr, L, C, tb);
     mamba3_conv4_vec_kernel<2><<<dim3((C / 8 + 127) / 128, B * ((L + MC_TB - 1) / MC_TB)), 128, 0, ST>>>((__nv_bfloat16*)dy, ld, col0,
