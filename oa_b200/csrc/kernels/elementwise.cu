@@ -670,6 +670,7 @@ extern "C" int oa_swiglu_bwd(int dtype, const void* gu, const void* dout, void* 
 extern "C" int oa_rope(int dtype, void* x, long long rows, int row_stride, int n_heads, int head_dim, int seq_len,
                        int pos_offset, float theta, int backward, const int* pos_dev, void* stream) {
   if (head_dim % 2) return OA_ERR_ARG;
+  if (n_heads <= 0) return OA_OK;                         // nothing to turn; the heads per thread below divide
   if (dtype == OA_BF16 && head_dim % 16 == 0 && row_stride % 8 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
     // One thread turns all heads of a row (the angle is theirs in common) while there are rows enough to fill the machine; a
     // decoding step has a handful of rows, where that loop was a chain of memory round trips, and spreads the heads,

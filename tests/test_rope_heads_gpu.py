@@ -23,3 +23,9 @@ def test_rope_head_groups(hd, rows, heads, seq):
         assert torch.equal(got[:, heads * hd:], x[:, heads * hd:])
         # angles up to 3007 in fp32 (2^-24 of them) and one rounding to bf16
         assert _rel(got[:, :heads * hd], ref[:, :heads * hd]) <= 2.0 ** -8
+
+
+def test_no_heads_and_no_rows():
+    x = torch.randn(4, 64, device="cuda").bfloat16()
+    assert torch.equal(K.rope_(x.clone(), 0, 64, 1), x)
+    assert K.rope_(x[:0].clone(), 1, 64, 1).shape == (0, 64)
