@@ -242,6 +242,7 @@ __global__ void rope_kernel(T* x, long long rows, int row_stride, int n_heads, i
 
 // bf16 fast path: one thread owns 8 consecutive pair indices j of one row, computes their 8 (cos, sin) once and applies
 // them to every head of the row with 16-byte accesses (the angle depends on the position and on j only).
+template <bool SPLIT>   // false: one thread turns all heads of a row (no division by the groups)
 __global__ void __launch_bounds__(256)
 rope_bf16_vec_kernel(__nv_bfloat16* x, long long rows, int row_stride, int n_heads, int hd, int seq_len, int pos_offset, float theta,
                      int backward, const int* __restrict__ pos_dev, int heads_per) {
@@ -249,12 +250,12 @@ rope_bf16_vec_kernel(__nv_bfloat16* x, long long rows, int row_stride, int n_hea
   pdl_wait();
   if (pos_dev) pos_offset += *pos_dev;
   const int half = hd >> 1, jv = half >> 3;                 // 8-wide vectors per half head
-  const int groups = (n_heads + heads_per - 1) / heads_per;
+  const int groups = SPLIT ? (n_heads + heads_per - 1) / heads_per : 1;
   const long long total = rows * groups * jv;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const int v = (int)(i % jv);
-    const int h_lo = (int)((i / jv) % groups) * heads_per, h_hi = min(n_heads, h_lo + heads_per);
-    const long long r = i / jv / groups;
+    const long long q = i / jv, r = SPLIT ? q / groups : q;
+    const int h_lo = SPLIT ? (int)(q - r * groups) * heads_per : 0, h_hi = SPLIT ? min(n_heads, h_lo + heads_per) : n_heads;
     const float pos = (float)((int)(r % seq_len) + pos_offset);
     float c[8], s[8];
 #pragma unroll
@@ -678,8 +679,13 @@ extern "C" int oa_rope(int dtype, void* x, long long rows, int row_stride, int n
     const long long per_head_group = rows * (head_dim / 16);
     int heads_per = n_heads;
     while (heads_per > 4 && per_head_group * ((n_heads + heads_per - 1) / heads_per) < 148 * 256) heads_per = (heads_per + 1) / 2;
-    launch_pdl(rope_bf16_vec_kernel, dim3(grid_for(per_head_group * ((n_heads + heads_per - 1) / heads_per), 256)), dim3(256), 0, ST,
-               (__nv_bfloat16*)x, rows, row_stride, n_heads, head_dim, seq_len, pos_offset, theta, backward, pos_dev, heads_per);
+    const dim3 grid(grid_for(per_head_group * ((n_heads + heads_per - 1) / heads_per), 256));
+    if (heads_per < n_heads)
+      launch_pdl(rope_bf16_vec_kernel<true>, grid, dim3(256), 0, ST, (__nv_bfloat16*)x, rows, row_stride, n_heads, head_dim, seq_len, pos_offset,
+                 theta, backward, pos_dev, heads_per);
+    else
+      launch_pdl(rope_bf16_vec_kernel<false>, grid, dim3(256), 0, ST, (__nv_bfloat16*)x, rows, row_stride, n_heads, head_dim, seq_len, pos_offset,
+                 theta, backward, pos_dev, heads_per);
     return CHECK_LAUNCH();
   }
   DISPATCH_T(dtype, rope_kernel<T><<<grid_for(rows * n_heads * head_dim / 2, 256), 256, 0, ST>>>(
