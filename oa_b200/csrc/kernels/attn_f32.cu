@@ -11,7 +11,7 @@
 // shared by TPR threads that each keep W (32 or 8) of the head dimensions in registers and combine their
 // partial dot products with shuffles.  W = 32 does the least work per score; W = 8 makes four times as many,
 // shorter CTAs (which under the causal mask also skip more of the other side) and is taken while W = 32 would
-// leave SMs without a second CTA: 16 x 4 heads of 32 dimensions and 128 positions are 64 CTAs of one warp per
+// leave SMs idle (af_split): 16 x 4 heads of 32 dimensions and 128 positions are 64 CTAs of one warp per
 // scheduler, 33 / 41 / 44 us for forward, dQ and dK / dV, against 19 / 29 / 27 us.  Forward and dQ rows are queries (keys / values stream through shared
 // memory), dK / dV rows are keys (queries and output gradients stream through shared memory together with
 // their log-sum-exp and delta = rowsum(dO * O)).
@@ -257,11 +257,15 @@ attn_f32_bwd_kv_kernel(const float* __restrict__ q, const float* __restrict__ k,
 
 using namespace oa;
 
-// threads per row, negative for eight dimensions per thread
-static inline int af_split(int hd, int batch, int heads, int seq) {
+// Threads per row, negative for eight dimensions per thread, which is taken up to `limit` CTAs of the wide form: one per SM, or somewhat
+// more where the causal mask lets the shorter CTAs skip work, or where a sequence leaves most rows of a wide CTA empty.  Wide against narrow
+// (4 heads of 64), forward 20 x 128 (160 CTAs) 37.7 / 36.3 us, 28 x 128 (224) 39.4 / 52.3; causal 28 x 128 39.5 / 37.5, 8 x 512 (256) 127 / 137;
+// 64 x 16 (256) 11.2 / 6.7.  Backward 20 x 128 128 / 105, 28 x 128 129 / 146, 2 x 1024 (128) 553 / 651; causal 28 x 128 127 / 113, 36 x 128
+// (288) 127 / 135.  One to two heads of 512 to 4096 positions (16 to 64 CTAs): 0.5 to 0.9 of the wide form throughout.
+static inline int af_split(int hd, int batch, int heads, int seq, int limit) {
   const int wide = hd <= 32 ? 1 : (hd <= 64 ? 2 : 4);
   const long long ctas = (long long)((seq + AF_THREADS / wide - 1) / (AF_THREADS / wide)) * heads * batch;
-  return hd <= 64 && ctas < 2 * 148 ? -4 * wide : wide;
+  return hd <= 64 && ctas <= (seq <= AF_TILE ? 295 : limit) ? -4 * wide : wide;
 }
 
 extern "C" int oa_attn_f32(const float* q, const float* k, const float* v, float* o, float* lse, int batch, int heads,
@@ -271,7 +275,7 @@ extern "C" int oa_attn_f32(const float* q, const float* k, const float* v, float
   if (batch <= 0 || heads <= 0 || seq <= 0) return OA_OK;
   if (heads > 65535 || batch > 65535) return OA_ERR_ARG;
   cudaStream_t st = (cudaStream_t)stream;
-  const int split = af_split(head_dim, batch, heads, seq), rows = AF_THREADS / (split < 0 ? -split : split);
+  const int split = af_split(head_dim, batch, heads, seq, causal && head_dim > 32 ? 224 : 160), rows = AF_THREADS / (split < 0 ? -split : split);
   dim3 grid((seq + rows - 1) / rows, heads, batch);
 #define AF_FWD(T, W) attn_f32_fwd_kernel<T, W><<<grid, AF_THREADS, 0, st>>>(q, k, v, o, lse, heads, seq, head_dim, row_stride, o_row_stride, scale, causal)
   if (split == -4) AF_FWD(4, 8);
@@ -291,7 +295,7 @@ extern "C" int oa_attn_f32_bwd(const float* q, const float* k, const float* v, c
   if (batch <= 0 || heads <= 0 || seq <= 0) return OA_OK;
   if (heads > 65535 || batch > 65535) return OA_ERR_ARG;
   cudaStream_t st = (cudaStream_t)stream;
-  const int split = af_split(head_dim, batch, heads, seq), rows = AF_THREADS / (split < 0 ? -split : split);
+  const int split = af_split(head_dim, batch, heads, seq, causal ? 240 : (seq > 128 ? 96 : head_dim > 32 ? 160 : 192)), rows = AF_THREADS / (split < 0 ? -split : split);
   dim3 grid((seq + rows - 1) / rows, heads, batch);
 #define AF_BWD(T, W)                                                                                                             \
   attn_f32_bwd_q_kernel<T, W><<<grid, AF_THREADS, 0, st>>>(q, k, v, o, dout, lse, dq, heads, seq, head_dim, row_stride, o_row_stride, \
