@@ -116,3 +116,21 @@ def test_sliced_epilogue():
 
     out = torch.empty(130, 126, device="cuda")
     assert graph_us(*[lambda: K.gemm(a, b, out=out, residual=res)] * 10) <= 2.5 * graph_us(*[lambda: K.gemm(a, b, out=out)] * 10)
+
+
+# Ragged extents on an aligned pitch: the last 16-byte piece of a row or a column is copied in part.  What lies behind it is NaN, so a
+# piece copied whole shows.  Tiles of 64 rows, of 32 rows, and a sliced reduction.
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, False), (True, True)])
+@pytest.mark.parametrize("m,n,k", [(70, 66, 17), (5, 3, 2), (33, 65, 130), (1001, 1000, 99), (1025, 903, 35), (90, 70, 514), (66, 62, 1027)])
+def test_partial_vectors(m, n, k, a_mn, b_mn):
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+
+    def sliced(rows, cols):
+        t = torch.full((rows, (cols + 3) // 4 * 4 + 4), float("nan"), device="cuda")
+        t[:, :cols] = torch.randn(rows, cols, device="cuda", generator=g)
+        return t[:, :cols]
+
+    a, b = sliced(k, m) if a_mn else sliced(m, k), sliced(k, n) if b_mn else sliced(n, k)
+    v = (a.t() if a_mn else a).double() @ (b if b_mn else b.t()).double()
+    y = K.gemm(a, b, a_mn=a_mn, b_mn=b_mn)
+    assert float((y.double() - v).norm() / v.norm()) <= 2e-6
