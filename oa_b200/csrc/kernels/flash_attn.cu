@@ -331,7 +331,8 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 // S0 | S1 | P0 | P1 | O0 | O1 = 128 + 128 + 64 + 64 + 64 + 64.
 // The running maximum is updated lazily, as above.
 // Two threads per row (sixteen softmax warps, maxima exchanged through shared memory) measured 127.7 instead of 121.7 us at head
-// dim 64 (8 x 2048 x 16) and 193 instead of 188 us at head dim 128 (4096 x 32): the warps' chains are not what bounds it.
+// dim 64 (8 x 2048 x 16) and 193 instead of 188 us at head dim 128 (4096 x 32): halving a row's share of the exponentials does not
+// shorten the chain scores -> exponentials -> P V -> next scores of a tile, which one partner tile covers only in part.
 // Head dim 128: O takes the columns of P, so P_t overwrites the first half of S_t (S0 | S1 | O0 | O1 = 4 x 128 columns).  Then
 // Q K_{j+1}^T is issued behind P V_j by the same thread, and it is the other tile's products and exponentials that fill the gap.
 template <int HD_>

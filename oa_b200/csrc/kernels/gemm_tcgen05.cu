@@ -1294,7 +1294,8 @@ extern "C" int oa_gemm_bf16_batched(const void* A, const void* B, void* out, int
   if ((N & 7) || (K & 7) || (a_mn && (M & 7))) return OA_ERR_ALIGN;
   if ((ldc & (out_f32 ? 3 : 7)) || (residual && (ldr & 7)) || ((aux_out || aux_in) && (ldaux & 7))) return OA_ERR_ALIGN;
   if (batch > 1 && ((sc_batch & 7) || (sr_batch & 7) || (saux_batch & 7) || (sbias_batch & 7))) return OA_ERR_ALIGN;
-  // A handful of rows against a large weight: the kernel that streams the weight (gemm_skinny.cu)
+  // A handful of rows against a large weight: the kernel that streams the weight (gemm_skinny.cu).  It adds the products up in another
+  // order, and the residual before the one rounding, so the last bits of a row depend on how many rows come with it.
   if (!force_bn && batch == 1 && !a_mn && !b_mn && M <= 64 && N >= 256 && K >= 512 && !accumulate && !aux_out && !aux_in && gemm_skinny_wins(M, N, K))
     return gemm_skinny(A, B, out, M, N, K, lda, ldb, ldc, bias, residual, ldr, act, out_f32, alpha, status, (cudaStream_t)stream);
   int bn = force_bn ? force_bn : ((N >= 256) ? 256 : 128);

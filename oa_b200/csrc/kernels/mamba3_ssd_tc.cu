@@ -200,7 +200,7 @@ ssd_chunk_fwd_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_const
 struct SsdChunkBwd {
   const float *cum, *scale, *gamma, *qk, *w;        // [G, 128]
   const float* D;
-  const __nv_bfloat16 *C, *Bt, *X;                  // [G, 128, 128], [G, 128, 128], [G, 128, 64]
+  const __nv_bfloat16* X;                           // [G, 128, 64]
   float *dC, *dB;                                   // [G, 128, 128]
   float *row_mm, *col_mm, *col_ge, *diag, *dcum_ce, *dw;   // [G, 128]
   __nv_bfloat16* dx; long long lddx;                // x columns of the projection gradient
@@ -537,7 +537,7 @@ int oa_ssd_chunk_bwd(const void* C, const void* Bt, const void* X, const void* X
       (rc = make_tmap_2d_bf16(&tdh, dH, CN, G * CP, CN, 64, CP)))
     return rc;
   SsdChunkBwd p{(const float*)cum, (const float*)scale, (const float*)gamma, (const float*)qk, (const float*)w, (const float*)D,
-                (const __nv_bfloat16*)C, (const __nv_bfloat16*)Bt, (const __nv_bfloat16*)X, (float*)dC, (float*)dB, (float*)row_mm, (float*)col_mm, (float*)col_ge,
+                (const __nv_bfloat16*)X, (float*)dC, (float*)dB, (float*)row_mm, (float*)col_mm, (float*)col_ge,
                 (float*)diag, (float*)dcum_ce, (float*)dw, (__nv_bfloat16*)dx, lddx, H, nC, L, (int)G, (int*)status};
   if (cudaFuncSetAttribute(ssd_chunk_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ChunkBwdSmem::BYTES) != cudaSuccess) return OA_ERR_LAUNCH;
   const int grid = (int)(G < num_sms() ? G : num_sms());

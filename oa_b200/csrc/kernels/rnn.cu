@@ -5,9 +5,10 @@
 //         with [h_r | h_z | h_n] = W_hh h + b_hh, gate order reset | update | candidate, h(0) = 0
 //   RNN:  h' = tanh(i + W_hh h + b_hh)
 // The input projection i = W_ih x + b_ih for all time steps is one GEMM done by the caller; only the serial part
-// runs here.  The reference runs one work-group per batch element with h in shared memory; here a CTA owns a tile
-// of BT batch rows so that every W_hh row fetched from L2 / shared memory is reused BT times, h and the gate
-// pre-activations live in shared memory, math is fp32.  The backward pass walks time in reverse from the saved
+// runs here.  The reference runs one work-group per batch element with h in shared memory.  Hidden widths up to 128 that
+// are multiples of 8 (rnn_reg_ok) do likewise, with W_hh in registers for the whole sequence (rnn_reg_*_kernel, further
+// down); for other widths (rnn_scan_*_kernel) a CTA owns a tile of BT batch rows so that every W_hh row fetched from L2 /
+// shared memory is reused BT times, and h and the gate pre-activations live in shared memory.  Math is fp32.  The backward pass walks time in reverse from the saved
 // h(t-1), emits the gate gradients dGi (for the input projection) and dGh; the weight gradient
 // dW_hh = dGh^T Hprev and db_hh are then ordinary (tensor-core) GEMM / column-sum calls.
 #include "common.cuh"
