@@ -7,6 +7,7 @@ to PyTorch math: a missing library or an unsupported shape raises.
 """
 from __future__ import annotations
 
+import functools
 import math
 import os
 from typing import Optional
@@ -150,9 +151,14 @@ def _f32_epilogue_takes(t: Optional[torch.Tensor], m: int, n: int) -> bool:
     return t is None or (t.dtype == torch.float32 and tuple(t.shape) == (m, n) and t.stride(1) == 1)
 
 
+@functools.lru_cache(maxsize=1024)
+def _f32_scratch_floats(m: int, n: int, k: int, batch: int) -> int:
+    return N.require().oa_gemm_f32_scratch_floats(m, n, k, batch)
+
+
 def _f32_scratch(m: int, n: int, k: int, batch: int, device: torch.device) -> Optional[torch.Tensor]:
     """The partial sums of a product whose reduction is sliced, from the current stream's allocator; None when it is not sliced."""
-    floats = N.require().oa_gemm_f32_scratch_floats(m, n, k, batch) if k >= 512 else 0
+    floats = _f32_scratch_floats(m, n, k, batch) if k >= 512 else 0
     return torch.empty(floats, dtype=torch.float32, device=device) if floats else None
 
 
