@@ -30,6 +30,11 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// One lane of a converged warp, the same one at every call with the full mask (elect.sync is deterministic in its mask).  Products,
+// commits and bulk copies are issued behind this and not behind `lane == 0`: their operands are per-warp values, and only elect.sync
+// tells the compiler that a single lane is active; behind a comparison it has to allow for several.  With no other change the
+// forward and data-gradient products of a 16384 x 4096 x 1024 MLP went from 105 and 103 to 94 and 92 us, the GELU-backward one from
+// 132 to 120, head dim 128 attention forward (1 x 4096 x 32, causal) from 187 to 180 us; attention backward did not move.
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred = 0;
   asm volatile(

@@ -128,7 +128,7 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   if (warp == 9) {
     // ------------- producer: the whole warp walks the loop and waits together; one lane issues the copies.  K block i is
     // loaded two iterations before V block i - 2... both rings are simply filled in order, K first.
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(q_full, Cfg::Q_BYTES);
 #pragma unroll
       for (int x = 0; x < HD / 64; ++x)
@@ -138,7 +138,7 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       if (i < n_kv) {
         const int st = i % NSK;
         if (!warp_wait(&k_empty[st], ((i / NSK) & 1) ^ 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_EMPTY); break; }
-        if (lane == 0) {
+        if (elect_one()) {
           mbar_expect_tx(&k_full[st], Cfg::KV_BYTES);
 #pragma unroll
           for (int x = 0; x < HD / 64; ++x)
@@ -149,7 +149,7 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       if (jv >= 0) {
         const int st = jv % NSV;
         if (!warp_wait(&v_empty[st], ((jv / NSV) & 1) ^ 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_EMPTY); break; }
-        if (lane == 0) {
+        if (elect_one()) {
           mbar_expect_tx(&v_full[st], Cfg::KV_BYTES);
 #pragma unroll
           for (int x = 0; x < HD / 64; ++x)
@@ -167,7 +167,7 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       const int st = i % NSK;
       if (!warp_wait(&k_full[st], (i / NSK) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_FULL); return false; }
       tc_fence_after();
-      if (lane == 0) {
+      if (elect_one()) {
         const uint32_t k_addr = smem_u32(smem + Cfg::OFF_K + st * Cfg::KV_BYTES);
 #pragma unroll
         for (int ks = 0; ks < HD / 16; ++ks) {
@@ -190,7 +190,7 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       if (!warp_wait(&v_full[st], (j / NSV) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_FULL); break; }
       if (!warp_wait(&p_full[j & 1], (j >> 1) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_SOFTMAX); break; }
       tc_fence_after();
-      if (lane == 0) {
+      if (elect_one()) {
         const uint32_t v_addr = smem_u32(smem + Cfg::OFF_V + st * Cfg::KV_BYTES);
 #pragma unroll
         for (int ks = 0; ks < FA_BN / 16; ++ks)
@@ -433,7 +433,7 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       decode(item, pr, h, b, nkv0, nkv1);
       const int n_it = max(nkv0, nkv1), row0 = b * p.seq;
       if (!warp_wait(q_empty, (itc & 1) ^ 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_EMPTY); break; }
-      if (lane == 0) {
+      if (elect_one()) {
         const int tiles = nkv1 > 0 ? 2 : 1;
         mbar_expect_tx(q_full, tiles * Cfg::Q_BYTES);
         for (int t = 0; t < tiles; ++t)
@@ -445,14 +445,14 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         const int st = blk % NS;
         const uint32_t ph = (blk / NS) & 1;
         if (!warp_wait(&k_empty[st], ph ^ 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_EMPTY); ok = false; break; }
-        if (lane == 0) {
+        if (elect_one()) {
           mbar_expect_tx(&k_full[st], Cfg::KV_BYTES);
 #pragma unroll
           for (int x = 0; x < HD / 64; ++x)
             tma_load_2d(smem + Cfg::OFF_K + st * Cfg::KV_BYTES + x * (FA_BN * 128), &tmK, &k_full[st], h * HD + x * 64, row0 + j * FA_BN);
         }
         if (!warp_wait(&v_empty[st], ph ^ 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_EMPTY); ok = false; break; }
-        if (lane == 0) {
+        if (elect_one()) {
           mbar_expect_tx(&v_full[st], Cfg::KV_BYTES);
 #pragma unroll
           for (int x = 0; x < HD / 64; ++x)
@@ -476,7 +476,7 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       if (!warp_wait(&k_full[st], (blk / NS) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_FULL); return false; }
       if (!ALIAS && sc > 0 && !warp_wait(&s_empty[t], (sc - 1) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_TMEM_EMPTY); return false; }
       tc_fence_after();
-      if (lane == 0) {
+      if (elect_one()) {
         const uint32_t k_addr = smem_u32(smem + Cfg::OFF_K + st * Cfg::KV_BYTES);
 #pragma unroll
         for (int ks = 0; ks < HD / 16; ++ks) {
@@ -507,7 +507,7 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         if (!warp_wait(&v_full[st], ((base + j) / NS) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_FULL); ok = false; break; }
         if (!warp_wait(&p_full[t], pc & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_SOFTMAX); ok = false; break; }
         tc_fence_after();
-        if (lane == 0) {
+        if (elect_one()) {
           const uint32_t v_addr = smem_u32(smem + Cfg::OFF_V + st * Cfg::KV_BYTES);
 #pragma unroll
           for (int ks = 0; ks < FA_BN / 16; ++ks)
@@ -853,7 +853,7 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       const int i0 = p.causal ? jb : 0, n_it = nblk - i0, row0 = b * p.seq;
       const long long stat_base = ((long long)b * p.heads + h) * p.seq;
       if (!warp_wait(kv_empty, (itc & 1) ^ 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_EMPTY); break; }
-      if (lane == 0) {
+      if (elect_one()) {
         mbar_expect_tx(kv_full, 2 * Cfg::T_BYTES);
 #pragma unroll
         for (int x = 0; x < HD / 64; ++x) {
@@ -865,7 +865,7 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         const int st = qc % NST;
         const uint32_t ph = (qc / NST) & 1;
         if (!warp_wait(&qdo_empty[st], ph ^ 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_EMPTY); ok = false; break; }
-        if (lane == 0) {
+        if (elect_one()) {
           mbar_expect_tx(&qdo_full[st], 2 * Cfg::T_BYTES);
           const int qrow = row0 + (i0 + it) * FA_BM;
 #pragma unroll
@@ -916,7 +916,7 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         // those columns, only once the previous gradient products have consumed them
         if (qc > 0 && !warp_wait(ALIAS ? pds_empty : s_empty, (qc - 1) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_TMEM_EMPTY); ok = false; break; }
         tc_fence_after();
-        if (lane == 0) {
+        if (elect_one()) {
           const uint32_t q_addr = smem_u32(smem + Cfg::OFF_Q + st * Cfg::T_BYTES);
           const uint32_t do_addr = smem_u32(smem + Cfg::OFF_DO + st * Cfg::T_BYTES);
 #pragma unroll
@@ -958,7 +958,7 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         if (!warp_wait(&qdo_full[st], (qc / NST) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_FULL); ok = false; break; }
         if (!warp_wait(pds_full, qc & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_SOFTMAX); ok = false; break; }
         tc_fence_after();
-        if (lane == 0) {
+        if (elect_one()) {
           const uint32_t b_addr = smem_u32(smem + (is_dv ? Cfg::OFF_DO : Cfg::OFF_Q) + st * Cfg::T_BYTES);
 #pragma unroll
           for (int ks = 0; ks < FA_BM / 16; ++ks)    // reduction over the 128 queries of this block
@@ -1170,7 +1170,7 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       decode(item, ib, h, b);
       const int n_kv = p.causal ? (ib + 1) : nblk, row0 = b * p.seq;
       if (!warp_wait(q_empty, (itc & 1) ^ 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_EMPTY); break; }
-      if (lane == 0) {
+      if (elect_one()) {
         mbar_expect_tx(q_full, 2 * Cfg::T_BYTES);
 #pragma unroll
         for (int x = 0; x < HD / 64; ++x) {
@@ -1182,7 +1182,7 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         const int st = kc % NST;
         const uint32_t ph = (kc / NST) & 1;
         if (!warp_wait(&kv_empty[st], ph ^ 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_EMPTY); ok = false; break; }
-        if (lane == 0) {
+        if (elect_one()) {
           mbar_expect_tx(&kv_full[st], 2 * Cfg::T_BYTES);
 #pragma unroll
           for (int x = 0; x < HD / 64; ++x) {
@@ -1212,7 +1212,7 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         if (!warp_wait(&kv_full[st], (kc / NST) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_FULL); ok = false; break; }
         if (kc > 0 && !warp_wait(s_empty, (kc - 1) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_TMEM_EMPTY); ok = false; break; }
         tc_fence_after();
-        if (lane == 0) {
+        if (elect_one()) {
           const uint32_t k_addr = smem_u32(smem + Cfg::OFF_K + st * Cfg::T_BYTES);
           const uint32_t v_addr = smem_u32(smem + Cfg::OFF_V + st * Cfg::T_BYTES);
 #pragma unroll
@@ -1250,7 +1250,7 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         if (!warp_wait(&kv_full[st], (kc / NST) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_FULL); ok = false; break; }
         if (!warp_wait(ds_full, kc & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_SOFTMAX); ok = false; break; }
         tc_fence_after();
-        if (lane == 0) {
+        if (elect_one()) {
           const uint32_t k_addr = smem_u32(smem + Cfg::OFF_K + st * Cfg::T_BYTES);
 #pragma unroll
           for (int ks = 0; ks < FA_BN / 16; ++ks)

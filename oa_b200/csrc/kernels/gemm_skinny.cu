@@ -81,7 +81,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     for (int i = kb0 + NS; i < kb1; ++i) {
       const int j = i - kb0, st = j % NS;
       if (!warp_wait(&empty[st], ((j / NS) & 1) ^ 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_EMPTY); break; }
-      if (lane == 0) {
+      if (elect_one()) {
         uint8_t* d = ring + st * Cfg::STAGE_BYTES;
         mbar_expect_tx(&full[st], Cfg::STAGE_BYTES);
         tma_load_3d(d, &tmW, &full[st], i * SK_BK, n0, 0);
@@ -95,7 +95,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       const int j = i - kb0, st = j % NS;
       if (!warp_wait(&full[st], (j / NS) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_FULL); break; }
       tc_fence_after();
-      if (lane == 0) {
+      if (elect_one()) {
         const uint32_t wa = smem_u32(ring + st * Cfg::STAGE_BYTES), xa = wa + Cfg::W_BYTES;
 #pragma unroll
         for (int ks = 0; ks < SK_BK / 16; ++ks)

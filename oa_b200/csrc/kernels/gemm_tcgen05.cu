@@ -171,7 +171,7 @@ struct TmaStoreCtx {
 __device__ __forceinline__ void tma_store_packed(TmaStoreCtx* ts, const CUtensorMap* m, const uint32_t* w, int col0) {
   const int lane = threadIdx.x & 31;
   uint8_t* b = ts->buf + (ts->n & 1) * 2048;
-  if (lane == 0) tma_store_wait_read1();
+  if (elect_one()) tma_store_wait_read1();
   __syncwarp();
   const uint32_t base = smem_u32(b) + lane * 64;
   const int sw = (lane >> 1) & 3;                       // 64-byte swizzle: 16-byte piece index ^= address bits 7..8
@@ -179,7 +179,7 @@ __device__ __forceinline__ void tma_store_packed(TmaStoreCtx* ts, const CUtensor
   for (int g = 0; g < 4; ++g) st_shared_v4(base + ((g ^ sw) << 4), make_uint4(w[g * 4], w[g * 4 + 1], w[g * 4 + 2], w[g * 4 + 3]));
   fence_proxy_async_smem();
   __syncwarp();
-  if (lane == 0) {
+  if (elect_one()) {
     if (ts->z < 0) tma_store_2d(m, b, col0, ts->row0);
     else tma_store_3d(m, b, col0, ts->row0, ts->z);
     tma_store_commit();
@@ -509,7 +509,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   if (p.tp_mode) tp_epoch = *reinterpret_cast<volatile unsigned long long*>(p.tp_sync) + 1;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       // ---------------- TMA producer
       int stage = 0;
       uint32_t phase = 0;
@@ -561,7 +561,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       // ---------------- MMA issuer
       constexpr uint32_t idesc = umma_idesc_bf16(BM, BN, A_MN, B_MN);
       // K-major: 8-row groups are 1024 B apart; one UMMA_K step is 32 B inside the swizzled row.
@@ -696,7 +696,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       acc ^= 1;
       if (acc == 0) acc_phase ^= 1;
     }
-    if (ts && lane == 0) tma_store_wait_read0();       // the staging buffers stay valid until the last store has read them
+    if (ts && elect_one()) tma_store_wait_read0();       // the staging buffers stay valid until the last store has read them
     if (n_pend > 0) {
       __threadfence_system();
       __syncwarp();
@@ -814,7 +814,7 @@ gemm_pair_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   pdl_wait();                            // everything above ran under the previous kernel's tail; global memory from here on
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       // ---------------- TMA producer (both CTAs; the bytes are credited to the even CTA's barrier)
       int stage = 0;
       uint32_t phase = 0;
@@ -864,7 +864,7 @@ gemm_pair_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
 #endif
     }
   } else if (warp == 1) {
-    if (lane == 0 && leader) {
+    if (elect_one() && leader) {
       // ---------------- MMA issuer of the pair
       constexpr uint32_t idesc_full = umma_idesc_bf16(256, 256, A_MN, B_MN);
       constexpr uint32_t idesc_half = umma_idesc_bf16(256, 128, A_MN, B_MN);
@@ -1081,7 +1081,7 @@ gemm_pair_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       acc ^= 1;
       if (acc == 0) acc_phase ^= 1;
     }
-    if (ts && lane == 0) tma_store_wait_read0();         // the staging buffers stay valid until the last store has read them
+    if (ts && elect_one()) tma_store_wait_read0();         // the staging buffers stay valid until the last store has read them
   }
   pdl_launch_dependents();               // this CTA's work is issued: the next kernel's CTAs may take the SM as it drains
   tc_fence_before();

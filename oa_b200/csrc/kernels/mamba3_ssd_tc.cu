@@ -64,7 +64,7 @@ ssd_chunk_fwd_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_const
   const uint32_t tm = tmem_slot;                    // G (M over its first half) | M X | C~ Hin^T = 128 + 64 + 64 columns
 
   if (warp == 4) {
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(&cb_full, 4 * HALF);
       for (int x = 0; x < 2; ++x) {
         tma_load_2d(sm + S::OFF_C + x * HALF, &tmC, &cb_full, x * 64, g * CQ);
@@ -80,7 +80,7 @@ ssd_chunk_fwd_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_const
     bool ok = warp_wait(&cb_full, 0);
     if (ok) {
       tc_fence_after();
-      if (lane == 0) {
+      if (elect_one()) {
 #pragma unroll
         for (int ks = 0; ks < CN / 16; ++ks)
           umma_f16(tm, desc_k(c_addr, ks, HALF), desc_k(b_addr, ks, HALF), umma_idesc_bf16(CQ, CQ, 0, 0), ks > 0);
@@ -91,7 +91,7 @@ ssd_chunk_fwd_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_const
     }
     if (ok) {
       tc_fence_after();
-      if (lane == 0)
+      if (elect_one())
 #pragma unroll
         for (int ks = 0; ks < CN / 16; ++ks)
           umma_f16(tm + 192, desc_k(c_addr, ks, HALF), desc_k(h_addr, ks, HALF / 2), umma_idesc_bf16(CQ, CP, 0, 0), ks > 0);
@@ -100,7 +100,7 @@ ssd_chunk_fwd_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_const
     }
     if (ok) {
       tc_fence_after();
-      if (lane == 0) {
+      if (elect_one()) {
 #pragma unroll
         for (int ks = 0; ks < CQ / 16; ++ks)
           umma_f16_ts(tm + 128, tm + ks * 8, desc_mn(x_addr, ks, HALF), umma_idesc_bf16(CQ, CP, 0, 1), ks > 0);
@@ -271,7 +271,7 @@ ssd_chunk_bwd_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_const
     for (int g = blockIdx.x; g < p.G && ok; g += gridDim.x, ++n) {
       // operands that only the products read are free when the previous chunk's products are done; C~ and B~ when its epilogue is
       ok = warp_wait(&ops_free, (n & 1) ^ 1);
-      if (ok && lane == 0) {
+      if (ok && elect_one()) {
         mbar_expect_tx(&ops_full, 5 * HALF);
         tma_load_2d(sm + S::OFF_DY, &tmDY, &ops_full, 0, g * CQ);
         tma_load_2d(sm + S::OFF_X, &tmX, &ops_full, 0, g * CQ);
@@ -283,7 +283,7 @@ ssd_chunk_bwd_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_const
       }
       __syncwarp();
       ok = ok && warp_wait(&cb_free, (n & 1) ^ 1);
-      if (ok && lane == 0) {
+      if (ok && elect_one()) {
         mbar_expect_tx(&cb_full, 4 * HALF);
         for (int x = 0; x < 2; ++x) {
           tma_load_2d(sm + S::OFF_C + x * HALF, &tmC, &cb_full, x * 64, g * CQ);
@@ -294,7 +294,7 @@ ssd_chunk_bwd_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_const
       ok = ok && warp_wait(&ops_full, n & 1) && warp_wait(&cb_full, n & 1);
       if (!ok) break;
       tc_fence_after();
-      if (lane == 0) {
+      if (elect_one()) {
 #pragma unroll
         for (int ks = 0; ks < CN / 16; ++ks)        // G = C~ B~^T
           umma_f16(tm + TM_A, desc_k(c_a, ks, HALF), desc_k(b_a, ks, HALF), umma_idesc_bf16(CQ, CQ, 0, 0), ks > 0);
@@ -313,7 +313,7 @@ ssd_chunk_bwd_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_const
       ok = warp_wait(&m_full, n & 1);
       if (!ok) break;
       tc_fence_after();
-      if (lane == 0) {
+      if (elect_one()) {
 #pragma unroll
         for (int ks = 0; ks < CQ / 16; ++ks)        // M^T dY
           umma_f16(tm + TM_X, desc_mn(m_a, ks, HALF), desc_mn(dy_a, ks, HALF), umma_idesc_bf16(CQ, CP, 1, 1), ks > 0);
