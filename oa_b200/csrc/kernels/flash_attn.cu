@@ -749,22 +749,30 @@ flash_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __r
   }
 }
 
-constexpr int FA_BWD_THREADS = 384;   // 8 softmax warps + 3 MMA issuer warps (the dQ kernel uses 2) + 1 TMA warp
+constexpr int FA_BWD_THREADS = 352;   // 8 softmax warps + 2 MMA issuer warps + 1 TMA warp
 
-// Backward pipeline (both kernels).  The score products of a tile land in TMEM; the eight softmax warps (two threads
-// per TMEM lane) copy them to registers and release the buffers at once, so the first MMA warp issues the score products
-// of the NEXT tile while this tile's exponentials run.  The bf16 results (P^T and dS^T in the dK/dV kernel, dS in the dQ
-// kernel) are written back to TMEM and are the A operands of the gradient products, which the second MMA warp issues:
-// nothing passes through shared memory.  One tcgen05.mma costs about 50 cycles to issue from a thread and the
-// N = head_dim products are issue bound, hence two issuing warps.
+// Backward pipeline (both kernels).  A tile passes through two phases in the eight softmax warps (two threads per TMEM lane, 64 columns
+// each): scores -> probabilities, then dP -> dS.  The phases have barriers of their own, so the tensor pipe always has the other
+// phase's products to run: under the exponentials of tile i it works on dS_{i-1}'s gradient product and on dP_i, and under
+// the dS phase of tile i it consumes P_i and forms the scores of tile i + 1.  One warp issues the products that hang on the
+// probabilities (scores and dV), the other those that hang on dS (dP and dK, or dP and dQ); within a warp the products that reuse
+// tensor-memory columns are ordered by the pipe.  The bf16 results overwrite the columns they were computed from, each half of the
+// columns within its own 64, so neither half waits for the other before it stores, and the gradient products start on the first half.
+// Bound by the latency of that chain: at head dim 64 the exponentials take 1024 of about 2,900 clocks per tile, at head dim 128 the
+// products 2,200 of about 4,000, and a barrier that is already complete costs a warp 100 clocks or more while the pipes are busy.
+// Measured, dK/dV and dQ kernel, with one barrier for both phases (scores and dP issued together, both read before either was
+// computed on) -> this: 2 x 3001 x 16 heads of 128 194 and 129 -> 161 and 109 us, 1 x 4096 x 32 of 128 325 and 206 -> 268 and 182,
+// 8 x 2048 x 16 of 64 195 and 164 -> 191 and 160.  Slower: one issuing warp for all four products (172 us, 260 us at head dim 64),
+// sixteen softmax warps (300 us at head dim 64 with the two phases merged into one pass; every wait is made by twice the warps),
+// one lane waiting for its warp (261 us), partner warps of a scheduler taking turns at the exponentials (212 us).
 //
 // The dK/dV kernel works on the TRANSPOSED tile, S^T = K Q^T with keys on the TMEM lanes, because dV = P^T dO and
 // dK = dS^T Q need P^T / dS^T with keys as the M dimension.  Per-query statistics (log-sum-exp, delta) are then per
-// COLUMN: the softmax warps stage them in shared memory (double buffered by iteration parity) and read them as broadcasts.
+// COLUMN: the producer warp stages them in shared memory beside the Q tile and they are read as broadcasts.
 template <int HD>
 struct BwdKvCfg {
-  static constexpr int NST = (HD == 64) ? 3 : 2;       // Q / dO ring: a stage is held from the score products to the end of dK
-  static constexpr bool ALIAS = HD != 64;               // head_dim 128: P^T / dS^T overwrite S^T / dP^T (no spare TMEM columns)
+  static constexpr int NST = (HD == 64) ? 3 : 2;       // Q and dO rings
+  static constexpr int NS = (HD == 64) ? 2 : 1;        // score buffers in TMEM (P^T lies over S^T, dS^T over dP^T)
   static constexpr int T_BYTES = FA_BM * HD * 2;        // one [128 x HD] tile
   static constexpr int OFF_K = 0;
   static constexpr int OFF_V = OFF_K + T_BYTES;
@@ -772,12 +780,34 @@ struct BwdKvCfg {
   static constexpr int OFF_DO = OFF_Q + NST * T_BYTES;
   static constexpr int OFF_STAT = OFF_DO + NST * T_BYTES;   // float[NST][256]: -lse*log2e | -delta*scale of the query block
   static constexpr int OFF_BAR = OFF_STAT + NST * 256 * 4;
-  static constexpr int SMEM_BYTES = OFF_BAR + 128;
+  static constexpr int SMEM_BYTES = OFF_BAR + 208;
   static constexpr int TMEM_COLS = 512;
-  static constexpr int TM_S = 0, TM_DP = 128;
-  static constexpr int TM_P = ALIAS ? 0 : 256, TM_DS = ALIAS ? 128 : 320;
-  static constexpr int TM_DV = ALIAS ? 256 : 384, TM_DK = TM_DV + HD;
+  static constexpr int TM_S = 0, TM_DP = NS * FA_BN, TM_DV = TM_DP + FA_BN, TM_DK = TM_DV + HD;
 };
+
+// two fp32 values per instruction
+__device__ __forceinline__ unsigned long long f2_of(uint32_t a, uint32_t b) { unsigned long long r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(a), "r"(b)); return r; }
+__device__ __forceinline__ void f2_to(unsigned long long v, uint32_t& a, uint32_t& b) { asm("mov.b64 {%0, %1}, %2;" : "=r"(a), "=r"(b) : "l"(v)); }
+__device__ __forceinline__ unsigned long long f2_fma(unsigned long long a, unsigned long long b, unsigned long long c) { unsigned long long d; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c)); return d; }
+__device__ __forceinline__ unsigned long long f2_mul(unsigned long long a, unsigned long long b) { unsigned long long d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+__device__ __forceinline__ void bwd_prob2(uint32_t& a, uint32_t& b, unsigned long long sl2, unsigned long long nl) {
+  f2_to(f2_fma(f2_of(a, b), sl2, nl), a, b);
+  a = __float_as_uint(fast_exp2(__uint_as_float(a))); b = __float_as_uint(fast_exp2(__uint_as_float(b)));
+}
+__device__ __forceinline__ void bwd_ds2(uint32_t& a, uint32_t& b, uint32_t d0, uint32_t d1, unsigned long long scale, unsigned long long nd) {
+  f2_to(f2_mul(f2_of(a, b), f2_fma(f2_of(d0, d1), scale, nd)), a, b);
+}
+// exp2(s sl2 + nl); p (dp scale + nd); 32 values of a lane as bf16 over 16 columns
+__device__ __forceinline__ uint32_t bwd_prob(uint32_t s, float sl2, float nl) { return __float_as_uint(fast_exp2(fmaf(__uint_as_float(s), sl2, nl))); }
+__device__ __forceinline__ uint32_t bwd_ds(uint32_t p, uint32_t dp, float scale, float nd) {
+  return __float_as_uint(__uint_as_float(p) * fmaf(__uint_as_float(dp), scale, nd));
+}
+__device__ __forceinline__ void bwd_store16(uint32_t taddr, const uint32_t* v) {
+  uint32_t w[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) w[i] = pack_bf16x2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
+  tmem_st16(taddr, w);
+}
 
 // Persistent: one CTA per SM walks the work items (key block, head, batch) it owns, heaviest causal key blocks first, items
 // dealt in snake order; dK, dV of an item accumulate in TMEM over its query blocks.  Barrier phases come from running counts.
@@ -787,20 +817,21 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
                     const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
                     const FlashBwdParams p) {
   using Cfg = BwdKvCfg<HD>;
-  constexpr int NST = Cfg::NST;
-  constexpr bool ALIAS = Cfg::ALIAS;
+  constexpr int NST = Cfg::NST, NS = Cfg::NS;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::OFF_BAR);
   uint64_t* kv_full = bars + 0;
-  uint64_t* kv_empty = bars + 1;   // the item's last score products have read K, V
-  uint64_t* qdo_full = bars + 2;   // [3]
-  uint64_t* qdo_empty = bars + 5;  // [3]  (dV and dK issuers both arrive)
-  uint64_t* s_full = bars + 8;     // S^T, dP^T of this tile are in TMEM
-  uint64_t* s_empty = bars + 9;    // ... and have been copied to registers (8 warps)
-  uint64_t* pds_full = bars + 10;  // P^T, dS^T of this tile are in TMEM (8 warps)
-  uint64_t* pds_empty = bars + 11; // ... and have been consumed by the gradient products (dV and dK issuers both arrive)
-  uint64_t* fin_full = bars + 12;  // dV, dK of the item are complete (both issuers arrive)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 13);
+  uint64_t* kv_empty = bars + 1;   // the item's last score and dP products have read K, V
+  uint64_t* q_full = bars + 2;     // [3]  Q bytes and the statistics
+  uint64_t* q_empty = bars + 5;    // [3]  dK has read Q (the scores and the statistics were read before)
+  uint64_t* do_full = bars + 8;    // [3]
+  uint64_t* do_empty = bars + 11;  // [3]  dP and dV have read dO
+  uint64_t* s_full = bars + 14;    // [2]  S^T of this tile is in TMEM
+  uint64_t* p_full = bars + 16;    // [2][2]  P^T, by score buffer and column half (4 warps each)
+  uint64_t* dp_full = bars + 20;   // dP^T
+  uint64_t* ds_full = bars + 21;   // [2]  dS^T, by column half (4 warps each)
+  uint64_t* fin_full = bars + 23;  // dV, dK of the item are complete (both issuers arrive)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 24);
   float* stat = reinterpret_cast<float*>(smem + Cfg::OFF_STAT);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -825,12 +856,11 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV); tma_prefetch_desc(&tmDO);
     mbar_init(kv_full, 1);
-    mbar_init(kv_empty, 1);
-    for (int s = 0; s < NST; ++s) { mbar_init(&qdo_full[s], 2); mbar_init(&qdo_empty[s], 2); }   // full: TMA bytes + the statistics
-    mbar_init(s_full, 1);
-    mbar_init(s_empty, 8);
-    mbar_init(pds_full, 8);
-    mbar_init(pds_empty, 2);
+    mbar_init(kv_empty, 2);
+    for (int s = 0; s < NST; ++s) { mbar_init(&q_full[s], 2); mbar_init(&q_empty[s], 1); mbar_init(&do_full[s], 1); mbar_init(&do_empty[s], 2); }
+    for (int s = 0; s < 2; ++s) { mbar_init(&s_full[s], 1); mbar_init(&ds_full[s], 4); }
+    for (int s = 0; s < 4; ++s) mbar_init(&p_full[s], 4);
+    mbar_init(dp_full, 1);
     mbar_init(fin_full, 2);
     mbar_fence_init();
   }
@@ -841,7 +871,7 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   const uint32_t tmem_base = *tmem_slot;
   pdl_wait();                            // the prologue above ran under the previous kernel's tail; global memory from here on
 
-  if (warp == 11) {
+  if (warp == 10) {
     // ------------- TMA producer (also stages the per-query statistics of each block)
     uint32_t itc = 0, qc = 0;       // items and Q / dO blocks loaded so far
     bool ok = true;
@@ -864,15 +894,20 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       for (int it = 0; it < n_it; ++it, ++qc) {
         const int st = qc % NST;
         const uint32_t ph = (qc / NST) & 1;
-        if (!warp_wait(&qdo_empty[st], ph ^ 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_EMPTY); ok = false; break; }
+        const int qrow = row0 + (i0 + it) * FA_BM;
+        if (!warp_wait(&q_empty[st], ph ^ 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_EMPTY); ok = false; break; }
         if (elect_one()) {
-          mbar_expect_tx(&qdo_full[st], 2 * Cfg::T_BYTES);
-          const int qrow = row0 + (i0 + it) * FA_BM;
+          mbar_expect_tx(&q_full[st], Cfg::T_BYTES);
 #pragma unroll
-          for (int x = 0; x < HD / 64; ++x) {
-            tma_load_2d(smem + Cfg::OFF_Q + st * Cfg::T_BYTES + x * (FA_BM * 128), &tmQ, &qdo_full[st], h * HD + x * 64, qrow);
-            tma_load_2d(smem + Cfg::OFF_DO + st * Cfg::T_BYTES + x * (FA_BM * 128), &tmDO, &qdo_full[st], h * HD + x * 64, qrow);
-          }
+          for (int x = 0; x < HD / 64; ++x)
+            tma_load_2d(smem + Cfg::OFF_Q + st * Cfg::T_BYTES + x * (FA_BM * 128), &tmQ, &q_full[st], h * HD + x * 64, qrow);
+        }
+        if (!warp_wait(&do_empty[st], ph ^ 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_EMPTY); ok = false; break; }
+        if (elect_one()) {
+          mbar_expect_tx(&do_full[st], Cfg::T_BYTES);
+#pragma unroll
+          for (int x = 0; x < HD / 64; ++x)
+            tma_load_2d(smem + Cfg::OFF_DO + st * Cfg::T_BYTES + x * (FA_BM * 128), &tmDO, &do_full[st], h * HD + x * 64, qrow);
         }
         // per-query statistics of this block, negated and pre-scaled: lane l stages queries 4l .. 4l+3
         {
@@ -891,17 +926,36 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           reinterpret_cast<float4*>(dst + 128)[lane] = nd;
         }
         __syncwarp();
-        if (lane == 0) mbar_arrive(&qdo_full[st]);
+        if (lane == 0) mbar_arrive(&q_full[st]);
         __syncwarp();
       }
       ++itc;
     }
   } else if (warp == 8) {
-    // ------------- MMA issuer A: transposed score products S^T = K Q^T, dP^T = V dO^T
+    // ------------- MMA issuer A: S^T = K Q^T and dV += P^T dO.  S^T of a tile goes over the P^T that dV read NS tiles ago.
     constexpr uint32_t idesc_s = umma_idesc_bf16(FA_BN, FA_BM, 0, 0);
-    const uint32_t k_addr = smem_u32(smem + Cfg::OFF_K), v_addr = smem_u32(smem + Cfg::OFF_V);
+    constexpr uint32_t idesc_g = umma_idesc_bf16(FA_BN, HD, 0, 1);   // [keys x HD] += X^T[keys x q] (TMEM) * Y[q x HD]
+    const uint32_t k_addr = smem_u32(smem + Cfg::OFF_K);
     uint32_t itc = 0, qc = 0;
     bool ok = true;
+    auto issue_s = [&](uint32_t n, bool last) -> bool {
+      const int st = n % NST;
+      if (!warp_wait(&q_full[st], (n / NST) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_FULL); return false; }
+      tc_fence_after();
+      if (elect_one()) {
+        const uint32_t q_addr = smem_u32(smem + Cfg::OFF_Q + st * Cfg::T_BYTES);
+        const uint32_t s_tm = tmem_base + Cfg::TM_S + (n % NS) * FA_BN;
+#pragma unroll
+        for (int ks = 0; ks < HD / 16; ++ks) {
+          const uint32_t off = (ks >> 2) * (FA_BM * 128) + (ks & 3) * 32;
+          umma_f16(s_tm, umma_smem_desc_sw128(k_addr + off, 16, 1024), umma_smem_desc_sw128(q_addr + off, 16, 1024), idesc_s, ks > 0 ? 1u : 0u);
+        }
+        umma_commit(&s_full[n % NS]);
+        if (last) umma_commit(kv_empty);
+      }
+      __syncwarp();
+      return true;
+    };
     for (int round = 0; round < n_rounds && ok; ++round) {
       const int item = item_of(round);
       if (item >= n_items) continue;
@@ -909,74 +963,102 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       decode(item, jb, h, b);
       const int n_it = nblk - (p.causal ? jb : 0);
       if (!warp_wait(kv_full, itc & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_FULL); break; }
-      for (int it = 0; it < n_it; ++it, ++qc) {
+      ok = issue_s(qc, n_it == 1);
+      // the previous item's dV / dK were read by the softmax warps before they produced this item's first P^T, dS^T
+      for (int it = 0; it < n_it && ok; ++it, ++qc) {
+        if (NS == 2 && it + 1 < n_it) { ok = issue_s(qc + 1, it + 2 == n_it); if (!ok) break; }
         const int st = qc % NST;
-        if (!warp_wait(&qdo_full[st], (qc / NST) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_FULL); ok = false; break; }
-        // S^T / dP^T may be overwritten once the softmax warps hold the previous tile in registers; when P^T / dS^T share
-        // those columns, only once the previous gradient products have consumed them
-        if (qc > 0 && !warp_wait(ALIAS ? pds_empty : s_empty, (qc - 1) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_TMEM_EMPTY); ok = false; break; }
-        tc_fence_after();
-        if (elect_one()) {
-          const uint32_t q_addr = smem_u32(smem + Cfg::OFF_Q + st * Cfg::T_BYTES);
-          const uint32_t do_addr = smem_u32(smem + Cfg::OFF_DO + st * Cfg::T_BYTES);
+        if (!warp_wait(&do_full[st], (qc / NST) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_FULL); ok = false; break; }
+        const uint32_t b_addr = smem_u32(smem + Cfg::OFF_DO + st * Cfg::T_BYTES);
+        const uint32_t a_addr = tmem_base + Cfg::TM_S + (qc % NS) * FA_BN;
+        for (int half = 0; half < 2; ++half) {
+          // an item's first product replaces the accumulator: wait until both halves' warps have read the previous item's
+          if (it == 0 && half == 0) ok = warp_wait(&p_full[(qc % NS) * 2 + 1], (qc / NS) & 1);
+          if (!ok || !warp_wait(&p_full[(qc % NS) * 2 + half], (qc / NS) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_SOFTMAX); ok = false; break; }
+          tc_fence_after();
+          if (elect_one()) {
 #pragma unroll
-          for (int ks = 0; ks < HD / 16; ++ks) {
-            const uint32_t off = (ks >> 2) * (FA_BM * 128) + (ks & 3) * 32;
-            umma_f16(tmem_base + Cfg::TM_S, umma_smem_desc_sw128(k_addr + off, 16, 1024),
-                     umma_smem_desc_sw128(q_addr + off, 16, 1024), idesc_s, ks > 0 ? 1u : 0u);
+            for (int ks = 0; ks < 4; ++ks)    // reduction over the 64 queries of this half
+              umma_f16_ts(tmem_base + Cfg::TM_DV, a_addr + half * 64 + ks * 8, umma_smem_desc_sw128(b_addr + (half * 4 + ks) * 2048, FA_BM * 128, 1024),
+                          idesc_g, (it > 0 || half > 0 || ks > 0) ? 1u : 0u);
+            if (half == 1) {
+              umma_commit(&do_empty[st]);
+              if (it + 1 == n_it) umma_commit(fin_full);
+            }
           }
-#pragma unroll
-          for (int ks = 0; ks < HD / 16; ++ks) {
-            const uint32_t off = (ks >> 2) * (FA_BM * 128) + (ks & 3) * 32;
-            umma_f16(tmem_base + Cfg::TM_DP, umma_smem_desc_sw128(v_addr + off, 16, 1024),
-                     umma_smem_desc_sw128(do_addr + off, 16, 1024), idesc_s, ks > 0 ? 1u : 0u);
-          }
-          umma_commit(s_full);
-          if (it + 1 == n_it) umma_commit(kv_empty);
+          __syncwarp();
         }
-        __syncwarp();
+        if (!ok) break;
+        if (NS == 1 && it + 1 < n_it) ok = issue_s(qc + 1, it + 2 == n_it);
       }
       ++itc;
     }
-  } else if (warp == 9 || warp == 10) {
-    // ------------- MMA issuers B (warp 9: dV += P^T dO) and C (warp 10: dK += dS^T Q), A operands from TMEM
-    constexpr uint32_t idesc_g = umma_idesc_bf16(FA_BN, HD, 0, 1);   // [keys x HD] += X^T[keys x q] (TMEM) * Y[q x HD]
-    const bool is_dv = warp == 9;
-    const uint32_t acc_addr = tmem_base + (is_dv ? Cfg::TM_DV : Cfg::TM_DK);
-    const uint32_t a_addr = tmem_base + (is_dv ? Cfg::TM_P : Cfg::TM_DS);
-    uint32_t qc = 0;
+  } else if (warp == 9) {
+    // ------------- MMA issuer B: dP^T = V dO^T and dK += dS^T Q.  dP^T of a tile goes over the dS^T that dK has read.
+    constexpr uint32_t idesc_s = umma_idesc_bf16(FA_BN, FA_BM, 0, 0);
+    constexpr uint32_t idesc_g = umma_idesc_bf16(FA_BN, HD, 0, 1);
+    const uint32_t v_addr = smem_u32(smem + Cfg::OFF_V);
+    const uint32_t dp_tm = tmem_base + Cfg::TM_DP;
+    uint32_t itc = 0, qc = 0;
     bool ok = true;
+    auto issue_dp = [&](uint32_t n, bool last) -> bool {
+      const int st = n % NST;
+      if (!warp_wait(&do_full[st], (n / NST) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_FULL); return false; }
+      tc_fence_after();
+      if (elect_one()) {
+        const uint32_t do_addr = smem_u32(smem + Cfg::OFF_DO + st * Cfg::T_BYTES);
+#pragma unroll
+        for (int ks = 0; ks < HD / 16; ++ks) {
+          const uint32_t off = (ks >> 2) * (FA_BM * 128) + (ks & 3) * 32;
+          umma_f16(dp_tm, umma_smem_desc_sw128(v_addr + off, 16, 1024), umma_smem_desc_sw128(do_addr + off, 16, 1024), idesc_s, ks > 0 ? 1u : 0u);
+        }
+        umma_commit(dp_full);
+        umma_commit(&do_empty[st]);
+        if (last) umma_commit(kv_empty);
+      }
+      __syncwarp();
+      return true;
+    };
     for (int round = 0; round < n_rounds && ok; ++round) {
       const int item = item_of(round);
       if (item >= n_items) continue;
       int jb, h, b;
       decode(item, jb, h, b);
       const int n_it = nblk - (p.causal ? jb : 0);
-      // the previous item's dV / dK were read by the softmax warps before they produced this item's first P^T, dS^T
-      for (int it = 0; it < n_it; ++it, ++qc) {
+      if (!warp_wait(kv_full, itc & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_FULL); break; }
+      ok = issue_dp(qc, n_it == 1);
+      for (int it = 0; it < n_it && ok; ++it, ++qc) {
         const int st = qc % NST;
-        if (!warp_wait(&qdo_full[st], (qc / NST) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_FULL); ok = false; break; }
-        if (!warp_wait(pds_full, qc & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_SOFTMAX); ok = false; break; }
-        tc_fence_after();
-        if (elect_one()) {
-          const uint32_t b_addr = smem_u32(smem + (is_dv ? Cfg::OFF_DO : Cfg::OFF_Q) + st * Cfg::T_BYTES);
+        if (!warp_wait(&q_full[st], (qc / NST) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_FULL); ok = false; break; }
+        const uint32_t b_addr = smem_u32(smem + Cfg::OFF_Q + st * Cfg::T_BYTES);
+        for (int half = 0; half < 2; ++half) {
+          if (it == 0 && half == 0) ok = warp_wait(&ds_full[1], qc & 1);   // as for dV
+          if (!ok || !warp_wait(&ds_full[half], qc & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_SOFTMAX); ok = false; break; }
+          tc_fence_after();
+          if (elect_one()) {
 #pragma unroll
-          for (int ks = 0; ks < FA_BM / 16; ++ks)    // reduction over the 128 queries of this block
-            umma_f16_ts(acc_addr, a_addr + ks * 8, umma_smem_desc_sw128(b_addr + ks * 2048, FA_BM * 128, 1024), idesc_g,
-                        (it > 0 || ks > 0) ? 1u : 0u);
-          umma_commit(&qdo_empty[st]);
-          umma_commit(pds_empty);
-          if (it + 1 == n_it) umma_commit(fin_full);
+            for (int ks = 0; ks < 4; ++ks)
+              umma_f16_ts(tmem_base + Cfg::TM_DK, dp_tm + half * 64 + ks * 8, umma_smem_desc_sw128(b_addr + (half * 4 + ks) * 2048, FA_BM * 128, 1024),
+                          idesc_g, (it > 0 || half > 0 || ks > 0) ? 1u : 0u);
+            if (half == 1) {
+              umma_commit(&q_empty[st]);
+              if (it + 1 == n_it) umma_commit(fin_full);
+            }
+          }
+          __syncwarp();
         }
-        __syncwarp();
+        if (!ok) break;
+        if (it + 1 < n_it) ok = issue_dp(qc + 1, it + 2 == n_it);
       }
+      ++itc;
     }
   } else {
     const int quad = warp & 3;
     const int half = warp >> 2;                  // this thread owns query columns [64*half, 64*half+64) of the tile
     const int r = quad * 32 + lane;              // key row inside the block = TMEM lane
-    const uint32_t t_lane = (uint32_t)(quad * 32) << 16;
-    const float sl2 = p.scale * LOG2E;
+    const uint32_t t_lane = tmem_base + ((uint32_t)(quad * 32) << 16);
+    const float sl2 = p.scale * LOG2E, scale = p.scale;
+    const unsigned long long sl22 = f2_of(__float_as_uint(sl2), __float_as_uint(sl2)), scale2 = f2_of(__float_as_uint(scale), __float_as_uint(scale));
     uint32_t itc = 0, qc = 0;
     bool ok = true;
     for (int round = 0; round < n_rounds && ok; ++round) {
@@ -986,69 +1068,63 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       decode(item, jb, h, b);
       const int i0 = p.causal ? jb : 0, n_it = nblk - i0, row0 = b * p.seq;
       for (int it = 0; it < n_it; ++it, ++qc) {
-        const int ib = i0 + it;
         const int st = qc % NST;
-        const float* st_cur = stat + st * 256;
-        ok = warp_wait(&qdo_full[st], (qc / NST) & 1);   // statistics of this block are staged
-        if (ok) ok = warp_wait(s_full, qc & 1);
+        const float* st_cur = stat + st * 256 + half * 64;
+        ok = warp_wait(&q_full[st], (qc / NST) & 1);   // statistics of this block are staged
+        if (ok) ok = warp_wait(&s_full[qc % NS], (qc / NS) & 1);
         if (!ok) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_TMEM_FULL); break; }
         tc_fence_after();
-        uint32_t s[64], dp[64];
-        tmem_ld32(tmem_base + t_lane + Cfg::TM_S + half * 64, s);
-        tmem_ld32(tmem_base + t_lane + Cfg::TM_S + half * 64 + 32, s + 32);
-        tmem_ld32(tmem_base + t_lane + Cfg::TM_DP + half * 64, dp);
-        tmem_ld32(tmem_base + t_lane + Cfg::TM_DP + half * 64 + 32, dp + 32);
+        const uint32_t s_addr = t_lane + Cfg::TM_S + (qc % NS) * FA_BN + half * 64;
+        const uint32_t dp_addr = t_lane + Cfg::TM_DP + half * 64;
+        uint32_t s[64];
+        tmem_ld32(s_addr, s);
+        tmem_ld32(s_addr + 32, s + 32);
         tmem_ld_wait();
-        if (ALIAS) {
-          pair_sync(quad);                         // both threads of the lane hold their columns before either overwrites them
-        } else {
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(s_empty);     // the next tile's score products may overwrite S^T, dP^T now
-        }
-        const float4* nl4 = reinterpret_cast<const float4*>(st_cur + half * 64);
-        const float4* nd4 = reinterpret_cast<const float4*>(st_cur + 128 + half * 64);
-        const bool diag = p.causal && ib == jb;    // alive iff key <= query: column >= row
+        const ulonglong2* nl4 = reinterpret_cast<const ulonglong2*>(st_cur);
+        const ulonglong2* nd4 = reinterpret_cast<const ulonglong2*>(st_cur + 128);
+        const bool diag = p.causal && it == 0;     // alive iff key <= query: column >= row
         const int first = r - half * 64;           // first alive column of this thread on the diagonal tile
-        uint32_t pw[32], dw[32];
-        if (diag) {
 #pragma unroll
-          for (int i = 0; i < 64; i += 4) {
-            const float4 nl = nl4[i >> 2], nd = nd4[i >> 2];
-            const float p0 = (i >= first) ? fast_exp2(fmaf(__uint_as_float(s[i]), sl2, nl.x)) : 0.f;
-            const float p1 = (i + 1 >= first) ? fast_exp2(fmaf(__uint_as_float(s[i + 1]), sl2, nl.y)) : 0.f;
-            const float p2 = (i + 2 >= first) ? fast_exp2(fmaf(__uint_as_float(s[i + 2]), sl2, nl.z)) : 0.f;
-            const float p3 = (i + 3 >= first) ? fast_exp2(fmaf(__uint_as_float(s[i + 3]), sl2, nl.w)) : 0.f;
-            pw[i >> 1] = pack_bf16x2(p0, p1);
-            pw[(i >> 1) + 1] = pack_bf16x2(p2, p3);
-            dw[i >> 1] = pack_bf16x2(p0 * fmaf(__uint_as_float(dp[i]), p.scale, nd.x), p1 * fmaf(__uint_as_float(dp[i + 1]), p.scale, nd.y));
-            dw[(i >> 1) + 1] = pack_bf16x2(p2 * fmaf(__uint_as_float(dp[i + 2]), p.scale, nd.z), p3 * fmaf(__uint_as_float(dp[i + 3]), p.scale, nd.w));
-          }
-        } else {
+        for (int c = 0; c < 2; ++c) {
 #pragma unroll
-          for (int i = 0; i < 64; i += 4) {
-            const float4 nl = nl4[i >> 2], nd = nd4[i >> 2];
-            const float p0 = fast_exp2(fmaf(__uint_as_float(s[i]), sl2, nl.x));
-            const float p1 = fast_exp2(fmaf(__uint_as_float(s[i + 1]), sl2, nl.y));
-            const float p2 = fast_exp2(fmaf(__uint_as_float(s[i + 2]), sl2, nl.z));
-            const float p3 = fast_exp2(fmaf(__uint_as_float(s[i + 3]), sl2, nl.w));
-            pw[i >> 1] = pack_bf16x2(p0, p1);
-            pw[(i >> 1) + 1] = pack_bf16x2(p2, p3);
-            dw[i >> 1] = pack_bf16x2(p0 * fmaf(__uint_as_float(dp[i]), p.scale, nd.x), p1 * fmaf(__uint_as_float(dp[i + 1]), p.scale, nd.y));
-            dw[(i >> 1) + 1] = pack_bf16x2(p2 * fmaf(__uint_as_float(dp[i + 2]), p.scale, nd.z), p3 * fmaf(__uint_as_float(dp[i + 3]), p.scale, nd.w));
+          for (int i = 0; i < 32; i += 4) {
+            const ulonglong2 nl = nl4[c * 8 + (i >> 2)];
+            uint32_t* sc = s + c * 32 + i;
+            bwd_prob2(sc[0], sc[1], sl22, nl.x);
+            bwd_prob2(sc[2], sc[3], sl22, nl.y);
           }
+          if (diag) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) s[c * 32 + i] = (c * 32 + i >= first) ? s[c * 32 + i] : 0u;
+          }
+          bwd_store16(s_addr + c * 16, s + c * 32);
         }
-        if (!ALIAS && qc > 0) {                     // the previous tile's gradient products still read P^T, dS^T
-          ok = warp_wait(pds_empty, (qc - 1) & 1);
-          if (!ok) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_EMPTY); break; }
-          tc_fence_after();
-        }
-        tmem_st32(tmem_base + t_lane + Cfg::TM_P + half * 32, pw);
-        tmem_st32(tmem_base + t_lane + Cfg::TM_DS + half * 32, dw);
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(pds_full);
+        if (lane == 0) mbar_arrive(&p_full[(qc % NS) * 2 + half]);
+        ok = warp_wait(dp_full, qc & 1);
+        if (!ok) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_TMEM_FULL); break; }
+        tc_fence_after();
+        uint32_t dp[64];
+        tmem_ld32(dp_addr, dp);
+        tmem_ld32(dp_addr + 32, dp + 32);
+        tmem_ld_wait();
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+#pragma unroll
+          for (int i = 0; i < 32; i += 4) {
+            const ulonglong2 nd = nd4[c * 8 + (i >> 2)];
+            uint32_t *sc = s + c * 32 + i, *dc = dp + c * 32 + i;
+            bwd_ds2(sc[0], sc[1], dc[0], dc[1], scale2, nd.x);
+            bwd_ds2(sc[2], sc[3], dc[2], dc[3], scale2, nd.y);
+          }
+          bwd_store16(dp_addr + c * 16, s + c * 32);
+        }
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&ds_full[half]);
       }
       if (!ok) break;
       ok = warp_wait(fin_full, itc & 1);
@@ -1064,7 +1140,7 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         for (int cc = 0; cc < HD / 64; ++cc) {
           const int c = half * (HD / 64) + cc;
           uint32_t a[32];
-          tmem_ld32(tmem_base + t_lane + tcol + c * 32, a);
+          tmem_ld32(t_lane + tcol + c * 32, a);
           tmem_ld_wait();
           if (kj < p.seq) {
 #pragma unroll
@@ -1077,7 +1153,7 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           }
         }
       }
-      tc_fence_before();   // dV / dK are read before this warp's next pds_full arrival lets the next item's products overwrite them
+      tc_fence_before();   // dV / dK are read before this warp's next p_full / ds_full arrivals let the next item's products overwrite them
     }
   }
   pdl_launch_dependents();
@@ -1088,39 +1164,42 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 
 template <int HD>
 struct BwdQCfg {
-  static constexpr int NST = (HD == 64) ? 3 : 2;       // K / V ring
+  static constexpr int NK = (HD == 64) ? 4 : 3;        // K ring: a tile is held from its scores to dQ
+  static constexpr int NV = (HD == 64) ? 3 : 2;        // V ring: held for dP only
   static constexpr int T_BYTES = FA_BM * HD * 2;
   static constexpr int OFF_Q = 0;
   static constexpr int OFF_DO = OFF_Q + T_BYTES;
   static constexpr int OFF_K = OFF_DO + T_BYTES;
-  static constexpr int OFF_V = OFF_K + NST * T_BYTES;
-  static constexpr int OFF_BAR = OFF_V + NST * T_BYTES;
-  static constexpr int SMEM_BYTES = OFF_BAR + 128;
+  static constexpr int OFF_V = OFF_K + NK * T_BYTES;
+  static constexpr int OFF_BAR = OFF_V + NV * T_BYTES;
+  static constexpr int SMEM_BYTES = OFF_BAR + 208;
   static constexpr int TMEM_COLS = 512;
-  static constexpr int TM_S = 0, TM_DP = 128, TM_DS = 256, TM_DQ = 320;
+  static constexpr int TM_S = 0, TM_DP = 256, TM_DQ = 384;   // two score buffers; dS over dP
 };
 
 // Persistent, like the dK / dV kernel: items are (query block, head, batch), heaviest causal query blocks first; dQ of an item
-// accumulates in TMEM over its key blocks.
+// accumulates in TMEM over its key blocks.  P is needed in registers only, so a score buffer is free once it has been read.
 template <int HD>
 __global__ void __launch_bounds__(FA_BWD_THREADS, 1)
 flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                    const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
                    const FlashBwdParams p) {
   using Cfg = BwdQCfg<HD>;
-  constexpr int NST = Cfg::NST;
+  constexpr int NK = Cfg::NK, NV = Cfg::NV;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::OFF_BAR);
   uint64_t* q_full = bars + 0;
-  uint64_t* q_empty = bars + 1;    // the item's last score products have read Q, dO
-  uint64_t* kv_full = bars + 2;    // [3]
-  uint64_t* kv_empty = bars + 5;   // [3]
-  uint64_t* s_full = bars + 8;
-  uint64_t* s_empty = bars + 9;
-  uint64_t* ds_full = bars + 10;
-  uint64_t* ds_empty = bars + 11;
-  uint64_t* fin_full = bars + 12;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 13);
+  uint64_t* q_empty = bars + 1;    // the item's last score and dP products have read Q, dO
+  uint64_t* k_full = bars + 2;     // [4]
+  uint64_t* k_empty = bars + 6;    // [4]  dQ has read K
+  uint64_t* v_full = bars + 10;    // [3]
+  uint64_t* v_empty = bars + 13;   // [3]
+  uint64_t* s_full = bars + 16;    // [2]
+  uint64_t* s_empty = bars + 18;   // [2]  (8 warps)
+  uint64_t* dp_full = bars + 20;
+  uint64_t* ds_full = bars + 21;   // [2]  by column half (4 warps each)
+  uint64_t* fin_full = bars + 23;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 24);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nblk = (p.seq + FA_BM - 1) / FA_BM;
@@ -1144,12 +1223,11 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV); tma_prefetch_desc(&tmDO);
     mbar_init(q_full, 1);
-    mbar_init(q_empty, 1);
-    for (int s = 0; s < NST; ++s) { mbar_init(&kv_full[s], 1); mbar_init(&kv_empty[s], 1); }
-    mbar_init(s_full, 1);
-    mbar_init(s_empty, 8);
-    mbar_init(ds_full, 8);
-    mbar_init(ds_empty, 1);
+    mbar_init(q_empty, 2);
+    for (int s = 0; s < NK; ++s) { mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1); }
+    for (int s = 0; s < NV; ++s) { mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1); }
+    for (int s = 0; s < 2; ++s) { mbar_init(&s_full[s], 1); mbar_init(&s_empty[s], 8); mbar_init(&ds_full[s], 4); }
+    mbar_init(dp_full, 1);
     mbar_init(fin_full, 1);
     mbar_fence_init();
   }
@@ -1179,25 +1257,29 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         }
       }
       for (int j = 0; j < n_kv; ++j, ++kc) {
-        const int st = kc % NST;
-        const uint32_t ph = (kc / NST) & 1;
-        if (!warp_wait(&kv_empty[st], ph ^ 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_EMPTY); ok = false; break; }
+        const int sk = kc % NK, sv = kc % NV;
+        if (!warp_wait(&k_empty[sk], ((kc / NK) & 1) ^ 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_EMPTY); ok = false; break; }
         if (elect_one()) {
-          mbar_expect_tx(&kv_full[st], 2 * Cfg::T_BYTES);
+          mbar_expect_tx(&k_full[sk], Cfg::T_BYTES);
 #pragma unroll
-          for (int x = 0; x < HD / 64; ++x) {
-            tma_load_2d(smem + Cfg::OFF_K + st * Cfg::T_BYTES + x * (FA_BN * 128), &tmK, &kv_full[st], h * HD + x * 64, row0 + j * FA_BN);
-            tma_load_2d(smem + Cfg::OFF_V + st * Cfg::T_BYTES + x * (FA_BN * 128), &tmV, &kv_full[st], h * HD + x * 64, row0 + j * FA_BN);
-          }
+          for (int x = 0; x < HD / 64; ++x)
+            tma_load_2d(smem + Cfg::OFF_K + sk * Cfg::T_BYTES + x * (FA_BN * 128), &tmK, &k_full[sk], h * HD + x * 64, row0 + j * FA_BN);
+        }
+        if (!warp_wait(&v_empty[sv], ((kc / NV) & 1) ^ 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_EMPTY); ok = false; break; }
+        if (elect_one()) {
+          mbar_expect_tx(&v_full[sv], Cfg::T_BYTES);
+#pragma unroll
+          for (int x = 0; x < HD / 64; ++x)
+            tma_load_2d(smem + Cfg::OFF_V + sv * Cfg::T_BYTES + x * (FA_BN * 128), &tmV, &v_full[sv], h * HD + x * 64, row0 + j * FA_BN);
         }
         __syncwarp();
       }
       ++itc;
     }
   } else if (warp == 8) {
-    // ------------- MMA issuer A: S = Q K_j^T, dP = dO V_j^T
+    // ------------- MMA issuer A: S = Q K_j^T
     constexpr uint32_t idesc_s = umma_idesc_bf16(FA_BM, FA_BN, 0, 0);
-    const uint32_t q_addr = smem_u32(smem + Cfg::OFF_Q), do_addr = smem_u32(smem + Cfg::OFF_DO);
+    const uint32_t q_addr = smem_u32(smem + Cfg::OFF_Q);
     uint32_t itc = 0, kc = 0;
     bool ok = true;
     for (int round = 0; round < n_rounds && ok; ++round) {
@@ -1208,26 +1290,19 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       const int n_kv = p.causal ? (ib + 1) : nblk;
       if (!warp_wait(q_full, itc & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_FULL); break; }
       for (int j = 0; j < n_kv; ++j, ++kc) {
-        const int st = kc % NST;
-        if (!warp_wait(&kv_full[st], (kc / NST) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_FULL); ok = false; break; }
-        if (kc > 0 && !warp_wait(s_empty, (kc - 1) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_TMEM_EMPTY); ok = false; break; }
+        const int st = kc % NK;
+        if (!warp_wait(&k_full[st], (kc / NK) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_FULL); ok = false; break; }
+        if (kc > 1 && !warp_wait(&s_empty[kc & 1], ((kc >> 1) - 1) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_TMEM_EMPTY); ok = false; break; }
         tc_fence_after();
         if (elect_one()) {
           const uint32_t k_addr = smem_u32(smem + Cfg::OFF_K + st * Cfg::T_BYTES);
-          const uint32_t v_addr = smem_u32(smem + Cfg::OFF_V + st * Cfg::T_BYTES);
 #pragma unroll
           for (int ks = 0; ks < HD / 16; ++ks) {
             const uint32_t off = (ks >> 2) * (FA_BM * 128) + (ks & 3) * 32;
-            umma_f16(tmem_base + Cfg::TM_S, umma_smem_desc_sw128(q_addr + off, 16, 1024),
+            umma_f16(tmem_base + Cfg::TM_S + (kc & 1) * FA_BN, umma_smem_desc_sw128(q_addr + off, 16, 1024),
                      umma_smem_desc_sw128(k_addr + off, 16, 1024), idesc_s, ks > 0 ? 1u : 0u);
           }
-#pragma unroll
-          for (int ks = 0; ks < HD / 16; ++ks) {
-            const uint32_t off = (ks >> 2) * (FA_BM * 128) + (ks & 3) * 32;
-            umma_f16(tmem_base + Cfg::TM_DP, umma_smem_desc_sw128(do_addr + off, 16, 1024),
-                     umma_smem_desc_sw128(v_addr + off, 16, 1024), idesc_s, ks > 0 ? 1u : 0u);
-          }
-          umma_commit(s_full);
+          umma_commit(&s_full[kc & 1]);
           if (j + 1 == n_kv) umma_commit(q_empty);
         }
         __syncwarp();
@@ -1235,40 +1310,72 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       ++itc;
     }
   } else if (warp == 9) {
-    // ------------- MMA issuer B: dQ += dS K_j (dS from TMEM)
+    // ------------- MMA issuer B: dP = dO V_j^T and dQ += dS K_j (dS from TMEM, over dP)
+    constexpr uint32_t idesc_s = umma_idesc_bf16(FA_BM, FA_BN, 0, 0);
     constexpr uint32_t idesc_q = umma_idesc_bf16(FA_BM, HD, 0, 1);   // dQ[q x HD] += dS[q x keys] * K[keys x HD]
-    uint32_t kc = 0;
+    const uint32_t do_addr = smem_u32(smem + Cfg::OFF_DO);
+    const uint32_t dp_tm = tmem_base + Cfg::TM_DP;
+    uint32_t itc = 0, kc = 0;
     bool ok = true;
+    auto issue_dp = [&](uint32_t n, bool last) -> bool {
+      const int st = n % NV;
+      if (!warp_wait(&v_full[st], (n / NV) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_FULL); return false; }
+      tc_fence_after();
+      if (elect_one()) {
+        const uint32_t v_addr = smem_u32(smem + Cfg::OFF_V + st * Cfg::T_BYTES);
+#pragma unroll
+        for (int ks = 0; ks < HD / 16; ++ks) {
+          const uint32_t off = (ks >> 2) * (FA_BM * 128) + (ks & 3) * 32;
+          umma_f16(dp_tm, umma_smem_desc_sw128(do_addr + off, 16, 1024), umma_smem_desc_sw128(v_addr + off, 16, 1024), idesc_s, ks > 0 ? 1u : 0u);
+        }
+        umma_commit(dp_full);
+        umma_commit(&v_empty[st]);
+        if (last) umma_commit(q_empty);
+      }
+      __syncwarp();
+      return true;
+    };
     for (int round = 0; round < n_rounds && ok; ++round) {
       const int item = item_of(round);
       if (item >= n_items) continue;
       int ib, h, b;
       decode(item, ib, h, b);
       const int n_kv = p.causal ? (ib + 1) : nblk;
-      for (int j = 0; j < n_kv; ++j, ++kc) {
-        const int st = kc % NST;
-        if (!warp_wait(&kv_full[st], (kc / NST) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_FULL); ok = false; break; }
-        if (!warp_wait(ds_full, kc & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_SOFTMAX); ok = false; break; }
-        tc_fence_after();
-        if (elect_one()) {
-          const uint32_t k_addr = smem_u32(smem + Cfg::OFF_K + st * Cfg::T_BYTES);
+      if (!warp_wait(q_full, itc & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_FULL); break; }
+      ok = issue_dp(kc, n_kv == 1);
+      for (int j = 0; j < n_kv && ok; ++j, ++kc) {
+        const int st = kc % NK;
+        if (!warp_wait(&k_full[st], (kc / NK) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_FULL); ok = false; break; }
+        const uint32_t k_addr = smem_u32(smem + Cfg::OFF_K + st * Cfg::T_BYTES);
+        for (int half = 0; half < 2; ++half) {
+          // an item's first product replaces the accumulator: wait until both halves' warps have read the previous item's
+          if (j == 0 && half == 0) ok = warp_wait(&ds_full[1], kc & 1);
+          if (!ok || !warp_wait(&ds_full[half], kc & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_SOFTMAX); ok = false; break; }
+          tc_fence_after();
+          if (elect_one()) {
 #pragma unroll
-          for (int ks = 0; ks < FA_BN / 16; ++ks)
-            umma_f16_ts(tmem_base + Cfg::TM_DQ, tmem_base + Cfg::TM_DS + ks * 8,
-                        umma_smem_desc_sw128(k_addr + ks * 2048, FA_BN * 128, 1024), idesc_q, (j > 0 || ks > 0) ? 1u : 0u);
-          umma_commit(&kv_empty[st]);
-          umma_commit(ds_empty);
-          if (j + 1 == n_kv) umma_commit(fin_full);
+            for (int ks = 0; ks < 4; ++ks)
+              umma_f16_ts(tmem_base + Cfg::TM_DQ, dp_tm + half * 64 + ks * 8, umma_smem_desc_sw128(k_addr + (half * 4 + ks) * 2048, FA_BN * 128, 1024),
+                          idesc_q, (j > 0 || half > 0 || ks > 0) ? 1u : 0u);
+            if (half == 1) {
+              umma_commit(&k_empty[st]);
+              if (j + 1 == n_kv) umma_commit(fin_full);
+            }
+          }
+          __syncwarp();
         }
-        __syncwarp();
+        if (!ok) break;
+        if (j + 1 < n_kv) ok = issue_dp(kc + 1, j + 2 == n_kv);
       }
+      ++itc;
     }
   } else if (warp < 8) {
     const int quad = warp & 3;
     const int half = warp >> 2;
     const int r = quad * 32 + lane;
-    const uint32_t t_lane = (uint32_t)(quad * 32) << 16;
-    const float sl2 = p.scale * LOG2E;
+    const uint32_t t_lane = tmem_base + ((uint32_t)(quad * 32) << 16);
+    const float sl2 = p.scale * LOG2E, scale = p.scale;
+    const unsigned long long sl22 = f2_of(__float_as_uint(sl2), __float_as_uint(sl2)), scale2 = f2_of(__float_as_uint(scale), __float_as_uint(scale));
     uint32_t itc = 0, kc = 0;
     bool ok = true;
     for (int round = 0; round < n_rounds && ok; ++round) {
@@ -1280,51 +1387,48 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       const long long stat_base = ((long long)b * p.heads + h) * p.seq;
       const int qi = ib * FA_BM + r;
       const bool q_ok = qi < p.seq;
-      const float lse2 = q_ok ? p.lse[stat_base + qi] * LOG2E : INFINITY;
-      const float dlt = q_ok ? p.delta[stat_base + qi] : 0.f;
-      const float nlse = -lse2, ndlt = -dlt * p.scale;
+      const float nlse = q_ok ? -p.lse[stat_base + qi] * LOG2E : -INFINITY;
+      const float ndlt = q_ok ? -p.delta[stat_base + qi] * scale : 0.f;
+      const unsigned long long nlse2 = f2_of(__float_as_uint(nlse), __float_as_uint(nlse)), ndlt2 = f2_of(__float_as_uint(ndlt), __float_as_uint(ndlt));
       for (int j = 0; j < n_kv; ++j, ++kc) {
-        ok = warp_wait(s_full, kc & 1);
+        ok = warp_wait(&s_full[kc & 1], (kc >> 1) & 1);
         if (!ok) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_TMEM_FULL); break; }
         tc_fence_after();
-        uint32_t s[64], dp[64];
-        tmem_ld32(tmem_base + t_lane + Cfg::TM_S + half * 64, s);
-        tmem_ld32(tmem_base + t_lane + Cfg::TM_S + half * 64 + 32, s + 32);
-        tmem_ld32(tmem_base + t_lane + Cfg::TM_DP + half * 64, dp);
-        tmem_ld32(tmem_base + t_lane + Cfg::TM_DP + half * 64 + 32, dp + 32);
+        const uint32_t s_addr = t_lane + Cfg::TM_S + (kc & 1) * FA_BN + half * 64;
+        const uint32_t dp_addr = t_lane + Cfg::TM_DP + half * 64;
+        uint32_t s[64];
+        tmem_ld32(s_addr, s);
+        tmem_ld32(s_addr + 32, s + 32);
         tmem_ld_wait();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(s_empty);
+        if (lane == 0) mbar_arrive(&s_empty[kc & 1]);
         const int k0 = j * FA_BN;
         const bool need_mask = (p.causal && j == ib) || (k0 + FA_BN > p.seq) || !q_ok;
-        uint32_t dw[32];
+#pragma unroll
+        for (int i = 0; i < 64; i += 2) bwd_prob2(s[i], s[i + 1], sl22, nlse2);
         if (need_mask) {
           const int lim = q_ok ? (min(p.causal ? qi : 0x7fffffff, p.seq - 1) - (k0 + half * 64)) : -1;
 #pragma unroll
-          for (int i = 0; i < 64; i += 2) {
-            const float p0 = (i <= lim) ? fast_exp2(fmaf(__uint_as_float(s[i]), sl2, nlse)) : 0.f;
-            const float p1 = (i + 1 <= lim) ? fast_exp2(fmaf(__uint_as_float(s[i + 1]), sl2, nlse)) : 0.f;
-            dw[i >> 1] = pack_bf16x2(p0 * fmaf(__uint_as_float(dp[i]), p.scale, ndlt), p1 * fmaf(__uint_as_float(dp[i + 1]), p.scale, ndlt));
-          }
-        } else {
+          for (int i = 0; i < 64; ++i) s[i] = (i <= lim) ? s[i] : 0u;
+        }
+        ok = warp_wait(dp_full, kc & 1);
+        if (!ok) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_TMEM_FULL); break; }
+        tc_fence_after();
+        uint32_t dp[64];
+        tmem_ld32(dp_addr, dp);
+        tmem_ld32(dp_addr + 32, dp + 32);
+        tmem_ld_wait();
 #pragma unroll
-          for (int i = 0; i < 64; i += 2) {
-            const float p0 = fast_exp2(fmaf(__uint_as_float(s[i]), sl2, nlse));
-            const float p1 = fast_exp2(fmaf(__uint_as_float(s[i + 1]), sl2, nlse));
-            dw[i >> 1] = pack_bf16x2(p0 * fmaf(__uint_as_float(dp[i]), p.scale, ndlt), p1 * fmaf(__uint_as_float(dp[i + 1]), p.scale, ndlt));
-          }
+        for (int c = 0; c < 2; ++c) {
+#pragma unroll
+          for (int i = c * 32; i < c * 32 + 32; i += 2) bwd_ds2(s[i], s[i + 1], dp[i], dp[i + 1], scale2, ndlt2);
+          bwd_store16(dp_addr + c * 16, s + c * 32);
         }
-        if (kc > 0) {
-          ok = warp_wait(ds_empty, (kc - 1) & 1);
-          if (!ok) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_EMPTY); break; }
-          tc_fence_after();
-        }
-        tmem_st32(tmem_base + t_lane + Cfg::TM_DS + half * 32, dw);
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(ds_full);
+        if (lane == 0) mbar_arrive(&ds_full[half]);
       }
       if (!ok) break;
       ok = warp_wait(fin_full, itc & 1);
@@ -1336,7 +1440,7 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       for (int cc = 0; cc < HD / 64; ++cc) {
         const int c = half * (HD / 64) + cc;
         uint32_t a[32];
-        tmem_ld32(tmem_base + t_lane + Cfg::TM_DQ + c * 32, a);
+        tmem_ld32(t_lane + Cfg::TM_DQ + c * 32, a);
         tmem_ld_wait();
         if (q_ok) {
 #pragma unroll
