@@ -40,6 +40,11 @@ int oa_gemm_bf16(const void* A, const void* B, void* out, int M, int N, int K, i
                  int b_mn, const void* bias, const void* residual, int ldr, void* aux_out, const void* aux_in,
                  int ldaux, int act, int out_f32, int accumulate, float alpha, void* workspace,
                  size_t workspace_bytes, int force_bn, int* status, void* stream);
+// y = act(alpha x W^T + bias) + residual for at most 64 rows of x; OA_ERR_UNSUPPORTED where oa_gemm_bf16 takes a tile kernel.
+// w_at_rest: nothing still in flight on the stream writes W.
+int oa_gemm_bf16_few_rows(const void* x, const void* w, void* out, int M, int N, int K, int ldx, int ldw, int ldc,
+                          const void* bias, const void* residual, int ldr, int act, int out_f32, float alpha, int w_at_rest,
+                          int* status, void* stream);
 // `batch` independent problems of one shape; s*_batch are element strides between problems (sbias_batch may be 0).
 int oa_gemm_bf16_batched(const void* A, const void* B, void* out, int M, int N, int K, int lda, int ldb, int ldc, int a_mn,
                          int b_mn, const void* bias, const void* residual, int ldr, void* aux_out, const void* aux_in,

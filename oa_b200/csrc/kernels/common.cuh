@@ -182,7 +182,7 @@ inline bool pdl_enabled() {
 }
 // Only for kernels that call pdl_wait() before their first global access.
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
+inline cudaError_t launch_pdl_if(bool on, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -192,8 +192,22 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = pdl_enabled() ? 1 : 0;
+  cfg.numAttrs = on ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
+  return launch_pdl_if(pdl_enabled(), kernel, grid, block, smem, st, static_cast<KArgs>(args)...);
+}
+// Kernels of a few microseconds, which follow one another in a decoding step or in the step of a small model: there the start of a
+// launch (1 to 2 us from its predecessor's last store to its own first load) is a good part of the time, and with the trigger at the
+// kernel's start it runs under the predecessor.  Up to PDL_SHORT_BLOCKS blocks, where all of them are resident at once or nearly so;
+// for grids of many waves the flag bought nothing (above).
+constexpr long long PDL_SHORT_BLOCKS = 1024;
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_short(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
+  const bool few = (long long)grid.x * grid.y * grid.z <= PDL_SHORT_BLOCKS;
+  return launch_pdl_if(few || pdl_enabled(), kernel, grid, block, smem, st, static_cast<KArgs>(args)...);
 }
 
 // ---------------------------------------------------------------- proxies / fences

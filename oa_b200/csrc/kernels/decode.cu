@@ -13,6 +13,8 @@ namespace oa {
 __global__ void kv_append_kernel(const __nv_bfloat16* __restrict__ k_src, const __nv_bfloat16* __restrict__ v_src, long long src_stride,
                                  __nv_bfloat16* __restrict__ kc, __nv_bfloat16* __restrict__ vc, int batch, int s_new, int heads, int hd,
                                  int pos0, int max_seq, const int* __restrict__ pos_dev) {
+  pdl_launch_dependents();
+  pdl_wait();
   // one thread per 8 elements of one (token, head) row; pos_dev (optional) adds a device-resident offset so that a decode
   // step captured in a CUDA graph advances without host-side parameters
   if (pos_dev) pos0 += *pos_dev;
@@ -37,6 +39,8 @@ __global__ void __launch_bounds__(128)
 decode_attn_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride, const __nv_bfloat16* __restrict__ kc,
                    const __nv_bfloat16* __restrict__ vc, __nv_bfloat16* __restrict__ out, long long out_stride, int heads, int len,
                    int max_seq, float scale_log2, const int* __restrict__ pos_dev) {
+  pdl_launch_dependents();
+  pdl_wait();
   if (pos_dev) len = min(len + *pos_dev, max_seq);
   constexpr int PER = HD / 32;                  // head-dim elements per lane in the p.v phase
   __shared__ float s_q[HD];
@@ -146,16 +150,18 @@ decode_attn_stream_kernel(const __nv_bfloat16* __restrict__ q, long long q_strid
   __shared__ float s_m[4], s_l[4];
   __shared__ float s_acc[4][HD];
   __shared__ int s_fail;
-  if (pos_dev) len = min(len + *pos_dev, max_seq);
+  pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_items = n_bh * splits;
-  const int per = (((len + splits - 1) / splits + TILE - 1) / TILE) * TILE;     // positions per split, whole tiles
   if (threadIdx.x == 0) {
     for (int i = 0; i < DA_STAGES; ++i) { mbar_init(&full_bar[i], 1); mbar_init(&empty_bar[i], 4); }
     mbar_fence_init();
     s_fail = 0;
   }
   __syncthreads();
+  pdl_wait();
+  if (pos_dev) len = min(len + *pos_dev, max_seq);
+  const int per = (((len + splits - 1) / splits + TILE - 1) / TILE) * TILE;     // positions per split, whole tiles
   unsigned char* tiles = da_smem;
 
   if (warp == 4) {
@@ -273,6 +279,8 @@ decode_attn_stream_kernel(const __nv_bfloat16* __restrict__ q, long long q_strid
 template <int HD>
 __global__ void decode_merge_kernel(const float* __restrict__ partial, __nv_bfloat16* __restrict__ out, long long out_stride, int heads,
                                     int splits) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int bh = blockIdx.x, b = bh / heads, h = bh - b * heads, d = threadIdx.x;
   const float* src = partial + (long long)bh * splits * (HD + 2);
   float M = -INFINITY;
@@ -299,9 +307,8 @@ extern "C" int oa_kv_append(const void* k_src, const void* v_src, long long src_
   const long long total = (long long)batch * s_new * heads * (head_dim / 8);
   const int threads = 256;
   const int blocks = (int)((total + threads - 1) / threads < 148 * 16 ? (total + threads - 1) / threads : 148 * 16);
-  kv_append_kernel<<<blocks, threads, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)k_src, (const __nv_bfloat16*)v_src, src_stride,
-                                                                 (__nv_bfloat16*)k_cache, (__nv_bfloat16*)v_cache, batch, s_new, heads,
-                                                                 head_dim, pos0, max_seq, pos_dev);
+  launch_short(kv_append_kernel, dim3(blocks), dim3(threads), 0, (cudaStream_t)stream, (const __nv_bfloat16*)k_src, (const __nv_bfloat16*)v_src,
+               src_stride, (__nv_bfloat16*)k_cache, (__nv_bfloat16*)v_cache, batch, s_new, heads, head_dim, pos0, max_seq, pos_dev);
   return cudaGetLastError() == cudaSuccess ? OA_OK : OA_ERR_LAUNCH;
 }
 
@@ -340,9 +347,9 @@ static int launch_decode_stream(const void* q, long long q_stride, const void* k
   }
   const int n_bh = batch * heads, items = n_bh * splits;
   const int grid = items < 2 * 148 ? items : 2 * 148;
-  decode_attn_stream_kernel<HD><<<grid, 160, smem, st>>>((const __nv_bfloat16*)q, q_stride, (const __nv_bfloat16*)kc, (const __nv_bfloat16*)vc,
-                                                         (float*)partial, heads, n_bh, splits, len, max_seq, sl2, pos_dev, status);
-  decode_merge_kernel<HD><<<n_bh, HD, 0, st>>>((const float*)partial, (__nv_bfloat16*)out, out_stride, heads, splits);
+  launch_short(decode_attn_stream_kernel<HD>, dim3(grid), dim3(160), smem, st, (const __nv_bfloat16*)q, q_stride, (const __nv_bfloat16*)kc,
+               (const __nv_bfloat16*)vc, (float*)partial, heads, n_bh, splits, len, max_seq, sl2, pos_dev, status);
+  launch_short(decode_merge_kernel<HD>, dim3(n_bh), dim3(HD), 0, st, (const float*)partial, (__nv_bfloat16*)out, out_stride, heads, splits);
   return cudaGetLastError() == cudaSuccess ? OA_OK : OA_ERR_LAUNCH;
 }
 

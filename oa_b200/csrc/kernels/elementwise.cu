@@ -175,6 +175,8 @@ __global__ void fill_vec_kernel(uint4* y, long long n16, uint4 pattern) {
 // I: 32-bit indices unless there are 2^31 vectors; the 64-bit division by the row length was most of the instructions.
 template <typename T, typename I>
 __global__ void swiglu_fwd_kernel(const T* __restrict__ gu, T* __restrict__ out, long long rows, int F) {
+  pdl_launch_dependents();
+  pdl_wait();
   constexpr int V = IO<T>::VEC;
   const I per_row = F / V, total = (I)rows * per_row, stride = (I)gridDim.x * blockDim.x;
   for (I i = (I)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -299,6 +301,8 @@ rope_bf16_vec_kernel(__nv_bfloat16* x, long long rows, int row_stride, int n_hea
 template <typename T>
 __global__ void embedding_fwd_kernel(const T* __restrict__ table, const int* __restrict__ ids, T* __restrict__ out,
                                      long long n_ids, int dim, int vocab, const T* __restrict__ pos, int seq_len) {
+  pdl_launch_dependents();
+  pdl_wait();
   constexpr int V = IO<T>::VEC;
   int per_row = dim / V;
   long long total = n_ids * per_row;
@@ -653,9 +657,9 @@ extern "C" int oa_fill(int dtype, void* y, long long n, float value, void* strea
 extern "C" int oa_swiglu_fwd(int dtype, const void* gu, void* out, long long rows, int F, void* stream) {
   if (F % 8) return OA_ERR_ALIGN;
   if (rows * F / 4 < 0x70000000LL) {
-    DISPATCH_T(dtype, swiglu_fwd_kernel<T, unsigned><<<grid_for(rows * F / IO<T>::VEC, 256), 256, 0, ST>>>((const T*)gu, (T*)out, rows, F));
+    DISPATCH_T(dtype, launch_short(swiglu_fwd_kernel<T, unsigned>, dim3(grid_for(rows * F / IO<T>::VEC, 256)), dim3(256), 0, ST, (const T*)gu, (T*)out, rows, F));
   } else {
-    DISPATCH_T(dtype, swiglu_fwd_kernel<T, long long><<<grid_for(rows * F / IO<T>::VEC, 256), 256, 0, ST>>>((const T*)gu, (T*)out, rows, F));
+    DISPATCH_T(dtype, launch_short(swiglu_fwd_kernel<T, long long>, dim3(grid_for(rows * F / IO<T>::VEC, 256)), dim3(256), 0, ST, (const T*)gu, (T*)out, rows, F));
   }
   return CHECK_LAUNCH();
 }
@@ -681,7 +685,7 @@ extern "C" int oa_rope(int dtype, void* x, long long rows, int row_stride, int n
     while (heads_per > 4 && per_head_group * ((n_heads + heads_per - 1) / heads_per) < 148 * 256) heads_per = (heads_per + 1) / 2;
     const dim3 grid(grid_for(per_head_group * ((n_heads + heads_per - 1) / heads_per), 256));
     if (heads_per < n_heads)
-      launch_pdl(rope_bf16_vec_kernel<true>, grid, dim3(256), 0, ST, (__nv_bfloat16*)x, rows, row_stride, n_heads, head_dim, seq_len, pos_offset,
+      launch_short(rope_bf16_vec_kernel<true>, grid, dim3(256), 0, ST, (__nv_bfloat16*)x, rows, row_stride, n_heads, head_dim, seq_len, pos_offset,
                  theta, backward, pos_dev, heads_per);
     else
       launch_pdl(rope_bf16_vec_kernel<false>, grid, dim3(256), 0, ST, (__nv_bfloat16*)x, rows, row_stride, n_heads, head_dim, seq_len, pos_offset,
@@ -695,7 +699,7 @@ extern "C" int oa_rope(int dtype, void* x, long long rows, int row_stride, int n
 extern "C" int oa_embedding_fwd(int dtype, const void* table, const int* ids, void* out, long long n_ids, int dim,
                                 int vocab, const void* pos_table, int seq_len, void* stream) {
   if (dim % 8) return OA_ERR_ALIGN;
-  DISPATCH_T(dtype, embedding_fwd_kernel<T><<<grid_for(n_ids * dim / IO<T>::VEC, 256), 256, 0, ST>>>(
+  DISPATCH_T(dtype, launch_short(embedding_fwd_kernel<T>, dim3(grid_for(n_ids * dim / IO<T>::VEC, 256)), dim3(256), 0, ST,
                         (const T*)table, ids, (T*)out, n_ids, dim, vocab, (const T*)pos_table, seq_len > 0 ? seq_len : 1));
   return CHECK_LAUNCH();
 }

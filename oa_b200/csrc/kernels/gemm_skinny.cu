@@ -11,7 +11,11 @@
 // to be large enough to have enough bytes in flight.  Wider products run further waves, whose tiles do not overlap their epilogues
 // with the next tile's loads as the persistent tile kernel does; gemm_skinny_wins says where that costs more than it saves.
 //
-// What bounds it: the weights' bytes at about 70 % of the copy rate (128-byte pieces of 128 rows; the rest is the ramp of a launch).
+// What bounds it: the weights' bytes, at 5.6 TB/s in a long product (128-byte pieces of 128 rows), plus 4 to 6 us to start, to meet in
+// the cluster and to store.  The start is taken off where the caller knows that nothing in flight writes W (w_at_rest, a decoding
+// step replayed as a graph): a CTA fills its ring, 27 MB over the chip, under the kernels between two products.  With the launches
+// between them chained the same way (launch_short) a 7B-class two-block step with one row went from 268 to 233 us, 32 + 1 of
+// them with their prompt from 9.45 to 8.23 ms (32 rows, 48 steps: 21.65 to 21.04 ms).
 // One row against 12288 x 4096 / 4096 x 4096 / 32000 x 4096: 31 / 18 / 66 us, with the tile kernel 38 / 22 / 69; a decoding step of
 // two 7B-class blocks and the head with 32 rows: 233 us of products, 336 us before (tile kernel on the transposed product, split-K
 // reduction, transposing copy and residual add as launches of their own).  Below 512 columns of K or 256 of N the tile kernel's
@@ -28,7 +32,7 @@ int num_sms();
 constexpr int SK_BN = 128, SK_BK = 64, SK_THREADS = 128, SK_MAX_CLUSTER = 8;
 
 struct SkinnyParams {
-  int M, N, K, ldc, ldr, act, out_f32, cluster;
+  int M, N, K, ldc, ldr, act, out_f32, cluster, w_at_rest;
   float alpha;
   void* out;
   const __nv_bfloat16 *bias, *residual;
@@ -54,6 +58,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   __shared__ uint64_t full[NS], empty[NS], done;
   __shared__ uint32_t tmem_slot;
   uint8_t* ring = sk_raw + ((1024u - (smem_u32(sk_raw) & 1023u)) & 1023u);   // the same offset in every CTA of the kernel
+  pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int c = p.cluster, rank = (int)cluster_ctarank();
   const int n0 = (int)(blockIdx.x / c) * SK_BN;
@@ -64,18 +69,23 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     for (int s = 0; s < NS; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
     mbar_init(&done, 1);
     mbar_fence_init();
-    for (int j = 0; j < NS && kb0 + j < kb1; ++j) {   // the ring is empty: fill it before the block meets
-      uint8_t* d = ring + j * Cfg::STAGE_BYTES;
+    // The ring is empty: fill it before the block meets, and with weights that no kernel still in flight writes even before the
+    // previous kernel has finished (only x comes from it).
+    if (!p.w_at_rest) pdl_wait();
+    for (int j = 0; j < NS && kb0 + j < kb1; ++j) {
       mbar_expect_tx(&full[j], Cfg::STAGE_BYTES);
-      tma_load_3d(d, &tmW, &full[j], (kb0 + j) * SK_BK, n0, 0);
-      tma_load_3d(d + Cfg::W_BYTES, &tmX, &full[j], (kb0 + j) * SK_BK, 0, 0);
+      tma_load_3d(ring + j * Cfg::STAGE_BYTES, &tmW, &full[j], (kb0 + j) * SK_BK, n0, 0);
     }
+    pdl_wait();
+    for (int j = 0; j < NS && kb0 + j < kb1; ++j)
+      tma_load_3d(ring + j * Cfg::STAGE_BYTES + Cfg::W_BYTES, &tmX, &full[j], (kb0 + j) * SK_BK, 0, 0);
   }
   if (warp == 1) { tmem_alloc<Cfg::TMEM_COLS>(&tmem_slot); tmem_relinquish(); }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t acc = tmem_slot;
+  pdl_wait();                                       // the residual and the output are touched by all threads
 
   if (warp == 0) {
     for (int i = kb0 + NS; i < kb1; ++i) {
@@ -178,12 +188,14 @@ static int launch_skinny(const CUtensorMap& tw, const CUtensorMap& tx, const Ski
   cfg.blockDim = dim3(SK_THREADS);
   cfg.dynamicSmemBytes = SkinnyCfg<MT>::SMEM_BYTES;
   cfg.stream = st;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = (unsigned)p.cluster;
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   return cudaLaunchKernelEx(&cfg, gemm_skinny_kernel<MT>, tw, tx, p) == cudaSuccess && cudaGetLastError() == cudaSuccess ? OA_OK : OA_ERR_LAUNCH;
 }
 
@@ -201,7 +213,7 @@ bool gemm_skinny_wins(int M, int N, int K) {
 
 // Called by oa_gemm_bf16 for the shapes its dispatch names; the arguments have passed its checks.
 int gemm_skinny(const void* x, const void* w, void* out, int M, int N, int K, int ldx, int ldw, int ldc, const void* bias, const void* residual,
-                int ldr, int act, int out_f32, float alpha, int* status, cudaStream_t st) {
+                int ldr, int act, int out_f32, float alpha, int w_at_rest, int* status, cudaStream_t st) {
   const int mt = (M + 15) / 16 * 16, tiles = (N + SK_BN - 1) / SK_BN, kb = (K + SK_BK - 1) / SK_BK;
   int c = 1;                                        // powers of two: a cluster of three left holes in the SMs' slots and a second wave
   while (c < SK_MAX_CLUSTER && 2 * c * tiles <= 2 * num_sms() && 2 * c <= kb / 4) c *= 2;
@@ -210,7 +222,7 @@ int gemm_skinny(const void* x, const void* w, void* out, int M, int N, int K, in
   if ((rc = make_tmap_3d_bf16(&tw, w, (uint64_t)K, (uint64_t)N, 1, (uint64_t)ldw, 0, SK_BK, SK_BN))) return rc;
   if ((rc = make_tmap_3d_bf16(&tx, x, (uint64_t)K, (uint64_t)M, 1, (uint64_t)ldx, 0, SK_BK, (uint32_t)mt))) return rc;
   SkinnyParams p;
-  p.M = M; p.N = N; p.K = K; p.ldc = ldc; p.ldr = ldr; p.act = act; p.out_f32 = out_f32; p.cluster = c; p.alpha = alpha;
+  p.M = M; p.N = N; p.K = K; p.ldc = ldc; p.ldr = ldr; p.act = act; p.out_f32 = out_f32; p.cluster = c; p.alpha = alpha; p.w_at_rest = w_at_rest;
   p.out = out; p.bias = (const __nv_bfloat16*)bias; p.residual = (const __nv_bfloat16*)residual; p.status = status;
   if (mt == 16) return launch_skinny<16>(tw, tx, p, tiles, st);
   if (mt == 32) return launch_skinny<32>(tw, tx, p, tiles, st);

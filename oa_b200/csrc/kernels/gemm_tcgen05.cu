@@ -1224,7 +1224,7 @@ static void try_store_map(GemmParams& p, void* out, uint64_t cols, uint64_t rows
 }
 
 int gemm_skinny(const void* x, const void* w, void* out, int M, int N, int K, int ldx, int ldw, int ldc, const void* bias, const void* residual,
-                int ldr, int act, int out_f32, float alpha, int* status, cudaStream_t st);
+                int ldr, int act, int out_f32, float alpha, int w_at_rest, int* status, cudaStream_t st);
 bool gemm_skinny_wins(int M, int N, int K);
 
 int num_sms() {
@@ -1284,6 +1284,20 @@ extern "C" size_t oa_gemm_workspace_bytes(int M, int N, int K) {
   return s > 1 ? (size_t)s * M * N * sizeof(float) : 0;
 }
 
+static bool few_rows(int M, int N, int K) { return M <= 64 && N >= 256 && K >= 512 && gemm_skinny_wins(M, N, K); }
+
+// The few-row product by itself.  w_at_rest: no work that may still be in flight on the stream writes W or its bytes (a replayed
+// graph in which nothing writes the weights), so W is requested before the previous kernel has finished.  OA_ERR_UNSUPPORTED for the
+// shapes that oa_gemm_bf16 gives to the tile kernels.
+extern "C" int oa_gemm_bf16_few_rows(const void* x, const void* w, void* out, int M, int N, int K, int ldx, int ldw, int ldc, const void* bias,
+                                     const void* residual, int ldr, int act, int out_f32, float alpha, int w_at_rest, int* status, void* stream) {
+  if (M <= 0 || N <= 0 || K <= 0) return OA_ERR_ARG;
+  if ((N & 7) || (K & 7) || (ldc & (out_f32 ? 3 : 7)) || (residual && (ldr & 7))) return OA_ERR_ALIGN;
+  if (act != OA_ACT_NONE && act != OA_ACT_GELU && act != OA_ACT_RELU && act != OA_ACT_SILU) return OA_ERR_UNSUPPORTED;
+  if (!few_rows(M, N, K)) return OA_ERR_UNSUPPORTED;
+  return gemm_skinny(x, w, out, M, N, K, ldx, ldw, ldc, bias, residual, ldr, act, out_f32, alpha, w_at_rest, status, (cudaStream_t)stream);
+}
+
 extern "C" int oa_gemm_bf16_batched(const void* A, const void* B, void* out, int M, int N, int K, int lda, int ldb, int ldc,
                                     int a_mn, int b_mn, const void* bias, const void* residual, int ldr, void* aux_out,
                                     const void* aux_in, int ldaux, int act, int out_f32, int accumulate, float alpha,
@@ -1296,8 +1310,8 @@ extern "C" int oa_gemm_bf16_batched(const void* A, const void* B, void* out, int
   if (batch > 1 && ((sc_batch & 7) || (sr_batch & 7) || (saux_batch & 7) || (sbias_batch & 7))) return OA_ERR_ALIGN;
   // A handful of rows against a large weight: the kernel that streams the weight (gemm_skinny.cu).  It adds the products up in another
   // order, and the residual before the one rounding, so the last bits of a row depend on how many rows come with it.
-  if (!force_bn && batch == 1 && !a_mn && !b_mn && M <= 64 && N >= 256 && K >= 512 && !accumulate && !aux_out && !aux_in && gemm_skinny_wins(M, N, K))
-    return gemm_skinny(A, B, out, M, N, K, lda, ldb, ldc, bias, residual, ldr, act, out_f32, alpha, status, (cudaStream_t)stream);
+  if (!force_bn && batch == 1 && !a_mn && !b_mn && !accumulate && !aux_out && !aux_in && few_rows(M, N, K))
+    return gemm_skinny(A, B, out, M, N, K, lda, ldb, ldc, bias, residual, ldr, act, out_f32, alpha, 0, status, (cudaStream_t)stream);
   int bn = force_bn ? force_bn : ((N >= 256) ? 256 : 128);
   int sms = num_sms();
   if (!force_bn && bn == 256) {

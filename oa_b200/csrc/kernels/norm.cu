@@ -649,10 +649,10 @@ extern "C" int oa_rmsnorm_fwd(int dtype, const void* x, const void* w, void* y, 
   const int nv = (cols + 32 * vec - 1) / (32 * vec);
   if ((at & 15) == 0 && rows <= 148 && nv > 2 && cols / vec <= 2 * NORM_THREADS) {
     if (dtype == OA_F32)
-      launch_pdl(rmsnorm_fwd_row_kernel<float>, dim3((unsigned)rows), dim3(NORM_THREADS), 0, ST, (const float*)x, (const float*)w, (float*)y, rstd, cols, eps,
+      launch_short(rmsnorm_fwd_row_kernel<float>, dim3((unsigned)rows), dim3(NORM_THREADS), 0, ST, (const float*)x, (const float*)w, (float*)y, rstd, cols, eps,
                  (const float*)residual_in, (float*)residual_out);
     else
-      launch_pdl(rmsnorm_fwd_row_kernel<__nv_bfloat16>, dim3((unsigned)rows), dim3(NORM_THREADS), 0, ST, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w,
+      launch_short(rmsnorm_fwd_row_kernel<__nv_bfloat16>, dim3((unsigned)rows), dim3(NORM_THREADS), 0, ST, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w,
                  (__nv_bfloat16*)y, rstd, cols, eps, (const __nv_bfloat16*)residual_in, (__nv_bfloat16*)residual_out);
     return CHECK_LAUNCH();
   }

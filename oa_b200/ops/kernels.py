@@ -7,10 +7,12 @@ to PyTorch math: a missing library or an unsupported shape raises.
 """
 from __future__ import annotations
 
+import contextlib
 import functools
 import math
 import os
-from typing import Optional
+import threading
+from typing import Iterable, Optional
 
 import torch
 
@@ -177,6 +179,22 @@ def set_gemm_planner(fn) -> None:
     _gemm_planner = fn
 
 
+_weights_at_rest = threading.local()
+
+
+@contextlib.contextmanager
+def weights_at_rest(weights: Iterable[torch.Tensor]):
+    """Within it, on this thread: no work that may be in flight on the stream writes the storages of these tensors (a graph is being
+    captured that only reads them), so products of a few rows with one of them as second operand request it before the
+    previous kernel has finished.  Copies made on the way have storages of their own and are not meant."""
+    before = getattr(_weights_at_rest, "storages", ())
+    _weights_at_rest.storages = {t.untyped_storage().data_ptr() for t in weights}
+    try:
+        yield
+    finally:
+        _weights_at_rest.storages = before
+
+
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = False,
          bias: Optional[torch.Tensor] = None, residual: Optional[torch.Tensor] = None, act: int = ACT_NONE,
          aux_out: Optional[torch.Tensor] = None, aux_in: Optional[torch.Tensor] = None,
@@ -238,6 +256,16 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
             V.OA_VALIDATE(Nn % 8 == 0 and K % 8 == 0, V.OaValidationSeverity.Error, "Kernel", "gemm: N=%d and K=%d must be multiples of 8", Nn, K)
             if force_bn == 0 and (M < 128 or Nn < 128):
                 V.OaValidation.Report(V.OaValidationSeverity.Info, "Kernel", "gemm M=%d N=%d K=%d: tile larger than the problem", M, Nn, K)
+        resting = getattr(_weights_at_rest, "storages", ())
+        if resting and M <= 64 and not (a_mn or b_mn or accumulate or force_bn) and aux_out is None and aux_in is None and _gemm_planner is None \
+                and b.untyped_storage().data_ptr() in resting:
+            rc = lib.oa_gemm_bf16_few_rows(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, Nn, K, a.stride(0), b.stride(0), out.stride(0), N.ptr(bias),
+                                           N.ptr(residual), residual.stride(0) if residual is not None else 0, act, int(out.dtype == torch.float32),
+                                           float(alpha), 1, status.data_ptr(), st)
+            if rc != C["OA_ERR_UNSUPPORTED"]:
+                _launch(rc, f"oa_gemm_bf16_few_rows M={M} N={Nn} K={K}", outputs=(out,))
+                return out
+
         def launch(bn: int) -> int:
             return lib.oa_gemm_bf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, Nn, K, a.stride(0), b.stride(0),
                                     out.stride(0), int(a_mn), int(b_mn), N.ptr(bias), N.ptr(residual),

@@ -47,14 +47,16 @@ class _GraphedStep:
         self.graph: Optional[torch.cuda.CUDAGraph] = None
         self.out = None
 
-    def run(self, ids: torch.Tensor, fn):
+    def run(self, ids: torch.Tensor, fn, weights=lambda: ()):
+        """`weights()`: tensors that the step reads and never writes."""
         self.ids.copy_(ids.reshape(self.ids.shape))
         if self.graph is None:
             fn(self.ids)                              # eager once: lazily created buffers (workspaces) exist before the capture
             self.pos.sub_(1)
             torch.cuda.synchronize()
             g = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(g, capture_error_mode="thread_local"):
+            # a replay begins after everything before it on the stream, so whatever changed the weights has finished by then
+            with torch.cuda.graph(g, capture_error_mode="thread_local"), K.weights_at_rest(weights()):
                 self.out = fn(self.ids)
             self.graph = g
         self.graph.replay()
@@ -149,7 +151,7 @@ class OaGptDecoder:
             return self._forward(ids.reshape(-1, 1))
         if self.Cache.Length + 1 > self.Cache.MaxSeq:
             raise ValueError("KV cache is full")
-        out = g.run(ids, self._graph_body)
+        out = g.run(ids, self._graph_body, lambda: [p.Data.Tensor() for p in self.Model.AllParameterPtrs()])
         self.Cache.Length += 1
         return out
 
