@@ -785,11 +785,6 @@ struct BwdKvCfg {
   static constexpr int TM_S = 0, TM_DP = NS * FA_BN, TM_DV = TM_DP + FA_BN, TM_DK = TM_DV + HD;
 };
 
-// two fp32 values per instruction
-__device__ __forceinline__ unsigned long long f2_of(uint32_t a, uint32_t b) { unsigned long long r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(a), "r"(b)); return r; }
-__device__ __forceinline__ void f2_to(unsigned long long v, uint32_t& a, uint32_t& b) { asm("mov.b64 {%0, %1}, %2;" : "=r"(a), "=r"(b) : "l"(v)); }
-__device__ __forceinline__ unsigned long long f2_fma(unsigned long long a, unsigned long long b, unsigned long long c) { unsigned long long d; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c)); return d; }
-__device__ __forceinline__ unsigned long long f2_mul(unsigned long long a, unsigned long long b) { unsigned long long d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
 __device__ __forceinline__ void bwd_prob2(uint32_t& a, uint32_t& b, unsigned long long sl2, unsigned long long nl) {
   f2_to(f2_fma(f2_of(a, b), sl2, nl), a, b);
   a = __float_as_uint(fast_exp2(__uint_as_float(a))); b = __float_as_uint(fast_exp2(__uint_as_float(b)));

@@ -11,12 +11,14 @@
 // Bmm need no transposed copies: gemm_f32_tile_kernel where each operand has one contiguous direction and 16-byte rows (an
 // asynchronous ring of K tiles), gemm_f32_kernel for any other strides (the next K tile prefetched into registers).  Few tiles with a
 // long reduction: K is sliced over more blocks, and the kernel that adds the slices up carries the epilogue.
+#include <type_traits>
+
 #include "common.cuh"
 #include "api.h"
 
 namespace oa {
 
-constexpr int FT = 64, FK = 16;
+constexpr int FT = 64, FK = 16;   // output tile width (and height of the plain kernel), columns of K per stage of the plain kernel
 
 struct F32Epi {
   const float *bias, *residual, *aux_in;
@@ -118,13 +120,206 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ B, float*
   }
 }
 
-// Operands with one contiguous direction and 16-byte rows: the tile arrives through a ring of three 16-byte cp.async stages and
-// the fourth is multiplied, so that a block waits for memory once instead of once per 16 columns.  An operand keeps the layout it
-// has in memory ([row][k] with a pitch of 20 floats, or [k][row]); the columns a thread owns follow it, which leaves its 16-byte
-// reads free of bank conflicts.  TM x 4 outputs per thread: 32-row tiles while 64-row tiles would leave SMs without a block.  What
-// bounds it at these sizes: the ramp of a launch and the shared-memory reads.  The 51 products of a character-model step (2048
-// rows, widths 128 to 512): 852 us before, 650 us now.  128 threads with twice the outputs each measured 760 us.
-constexpr int F_THREADS = 256, F_TM = FT * 16 / F_THREADS, FS = 4, FP_K = FK + 4, FP_MN = FT + 4, F_STAGE = FT * FP_K;
+// Operands with one contiguous direction and 16-byte rows: the tile arrives through a ring of 16-byte cp.async stages, so that a block
+// waits for memory once instead of once per stage.  An operand keeps the layout it has in memory ([row][k], or [k][row], with
+// four floats of padding); the columns a thread owns follow it, which leaves its 16-byte reads free of bank conflicts.
+// A thread owns 8 x 4 outputs, whatever the tile: 64 threads cover 32 x 64, 128 cover 64 x 64, and the block's 256 threads are KG = 4 or
+// 2 such groups that each take their own eight columns of a stage and add their sums up, in group order, through shared memory at the
+// end.  That is twelve 16-byte reads per 128 multiply-adds; two or four rows per thread over all of K, the shape of the tile kernel
+// before this one, read six or eight per 32 or 64, ran at 320 clocks per four columns of K where the reads alone need 80, and left a
+// block of 2048 x 128 x 512 with 8 warps in step and nothing to hide their latencies.
+// What bounds it: multiply-adds at half their rate in long reductions, the ramp of a launch and the two passes through the epilogue's
+// shared memory in short ones.  Before -> now: 2048 x 128 x 512 20.3 -> 13.1 us,
+// 512 x 512 x 512 20.5 -> 13.2, 128 x 128 x 4096 in slices 14.2 -> 11.6 to 13.3, 4096^3 with both operands row-contiguous 3.50 -> 2.72 ms,
+// with both K-contiguous 3.57 -> 3.4 (there the pairs of a register file's double width do not lie side by side).
+// The next kernel's launch is let in at the end, not at the start: blocks that were resident early sit where this kernel left
+// room, not one per SM, and products that followed one another took up to 1.5 times as long.
+constexpr int F_THREADS = 256;
+template <int ROWS, int MN, int KW>   // a [ROWS x KW] tile: [k][row] when MN, else [row][k]
+struct F32Tile {
+  static constexpr int PITCH = (MN ? ROWS : KW) + 4;
+  static constexpr int FLOATS = (MN ? KW : ROWS) * PITCH;
+  static constexpr int PIECES = ROWS * KW / 4 / F_THREADS;      // 16-byte pieces per thread
+  static_assert(PIECES * 4 * F_THREADS == ROWS * KW, "whole pieces per thread");
+  const float* src[PIECES];        // this thread's pieces of the next stage (rows outside the matrix: any valid address, no bytes)
+  uint32_t dst[PIECES];            // byte offset inside a stage
+  int bytes[PIECES], left[PIECES]; // bytes of a whole stage; columns of K from the piece to the end of the slice
+  long long step;
+  __device__ __forceinline__ void start(const float* __restrict__ g, long long ld, int r0, int k_lo, int rows, int k_hi) {
+    step = MN ? (long long)KW * ld : KW;
+#pragma unroll
+    for (int q = 0; q < PIECES; ++q) {
+      const int i = threadIdx.x + q * F_THREADS;
+      constexpr int PER = (MN ? ROWS : KW) / 4;
+      const int major = i / PER, minor = (i % PER) * 4, r = MN ? minor : major, k = MN ? major : minor;
+      bytes[q] = max(0, min(4, MN ? rows - (r0 + r) : (r0 + r < rows ? 4 : 0))) * 4;
+      left[q] = k_hi - (k_lo + k);
+      dst[q] = (uint32_t)(major * PITCH + minor) * 4u;
+      src[q] = bytes[q] ? g + (MN ? (long long)(k_lo + k) * ld + r0 + r : (long long)(r0 + r) * ld + k_lo + k) : g;
+    }
+  }
+  __device__ __forceinline__ void fetch(uint32_t stage, const float* g, bool whole) {
+#pragma unroll
+    for (int q = 0; q < PIECES; ++q) {
+      int n = bytes[q];
+      const float* p = src[q];
+      if (!whole) {                                             // the slice ends inside this stage
+        n = MN ? (left[q] > 0 ? n : 0) : min(n, max(0, min(4, left[q])) * 4);
+        if (n == 0) p = g;
+      }
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(stage + dst[q]), "l"(p), "r"(n) : "memory");
+      if (bytes[q]) src[q] += step;
+      left[q] -= KW;
+    }
+  }
+};
+
+template <int A_MN, int B_MN, int ROWS>
+__global__ void __launch_bounds__(F_THREADS, 2)
+gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ B, float* __restrict__ C, int M, int N, int K, long long lda,
+                     long long ldb, int ldc, long long batch_a, long long batch_b, long long batch_c, const F32Epi epi, int k_chunk) {
+  constexpr int KG = 128 / ROWS, KW = 8 * KG, STAGES = ROWS == 32 ? 3 : 4, TY = ROWS / 8;
+  using TA = F32Tile<ROWS, A_MN, KW>;
+  using TB = F32Tile<FT, B_MN, KW>;
+  constexpr int STAGE = TA::FLOATS + TB::FLOATS;
+  __shared__ __align__(16) float ring[STAGES * STAGE];
+  static_assert(KG * ROWS * FT <= STAGES * STAGE, "the groups' sums reuse the ring");
+  const int b = blockIdx.z;
+  const int k_lo = k_chunk > 0 ? b * k_chunk : 0, k_hi = k_chunk > 0 ? min(K, k_lo + k_chunk) : K;
+  if (k_chunk == 0) { A += (long long)b * batch_a; B += (long long)b * batch_b; }
+  C += (long long)b * batch_c;
+  const int m0 = blockIdx.y * ROWS, n0 = blockIdx.x * FT;
+  const int group = threadIdx.x / (F_THREADS / KG), t = threadIdx.x % (F_THREADS / KG);
+  const int tx = t & 15, ty = t >> 4;
+  const int steps = (k_hi - k_lo + KW - 1) / KW, whole = (k_hi - k_lo) / KW;
+  TA ta;
+  TB tb;
+  ta.start(A, lda, m0, k_lo, M, k_hi);
+  tb.start(B, ldb, n0, k_lo, N, k_hi);
+  const uint32_t ring0 = smem_u32(ring);
+  int filled = 0, slot = 0;                           // stages requested so far, and the place of the next
+  auto load = [&]() {
+    if (filled < steps) {
+      const uint32_t st = ring0 + slot * (STAGE * 4);
+      ta.fetch(st, A, filled < whole);
+      tb.fetch(st + TA::FLOATS * 4, B, filled < whole);
+    }
+    ++filled;
+    if (++slot == STAGES) slot = 0;
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  pdl_wait();
+#pragma unroll
+  for (int i = 0; i < STAGES - 1; ++i) load();
+  // Sums of two outputs, or of the even and the odd columns of K of one output, per register pair: whichever way the operands' 16-byte
+  // reads leave pairs side by side (K-major both: along K; A row-contiguous: two rows; else two columns).
+  constexpr int PAIR = A_MN ? 1 : (B_MN ? 2 : 0);
+  constexpr int PR = PAIR == 1 ? 4 : 8, PC = PAIR == 2 ? 2 : 4;
+  using Acc = typename std::conditional<PAIR == 0, float, unsigned long long>::type;
+  Acc acc[PR][PC] = {};
+  int at = 0;
+  for (int i = 0; i < steps; ++i) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+    __syncthreads();                                  // stage i has landed everywhere, stage i - 1 has been read
+    load();
+    const float *pa = ring + at * STAGE, *pb = pa + TA::FLOATS;
+    if (++at == STAGES) at = 0;
+#pragma unroll
+    for (int kk = 0; kk < 8; kk += 4) {
+      const int k0 = group * 8 + kk;
+      if constexpr (PAIR == 0) {
+        float a[8][4], bb[4][4];                      // [row][k], [column][k]
+#pragma unroll
+        for (int c = 0; c < 4; ++c) *reinterpret_cast<float4*>(bb[c]) = *reinterpret_cast<const float4*>(pb + (tx + 16 * c) * TB::PITCH + k0);
+#pragma unroll
+        for (int r = 0; r < 8; ++r) *reinterpret_cast<float4*>(a[r]) = *reinterpret_cast<const float4*>(pa + (ty + TY * r) * TA::PITCH + k0);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+#pragma unroll
+          for (int r = 0; r < 8; ++r)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) acc[r][c] = fmaf(a[r][k], bb[c][k], acc[r][c]);
+      } else if constexpr (PAIR == 1) {
+        float bk[4][4];                               // [column][k]
+        if constexpr (!B_MN) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) *reinterpret_cast<float4*>(bk[c]) = *reinterpret_cast<const float4*>(pb + (tx + 16 * c) * TB::PITCH + k0);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const ulonglong2 lo = *reinterpret_cast<const ulonglong2*>(pa + (k0 + k) * TA::PITCH + ty * 8);
+          const ulonglong2 hi = *reinterpret_cast<const ulonglong2*>(pa + (k0 + k) * TA::PITCH + ty * 8 + 4);
+          const unsigned long long a[4] = {lo.x, lo.y, hi.x, hi.y};
+          float b[4];
+          if constexpr (B_MN) *reinterpret_cast<float4*>(b) = *reinterpret_cast<const float4*>(pb + (k0 + k) * TB::PITCH + tx * 4);
+          else { b[0] = bk[0][k]; b[1] = bk[1][k]; b[2] = bk[2][k]; b[3] = bk[3][k]; }
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            const unsigned long long b2 = f2_of(__float_as_uint(b[c]), __float_as_uint(b[c]));
+#pragma unroll
+            for (int r = 0; r < 4; ++r) acc[r][c] = f2_fma(a[r], b2, acc[r][c]);
+          }
+        }
+      } else {
+        ulonglong2 b[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) b[k] = *reinterpret_cast<const ulonglong2*>(pb + (k0 + k) * TB::PITCH + tx * 4);
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          const float4 v = *reinterpret_cast<const float4*>(pa + (ty + TY * r) * TA::PITCH + k0);
+          const float a[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const unsigned long long a2 = f2_of(__float_as_uint(a[k]), __float_as_uint(a[k]));
+            acc[r][0] = f2_fma(a2, b[k].x, acc[r][0]);
+            acc[r][1] = f2_fma(a2, b[k].y, acc[r][1]);
+          }
+        }
+      }
+    }
+  }
+  pdl_launch_dependents();
+  __syncthreads();                                    // the last stage has been read; the copies still counted are empty
+  {
+    float* mine = ring + group * (ROWS * FT);
+    auto half = [](unsigned long long v, int h) -> float { return __uint_as_float((uint32_t)(h ? v >> 32 : v)); };
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      float* row = mine + (A_MN ? ty * 8 + r : ty + TY * r) * FT;
+      float v[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        if constexpr (PAIR == 0) v[c] = acc[r][c];
+        else if constexpr (PAIR == 1) v[c] = half(acc[r >> 1][c], r & 1);
+        else v[c] = half(acc[r][c >> 1], c & 1);
+      }
+      if (B_MN) {
+        *reinterpret_cast<float4*>(row + tx * 4) = make_float4(v[0], v[1], v[2], v[3]);
+      } else {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) row[tx + 16 * c] = v[c];
+      }
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < ROWS * FT / F_THREADS; ++i) {
+    const int e = i * F_THREADS + threadIdx.x, gm = m0 + e / FT, gn = n0 + e % FT;
+    if (gm >= M || gn >= N) continue;
+    float v = ring[e];
+#pragma unroll
+    for (int g = 1; g < KG; ++g) v += ring[g * (ROWS * FT) + e];
+    float* o = C + (long long)gm * ldc + gn;
+    *o = f32_epilogue(epi, v, gm, gn, o);
+  }
+}
+
+// The same products over fewer than F_BRIEF_K columns of K with tiles for every SM: 4 x 4 outputs per thread over all of K, stored from
+// registers.  Fewer registers leave room for three blocks per SM, and of a few stages of arithmetic what counts is how many blocks
+// overlap their loads and stores.  Against the kernel above: 2048 x 512 x 128 11.9 / 12.9 us, 8192 x 384 x 64 17 / 24, 4096 x 1024 x 160
+// 40 / 48, 50000 x 32 x 32 10.5 / 17; 1024 x 1024 x 256 21.1 / 20.6 (18 with both operands row-contiguous), 512 x 512 x 512 20.5 / 13.2.
+constexpr int F_BRIEF_K = 192;
+constexpr int FS = 4, FP_K = FK + 4, FP_MN = FT + 4, F_STAGE = FT * FP_K;
 __device__ __forceinline__ void f32_cp16(float* dst, const float* src, int bytes) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
 }
@@ -146,13 +341,14 @@ __device__ __forceinline__ void f32_fetch(float* sm, const float* __restrict__ g
   }
 }
 
-template <int A_MN, int B_MN, int TM>
+template <int A_MN, int B_MN>
 __global__ void __launch_bounds__(F_THREADS)
-gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ B, float* __restrict__ C, int M, int N, int K, long long lda,
+gemm_f32_brief_kernel(const float* __restrict__ A, const float* __restrict__ B, float* __restrict__ C, int M, int N, int K, long long lda,
                      long long ldb, int ldc, long long batch_a, long long batch_b, long long batch_c, const F32Epi epi, int k_chunk) {
-  constexpr int TY = F_THREADS / 16, ROWS = TY * TM;
+  constexpr int TM = 4, TY = F_THREADS / 16, ROWS = TY * TM;
   __shared__ __align__(16) float sA[FS][F_STAGE], sB[FS][F_STAGE];
   const int b = blockIdx.z;
+  pdl_wait();
   const int k_lo = k_chunk > 0 ? b * k_chunk : 0, k_hi = k_chunk > 0 ? min(K, k_lo + k_chunk) : K;
   if (k_chunk == 0) { A += (long long)b * batch_a; B += (long long)b * batch_b; }
   C += (long long)b * batch_c;
@@ -240,21 +436,26 @@ static bool gemm_f32_tiles(const float* A, const float* B, float* C, int M, int 
   const int z = k_chunk > 0 ? slices : batch;
   const long long tiles = (long long)((N + FT - 1) / FT) * ((M + FT - 1) / FT) * z;
   const int rows = tiles >= 148 ? 64 : 32;
+  const bool brief = rows == 64 && (k_chunk > 0 ? k_chunk : K) < F_BRIEF_K;
   const dim3 grid((N + FT - 1) / FT, (M + rows - 1) / rows, z);
   if (grid.y > 65535) return false;
-#define OA_F32_TILE(AM, BMN)                                                                                                                  \
-  if (rows == 64) gemm_f32_tile_kernel<AM, BMN, F_TM><<<grid, F_THREADS, 0, st>>>(A, B, C, M, N, K, lda, ldb, ldc, batch_a, batch_b, batch_c, epi, k_chunk); \
-  else gemm_f32_tile_kernel<AM, BMN, F_TM / 2><<<grid, F_THREADS, 0, st>>>(A, B, C, M, N, K, lda, ldb, ldc, batch_a, batch_b, batch_c, epi, k_chunk)
+#define OA_F32_RUN(KERNEL) launch_short(KERNEL, grid, dim3(F_THREADS), 0, st, A, B, C, M, N, K, lda, ldb, ldc, batch_a, batch_b, batch_c, epi, k_chunk)
+#define OA_F32_TILE(AM, BMN)                                              \
+  if (brief) OA_F32_RUN((gemm_f32_brief_kernel<AM, BMN>));                \
+  else if (rows == 64) OA_F32_RUN((gemm_f32_tile_kernel<AM, BMN, 64>));   \
+  else OA_F32_RUN((gemm_f32_tile_kernel<AM, BMN, 32>))
   if (a_k && b_k) { OA_F32_TILE(0, 0); }
   else if (a_k) { OA_F32_TILE(0, 1); }
   else if (b_k) { OA_F32_TILE(1, 0); }
   else { OA_F32_TILE(1, 1); }
 #undef OA_F32_TILE
+#undef OA_F32_RUN
   return true;
 }
 
 // C[m,n] = epilogue(sum_s part[s][m,n]): fixed slice order, so the split-K result is reproducible
 __global__ void gemm_f32_splitk_reduce_kernel(const float* __restrict__ part, float* __restrict__ C, int M, int N, int ldc, int splits, const F32Epi epi) {
+  pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (long long)M * N) return;
   const int m = (int)(i / N), n = (int)(i % N);
@@ -294,7 +495,7 @@ static int gemm_f32(const float* A, const float* B, float* C, int M, int N, int 
     if (!oa::gemm_f32_tiles(A, B, scratch, M, N, K, sam, sak, sbn, sbk, N, 1, 0, 0, (long long)M * N, part_epi, k_chunk, splits, st))
       oa::gemm_f32_kernel<<<grid, 256, 0, st>>>(A, B, scratch, M, N, K, sam, sak, sbn, sbk, N, 0, 0, (long long)M * N, part_epi, k_chunk);
     const long long n = (long long)M * N;
-    oa::gemm_f32_splitk_reduce_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(scratch, C, M, N, ldc, splits, epi);
+    oa::launch_short(oa::gemm_f32_splitk_reduce_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, st, (const float*)scratch, C, M, N, ldc, splits, epi);
     return cudaGetLastError() == cudaSuccess ? OA_OK : OA_ERR_LAUNCH;
   }
   if (!oa::gemm_f32_tiles(A, B, C, M, N, K, sam, sak, sbn, sbk, ldc, batch, batch_a, batch_b, batch_c, epi, 0, 0, st))
