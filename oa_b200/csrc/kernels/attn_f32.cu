@@ -7,14 +7,16 @@
 // product is streamed through shared memory 32 rows at a time with an online softmax, so there is no
 // sequence-length cap and global memory is read in whole rows.
 //
-// Work split (all three kernels): a CTA of 128 threads owns 128 / TPR rows of one (batch, head); a row is
-// shared by TPR threads that each keep W (32 or 8) of the head dimensions in registers and combine their
-// partial dot products with shuffles.  W = 32 does the least work per score; W = 8 makes four times as many,
-// shorter CTAs (which under the causal mask also skip more of the other side) and is taken while W = 32 would
-// leave SMs idle (af_split): 16 x 4 heads of 32 dimensions and 128 positions are 64 CTAs of one warp per
-// scheduler, 33 / 41 / 44 us for forward, dQ and dK / dV, against 19 / 29 / 27 us.  Forward and dQ rows are queries (keys / values stream through shared
-// memory), dK / dV rows are keys (queries and output gradients stream through shared memory together with
-// their log-sum-exp and delta = rowsum(dO * O)).
+// Work split (all three kernels): a CTA of 128 threads owns 128 / (DS KS) rows of one (batch, head).  A row is shared by DS threads that
+// keep 32 head dimensions each in registers (their partial dot products meet in shuffles) and by KS groups of those that take every
+// KS-th row of the other side, with a running maximum and sums of their own that meet once, at the end.  KS = 1 does the least
+// work per score; KS = 4 makes four times as many, shorter CTAs (which under the causal mask also skip more of the other side), lets
+// the next tile arrive through cp.async under this one, and is taken while KS = 1 would leave SMs idle (af_split).
+// 16 x 4 heads of 32 dimensions and 128 positions are 64 CTAs with KS = 1, one warp per scheduler: 29 us forward
+// and 83 us both gradients.  With KS = 4: 14 us, and 38 for both gradients (19, and 53, with eight
+// dimensions per thread, whose dot products each took two shuffles).
+// Forward and dQ rows are queries (keys / values stream through shared memory), dK / dV rows are keys (queries and output gradients
+// stream through shared memory together with their log-sum-exp and delta = rowsum(dO * O)).
 #include "common.cuh"
 #include "api.h"
 
@@ -23,229 +25,321 @@ namespace oa {
 constexpr int AF_THREADS = 128;
 constexpr int AF_TILE = 32;     // streamed rows per step
 
-// floats per W-dimension segment in shared memory (padded: segments land in different banks)
-template <int W> constexpr int af_seg = W + 4;
+constexpr int AF_W = 32;        // head dimensions per thread
+constexpr int AF_SEG = AF_W + 4;   // floats per such segment in shared memory (padded: rows and segments land in different banks)
 
-// Loads rows [r0, r0 + 32) of a [rows, stride] matrix (columns [col0, col0 + hd)) into sm[32][TPR][af_seg<W>]; rows >= limit
-// and dimensions >= hd become 0.
-template <int TPR, int W>
-__device__ __forceinline__ void af_load_tile(float* sm, const float* __restrict__ g, long long stride, long long row_base, int r0,
-                                             int limit, int col0, int hd) {
+// A streamed tile of rows [r0, r0 + 32) of a [rows, stride] matrix, columns [col0, col0 + hd), as [32][DS][AF_SEG]; rows >= limit and
+// dimensions >= hd become 0.  `vec`: 16-byte pieces (hd, stride and the pointer allow it), asynchronously when ASYNC.
+template <int DS, bool ASYNC>
+__device__ __forceinline__ void af_load_tile(float* sm, const float* __restrict__ g, long long stride, long long row_base, int r0, int limit, int col0,
+                                             int hd, bool vec) {
+  constexpr int COLS = DS * AF_W;
+  if (vec) {
+#pragma unroll
+    for (int idx = threadIdx.x; idx < AF_TILE * COLS / 4; idx += AF_THREADS) {
+      const int r = idx / (COLS / 4), c = idx % (COLS / 4) * 4;
+      const bool ok = r0 + r < limit && c < hd;
+      const float* src = ok ? g + (row_base + r0 + r) * stride + col0 + c : g;
+      float* dst = sm + (r * DS + c / AF_W) * AF_SEG + c % AF_W;
+      if (ASYNC) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(ok ? 16 : 0) : "memory");
+      else *reinterpret_cast<float4*>(dst) = ok ? *reinterpret_cast<const float4*>(src) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  } else {
 #pragma unroll 4
-  for (int idx = threadIdx.x; idx < AF_TILE * TPR * W; idx += AF_THREADS) {
-    const int r = idx / (TPR * W), c = idx % (TPR * W);
-    float x = 0.f;
-    if (r0 + r < limit && c < hd) x = g[(row_base + r0 + r) * stride + col0 + c];
-    sm[(r * TPR + c / W) * af_seg<W> + c % W] = x;
+    for (int idx = threadIdx.x; idx < AF_TILE * COLS; idx += AF_THREADS) {
+      const int r = idx / COLS, c = idx % COLS;
+      float x = 0.f;
+      if (r0 + r < limit && c < hd) x = g[(row_base + r0 + r) * stride + col0 + c];
+      sm[(r * DS + c / AF_W) * AF_SEG + c % AF_W] = x;
+    }
   }
 }
+__device__ __forceinline__ void af_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void af_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-template <int TPR>
+// sum over the DS threads that share a row's dot products (neighbouring lanes)
+template <int DS>
 __device__ __forceinline__ float af_reduce(float x) {
-  if (TPR >= 2) x += __shfl_xor_sync(0xffffffffu, x, 1);
-  if (TPR >= 4) x += __shfl_xor_sync(0xffffffffu, x, 2);
-  if (TPR >= 8) x += __shfl_xor_sync(0xffffffffu, x, 4);
+  if (DS >= 2) x += __shfl_xor_sync(0xffffffffu, x, 1);
+  if (DS >= 4) x += __shfl_xor_sync(0xffffffffu, x, 2);
   return x;
 }
+// Sums of v[0..31] over the KS groups of a row: every group ends up with 32 / KS of them, v[0 .. 32 / KS), which are dimensions
+// af_first<KS>(ks) and on.
+template <int DS, int KS>
+__device__ __forceinline__ void af_scatter_sum(float* v, int ks) {
+  if constexpr (KS == 4) {
+#pragma unroll
+    for (int t = 0; t < 16; ++t) {
+      const float mine = ks & 1 ? v[t + 16] : v[t], theirs = ks & 1 ? v[t] : v[t + 16];
+      v[t] = mine + __shfl_xor_sync(0xffffffffu, theirs, DS);
+    }
+#pragma unroll
+    for (int t = 0; t < 8; ++t) {
+      const float mine = ks & 2 ? v[t + 8] : v[t], theirs = ks & 2 ? v[t] : v[t + 8];
+      v[t] = mine + __shfl_xor_sync(0xffffffffu, theirs, 2 * DS);
+    }
+  }
+}
+template <int KS>
+__device__ __forceinline__ int af_first(int ks) { return KS == 4 ? (ks & 1) * 16 + (ks >> 1) * 8 : 0; }
 
-template <int W>
 __device__ __forceinline__ float af_dot(const float* a, const float* __restrict__ sm_row) {
   float d0 = 0.f, d1 = 0.f, d2 = 0.f, d3 = 0.f;
 #pragma unroll
-  for (int t = 0; t < W; t += 4) {
+  for (int t = 0; t < AF_W; t += 4) {
     const float4 x = *reinterpret_cast<const float4*>(sm_row + t);
     d0 = fmaf(a[t], x.x, d0); d1 = fmaf(a[t + 1], x.y, d1); d2 = fmaf(a[t + 2], x.z, d2); d3 = fmaf(a[t + 3], x.w, d3);
   }
   return (d0 + d1) + (d2 + d3);
 }
 
-template <int W>
 __device__ __forceinline__ void af_axpy(float* acc, float a, const float* __restrict__ sm_row) {
 #pragma unroll
-  for (int t = 0; t < W; t += 4) {
+  for (int t = 0; t < AF_W; t += 4) {
     const float4 x = *reinterpret_cast<const float4*>(sm_row + t);
     acc[t] = fmaf(a, x.x, acc[t]); acc[t + 1] = fmaf(a, x.y, acc[t + 1]);
     acc[t + 2] = fmaf(a, x.z, acc[t + 2]); acc[t + 3] = fmaf(a, x.w, acc[t + 3]);
   }
 }
 
-template <int TPR, int W>
+template <int DS, int KS>
+struct AfCfg {
+  static constexpr int TPR = DS * KS, ROWS = AF_THREADS / TPR;
+  static constexpr bool ASYNC = KS > 1;                        // two buffers, the next tile in flight
+  static constexpr int BUFS = ASYNC ? 2 : 1, TILE = AF_TILE * DS * AF_SEG;
+};
+
+// The two streamed matrices of all three kernels, tile by tile: body(j0, x tile, y tile) for j0 in [lo, hi) in steps of 32.
+template <int DS, int KS, typename Body>
+__device__ __forceinline__ void af_stream(float* sx, float* sy, const float* __restrict__ x, long long xs, const float* __restrict__ y, long long ys,
+                                          long long row0, int lo, int hi, int limit, int col0, int hd, bool vec, Body body) {
+  using Cfg = AfCfg<DS, KS>;
+  auto load = [&](int j0, int buf) {
+    af_load_tile<DS, Cfg::ASYNC>(sx + buf * Cfg::TILE, x, xs, row0, j0, limit, col0, hd, vec);
+    af_load_tile<DS, Cfg::ASYNC>(sy + buf * Cfg::TILE, y, ys, row0, j0, limit, col0, hd, vec);
+    if (Cfg::ASYNC) af_commit();
+  };
+  if constexpr (Cfg::ASYNC) {
+    load(lo, 0);
+    for (int j0 = lo, buf = 0; j0 < hi; j0 += AF_TILE, buf ^= 1) {
+      if (j0 + AF_TILE < hi) { load(j0 + AF_TILE, buf ^ 1); af_wait<1>(); } else { af_wait<0>(); }
+      __syncthreads();
+      body(j0, sx + buf * Cfg::TILE, sy + buf * Cfg::TILE);
+      __syncthreads();                                         // the buffer may be filled again
+    }
+  } else {
+    for (int j0 = lo; j0 < hi; j0 += AF_TILE) {
+      __syncthreads();
+      load(j0, 0);
+      __syncthreads();
+      body(j0, sx, sy);
+    }
+  }
+}
+
+template <int DS, int KS>
 __global__ void __launch_bounds__(AF_THREADS)
 attn_f32_fwd_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
                     float* __restrict__ o, float* __restrict__ lse, int heads, int seq, int hd, long long rs, long long os,
-                    float scale, int causal) {
-  constexpr int ROWS = AF_THREADS / TPR;
-  __shared__ __align__(16) float sK[AF_TILE * TPR * af_seg<W>];
-  __shared__ __align__(16) float sV[AF_TILE * TPR * af_seg<W>];
+                    float scale, int causal, int vec) {
+  using Cfg = AfCfg<DS, KS>;
+  constexpr int NJ = AF_TILE / KS;                             // keys of a tile that this thread takes: ks, ks + KS, ...
+  __shared__ __align__(16) float sK[Cfg::BUFS * Cfg::TILE], sV[Cfg::BUFS * Cfg::TILE];
+  pdl_wait();
   const int h = blockIdx.y, b = blockIdx.z;
-  const int i0 = blockIdx.x * ROWS;
-  const int i = i0 + threadIdx.x / TPR, seg = threadIdx.x % TPR;
+  const int i0 = blockIdx.x * Cfg::ROWS;
+  const int i = i0 + threadIdx.x / Cfg::TPR, seg = threadIdx.x % DS, ks = threadIdx.x % Cfg::TPR / DS;
   const long long row0 = (long long)b * seq;
   const bool row_ok = i < seq;
-  float qr[W], acc[W];
+  float qr[AF_W], acc[AF_W];
 #pragma unroll
-  for (int t = 0; t < W; ++t) {
-    const int d = seg * W + t;
+  for (int t = 0; t < AF_W; ++t) {
+    const int d = seg * AF_W + t;
     qr[t] = (row_ok && d < hd) ? q[(row0 + i) * rs + h * hd + d] * scale : 0.f;
     acc[t] = 0.f;
   }
   float m = -INFINITY, l = 0.f;
-  const int kend = causal ? min(seq, i0 + ROWS) : seq;       // keys this CTA needs
-  for (int j0 = 0; j0 < kend; j0 += AF_TILE) {
-    __syncthreads();
-    af_load_tile<TPR, W>(sK, k, rs, row0, j0, seq, h * hd, hd);
-    af_load_tile<TPR, W>(sV, v, rs, row0, j0, seq, h * hd, hd);
-    __syncthreads();
-    float s[AF_TILE];
+  const int kend = causal ? min(seq, i0 + Cfg::ROWS) : seq;       // keys this CTA needs
+  af_stream<DS, KS>(sK, sV, k, rs, v, rs, row0, 0, kend, seq, h * hd, hd, vec, [&](int j0, const float* tk, const float* tv) {
+    float s[NJ];
     float mt = -INFINITY;
 #pragma unroll
-    for (int j = 0; j < AF_TILE; ++j) {
-      float d = af_reduce<TPR>(af_dot<W>(qr, sK + (j * TPR + seg) * af_seg<W>));
+    for (int jj = 0; jj < NJ; ++jj) {
+      const int j = jj * KS + ks;
+      const float d = af_reduce<DS>(af_dot(qr, tk + (j * DS + seg) * AF_SEG));
       const int kj = j0 + j;
       const bool alive = kj < seq && (!causal || kj <= i);
-      s[j] = alive ? d : -INFINITY;
-      mt = fmaxf(mt, s[j]);
+      s[jj] = alive ? d : -INFINITY;
+      mt = fmaxf(mt, s[jj]);
     }
     const float mn = fmaxf(m, mt);
     const float mu = (mn == -INFINITY) ? 0.f : mn;
     const float alpha = __expf(m - mu);
     float ls = 0.f;
 #pragma unroll
-    for (int t = 0; t < W; ++t) acc[t] *= alpha;
+    for (int t = 0; t < AF_W; ++t) acc[t] *= alpha;
 #pragma unroll
-    for (int j = 0; j < AF_TILE; ++j) {
-      const float p = __expf(s[j] - mu);
+    for (int jj = 0; jj < NJ; ++jj) {
+      const float p = __expf(s[jj] - mu);
       ls += p;
-      af_axpy<W>(acc, p, sV + (j * TPR + seg) * af_seg<W>);
+      af_axpy(acc, p, tv + ((jj * KS + ks) * DS + seg) * AF_SEG);
     }
     l = l * alpha + ls;
     m = mn;
+  });
+  if constexpr (KS == 4) {
+    // the groups' maxima and sums meet
+    float mx = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, DS));
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2 * DS));
+    const float w = __expf(m - (mx == -INFINITY ? 0.f : mx));
+    l *= w;
+    l += __shfl_xor_sync(0xffffffffu, l, DS);
+    l += __shfl_xor_sync(0xffffffffu, l, 2 * DS);
+#pragma unroll
+    for (int t = 0; t < AF_W; ++t) acc[t] *= w;
+    m = mx;
+    af_scatter_sum<DS, KS>(acc, ks);
   }
   if (!row_ok) return;
   const float inv = l > 0.f ? 1.f / l : 0.f;
 #pragma unroll
-  for (int t = 0; t < W; ++t) {
-    const int d = seg * W + t;
+  for (int t = 0; t < AF_W / KS; ++t) {
+    const int d = seg * AF_W + af_first<KS>(ks) + t;
     if (d < hd) o[(row0 + i) * os + h * hd + d] = acc[t] * inv;
   }
-  if (seg == 0 && lse) lse[((long long)b * heads + h) * seq + i] = m + logf(l);
+  if (seg == 0 && ks == 0 && lse) lse[((long long)b * heads + h) * seq + i] = m + logf(l);
 }
 
 // dQ: rows are queries; K and V stream through shared memory.
-template <int TPR, int W>
+template <int DS, int KS>
 __global__ void __launch_bounds__(AF_THREADS)
 attn_f32_bwd_q_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
                       const float* __restrict__ o, const float* __restrict__ dout, const float* __restrict__ lse,
                       float* __restrict__ dq, int heads, int seq, int hd, long long rs, long long os, long long ds_, float scale,
-                      int causal) {
-  constexpr int ROWS = AF_THREADS / TPR;
-  __shared__ __align__(16) float sK[AF_TILE * TPR * af_seg<W>];
-  __shared__ __align__(16) float sV[AF_TILE * TPR * af_seg<W>];
+                      int causal, int vec) {
+  using Cfg = AfCfg<DS, KS>;
+  constexpr int NJ = AF_TILE / KS;
+  __shared__ __align__(16) float sK[Cfg::BUFS * Cfg::TILE], sV[Cfg::BUFS * Cfg::TILE];
+  pdl_wait();
   const int h = blockIdx.y, b = blockIdx.z;
-  const int i0 = blockIdx.x * ROWS;
-  const int i = i0 + threadIdx.x / TPR, seg = threadIdx.x % TPR;
+  const int i0 = blockIdx.x * Cfg::ROWS;
+  const int i = i0 + threadIdx.x / Cfg::TPR, seg = threadIdx.x % DS, ks = threadIdx.x % Cfg::TPR / DS;
   const long long row0 = (long long)b * seq;
   const bool row_ok = i < seq;
-  float qr[W], dor[W], acc[W];
+  float qr[AF_W], dor[AF_W], acc[AF_W];
   float delta = 0.f;
 #pragma unroll
-  for (int t = 0; t < W; ++t) {
-    const int d = seg * W + t;
+  for (int t = 0; t < AF_W; ++t) {
+    const int d = seg * AF_W + t;
     const bool ok = row_ok && d < hd;
     qr[t] = ok ? q[(row0 + i) * rs + h * hd + d] * scale : 0.f;
     dor[t] = ok ? dout[(row0 + i) * os + h * hd + d] : 0.f;
     if (ok) delta = fmaf(dor[t], o[(row0 + i) * os + h * hd + d], delta);
     acc[t] = 0.f;
   }
-  delta = af_reduce<TPR>(delta);
+  delta = af_reduce<DS>(delta);
   const float L = row_ok ? lse[((long long)b * heads + h) * seq + i] : 0.f;
-  const int kend = causal ? min(seq, i0 + ROWS) : seq;
-  for (int j0 = 0; j0 < kend; j0 += AF_TILE) {
-    __syncthreads();
-    af_load_tile<TPR, W>(sK, k, rs, row0, j0, seq, h * hd, hd);
-    af_load_tile<TPR, W>(sV, v, rs, row0, j0, seq, h * hd, hd);
-    __syncthreads();
+  const int kend = causal ? min(seq, i0 + Cfg::ROWS) : seq;
+  af_stream<DS, KS>(sK, sV, k, rs, v, rs, row0, 0, kend, seq, h * hd, hd, vec, [&](int j0, const float* tk, const float* tv) {
 #pragma unroll 4
-    for (int j = 0; j < AF_TILE; ++j) {
-      const float* kr = sK + (j * TPR + seg) * af_seg<W>;
-      const float d = af_reduce<TPR>(af_dot<W>(qr, kr));
-      const float dp = af_reduce<TPR>(af_dot<W>(dor, sV + (j * TPR + seg) * af_seg<W>));
+    for (int jj = 0; jj < NJ; ++jj) {
+      const int j = jj * KS + ks;
+      const float* kr = tk + (j * DS + seg) * AF_SEG;
+      const float d = af_reduce<DS>(af_dot(qr, kr));
+      const float dp = af_reduce<DS>(af_dot(dor, tv + (j * DS + seg) * AF_SEG));
       const int kj = j0 + j;
       const bool alive = row_ok && kj < seq && (!causal || kj <= i);
       const float ds = alive ? __expf(d - L) * (dp - delta) * scale : 0.f;
-      af_axpy<W>(acc, ds, kr);
+      af_axpy(acc, ds, kr);
     }
-  }
+  });
+  af_scatter_sum<DS, KS>(acc, ks);
   if (!row_ok) return;
 #pragma unroll
-  for (int t = 0; t < W; ++t) {
-    const int d = seg * W + t;
+  for (int t = 0; t < AF_W / KS; ++t) {
+    const int d = seg * AF_W + af_first<KS>(ks) + t;
     if (d < hd) dq[(row0 + i) * ds_ + h * hd + d] = acc[t];
   }
 }
 
 // dK, dV: rows are keys; Q and dO stream through shared memory with the queries' log-sum-exp and delta.
-template <int TPR, int W>
+template <int DS, int KS>
 __global__ void __launch_bounds__(AF_THREADS)
 attn_f32_bwd_kv_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
                        const float* __restrict__ o, const float* __restrict__ dout, const float* __restrict__ lse,
                        float* __restrict__ dk, float* __restrict__ dv, int heads, int seq, int hd, long long rs, long long os,
-                       long long ds_, float scale, int causal) {
-  constexpr int ROWS = AF_THREADS / TPR;
-  __shared__ __align__(16) float sQ[AF_TILE * TPR * af_seg<W>];
-  __shared__ __align__(16) float sDO[AF_TILE * TPR * af_seg<W>];
-  __shared__ float sL[AF_TILE], sDelta[AF_TILE];
+                       long long ds_, float scale, int causal, int vec) {
+  using Cfg = AfCfg<DS, KS>;
+  constexpr int NI = AF_TILE / KS;
+  __shared__ __align__(16) float sQ[Cfg::BUFS * Cfg::TILE], sDO[Cfg::BUFS * Cfg::TILE];
+  __shared__ float sL[2][AF_TILE], sDelta[2][AF_TILE];
+  pdl_wait();
   const int h = blockIdx.y, b = blockIdx.z;
-  const int j0 = blockIdx.x * ROWS;
-  const int j = j0 + threadIdx.x / TPR, seg = threadIdx.x % TPR;
+  const int j0 = blockIdx.x * Cfg::ROWS;
+  const int j = j0 + threadIdx.x / Cfg::TPR, seg = threadIdx.x % DS, ks = threadIdx.x % Cfg::TPR / DS;
   const long long row0 = (long long)b * seq;
   const bool row_ok = j < seq;
-  float kr[W], vr[W], acck[W], accv[W];
+  float kr[AF_W], vr[AF_W], acck[AF_W], accv[AF_W];
 #pragma unroll
-  for (int t = 0; t < W; ++t) {
-    const int d = seg * W + t;
+  for (int t = 0; t < AF_W; ++t) {
+    const int d = seg * AF_W + t;
     const bool ok = row_ok && d < hd;
     kr[t] = ok ? k[(row0 + j) * rs + h * hd + d] * scale : 0.f;
     vr[t] = ok ? v[(row0 + j) * rs + h * hd + d] : 0.f;
     acck[t] = 0.f; accv[t] = 0.f;
   }
-  const int istart = causal ? (j0 / AF_TILE) * AF_TILE : 0;    // first query tile any key of this CTA can see
-  for (int i0 = istart; i0 < seq; i0 += AF_TILE) {
-    __syncthreads();
-    af_load_tile<TPR, W>(sQ, q, rs, row0, i0, seq, h * hd, hd);
-    af_load_tile<TPR, W>(sDO, dout, os, row0, i0, seq, h * hd, hd);
-    {
-      // delta of the 32 queries: 4 threads per query, shuffle-combined
-      const int r = threadIdx.x >> 2, part = threadIdx.x & 3;
-      float dl = 0.f;
-      if (i0 + r < seq)
-        for (int d = part; d < hd; d += 4) dl = fmaf(dout[(row0 + i0 + r) * os + h * hd + d], o[(row0 + i0 + r) * os + h * hd + d], dl);
-      dl += __shfl_xor_sync(0xffffffffu, dl, 1);
-      dl += __shfl_xor_sync(0xffffffffu, dl, 2);
-      if (part == 0) {
-        sDelta[r] = dl;
-        sL[r] = (i0 + r < seq) ? lse[((long long)b * heads + h) * seq + i0 + r] : INFINITY;
+  // delta and log-sum-exp of the 32 queries of a tile: 4 threads per query, shuffle-combined.  Tiles alternate between two slots, so
+  // those of the next tile can be written while the last warps still read this one's.
+  auto stats = [&](int i0, int slot) {
+    const int r = threadIdx.x >> 2, part = threadIdx.x & 3;
+    float dl = 0.f;
+    if (i0 + r < seq) {
+      const float *pd = dout + (row0 + i0 + r) * os + h * hd, *po = o + (row0 + i0 + r) * os + h * hd;
+      if (vec) {
+        for (int d = part * 4; d < hd; d += 16) {
+          const float4 a = *reinterpret_cast<const float4*>(pd + d), c = *reinterpret_cast<const float4*>(po + d);
+          dl = fmaf(a.x, c.x, fmaf(a.y, c.y, fmaf(a.z, c.z, fmaf(a.w, c.w, dl))));
+        }
+      } else {
+        for (int d = part; d < hd; d += 4) dl = fmaf(pd[d], po[d], dl);
       }
     }
-    __syncthreads();
+    dl += __shfl_xor_sync(0xffffffffu, dl, 1);
+    dl += __shfl_xor_sync(0xffffffffu, dl, 2);
+    if (part == 0) {
+      sDelta[slot][r] = dl;
+      sL[slot][r] = (i0 + r < seq) ? lse[((long long)b * heads + h) * seq + i0 + r] : INFINITY;
+    }
+  };
+  const int istart = causal ? (j0 / AF_TILE) * AF_TILE : 0;    // first query tile any key of this CTA can see
+  int slot = 0;
+  stats(istart, 0);
+  af_stream<DS, KS>(sQ, sDO, q, rs, dout, os, row0, istart, seq, seq, h * hd, hd, vec, [&](int i0, const float* tq, const float* td) {
+    if (i0 + AF_TILE < seq) stats(i0 + AF_TILE, slot ^ 1);
 #pragma unroll 4
-    for (int ii = 0; ii < AF_TILE; ++ii) {
-      const float* qrow = sQ + (ii * TPR + seg) * af_seg<W>;
-      const float* dorow = sDO + (ii * TPR + seg) * af_seg<W>;
-      const float d = af_reduce<TPR>(af_dot<W>(kr, qrow));
-      const float dp = af_reduce<TPR>(af_dot<W>(vr, dorow));
+    for (int jj = 0; jj < NI; ++jj) {
+      const int ii = jj * KS + ks;
+      const float* qrow = tq + (ii * DS + seg) * AF_SEG;
+      const float* dorow = td + (ii * DS + seg) * AF_SEG;
+      const float d = af_reduce<DS>(af_dot(kr, qrow));
+      const float dp = af_reduce<DS>(af_dot(vr, dorow));
       const int qi = i0 + ii;
       const bool alive = row_ok && qi < seq && (!causal || j <= qi);
-      const float p = alive ? __expf(d - sL[ii]) : 0.f;
-      const float ds = p * (dp - sDelta[ii]);     // the key registers carry the scale: dK = scale * dS^T Q restored below
-      af_axpy<W>(accv, p, dorow);
-      af_axpy<W>(acck, ds, qrow);
+      const float p = alive ? __expf(d - sL[slot][ii]) : 0.f;
+      const float ds = p * (dp - sDelta[slot][ii]);     // the key registers carry the scale: dK = scale * dS^T Q restored below
+      af_axpy(accv, p, dorow);
+      af_axpy(acck, ds, qrow);
     }
-  }
+    slot ^= 1;
+  });
+  af_scatter_sum<DS, KS>(acck, ks);
+  af_scatter_sum<DS, KS>(accv, ks);
   if (!row_ok) return;
 #pragma unroll
-  for (int t = 0; t < W; ++t) {
-    const int d = seg * W + t;
+  for (int t = 0; t < AF_W / KS; ++t) {
+    const int d = seg * AF_W + af_first<KS>(ks) + t;
     if (d < hd) {
       dk[(row0 + j) * ds_ + h * hd + d] = acck[t] * scale;
       dv[(row0 + j) * ds_ + h * hd + d] = accv[t];
@@ -257,15 +351,22 @@ attn_f32_bwd_kv_kernel(const float* __restrict__ q, const float* __restrict__ k,
 
 using namespace oa;
 
-// Threads per row, negative for eight dimensions per thread, which is taken up to `limit` CTAs of the wide form: one per SM, or somewhat
-// more where the causal mask lets the shorter CTAs skip work, or where a sequence leaves most rows of a wide CTA empty.  Wide against narrow
-// (4 heads of 64), forward 20 x 128 (160 CTAs) 37.7 / 36.3 us, 28 x 128 (224) 39.4 / 52.3; causal 28 x 128 39.5 / 37.5, 8 x 512 (256) 127 / 137;
-// 64 x 16 (256) 11.2 / 6.7.  Backward 20 x 128 128 / 105, 28 x 128 129 / 146, 2 x 1024 (128) 553 / 651; causal 28 x 128 127 / 113, 36 x 128
-// (288) 127 / 135.  One to two heads of 512 to 4096 positions (16 to 64 CTAs): 0.5 to 0.9 of the wide form throughout.
+// DS, or -4 DS for KS = 4, which is taken up to `limit` CTAs of the KS = 1 form: one per SM, or somewhat more where the causal mask lets the
+// shorter CTAs skip work, and wherever a sequence would leave most rows of a wide CTA empty.  KS = 1 against 4 (4 heads), forward, full mask,
+// 48 x 128 of 32 dimensions (192 CTAs) 33.8 / 33.5 us, 28 x 128 of 64 (224) 38.4 / 40.7; causal 16 x 512 of 32 (256) 107 / 98, 36 x 128 of 64 (288)
+// 38.7 / 39.4.  Backward, full, 48 x 128 of 32 (192) 123 / 103, 28 x 128 of 64 (224) 119 / 131, 14 x 128 of 64 (112) 79 / 76, but 2 x 1024 of 64 (128)
+// 470 / 489; causal 36 x 128 of 64 (288) 117 / 114.  100 x 16 of 64 (400 CTAs) 13.3 / 8.2 and 50.9 / 28.2.
 static inline int af_split(int hd, int batch, int heads, int seq, int limit) {
   const int wide = hd <= 32 ? 1 : (hd <= 64 ? 2 : 4);
   const long long ctas = (long long)((seq + AF_THREADS / wide - 1) / (AF_THREADS / wide)) * heads * batch;
-  return hd <= 64 && ctas <= (seq <= AF_TILE ? 295 : limit) ? -4 * wide : wide;
+  return hd <= 64 && (seq <= AF_TILE || ctas <= limit) ? -4 * wide : wide;
+}
+
+// Whether every row of the streamed operands can be read in 16-byte pieces.
+static int af_vec(int hd, long long rs, long long os, const void* a, const void* b, const void* c, const void* d, const void* e) {
+  const uintptr_t at = reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c) |
+                       reinterpret_cast<uintptr_t>(d) | reinterpret_cast<uintptr_t>(e);
+  return ((hd | rs | os) & 3) == 0 && (at & 15) == 0;
 }
 
 extern "C" int oa_attn_f32(const float* q, const float* k, const float* v, float* o, float* lse, int batch, int heads,
@@ -275,14 +376,16 @@ extern "C" int oa_attn_f32(const float* q, const float* k, const float* v, float
   if (batch <= 0 || heads <= 0 || seq <= 0) return OA_OK;
   if (heads > 65535 || batch > 65535) return OA_ERR_ARG;
   cudaStream_t st = (cudaStream_t)stream;
-  const int split = af_split(head_dim, batch, heads, seq, causal && head_dim > 32 ? 224 : 160), rows = AF_THREADS / (split < 0 ? -split : split);
+  const int split = af_split(head_dim, batch, heads, seq, causal ? 260 : 192), rows = AF_THREADS / (split < 0 ? -split : split);
   dim3 grid((seq + rows - 1) / rows, heads, batch);
-#define AF_FWD(T, W) attn_f32_fwd_kernel<T, W><<<grid, AF_THREADS, 0, st>>>(q, k, v, o, lse, heads, seq, head_dim, row_stride, o_row_stride, scale, causal)
-  if (split == -4) AF_FWD(4, 8);
-  else if (split == -8) AF_FWD(8, 8);
-  else if (split == 1) AF_FWD(1, 32);
-  else if (split == 2) AF_FWD(2, 32);
-  else AF_FWD(4, 32);
+  const int vec = af_vec(head_dim, row_stride, o_row_stride, q, k, v, o, o);
+#define AF_FWD(D, S) launch_short(attn_f32_fwd_kernel<D, S>, grid, dim3(AF_THREADS), 0, st, q, k, v, o, lse, heads, seq, head_dim, row_stride, \
+                                  o_row_stride, scale, causal, vec)
+  if (split == -4) AF_FWD(1, 4);
+  else if (split == -8) AF_FWD(2, 4);
+  else if (split == 1) AF_FWD(1, 1);
+  else if (split == 2) AF_FWD(2, 1);
+  else AF_FWD(4, 1);
 #undef AF_FWD
   return cudaGetLastError() == cudaSuccess ? OA_OK : OA_ERR_LAUNCH;
 }
@@ -295,18 +398,19 @@ extern "C" int oa_attn_f32_bwd(const float* q, const float* k, const float* v, c
   if (batch <= 0 || heads <= 0 || seq <= 0) return OA_OK;
   if (heads > 65535 || batch > 65535) return OA_ERR_ARG;
   cudaStream_t st = (cudaStream_t)stream;
-  const int split = af_split(head_dim, batch, heads, seq, causal ? 240 : (seq > 128 ? 96 : head_dim > 32 ? 160 : 192)), rows = AF_THREADS / (split < 0 ? -split : split);
+  const int split = af_split(head_dim, batch, heads, seq, causal ? 300 : (seq > 128 ? 96 : 192)), rows = AF_THREADS / (split < 0 ? -split : split);
   dim3 grid((seq + rows - 1) / rows, heads, batch);
-#define AF_BWD(T, W)                                                                                                             \
-  attn_f32_bwd_q_kernel<T, W><<<grid, AF_THREADS, 0, st>>>(q, k, v, o, dout, lse, dq, heads, seq, head_dim, row_stride, o_row_stride, \
-                                                        d_row_stride, scale, causal);                                            \
-  attn_f32_bwd_kv_kernel<T, W><<<grid, AF_THREADS, 0, st>>>(q, k, v, o, dout, lse, dk, dv, heads, seq, head_dim, row_stride,          \
-                                                         o_row_stride, d_row_stride, scale, causal);
-  if (split == -4) { AF_BWD(4, 8) }
-  else if (split == -8) { AF_BWD(8, 8) }
-  else if (split == 1) { AF_BWD(1, 32) }
-  else if (split == 2) { AF_BWD(2, 32) }
-  else { AF_BWD(4, 32) }
+  const int vec = af_vec(head_dim, row_stride, o_row_stride, q, k, v, o, dout);
+#define AF_BWD(D, S)                                                                                                                        \
+  launch_short(attn_f32_bwd_q_kernel<D, S>, grid, dim3(AF_THREADS), 0, st, q, k, v, o, dout, lse, dq, heads, seq, head_dim, row_stride,       \
+               o_row_stride, d_row_stride, scale, causal, vec);                                                                             \
+  launch_short(attn_f32_bwd_kv_kernel<D, S>, grid, dim3(AF_THREADS), 0, st, q, k, v, o, dout, lse, dk, dv, heads, seq, head_dim, row_stride,  \
+               o_row_stride, d_row_stride, scale, causal, vec)
+  if (split == -4) { AF_BWD(1, 4); }
+  else if (split == -8) { AF_BWD(2, 4); }
+  else if (split == 1) { AF_BWD(1, 1); }
+  else if (split == 2) { AF_BWD(2, 1); }
+  else { AF_BWD(4, 1); }
 #undef AF_BWD
   return cudaGetLastError() == cudaSuccess ? OA_OK : OA_ERR_LAUNCH;
 }
