@@ -129,6 +129,7 @@ __global__ void unary_kernel(int op, const T* __restrict__ x, T* __restrict__ y,
 template <typename T>
 __global__ void binary_kernel(int op, const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ y, long long n,
                               long long inner, int mode, float s0) {
+  pdl_wait();
   long long stride = (long long)gridDim.x * blockDim.x;
   if (mode == OA_BC_NONE) {
     constexpr int V = IO<T>::VEC;
@@ -348,6 +349,7 @@ template <typename T>
 __global__ void __launch_bounds__(512)
 col_sum_partial_kernel(const T* __restrict__ x, float* __restrict__ partial, long long rows, int cols, int rows_per_block) {
   __shared__ float sm[4][128];
+  pdl_wait();
   const int c = blockIdx.x * 128 + threadIdx.x;
   const int lane = threadIdx.y;
   const long long r0 = (long long)blockIdx.y * rows_per_block;
@@ -380,6 +382,7 @@ col_sum_partial_kernel(const T* __restrict__ x, float* __restrict__ partial, lon
 template <typename D>
 __global__ void col_sum_final_kernel(const float* __restrict__ partial, D* __restrict__ out, int nparts, int cols,
                                      int accumulate) {
+  pdl_wait();
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= cols) return;
   float s = 0.f;
@@ -598,8 +601,8 @@ extern "C" int oa_binary(int op, int dtype, const void* a, const void* b, void* 
   long long work = bcast_mode == OA_BC_NONE ? n / 4 + 1 : n;
   // leaky-relu / elu slopes travel in `inner_b` is not possible; those backward ops use slope 0.01 / alpha 1.
   float s0 = (op == OA_B_LEAKY_RELU_BWD) ? 0.01f : 1.0f;
-  DISPATCH_T(dtype, binary_kernel<T><<<grid_for(work, 256), 256, 0, ST>>>(op, (const T*)a, (const T*)b, (T*)y, n,
-                                                                         inner_b > 0 ? inner_b : 1, bcast_mode, s0));
+  DISPATCH_T(dtype, launch_short(binary_kernel<T>, dim3(grid_for(work, 256)), dim3(256), 0, ST, op, (const T*)a, (const T*)b, (T*)y, n,
+                                 inner_b > 0 ? inner_b : 1, bcast_mode, s0));
   return CHECK_LAUNCH();
 }
 // parts[t][i] (t < terms) = successive bf16 roundings of x[i]: x ~ sum_t parts[t], each term carrying the next 8 mantissa bits.
@@ -714,9 +717,10 @@ extern "C" int oa_col_sum(int dtype, const void* x, void* out, int out_dtype, lo
   const int RPB = 256;
   int nparts = (int)((rows + RPB - 1) / RPB);
   dim3 g1((cols + 127) / 128, nparts);
-  DISPATCH_T(dtype, col_sum_partial_kernel<T><<<g1, dim3(128, 4), 0, ST>>>((const T*)x, scratch, rows, cols, RPB));
-  if (out_dtype == OA_F32) col_sum_final_kernel<float><<<(cols + 127) / 128, 128, 0, ST>>>(scratch, (float*)out, nparts, cols, accumulate);
-  else col_sum_final_kernel<__nv_bfloat16><<<(cols + 127) / 128, 128, 0, ST>>>(scratch, (__nv_bfloat16*)out, nparts, cols, accumulate);
+  DISPATCH_T(dtype, launch_short(col_sum_partial_kernel<T>, g1, dim3(128, 4), 0, ST, (const T*)x, scratch, rows, cols, RPB));
+  const dim3 g2((cols + 127) / 128);
+  if (out_dtype == OA_F32) launch_short(col_sum_final_kernel<float>, g2, dim3(128), 0, ST, (const float*)scratch, (float*)out, nparts, cols, accumulate);
+  else launch_short(col_sum_final_kernel<__nv_bfloat16>, g2, dim3(128), 0, ST, (const float*)scratch, (__nv_bfloat16*)out, nparts, cols, accumulate);
   return CHECK_LAUNCH();
 }
 extern "C" int oa_bias_add(int dtype, void* x, const void* bias, long long rows, int cols, void* stream) {

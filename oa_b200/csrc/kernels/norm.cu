@@ -475,6 +475,7 @@ template <typename T>
 __global__ void __launch_bounds__(NORM_THREADS)
 layernorm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ w, const T* __restrict__ b, T* __restrict__ y,
                      float* __restrict__ mean_out, float* __restrict__ rstd_out, long long rows, int cols, float eps) {
+  pdl_wait();
   constexpr int V = NIO<T>::VEC;
   const int lane = threadIdx.x & 31;
   const long long warp_global = (long long)blockIdx.x * NORM_WARPS + (threadIdx.x >> 5);
@@ -525,6 +526,7 @@ layernorm_bwd_kernel(const T* __restrict__ x, const T* __restrict__ w, const T* 
   const int warp = threadIdx.x >> 5;
   for (int i = threadIdx.x; i < warps_used * 2 * cols; i += blockDim.x) s_acc[i] = 0.f;
   __syncthreads();
+  pdl_wait();
   if (warp < warps_used) {
     float* my_dw = s_acc + (size_t)warp * 2 * cols;
     float* my_db = my_dw + cols;
@@ -690,7 +692,7 @@ static int set_smem(K kernel, size_t bytes) {
 
 static void partial_rows_sum(const float* partial, void* out, int out_dtype, int nparts, int cols, int accumulate, cudaStream_t st) {
   const dim3 grid((cols + 31) / 32);
-#define OA_PSUM(D, THREADS) launch_pdl(partial_rows_sum_kernel<D, THREADS>, grid, dim3(THREADS), 0, st, partial, (D*)out, nparts, cols, accumulate)
+#define OA_PSUM(D, THREADS) launch_short(partial_rows_sum_kernel<D, THREADS>, grid, dim3(THREADS), 0, st, partial, (D*)out, nparts, cols, accumulate)
   if (out_dtype == OA_F32) {
     if (nparts <= PSUM_FEW) OA_PSUM(float, 256);
     else OA_PSUM(float, 1024);
@@ -761,9 +763,9 @@ extern "C" int oa_layernorm_fwd(int dtype, const void* x, const void* w, const v
   long long nb = (rows + NORM_WARPS - 1) / NORM_WARPS;
   if (nb > 148 * 8) nb = 148 * 8;
   if (dtype == OA_F32)
-    layernorm_fwd_kernel<float><<<(int)nb, NORM_THREADS, 0, ST>>>((const float*)x, (const float*)w, (const float*)b, (float*)y, mean, rstd, rows, cols, eps);
+    launch_short(layernorm_fwd_kernel<float>, dim3((unsigned)nb), dim3(NORM_THREADS), 0, ST, (const float*)x, (const float*)w, (const float*)b, (float*)y, mean, rstd, rows, cols, eps);
   else if (dtype == OA_BF16)
-    layernorm_fwd_kernel<__nv_bfloat16><<<(int)nb, NORM_THREADS, 0, ST>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (const __nv_bfloat16*)b, (__nv_bfloat16*)y, mean, rstd, rows, cols, eps);
+    launch_short(layernorm_fwd_kernel<__nv_bfloat16>, dim3((unsigned)nb), dim3(NORM_THREADS), 0, ST, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (const __nv_bfloat16*)b, (__nv_bfloat16*)y, mean, rstd, rows, cols, eps);
   else return OA_ERR_UNSUPPORTED;
   return CHECK_LAUNCH();
 }
@@ -781,10 +783,10 @@ extern "C" int oa_layernorm_bwd(int dtype, const void* x, const void* w, const v
   int rc;
   if (dtype == OA_F32) {
     if ((rc = set_smem(layernorm_bwd_kernel<float>, smem))) return rc;
-    layernorm_bwd_kernel<float><<<blocks, NORM_THREADS, smem, ST>>>((const float*)x, (const float*)w, (const float*)dy, mean, rstd, (float*)dx, rows, cols, scratch, warps, blocks);
+    launch_short(layernorm_bwd_kernel<float>, dim3(blocks), dim3(NORM_THREADS), smem, ST, (const float*)x, (const float*)w, (const float*)dy, mean, rstd, (float*)dx, rows, cols, scratch, warps, blocks);
   } else if (dtype == OA_BF16) {
     if ((rc = set_smem(layernorm_bwd_kernel<__nv_bfloat16>, smem))) return rc;
-    layernorm_bwd_kernel<__nv_bfloat16><<<blocks, NORM_THREADS, smem, ST>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (const __nv_bfloat16*)dy, mean, rstd, (__nv_bfloat16*)dx, rows, cols, scratch, warps, blocks);
+    launch_short(layernorm_bwd_kernel<__nv_bfloat16>, dim3(blocks), dim3(NORM_THREADS), smem, ST, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (const __nv_bfloat16*)dy, mean, rstd, (__nv_bfloat16*)dx, rows, cols, scratch, warps, blocks);
   } else return OA_ERR_UNSUPPORTED;
   float* part_db = scratch + (size_t)blocks * cols;
   if (dw) partial_rows_sum(scratch, dw, dw_dtype, blocks, cols, accumulate_dw, ST);

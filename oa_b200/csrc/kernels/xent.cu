@@ -210,6 +210,7 @@ __global__ void __launch_bounds__(XENT_THREADS)
 xent_warp_kernel(const T* __restrict__ logits, const int* __restrict__ targets, float* __restrict__ row_loss, T* dlogits,
                  long long rows, int vocab, int ld, float grad_scale, int ignore_index) {
   constexpr int V = XIO<T>::VEC, NV = XENT_WARP_VECS;
+  pdl_wait();
   const long long row = (long long)blockIdx.x * (XENT_THREADS / 32) + (threadIdx.x >> 5);
   if (row >= rows) return;
   const int lane = threadIdx.x & 31, nvec = vocab / V;
@@ -266,7 +267,7 @@ static int launch_xent(const T* logits, const int* targets, float* row_loss, T* 
   const size_t smem = (size_t)nvec * 16;
   if (vec_ok && vocab % V == 0 && nvec <= XENT_WARP_VECS * 32) {
     const unsigned blocks = (unsigned)((rows + XENT_THREADS / 32 - 1) / (XENT_THREADS / 32));
-    xent_warp_kernel<T><<<blocks, XENT_THREADS, 0, st>>>(logits, targets, row_loss, dlogits, rows, vocab, ld, grad_scale, ignore_index);
+    launch_short(xent_warp_kernel<T>, dim3(blocks), dim3(XENT_THREADS), 0, st, logits, targets, row_loss, dlogits, rows, vocab, ld, grad_scale, ignore_index);
   } else if (vec_ok && smem > 0 && smem <= XENT_SMEM_MAX && xent_row_on_chip(smem, rows, dlogits != nullptr, sizeof(T))) {
     // eight vectors or so per thread: fewer threads leave the copies of short rows in flight together with the next CTA's
     auto go = [&](auto kernel, int threads) -> int {
@@ -288,6 +289,7 @@ static int launch_xent(const T* logits, const int* targets, float* row_loss, T* 
 // out[0] = scale * sum(x), one CTA, fixed reduction order.
 __global__ void mean_f32_kernel(const float* __restrict__ x, float* __restrict__ out, long long n, float scale) {
   __shared__ float red[32];
+  pdl_wait();
   float s = 0.f;
   for (long long i = threadIdx.x; i < n; i += blockDim.x) s += x[i];
   s = warp_sum(s);
@@ -423,6 +425,6 @@ extern "C" int oa_vp_xent_finish(int dtype, void* logits, const int* targets, co
 }
 
 extern "C" int oa_mean_f32(const float* x, float* out, long long n, float scale, void* stream) {
-  mean_f32_kernel<<<1, 1024, 0, (cudaStream_t)stream>>>(x, out, n, scale);
+  oa::launch_short(mean_f32_kernel, dim3(1), dim3(1024), 0, (cudaStream_t)stream, x, out, n, scale);
   return cudaGetLastError() == cudaSuccess ? OA_OK : OA_ERR_LAUNCH;
 }
