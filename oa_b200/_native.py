@@ -129,7 +129,8 @@ def ptr(t: Optional[torch.Tensor]) -> Optional[int]:
 
 
 def stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """The current stream's handle, without the Python object around it: every launch asks for it."""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 _launch_count = 0

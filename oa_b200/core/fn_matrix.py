@@ -553,7 +553,12 @@ def _repeat_bwd(g, shape, dim, repeats):
 
 # ======================================================================= reductions
 def _rows(t: torch.Tensor):
-    return _c(t).reshape(-1, t.shape[-1])
+    t = _c(t)
+    return t if t.dim() == 2 else t.reshape(-1, t.shape[-1])
+
+
+def _as(t: torch.Tensor, shape) -> torch.Tensor:
+    return t if t.shape == shape else t.reshape(shape)
 
 
 def Sum(m: OaMatrix, dim: Optional[int] = None) -> OaMatrix:
@@ -830,14 +835,14 @@ def RmsNorm(x: OaMatrix, w: OaMatrix, eps: float = 1e-6) -> OaMatrix:
     tx, tw = x.Tensor(), w.Tensor()
     x2 = _rows(tx)
     y, rstd, _ = K.rmsnorm_fwd(x2, tw, eps)
-    out = _w(y.reshape(tx.shape))
+    out = _w(_as(y, tx.shape))
 
     def back(g, pending=None):
         # `pending`: what x has already collected through the residual stream; the kernel adds it while it writes dx
         sink = w.GradSink() if (w.IsLeaf() and w.RequiresGrad()) else None
         dres = _rows(pending) if (pending is not None and pending.is_contiguous()) else None
         dx, dw = K.rmsnorm_bwd(x2, tw, _rows(g), rstd, dres=dres, dw_out=sink[0] if sink else None, accumulate_dw=bool(sink and sink[1]))
-        dx = dx.reshape(tx.shape)
+        dx = _as(dx, tx.shape)
         if pending is not None and dres is None:
             dx = K.binary("add", pending, dx)
         return (dx, None if sink else dw)
@@ -871,7 +876,7 @@ def LayerNorm(x: OaMatrix, w: OaMatrix, b: Optional[OaMatrix], eps: float = 1e-5
     x2 = _rows(tx)
     tw = w.Tensor()
     y, mean, rstd = K.layernorm_fwd(x2, tw, b.Tensor() if b is not None else None, eps)
-    out = _w(y.reshape(tx.shape))
+    out = _w(_as(y, tx.shape))
 
     def back(g):
         ws = w.GradSink() if (w.IsLeaf() and w.RequiresGrad()) else None
@@ -880,7 +885,7 @@ def LayerNorm(x: OaMatrix, w: OaMatrix, b: Optional[OaMatrix], eps: float = 1e-5
             ws = bs = None  # mixed states: fall back to returned gradients
         dx, dw, db = K.layernorm_bwd(x2, tw, _rows(g), mean, rstd, dw_out=ws[0] if ws else None,
                                      db_out=bs[0] if bs else None, accumulate=bool(ws and ws[1]), want_bias=b is not None)
-        return (dx.reshape(tx.shape), None if ws else dw, None if bs else db)
+        return (_as(dx, tx.shape), None if ws else dw, None if bs else db)
 
     return AG.attach("LayerNorm", out, [x, w, b], back)
 

@@ -151,7 +151,7 @@ class OaGradientTape:
                     if pending is not None:
                         _count_down(fn, pending, hook)
                     continue
-                if tuple(up.shape) != fn.out_shape and up.numel() == _numel(fn.out_shape):
+                if up.shape != fn.out_shape and up.numel() == _numel(fn.out_shape):
                     up = up.reshape(fn.out_shape)
                 folded = None
                 if fn.fold is None:
@@ -162,14 +162,15 @@ class OaGradientTape:
                     if fchild is not None:
                         prev = grad_map.get(id(fchild))
                         ft = fi.Tensor()
-                        if prev is not None and tuple(prev.shape) == tuple(ft.shape) and prev.dtype == ft.dtype:
+                        if prev is not None and prev.shape == ft.shape and prev.dtype == ft.dtype:
                             folded = prev
                     in_grads = fn.backward(up, folded)
                 for idx, (inp, d) in enumerate(zip(fn.inputs, in_grads)):
                     if inp is None or d is None or not inp.RequiresGrad():
                         continue
-                    if tuple(d.shape) != tuple(inp.Tensor().shape) and d.numel() == inp.NumElements():
-                        d = d.reshape(inp.Tensor().shape)
+                    shape = inp.Tensor().shape
+                    if d.shape != shape and d.numel() == inp.NumElements():
+                        d = d.reshape(shape)
                     if inp.IsLeaf():
                         inp.AccumulateGradTensor(d)
                         continue
@@ -180,7 +181,7 @@ class OaGradientTape:
                     if prev is None or (folded is not None and idx == fn.fold):
                         grad_map[id(child)] = d            # first contribution, or one that already contains the pending gradient
                     else:
-                        if tuple(d.shape) != tuple(prev.shape):
+                        if d.shape != prev.shape:
                             d = d.reshape(prev.shape)
                         grad_map[id(child)] = K.binary("add", prev, d if d.dtype == prev.dtype else d.to(prev.dtype))
                 if pending is not None:

@@ -684,6 +684,11 @@ def dropout(x: torch.Tensor, p: float, seed: int, offset: int, state: Optional[t
 
 
 # ---------------------------------------------------------------- norms
+@functools.lru_cache(maxsize=1024)
+def _norm_bwd_scratch_bytes(rows: int, cols: int) -> int:
+    return N.require().oa_norm_bwd_scratch_bytes(rows, cols)
+
+
 def rmsnorm_fwd(x, w, eps, residual=None):
     """Returns (y, rstd, residual_out).  With `residual`, normalises x + residual and also returns that sum."""
     rows, cols = x.shape
@@ -720,7 +725,7 @@ def rmsnorm_bwd(x, w, dy, rstd, *, dres=None, dw_out=None, accumulate_dw=False):
         s = (df * xh).sum(0)
         dw.copy_(s + dw.float() if accumulate_dw else s)
         return dx, dw
-    sc = scratch(x.device, N.require().oa_norm_bwd_scratch_bytes(rows, cols), "norm")
+    sc = scratch(x.device, _norm_bwd_scratch_bytes(rows, cols), "norm")
     _launch(N.require().oa_rmsnorm_bwd(dt(x), x.data_ptr(), w.data_ptr(), dy.data_ptr(), rstd.data_ptr(), dx.data_ptr(),
                                        dw.data_ptr(), dt(dw), rows, cols, N.ptr(dres), sc.data_ptr(), int(accumulate_dw),
                                        N.stream()), "oa_rmsnorm_bwd", 2)
@@ -764,7 +769,7 @@ def layernorm_bwd(x, w, dy, mean, rstd, *, dw_out=None, db_out=None, accumulate=
             sb = df.sum(0)
             db.copy_(sb + db.float() if accumulate else sb)
         return dx, dw, db
-    sc = scratch(x.device, N.require().oa_norm_bwd_scratch_bytes(rows, cols), "norm")
+    sc = scratch(x.device, _norm_bwd_scratch_bytes(rows, cols), "norm")
     _launch(N.require().oa_layernorm_bwd(dt(x), x.data_ptr(), w.data_ptr(), dy.data_ptr(), mean.data_ptr(), rstd.data_ptr(),
                                          dx.data_ptr(), dw.data_ptr(), N.ptr(db), dt(dw), rows, cols, sc.data_ptr(),
                                          int(accumulate), N.stream()), "oa_layernorm_bwd", 3)

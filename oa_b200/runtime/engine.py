@@ -127,6 +127,7 @@ class OaContext:
     """Recorder + executor bound to one CUDA stream (or to the CPU)."""
 
     _tls = threading.local()
+    _collect: Optional[list] = None       # nodes of the step being collected
 
     def __init__(self, engine: "OaEngine"):
         self._engine = engine
@@ -169,7 +170,7 @@ class OaContext:
     def Add(self, kernel: str, reads=(), writes=()) -> None:
         """Notes one recorded kernel node. Buffers are identified by their storage address."""
         self._interval_nodes += 1
-        collecting = getattr(self, "_collect", None) is not None
+        collecting = self._collect is not None
         if self._recording or collecting:
             node = (kernel, tuple(_buf_id(t) for t in reads), tuple(_buf_id(t) for t in writes))
             if self._recording:
