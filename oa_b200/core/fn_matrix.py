@@ -737,6 +737,21 @@ def _bias_grad(bias: Optional[OaMatrix], g2: torch.Tensor):
     return K.col_sum(g2)
 
 
+def _weight_bias_grad(w: OaMatrix, tw: torch.Tensor, b: Optional[OaMatrix], gz: torch.Tensor, x2: torch.Tensor):
+    """Gradients of a linear layer's weight and bias, None where there is none or a leaf's buffer has taken it."""
+    want_w, want_b = w is not None and w.RequiresGrad(), b is not None and b.RequiresGrad()
+    if not want_w:
+        return None, _bias_grad(b, gz)
+    buf, acc, direct = _grad_out(w, tw.shape, tw.dtype, tw.device)
+    if not want_b:
+        K.gemm(gz, x2, a_mn=True, b_mn=True, out=buf, accumulate=acc)
+        return (None if direct else buf), None
+    sink = b.GradSink() if b.IsLeaf() else None
+    db = sink[0] if sink is not None else torch.empty(gz.shape[1], dtype=gz.dtype, device=gz.device)
+    K.weight_grad(gz, x2, out=buf, accumulate=acc, bias_out=db, bias_accumulate=bool(sink and sink[1]))
+    return (None if direct else buf), (None if sink is not None else db)
+
+
 def Linear(x: OaMatrix, w: OaMatrix, b: Optional[OaMatrix] = None, act: int = K.ACT_NONE, name: str = "Linear",
            residual: Optional[OaMatrix] = None) -> OaMatrix:
     """y = act(x @ W^T + b) (+ residual); W is [out, in].  act in {none, gelu, relu} is fused in the GEMM epilogue,
@@ -759,12 +774,7 @@ def Linear(x: OaMatrix, w: OaMatrix, b: Optional[OaMatrix] = None, act: int = K.
         else:
             gz = g2
         dx = K.gemm(gz, tw, b_mn=True).reshape(tx.shape) if x.RequiresGrad() else None
-        dw = None
-        if w.RequiresGrad():
-            buf, acc, direct = _grad_out(w, tw.shape, tw.dtype, tw.device)
-            K.gemm(gz, x2, a_mn=True, b_mn=True, out=buf, accumulate=acc)
-            dw = None if direct else buf
-        db = _bias_grad(b, gz)
+        dw, db = _weight_bias_grad(w, tw, b, gz, x2)
         if residual is not None:
             return (dx, dw, db, g)
         return (dx, dw, db)

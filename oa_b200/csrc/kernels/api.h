@@ -63,6 +63,9 @@ int oa_gemm_bf16_grouped(int mode, const void* A, const void* B, void* out, int 
 // and, oa_gemm_f32_epi: v = alpha * sum + bias;  aux_out = v;  v = act(v) or v * act'(aux_in);  C = v + residual (+ C if accumulate).
 // residual and aux_* are [M, N] with unit column stride.  `scratch`: oa_gemm_f32_scratch_floats() floats of this call's own, or null:
 // the reduction is not sliced.
+// C (+)= A^T B and a_sum (+)= the column sums of A, A [K, M] and B [K, N] row-contiguous; OA_ERR_UNSUPPORTED where rows are not on 16 bytes.
+int oa_gemm_f32_weight_grad(const float* A, const float* B, float* C, int M, int N, int K, long long lda, long long ldb,
+                            int ldc, int accumulate, float* a_sum, int a_sum_accumulate, float* scratch, void* stream);
 size_t oa_gemm_f32_scratch_floats(int M, int N, int K, int batch);
 int oa_gemm_f32(const float* A, const float* B, float* C, int M, int N, int K, long long sam, long long sak,
                 long long sbn, long long sbk, int ldc, int batch, long long batch_a, long long batch_b,

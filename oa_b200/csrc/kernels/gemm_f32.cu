@@ -25,6 +25,8 @@ struct F32Epi {
   float* aux_out;
   int ldr, ldaux, act, accumulate;
   float alpha;
+  float* a_sum = nullptr;        // [M]: also the sums of A over K (bias gradient beside a weight gradient), by the blocks of the first columns
+  int a_sum_accumulate = 0;
 };
 
 // Not inlined: sixteen copies of tanhf and its gradient made the epilogue some tens of kilobytes of code, and a launch of a few
@@ -46,6 +48,20 @@ __device__ __forceinline__ float f32_epilogue(const F32Epi& e, float acc, int m,
   if (e.residual) v += e.residual[(long long)m * e.ldr + n];
   if (e.accumulate) v += *c;
   return v;
+}
+
+// sum += v with what the addition loses carried on (Kahan): a thread adds up all of K, where separate column sums had short chains, and
+// one after the other 500 terms lost four times as much
+__device__ __forceinline__ void f32_add_kept(float& sum, float& lost, float v) {
+  const float y = v - lost, t = sum + y;
+  const float e = (t - sum) - y;
+  lost = fabsf(e) <= 3.4028235e38f ? e : 0.f;            // an infinite sum stays one
+  sum = t;
+}
+__device__ __forceinline__ void f32_store_sum(const F32Epi& e, float s, int m, int M, int slice) {
+  if (m >= M) return;
+  float* o = e.a_sum + (long long)slice * M + m;
+  *o = e.a_sum_accumulate ? *o + s : s;
 }
 
 __global__ void __launch_bounds__(256)
@@ -217,6 +233,8 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ B, f
   constexpr int PR = PAIR == 1 ? 4 : 8, PC = PAIR == 2 ? 2 : 4;
   using Acc = typename std::conditional<PAIR == 0, float, unsigned long long>::type;
   Acc acc[PR][PC] = {};
+  const bool sums = A_MN && epi.a_sum && blockIdx.x == 0 && threadIdx.x < ROWS;
+  float a_sum = 0.f, a_lost = 0.f;
   int at = 0;
   for (int i = 0; i < steps; ++i) {
     asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
@@ -224,6 +242,14 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ B, f
     load();
     const float *pa = ring + at * STAGE, *pb = pa + TA::FLOATS;
     if (++at == STAGES) at = 0;
+    if constexpr (A_MN) {
+      if (sums) {
+        float v = 0.f;
+#pragma unroll
+        for (int k = 0; k < KW; ++k) v += pa[k * TA::PITCH + threadIdx.x];
+        f32_add_kept(a_sum, a_lost, v);
+      }
+    }
 #pragma unroll
     for (int kk = 0; kk < 8; kk += 4) {
       const int k0 = group * 8 + kk;
@@ -278,6 +304,7 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ B, f
       }
     }
   }
+  if (A_MN && sums) f32_store_sum(epi, a_sum, m0 + threadIdx.x, M, k_chunk > 0 ? b : 0);
   pdl_launch_dependents();
   __syncthreads();                                    // the last stage has been read; the copies still counted are empty
   {
@@ -365,11 +392,21 @@ gemm_f32_brief_kernel(const float* __restrict__ A, const float* __restrict__ B, 
 #pragma unroll
   for (int i = 0; i < FS - 1; ++i) load(i);
   float acc[TM][4] = {};
+  const bool sums = A_MN && epi.a_sum && blockIdx.x == 0 && threadIdx.x < ROWS;
+  float a_sum = 0.f, a_lost = 0.f;
   for (int i = 0; i < steps; ++i) {
     asm volatile("cp.async.wait_group %0;" ::"n"(FS - 2) : "memory");
     __syncthreads();                                  // stage i has landed everywhere, stage i - 1 has been read
     load(i + FS - 1);
     const float *pa = sA[i % FS], *pb = sB[i % FS];
+    if constexpr (A_MN) {
+      if (sums) {
+        float v = 0.f;
+#pragma unroll
+        for (int k = 0; k < FK; ++k) v += pa[k * FP_MN + threadIdx.x];
+        f32_add_kept(a_sum, a_lost, v);
+      }
+    }
 #pragma unroll
     for (int kk = 0; kk < FK; kk += 4) {
       float a[4][TM], bb[4][4];                       // [k][row], [k][column]
@@ -410,6 +447,7 @@ gemm_f32_brief_kernel(const float* __restrict__ A, const float* __restrict__ B, 
           for (int c = 0; c < 4; ++c) acc[r][c] = fmaf(a[k][r], bb[k][c], acc[r][c]);
     }
   }
+  if (A_MN && sums) f32_store_sum(epi, a_sum, m0 + threadIdx.x, M, k_chunk > 0 ? b : 0);
 #pragma unroll
   for (int r = 0; r < TM; ++r) {
     const int gm = m0 + (A_MN ? ty * TM + r : ty + TY * r);
@@ -454,9 +492,15 @@ static bool gemm_f32_tiles(const float* A, const float* B, float* C, int M, int 
 }
 
 // C[m,n] = epilogue(sum_s part[s][m,n]): fixed slice order, so the split-K result is reproducible
-__global__ void gemm_f32_splitk_reduce_kernel(const float* __restrict__ part, float* __restrict__ C, int M, int N, int ldc, int splits, const F32Epi epi) {
+__global__ void gemm_f32_splitk_reduce_kernel(const float* __restrict__ part, const float* __restrict__ part_sum, float* __restrict__ C, int M, int N, int ldc,
+                                              int splits, const F32Epi epi) {
   pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (epi.a_sum && i < M) {
+    float s = 0.f;
+    for (int k = 0; k < splits; ++k) s += part_sum[(long long)k * M + i];
+    f32_store_sum(epi, s, (int)i, M, 0);
+  }
   if (i >= (long long)M * N) return;
   const int m = (int)(i / N), n = (int)(i % N);
   float s = 0.f;
@@ -485,17 +529,19 @@ static int gemm_f32(const float* A, const float* B, float* C, int M, int N, int 
                     int ldc, int batch, long long batch_a, long long batch_b, long long batch_c, const oa::F32Epi& epi, float* scratch, void* stream) {
   if (M <= 0 || N <= 0 || batch <= 0) return OA_OK;
   if (K < 0 || batch > 65535) return OA_ERR_ARG;
-  const oa::F32Epi part_epi{nullptr, nullptr, nullptr, nullptr, 0, 0, OA_ACT_NONE, 0, 1.0f};
+  oa::F32Epi part_epi{nullptr, nullptr, nullptr, nullptr, 0, 0, OA_ACT_NONE, 0, 1.0f};
   dim3 grid((N + oa::FT - 1) / oa::FT, (M + oa::FT - 1) / oa::FT, batch);
   cudaStream_t st = (cudaStream_t)stream;
   int k_chunk = 0;
   const int splits = scratch ? oa::f32_splits(M, N, K, batch, &k_chunk) : 1;
   if (splits >= 2) {
     grid.z = splits;
+    float* part_sum = scratch + (long long)splits * M * N;
+    if (epi.a_sum) part_epi.a_sum = part_sum;
     if (!oa::gemm_f32_tiles(A, B, scratch, M, N, K, sam, sak, sbn, sbk, N, 1, 0, 0, (long long)M * N, part_epi, k_chunk, splits, st))
       oa::gemm_f32_kernel<<<grid, 256, 0, st>>>(A, B, scratch, M, N, K, sam, sak, sbn, sbk, N, 0, 0, (long long)M * N, part_epi, k_chunk);
     const long long n = (long long)M * N;
-    oa::launch_short(oa::gemm_f32_splitk_reduce_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, st, (const float*)scratch, C, M, N, ldc, splits, epi);
+    oa::launch_short(oa::gemm_f32_splitk_reduce_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, st, (const float*)scratch, (const float*)part_sum, C, M, N, ldc, splits, epi);
     return cudaGetLastError() == cudaSuccess ? OA_OK : OA_ERR_LAUNCH;
   }
   if (!oa::gemm_f32_tiles(A, B, C, M, N, K, sam, sak, sbn, sbk, ldc, batch, batch_a, batch_b, batch_c, epi, 0, 0, st))
@@ -509,7 +555,7 @@ extern "C" size_t oa_gemm_f32_scratch_floats(int M, int N, int K, int batch) {
   int k_chunk = 0;
   if (M <= 0 || N <= 0) return 0;
   const int splits = oa::f32_splits(M, N, K, batch, &k_chunk);
-  return splits >= 2 ? (size_t)splits * M * N : 0;
+  return splits >= 2 ? (size_t)splits * M * (N + 1) : 0;   // + the sums of A, when they are asked for
 }
 
 extern "C" int oa_gemm_f32(const float* A, const float* B, float* C, int M, int N, int K, long long sam, long long sak,
@@ -526,4 +572,17 @@ extern "C" int oa_gemm_f32_epi(const float* A, const float* B, float* C, int M, 
   if ((act == OA_ACT_GELU_BWD || act == OA_ACT_RELU_BWD) && !aux_in) return OA_ERR_ARG;
   return gemm_f32(A, B, C, M, N, K, sam, sak, sbn, sbk, ldc, 1, 0, 0, 0, oa::F32Epi{bias, residual, aux_in, aux_out, ldr, ldaux, act, accumulate, alpha},
                   scratch, stream);
+}
+
+// C[M, N] (+)= A^T B for row-contiguous A [K, M] and B [K, N] (a weight gradient), and a_sum[M] (+)= the column sums of A (the bias
+// gradient) from the same tiles.  OA_ERR_UNSUPPORTED: the operands do not fit the tile kernels, nothing was done.
+extern "C" int oa_gemm_f32_weight_grad(const float* A, const float* B, float* C, int M, int N, int K, long long lda, long long ldb, int ldc, int accumulate,
+                                       float* a_sum, int a_sum_accumulate, float* scratch, void* stream) {
+  if (M <= 0 || N <= 0 || K <= 0 || ((lda | ldb) & 3) || lda < 0 || ldb < 0 || ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B)) & 15) ||
+      (M + 31) / 32 > 65535)
+    return OA_ERR_UNSUPPORTED;
+  oa::F32Epi epi{nullptr, nullptr, nullptr, nullptr, 0, 0, OA_ACT_NONE, accumulate, 1.0f};
+  epi.a_sum = a_sum;
+  epi.a_sum_accumulate = a_sum_accumulate;
+  return gemm_f32(A, B, C, M, N, K, 1, lda, 1, ldb, ldc, 1, 0, 0, 0, epi, scratch, stream);
 }

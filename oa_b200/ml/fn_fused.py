@@ -72,8 +72,14 @@ def PackedProjection(x: OaMatrix, weights: Sequence[OaMatrix], biases: Sequence[
         g2 = F._rows(g)
         dx = K.gemm(g2, w, b_mn=True).reshape(tx.shape) if x.RequiresGrad() else None
         res = [dx]
+        with_bias = False
         if gw is not None and all(p.IsLeaf() for p in weights):
-            K.gemm(g2, x2, a_mn=True, b_mn=True, out=gw, accumulate=_sink_state(weights))
+            acc = _sink_state(weights)
+            with_bias = has_bias and gb is not None and all(p.IsLeaf() for p in biases)
+            if with_bias:
+                K.weight_grad(g2, x2, out=gw, accumulate=acc, bias_out=gb, bias_accumulate=_sink_state(biases))
+            else:
+                K.gemm(g2, x2, a_mn=True, b_mn=True, out=gw, accumulate=acc)
             res += [None] * len(weights)
         else:
             dw = K.gemm(g2, x2, a_mn=True, b_mn=True)
@@ -81,7 +87,9 @@ def PackedProjection(x: OaMatrix, weights: Sequence[OaMatrix], biases: Sequence[
             for p in weights:
                 res.append(dw[o:o + p.Size(0)])
                 o += p.Size(0)
-        if has_bias:
+        if with_bias:
+            res += [None] * len(biases)
+        elif has_bias:
             if gb is not None and all(p.IsLeaf() for p in biases):
                 K.col_sum(g2, out=gb, accumulate=_sink_state(biases))
                 res += [None] * len(biases)
@@ -115,23 +123,12 @@ def FfnGelu(x: OaMatrix, w1: OaMatrix, b1: Optional[OaMatrix], w2: OaMatrix, b2:
     def back(g):
         g2 = F._rows(g)
         dz = K.gemm(g2, tw2, b_mn=True, act=bwd_act, aux_in=z)
-        dw2 = _weight_grad(w2, g2, h)
-        db2 = F._bias_grad(b2, g2)
-        dw1 = _weight_grad(w1, dz, x2)
-        db1 = F._bias_grad(b1, dz)
+        dw2, db2 = F._weight_bias_grad(w2, tw2, b2, g2, h)
+        dw1, db1 = F._weight_bias_grad(w1, tw1, b1, dz, x2)
         dx = K.gemm(dz, tw1, b_mn=True).reshape(tx.shape) if x.RequiresGrad() else None
         return (dx, dw1, db1, dw2, db2, g if residual is not None else None)
 
     return AG.attach("FfnGelu", out, [x, w1, b1, w2, b2, residual], back)
-
-
-def _weight_grad(w: OaMatrix, g2: torch.Tensor, x2: torch.Tensor):
-    if w is None or not w.RequiresGrad():
-        return None
-    tw = w.Tensor()
-    buf, acc, direct = F._grad_out(w, tw.shape, tw.dtype, tw.device)
-    K.gemm(g2, x2, a_mn=True, b_mn=True, out=buf, accumulate=acc)
-    return None if direct else buf
 
 
 def FfnSwiglu(x: OaMatrix, gate_w: OaMatrix, up_w: OaMatrix, down_w: OaMatrix, residual: Optional[OaMatrix] = None) -> OaMatrix:

@@ -324,6 +324,23 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     raise N.OaKernelError(f"gemm: unsupported dtype {a.dtype}")
 
 
+def weight_grad(dy: torch.Tensor, x: torch.Tensor, *, out: torch.Tensor, accumulate: bool, bias_out: torch.Tensor, bias_accumulate: bool) -> None:
+    """out (+)= dy^T x and bias_out (+)= the column sums of dy; in fp32 the same tiles give both."""
+    if dy.is_cuda and dy.dtype == torch.float32 and not _f32_tensor_terms and dy.stride(1) == 1 and x.stride(1) == 1 and out.stride(1) == 1 \
+            and out.dtype == torch.float32 and bias_out.dtype == torch.float32 and bias_out.is_contiguous():
+        K, M = dy.shape
+        Nn = x.shape[1]
+        if x.shape[0] == K and tuple(out.shape) == (M, Nn) and bias_out.numel() == M:
+            sc = _f32_scratch(M, Nn, K, 1, dy.device)
+            rc = N.require().oa_gemm_f32_weight_grad(dy.data_ptr(), x.data_ptr(), out.data_ptr(), M, Nn, K, dy.stride(0), x.stride(0), out.stride(0),
+                                                     int(accumulate), bias_out.data_ptr(), int(bias_accumulate), N.ptr(sc), N.stream())
+            if rc != C["OA_ERR_UNSUPPORTED"]:
+                _launch(rc, "oa_gemm_f32_weight_grad", outputs=(out, bias_out))
+                return
+    gemm(dy, x, a_mn=True, b_mn=True, out=out, accumulate=accumulate)
+    col_sum(dy, out=bias_out, accumulate=bias_accumulate)
+
+
 def bgemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = False, out: Optional[torch.Tensor] = None,
           out_dtype: Optional[torch.dtype] = None, accumulate: bool = False, alpha: float = 1.0,
           residual: Optional[torch.Tensor] = None) -> torch.Tensor:

@@ -38,3 +38,24 @@ def test_attention_rows_off_16_bytes(hd, off):
     o2, lse2 = K.flash_fwd(*clean, batch, seq, heads, hd)
     for a, e in zip(got, (o2, *K.flash_bwd(*clean, o2, do, lse2, batch, seq, heads, hd))):
         assert float((a - e).norm() / e.norm()) <= 1e-6       # the same sums but for the delta's, whose order follows the loads
+
+
+# Weight and bias gradient from one product: in one piece, sliced, off the tile and with rows that the tile kernels do not take.
+@pytest.mark.parametrize("rows,m,n", [(1, 4, 4), (37, 65, 12), (600, 70, 33), (2048, 128, 512), (2048, 512, 128), (500, 1000, 1400), (130, 700, 1500)])
+@pytest.mark.parametrize("accumulate", [False, True])
+@pytest.mark.parametrize("off", [0, 1])
+def test_weight_and_bias_gradient(rows, m, n, accumulate, off):
+    g = torch.Generator(device="cuda").manual_seed(rows + m + n)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    dy, x = r(rows, (m + 7) // 4 * 4)[:, off:off + m], r(rows, (n + 3) // 4 * 4)[:, :n]
+    w, b = r(m, n), r(m)
+    want_w, want_b = dy.double().t() @ x.double(), dy.double().sum(0)
+    if accumulate:
+        want_w, want_b = want_w + w.double(), want_b + b.double()
+    K.weight_grad(dy, x, out=w, accumulate=accumulate, bias_out=b, bias_accumulate=accumulate)
+    assert float((w.double() - want_w).norm() / want_w.norm()) <= 2e-6
+    # a column sum of up to 2048 terms of unit variance: a few 2^-24 times the partial sums it runs through, at most sqrt(rows) each
+    assert float((b.double() - want_b).abs().max()) <= 2.0 ** -24 * 16 * (rows + 1) ** 0.5
+    dy[0, 1] = float("inf")
+    K.weight_grad(dy, x, out=w, accumulate=False, bias_out=b, bias_accumulate=False)
+    assert float(b[1]) == float("inf") and bool(torch.isfinite(b[2:]).all())
