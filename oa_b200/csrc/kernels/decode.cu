@@ -136,8 +136,8 @@ constexpr int DA_TILE_BYTES = 16384;
 template <int HD>
 __global__ void __launch_bounds__(160)
 decode_attn_stream_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride, const __nv_bfloat16* __restrict__ kc,
-                          const __nv_bfloat16* __restrict__ vc, float* __restrict__ partial, int heads, int n_bh, int splits, int len,
-                          int max_seq, float scale_log2, const int* __restrict__ pos_dev, int* __restrict__ status) {
+                          const __nv_bfloat16* __restrict__ vc, float* __restrict__ partial, __nv_bfloat16* __restrict__ out, long long out_stride,
+                          int heads, int n_bh, int splits, int len, int max_seq, float scale_log2, const int* __restrict__ pos_dev, int* __restrict__ status) {
   constexpr int LPR = HD / 64;            // lanes that share one row in the q.k phase (64 head-dim elements each)
   constexpr int RW = 32 / LPR;            // rows per warp and tile
   constexpr int TILE = 4 * RW;            // positions per tile: 64 (HD 128) or 128 (HD 64) -> 16 KB of K and of V
@@ -261,12 +261,17 @@ decode_attn_stream_kernel(const __nv_bfloat16* __restrict__ q, long long q_strid
       float w[4], L = 0.f;
 #pragma unroll
       for (int k = 0; k < 4; ++k) { w[k] = s_m[k] == -INFINITY ? 0.f : fast_exp2(s_m[k] - M); L += s_l[k] * w[k]; }
-      float* dst = partial + (long long)item * (HD + 2);
       if (threadIdx.x < HD) {
         const int d = threadIdx.x;
-        dst[d] = s_acc[0][d] * w[0] + s_acc[1][d] * w[1] + s_acc[2][d] * w[2] + s_acc[3][d] * w[3];
+        const float v = s_acc[0][d] * w[0] + s_acc[1][d] * w[1] + s_acc[2][d] * w[2] + s_acc[3][d] * w[3];
+        float* dst = partial + (long long)item * (HD + 2);
+        if (splits == 1) {                                // the only piece: nothing to merge
+          out[(long long)b * out_stride + h * HD + d] = __float2bfloat16_rn(L > 0.f ? v / L : 0.f);
+        } else {
+          dst[d] = v;
+          if (d == 0) { dst[HD] = M; dst[HD + 1] = L; }
+        }
       }
-      if (threadIdx.x == 0) { dst[HD] = M; dst[HD + 1] = L; }
       const bool stop = s_fail != 0;                      // the same for all four warps: they leave together
       consumer_sync();
       if (stop) break;
@@ -295,9 +300,69 @@ __global__ void decode_merge_kernel(const float* __restrict__ partial, __nv_bflo
   out[(long long)b * out_stride + h * HD + d] = __float2bfloat16_rn(L > 0.f ? v / L : 0.f);
 }
 
+// One new token per sequence: the rotate-half embedding of q and k in place and the append of k and v to the cache, which as launches of
+// their own cost a decoding step 4.2 and 1.9 us.  A block takes eight of a row's 2 H rotated heads (and the v heads beside its k
+// heads); its first hd / 2 threads compute one angle each, the same for every head, where the general kernel's threads compute
+// eight one after the other.
+constexpr int RA_HEADS = 8;
+__global__ void __launch_bounds__(128)
+rope_kv_append_kernel(__nv_bfloat16* x, long long row_stride, int heads, int hd, int pos, float theta, const int* __restrict__ pos_dev,
+                      __nv_bfloat16* __restrict__ kc, __nv_bfloat16* __restrict__ vc, int max_seq) {
+  __shared__ float s_cos[64], s_sin[64];
+  pdl_launch_dependents();
+  pdl_wait();
+  if (pos_dev) pos += *pos_dev;
+  const int b = blockIdx.x, half = hd >> 1;
+  if ((int)threadIdx.x < half) {
+    const float freq = __powf(theta, -2.f * (float)threadIdx.x / (float)hd);
+    sincosf((float)pos * freq, &s_sin[threadIdx.x], &s_cos[threadIdx.x]);
+  }
+  __syncthreads();
+  const bool fits = pos < max_seq;               // a full cache drops the token (the host checks capacity before replaying)
+  const int jv = half >> 3;                      // 8-wide vectors per half head
+  for (int i = threadIdx.x; i < RA_HEADS * jv; i += blockDim.x) {
+    const int head = blockIdx.y * RA_HEADS + i / jv, j = (i % jv) * 8;
+    if (head >= 2 * heads) break;
+    __nv_bfloat16* row = x + b * row_stride + (long long)head * hd + j;
+    const uint4 ua = *reinterpret_cast<const uint4*>(row), ub = *reinterpret_cast<const uint4*>(row + half);
+    const uint32_t wa[4] = {ua.x, ua.y, ua.z, ua.w}, wb[4] = {ub.x, ub.y, ub.z, ub.w};
+    uint32_t oa[4], ob[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float2 p = unpack_bf16x2(wa[k]), q = unpack_bf16x2(wb[k]);
+      const float c0 = s_cos[j + 2 * k], c1 = s_cos[j + 2 * k + 1], s0 = s_sin[j + 2 * k], s1 = s_sin[j + 2 * k + 1];
+      oa[k] = pack_bf16x2(p.x * c0 - q.x * s0, p.y * c1 - q.y * s1);
+      ob[k] = pack_bf16x2(q.x * c0 + p.x * s0, q.y * c1 + p.y * s1);
+    }
+    const uint4 ra = make_uint4(oa[0], oa[1], oa[2], oa[3]), rb = make_uint4(ob[0], ob[1], ob[2], ob[3]);
+    *reinterpret_cast<uint4*>(row) = ra;
+    *reinterpret_cast<uint4*>(row + half) = rb;
+    if (head >= heads && fits) {
+      const long long at = (((long long)b * heads + head - heads) * max_seq + pos) * hd + j;
+      const __nv_bfloat16* v = row + (long long)heads * hd;
+      *reinterpret_cast<uint4*>(kc + at) = ra;
+      *reinterpret_cast<uint4*>(kc + at + half) = rb;
+      *reinterpret_cast<uint4*>(vc + at) = *reinterpret_cast<const uint4*>(v);
+      *reinterpret_cast<uint4*>(vc + at + half) = *reinterpret_cast<const uint4*>(v + half);
+    }
+  }
+}
+
 }  // namespace oa
 
 using namespace oa;
+
+// x: [batch, row_stride] rows q | k | v of `heads` heads each.  OA_ERR_UNSUPPORTED for head dims the vector path does not take.
+extern "C" int oa_rope_kv_append(void* x, long long row_stride, int batch, int heads, int head_dim, int pos, float theta, const int* pos_dev, void* k_cache,
+                                 void* v_cache, int max_seq, void* stream) {
+  if (head_dim % 16 || head_dim < 16 || head_dim > 128 || heads <= 0 || batch > 0x7fffffff / 4) return OA_ERR_UNSUPPORTED;
+  if (row_stride % 8 || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache)) & 15)) return OA_ERR_ALIGN;
+  if (pos < 0 || (!pos_dev && pos >= max_seq)) return OA_ERR_ARG;
+  if (batch <= 0) return OA_OK;
+  launch_short(rope_kv_append_kernel, dim3((unsigned)batch, (unsigned)((2 * heads + RA_HEADS - 1) / RA_HEADS)), dim3(128), 0, (cudaStream_t)stream,
+               (__nv_bfloat16*)x, row_stride, heads, head_dim, pos, theta, pos_dev, (__nv_bfloat16*)k_cache, (__nv_bfloat16*)v_cache, max_seq);
+  return cudaGetLastError() == cudaSuccess ? OA_OK : OA_ERR_LAUNCH;
+}
 
 extern "C" int oa_kv_append(const void* k_src, const void* v_src, long long src_stride, void* k_cache, void* v_cache, int batch,
                             int s_new, int heads, int head_dim, int pos0, int max_seq, const int* pos_dev, void* stream) {
@@ -348,8 +413,8 @@ static int launch_decode_stream(const void* q, long long q_stride, const void* k
   const int n_bh = batch * heads, items = n_bh * splits;
   const int grid = items < 2 * 148 ? items : 2 * 148;
   launch_short(decode_attn_stream_kernel<HD>, dim3(grid), dim3(160), smem, st, (const __nv_bfloat16*)q, q_stride, (const __nv_bfloat16*)kc,
-               (const __nv_bfloat16*)vc, (float*)partial, heads, n_bh, splits, len, max_seq, sl2, pos_dev, status);
-  launch_short(decode_merge_kernel<HD>, dim3(n_bh), dim3(HD), 0, st, (const float*)partial, (__nv_bfloat16*)out, out_stride, heads, splits);
+               (const __nv_bfloat16*)vc, (float*)partial, (__nv_bfloat16*)out, out_stride, heads, n_bh, splits, len, max_seq, sl2, pos_dev, status);
+  if (splits > 1) launch_short(decode_merge_kernel<HD>, dim3(n_bh), dim3(HD), 0, st, (const float*)partial, (__nv_bfloat16*)out, out_stride, heads, splits);
   return cudaGetLastError() == cudaSuccess ? OA_OK : OA_ERR_LAUNCH;
 }
 

@@ -1097,6 +1097,21 @@ def kv_append(k_src: torch.Tensor, v_src: torch.Tensor, k_cache: torch.Tensor, v
                                      heads, hd, pos0, max_seq, N.ptr(pos_dev), N.stream()), "oa_kv_append")
 
 
+def rope_kv_append(qkv: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, pos: int, theta: float,
+                   pos_dev: Optional[torch.Tensor] = None) -> None:
+    """One new token per sequence: RoPE on q and k of the packed rows [batch, 3 * heads * head_dim] in place, then k and v into the caches
+    at `pos` (plus the device-resident offset)."""
+    _, heads, max_seq, hd = k_cache.shape
+    batch, D = qkv.shape[0], heads * hd
+    if qkv.is_cuda and qkv.dtype == torch.bfloat16 and k_cache.dtype == torch.bfloat16 and qkv.stride(1) == 1 and hd % 16 == 0 and 16 <= hd <= 128 \
+            and qkv.stride(0) % 8 == 0 and (qkv.data_ptr() | k_cache.data_ptr() | v_cache.data_ptr()) % 16 == 0:
+        _launch(N.require().oa_rope_kv_append(qkv.data_ptr(), qkv.stride(0), batch, heads, hd, pos, float(theta), N.ptr(pos_dev), k_cache.data_ptr(),
+                                              v_cache.data_ptr(), max_seq, N.stream()), "oa_rope_kv_append")
+        return
+    rope_(qkv[:, : 2 * D], 2 * heads, hd, 1, pos_offset=pos, theta=theta, pos_dev=pos_dev)
+    kv_append(qkv[:, D:2 * D], qkv[:, 2 * D:], k_cache, v_cache, batch, 1, pos, pos_dev=pos_dev)
+
+
 def decode_attn(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, length: int, scale: Optional[float] = None,
                 pos_dev: Optional[torch.Tensor] = None) -> torch.Tensor:
     """One query token per sequence, q [batch, heads*head_dim] (row stride allowed), against the first `length` cached
@@ -1118,7 +1133,7 @@ def decode_attn(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, l
         part = scratch(q.device, lib.oa_decode_attn_stream_scratch_bytes(batch, heads, hd, splits), "decode_attn_partial")
         _launch(lib.oa_decode_attn_stream(q.data_ptr(), q.stride(0), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(), out.stride(0),
                                           batch, heads, hd, length, max_seq, float(scale), N.ptr(pos_dev), part.data_ptr(), splits,
-                                          status_word(q.device).data_ptr(), N.stream()), "oa_decode_attn_stream", 2)
+                                          status_word(q.device).data_ptr(), N.stream()), "oa_decode_attn_stream", 1 if splits == 1 else 2)
         return out
     _launch(lib.oa_decode_attn(q.data_ptr(), q.stride(0), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(), out.stride(0), batch,
                                heads, hd, length, max_seq, float(scale), N.ptr(pos_dev), N.stream()), "oa_decode_attn")

@@ -90,8 +90,9 @@ class OaGptDecoder:
             K.kv_append(t[:, D:2 * D], t[:, 2 * D:], self.Cache.K[i], self.Cache.V[i], batch, s_new, 0)
         else:
             if a.RopeTheta > 0:
-                K.rope_(t[:, : 2 * D], 2 * H, hd, 1, pos_offset=pos0, theta=a.RopeTheta, pos_dev=pd)
-            K.kv_append(t[:, D:2 * D], t[:, 2 * D:], self.Cache.K[i], self.Cache.V[i], batch, 1, pos0, pos_dev=pd)
+                K.rope_kv_append(t, self.Cache.K[i], self.Cache.V[i], pos0, a.RopeTheta, pos_dev=pd)
+            else:
+                K.kv_append(t[:, D:2 * D], t[:, 2 * D:], self.Cache.K[i], self.Cache.V[i], batch, 1, pos0, pos_dev=pd)
             attn = OaMatrix(K.decode_attn(t[:, :D], self.Cache.K[i], self.Cache.V[i], pos0 + 1, pos_dev=pd))
         o = a.OutProj
         x = F.Linear(attn, o.Weight.Data, o.Bias.Data if o.Bias else None, residual=x)
