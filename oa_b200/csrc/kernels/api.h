@@ -168,6 +168,12 @@ int oa_attn_f32_bwd(const float* q, const float* k, const float* v, const float*
 // ---- recurrent scans (rnn.cu): gates = 3 (GRU: reset | update | candidate) or 1 (tanh RNN)
 int oa_rnn_scan_fwd(int dtype, int gates, const void* gates_i, const void* w_hh, const void* b_hh, const void* h0, void* out,
                     void* hprev, int batch, int seq, int H, void* stream);
+// A GRU forward scan that leaves the coefficients of the backward step (oa_gru_coef_floats, 0 where it does not), and the backward scan from them.
+size_t oa_gru_coef_floats(int gates, int batch, int seq, int H);
+int oa_gru_scan_fwd_coef(int dtype, const void* gates_i, const void* w_hh, const void* b_hh, const void* h0, void* out,
+                         void* hprev, float* coef, int batch, int seq, int H, void* stream);
+int oa_gru_scan_bwd_coef(int dtype, const float* coef, const void* w_hh, const void* dout, void* dgi, void* dgh, void* dh0,
+                         int batch, int seq, int H, void* stream);
 size_t oa_rnn_scan_bwd_scratch_floats(int gates, int batch, int seq, int H);
 int oa_rnn_scan_bwd(int dtype, int gates, const void* gates_i, const void* w_hh, const void* b_hh, const void* hprev,
                     const void* dout, void* dgi, void* dgh, void* dh0, float* scratch, int batch, int seq, int H, void* stream);

@@ -388,7 +388,163 @@ rnn_reg_bwd_kernel(const float* __restrict__ coef, const float* __restrict__ zg,
   if (dh0 && p == 0) rst<T>(dh0 + (long long)b * H + i, carry);
 }
 
+// GRU layers of 65 to 128 units (a multiple of 16): four lanes own TWO units, which halves the warps, and with them the passes through
+// the activations that all lanes of a quad make together, and the shared-memory reads per product.  After a reduce-scatter over the
+// quad two lanes hold each unit.  A thread's weights are 192 registers.  A forward scan that a backward scan follows also writes
+// the coefficients (below: rnn_reg_coef_kernel), which are by-products of its step, instead of leaving a kernel to run the recurrent
+// products of all steps again.
+// 64 sequences of 128 steps, 128 units, fp32: forward 127 -> 88 us, backward 74 + 151 -> 86 us.
+constexpr int GRU2_NM = 8;
+template <typename T>
+__device__ __forceinline__ void gru2_load(unsigned long long (&w)[2][3][GRU2_NM][2], const T* __restrict__ w_hh, int i0, int p, int H, bool by_row) {
+#pragma unroll
+  for (int u = 0; u < 2; ++u)
+#pragma unroll
+    for (int g = 0; g < 3; ++g)
+#pragma unroll
+      for (int m = 0; m < GRU2_NM; ++m) {
+        float v[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const int k = 4 * (p + 4 * m) + c;
+          v[c] = k < H ? (by_row ? rld<T>(w_hh + (long long)(g * H + i0 + u) * H + k) : rld<T>(w_hh + (long long)(g * H + k) * H + i0 + u)) : 0.f;
+        }
+        w[u][g][m][0] = pack2(v[0], v[1]);
+        w[u][g][m][1] = pack2(v[2], v[3]);
+      }
+}
+// the quad's sum of each of two units; lanes 0, 1 get the first one's, lanes 2, 3 the second one's
+__device__ __forceinline__ float gru2_sum(float a, float b, int p) {
+  const float mine = p & 2 ? b : a, theirs = p & 2 ? a : b;
+  const float v = mine + __shfl_xor_sync(0xffffffffu, theirs, 2);
+  return v + __shfl_xor_sync(0xffffffffu, v, 1);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256, 1)
+gru2_fwd_kernel(const T* __restrict__ gates_i, const T* __restrict__ w_hh, const T* __restrict__ b_hh, const T* __restrict__ h0, T* __restrict__ out,
+                T* __restrict__ hprev, float* __restrict__ coef, float* __restrict__ zg, int seq, int H) {
+  __shared__ __align__(16) float sh[2][16 * GRU2_NM];
+  const int p = threadIdx.x & 3, q = p & 1, i0 = (threadIdx.x >> 2) * 2, i = i0 + (p >> 1), b = blockIdx.x;
+  unsigned long long w[2][3][GRU2_NM][2];
+  gru2_load<T>(w, w_hh, i0, p, H, true);
+  float bias[3];
+#pragma unroll
+  for (int g = 0; g < 3; ++g) bias[g] = b_hh ? rld<T>(b_hh + g * H + i) : 0.f;
+  float hp = h0 ? rld<T>(h0 + (long long)b * H + i) : 0.f;
+  for (int k = threadIdx.x; k < 16 * GRU2_NM; k += blockDim.x) sh[0][k] = sh[1][k] = 0.f;
+  __syncthreads();
+  if (q == 0) sh[0][i] = hp;
+  __syncthreads();
+  constexpr int PF = 2;                                       // input gates are fetched two steps ahead
+  const T* gi = gates_i + (long long)b * seq * 3 * H + i;
+  float pf[PF][3];
+#pragma unroll
+  for (int u = 0; u < PF; ++u)
+#pragma unroll
+    for (int g = 0; g < 3; ++g) pf[u][g] = u < seq ? rld<T>(gi + ((long long)u * 3 + g) * H) : 0.f;
+  for (int t0 = 0; t0 < seq; t0 += PF) {
+#pragma unroll
+    for (int u = 0; u < PF; ++u) {
+      const int t = t0 + u;
+      if (t >= seq) break;
+      unsigned long long acc[2][3] = {};
+#pragma unroll
+      for (int m = 0; m < GRU2_NM; ++m) {
+        const ulonglong2 hv = *reinterpret_cast<const ulonglong2*>(&sh[u & 1][4 * (p + 4 * m)]);
+#pragma unroll
+        for (int v = 0; v < 2; ++v)
+#pragma unroll
+          for (int g = 0; g < 3; ++g) acc[v][g] = fma2(w[v][g][m][1], hv.y, fma2(w[v][g][m][0], hv.x, acc[v][g]));
+      }
+      float x[3], gh[3];
+#pragma unroll
+      for (int g = 0; g < 3; ++g) {
+        x[g] = pf[u][g];
+        if (t + PF < seq) pf[u][g] = rld<T>(gi + ((long long)(t + PF) * 3 + g) * H);
+        gh[g] = gru2_sum(sum2(acc[0][g]), sum2(acc[1][g]), p) + bias[g];
+      }
+      const float r = sigmoid_f(x[0] + gh[0]), z = sigmoid_f(x[1] + gh[1]), n = tanhf(x[2] + r * gh[2]);
+      const float hn = (1.f - z) * n + z * hp;
+      const long long at = ((long long)b * seq + t) * H + i;
+      if (q == 0) sh[(u & 1) ^ 1][i] = hn;
+      else rst<T>(out + at, hn);
+      if (q == 0 && hprev) rst<T>(hprev + at, hp);
+      if (coef) {
+        const float cn = (1.f - z) * (1.f - n * n);
+        const float2 c = q == 0 ? make_float2(cn * gh[2] * r * (1.f - r), (hp - n) * z * (1.f - z)) : make_float2(cn * r, cn);
+        *reinterpret_cast<float2*>(coef + at * 4 + 2 * q) = c;
+        if (q == 1) zg[at] = z;
+      }
+      hp = hn;
+      __syncthreads();
+    }
+  }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256, 1)
+gru2_bwd_kernel(const float* __restrict__ coef, const float* __restrict__ zg, const T* __restrict__ w_hh, const T* __restrict__ dout, T* __restrict__ dgi,
+                T* __restrict__ dgh, T* __restrict__ dh0, int seq, int H) {
+  __shared__ __align__(16) float sg[2][3][16 * GRU2_NM];
+  const int p = threadIdx.x & 3, q = p & 1, i0 = (threadIdx.x >> 2) * 2, i = i0 + (p >> 1), b = blockIdx.x;
+  unsigned long long w[2][3][GRU2_NM][2];
+  gru2_load<T>(w, w_hh, i0, p, H, false);
+  for (int k = threadIdx.x; k < 2 * 3 * 16 * GRU2_NM; k += blockDim.x) (&sg[0][0][0])[k] = 0.f;
+  __syncthreads();
+  constexpr int PF = 2;
+  const long long row0 = (long long)b * seq;
+  float2 cf[PF];
+  float zf[PF], df[PF];
+  auto fetch = [&](int t, float2& c, float& z, float& d) {
+    const long long at = (row0 + t) * H + i;
+    c = *reinterpret_cast<const float2*>(coef + at * 4 + 2 * q);
+    z = zg[at];
+    d = rld<T>(dout + at);
+  };
+#pragma unroll
+  for (int u = 0; u < PF; ++u)
+    if (seq - 1 - u >= 0) fetch(seq - 1 - u, cf[u], zf[u], df[u]);
+  float carry = 0.f;
+  for (int t0 = seq - 1; t0 >= 0; t0 -= PF) {
+#pragma unroll
+    for (int u = 0; u < PF; ++u) {
+      const int t = t0 - u;
+      if (t < 0) break;
+      const float d = df[u] + carry, g0 = d * cf[u].x, g1 = d * cf[u].y, direct = d * zf[u];
+      if (t - PF >= 0) fetch(t - PF, cf[u], zf[u], df[u]);
+      const long long at = (row0 + t) * 3 * H + i;
+      if (q == 0) {                                            // reset and update gate
+        sg[u & 1][0][i] = g0;
+        sg[u & 1][1][i] = g1;
+        rst<T>(dgh + at, g0); rst<T>(dgh + at + H, g1);
+        rst<T>(dgi + at, g0); rst<T>(dgi + at + H, g1);
+      } else {                                                 // candidate: through the recurrent and through the input projection
+        sg[u & 1][2][i] = g0;
+        rst<T>(dgh + at + 2 * H, g0);
+        rst<T>(dgi + at + 2 * H, g1);
+      }
+      __syncthreads();
+      unsigned long long acc[2][3] = {};
+#pragma unroll
+      for (int g = 0; g < 3; ++g)
+#pragma unroll
+        for (int m = 0; m < GRU2_NM; ++m) {
+          const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(&sg[u & 1][g][4 * (p + 4 * m)]);
+#pragma unroll
+          for (int x = 0; x < 2; ++x) acc[x][g] = fma2(w[x][g][m][1], v.y, fma2(w[x][g][m][0], v.x, acc[x][g]));
+        }
+      float s[2];
+#pragma unroll
+      for (int x = 0; x < 2; ++x) s[x] = sum2(acc[x][0]) + sum2(acc[x][1]) + sum2(acc[x][2]);
+      carry = direct + gru2_sum(s[0], s[1], p);
+    }
+  }
+  if (dh0 && q == 0) rst<T>(dh0 + (long long)b * H + i, carry);
+}
+
 constexpr int RNN_REG_MAX_H = 128;
+inline bool gru2_ok(int gates, int H) { return gates == 3 && H > 64 && H <= RNN_REG_MAX_H && H % 16 == 0; }
 inline bool rnn_reg_ok(int H) { return H >= 8 && H <= RNN_REG_MAX_H && H % 8 == 0; }   // whole warps of four lanes per unit
 #define OA_RNN_REG_NM(T, G, CALL)                                        \
   {                                                                      \
@@ -411,6 +567,45 @@ static int rnn_set_smem(K kernel, size_t bytes) {
 using namespace oa;
 #define ST ((cudaStream_t)stream)
 
+static void gru2_fwd(int dtype, const void* gates_i, const void* w_hh, const void* b_hh, const void* h0, void* out, void* hprev, float* coef, int batch, int seq,
+                     int H, cudaStream_t st) {
+  float* zg = coef ? coef + (size_t)batch * seq * H * 4 : nullptr;
+  if (dtype == OA_F32)
+    gru2_fwd_kernel<float><<<batch, 2 * H, 0, st>>>((const float*)gates_i, (const float*)w_hh, (const float*)b_hh, (const float*)h0, (float*)out, (float*)hprev,
+                                                    coef, zg, seq, H);
+  else
+    gru2_fwd_kernel<__nv_bfloat16><<<batch, 2 * H, 0, st>>>((const __nv_bfloat16*)gates_i, (const __nv_bfloat16*)w_hh, (const __nv_bfloat16*)b_hh,
+                                                            (const __nv_bfloat16*)h0, (__nv_bfloat16*)out, (__nv_bfloat16*)hprev, coef, zg, seq, H);
+}
+static void gru2_bwd(int dtype, const float* coef, const void* w_hh, const void* dout, void* dgi, void* dgh, void* dh0, int batch, int seq, int H,
+                     cudaStream_t st) {
+  const float* zg = coef + (size_t)batch * seq * H * 4;
+  if (dtype == OA_F32)
+    gru2_bwd_kernel<float><<<batch, 2 * H, 0, st>>>(coef, zg, (const float*)w_hh, (const float*)dout, (float*)dgi, (float*)dgh, (float*)dh0, seq, H);
+  else
+    gru2_bwd_kernel<__nv_bfloat16><<<batch, 2 * H, 0, st>>>(coef, zg, (const __nv_bfloat16*)w_hh, (const __nv_bfloat16*)dout, (__nv_bfloat16*)dgi,
+                                                            (__nv_bfloat16*)dgh, (__nv_bfloat16*)dh0, seq, H);
+}
+
+// Floats that a forward scan can leave for the backward one (0: it leaves none), and the two scans with them.
+extern "C" size_t oa_gru_coef_floats(int gates, int batch, int seq, int H) { return gru2_ok(gates, H) ? (size_t)batch * seq * H * 5 : 0; }
+extern "C" int oa_gru_scan_fwd_coef(int dtype, const void* gates_i, const void* w_hh, const void* b_hh, const void* h0, void* out, void* hprev, float* coef,
+                                    int batch, int seq, int H, void* stream) {
+  if (batch <= 0 || seq <= 0) return OA_OK;
+  if ((dtype != OA_F32 && dtype != OA_BF16) || !gru2_ok(3, H)) return OA_ERR_UNSUPPORTED;
+  if (!coef) return OA_ERR_ARG;
+  gru2_fwd(dtype, gates_i, w_hh, b_hh, h0, out, hprev, coef, batch, seq, H, ST);
+  return cudaGetLastError() == cudaSuccess ? OA_OK : OA_ERR_LAUNCH;
+}
+extern "C" int oa_gru_scan_bwd_coef(int dtype, const float* coef, const void* w_hh, const void* dout, void* dgi, void* dgh, void* dh0, int batch, int seq,
+                                    int H, void* stream) {
+  if (batch <= 0 || seq <= 0) return OA_OK;
+  if ((dtype != OA_F32 && dtype != OA_BF16) || !gru2_ok(3, H)) return OA_ERR_UNSUPPORTED;
+  if (!coef) return OA_ERR_ARG;
+  gru2_bwd(dtype, coef, w_hh, dout, dgi, dgh, dh0, batch, seq, H, ST);
+  return cudaGetLastError() == cudaSuccess ? OA_OK : OA_ERR_LAUNCH;
+}
+
 // gates = 3 (GRU) or 1 (RNN).  gates_i [B, S, gates*H], w_hh [gates*H, H], b_hh [gates*H] or null, h0 [B, H] or null,
 // out [B, S, H], hprev [B, S, H] or null (needed for the backward pass).
 extern "C" int oa_rnn_scan_fwd(int dtype, int gates, const void* gates_i, const void* w_hh, const void* b_hh, const void* h0,
@@ -418,6 +613,10 @@ extern "C" int oa_rnn_scan_fwd(int dtype, int gates, const void* gates_i, const 
   if (gates != 1 && gates != 3) return OA_ERR_ARG;
   if (batch <= 0 || seq <= 0) return OA_OK;
   if (dtype != OA_F32 && dtype != OA_BF16) return OA_ERR_UNSUPPORTED;
+  if (gru2_ok(gates, H)) {
+    gru2_fwd(dtype, gates_i, w_hh, b_hh, h0, out, hprev, nullptr, batch, seq, H, ST);
+    return cudaGetLastError() == cudaSuccess ? OA_OK : OA_ERR_LAUNCH;
+  }
   if (rnn_reg_ok(H)) {
 #define CALL_REG_FWD(T, G, NM)                                                                                              \
     rnn_reg_fwd_kernel<T, G, NM><<<batch, 4 * H, 0, ST>>>((const T*)gates_i, (const T*)w_hh, (const T*)b_hh, (const T*)h0, \
@@ -455,6 +654,16 @@ extern "C" int oa_rnn_scan_bwd(int dtype, int gates, const void* gates_i, const 
     const long long rows = (long long)batch * seq;
     float* zg = scratch + rows * H * 4;                       // GRU only
     const int grid = rows < 148 * 4 ? (int)rows : 148 * 4;
+    if (gru2_ok(gates, H)) {
+      if (dtype == OA_F32)
+        rnn_reg_coef_kernel<float, 3, 8><<<grid, 4 * H, 0, ST>>>((const float*)gates_i, (const float*)w_hh, (const float*)b_hh, (const float*)hprev, scratch, zg,
+                                                                 rows, H);
+      else
+        rnn_reg_coef_kernel<__nv_bfloat16, 3, 8><<<grid, 4 * H, 0, ST>>>((const __nv_bfloat16*)gates_i, (const __nv_bfloat16*)w_hh, (const __nv_bfloat16*)b_hh,
+                                                                         (const __nv_bfloat16*)hprev, scratch, zg, rows, H);
+      gru2_bwd(dtype, scratch, w_hh, dout, dgi, dgh, dh0, batch, seq, H, ST);
+      return cudaGetLastError() == cudaSuccess ? OA_OK : OA_ERR_LAUNCH;
+    }
 #define CALL_REG_BWD(T, G, NM)                                                                                               \
     rnn_reg_coef_kernel<T, G, NM><<<grid, 4 * H, 0, ST>>>((const T*)gates_i, (const T*)w_hh, (const T*)b_hh, (const T*)hprev, \
                                                           scratch, zg, rows, H);                                              \

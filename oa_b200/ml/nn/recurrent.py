@@ -25,12 +25,13 @@ def RecurrentScan(gates_i: OaMatrix, w_hh: OaMatrix, b_hh: Optional[OaMatrix], g
     tg, tw = F._c(gates_i.Tensor()), F._c(w_hh.Tensor())
     tb = b_hh.Tensor() if b_hh is not None else None
     need = AG.IsEnabled() and (gates_i.RequiresGrad() or w_hh.RequiresGrad())
-    out_t, hprev = K.rnn_scan_fwd(tg, tw, tb, gates, save=need)
+    coef = K.rnn_coef(tg, gates) if need else None
+    out_t, hprev = K.rnn_scan_fwd(tg, tw, tb, gates, save=need, coef=coef)
     out = OaMatrix(out_t)
 
     def back(g):
         F._ctx_add(name + "Bwd")
-        dgi, dgh, _ = K.rnn_scan_bwd(tg, tw, tb, hprev, F._c(g), gates)
+        dgi, dgh, _ = K.rnn_scan_bwd(tg, tw, tb, hprev, F._c(g), gates, coef=coef)
         B, S, GH = dgh.shape
         H = GH // gates
         dgh2, hp2 = dgh.reshape(B * S, GH), hprev.reshape(B * S, H)

@@ -1005,9 +1005,16 @@ def flash_bwd(q, k, v, o, dout, lse, batch: int, seq: int, heads: int, head_dim:
 
 
 # ---------------------------------------------------------------- recurrent scans
+def rnn_coef(gates_i: torch.Tensor, gates: int) -> Optional[torch.Tensor]:
+    """Room for the coefficients that a forward scan of this shape leaves for the backward one; None where it leaves none."""
+    B, S, GH = gates_i.shape
+    n = N.require().oa_gru_coef_floats(gates, B, S, GH // gates) if gates_i.is_cuda else 0
+    return torch.empty(n, dtype=torch.float32, device=gates_i.device) if n else None
+
+
 def rnn_scan_fwd(gates_i: torch.Tensor, w_hh: torch.Tensor, b_hh: Optional[torch.Tensor], gates: int, h0: Optional[torch.Tensor] = None,
-                 save: bool = True):
-    """gates_i [B, S, gates*H] (input projection of all steps) -> (out [B,S,H], hprev [B,S,H] or None)."""
+                 save: bool = True, coef: Optional[torch.Tensor] = None):
+    """gates_i [B, S, gates*H] (input projection of all steps) -> (out [B,S,H], hprev [B,S,H] or None); fills `coef` (rnn_coef) if given."""
     B, S, GH = gates_i.shape
     H = GH // gates
     out = torch.empty((B, S, H), dtype=gates_i.dtype, device=gates_i.device)
@@ -1031,13 +1038,17 @@ def rnn_scan_fwd(gates_i: torch.Tensor, w_hh: torch.Tensor, b_hh: Optional[torch
                 h = torch.tanh(gi + gh)
             out[:, t] = h
         return out, hprev
+    if coef is not None:
+        _launch(N.require().oa_gru_scan_fwd_coef(dt(gates_i), gates_i.contiguous().data_ptr(), w_hh.contiguous().data_ptr(), N.ptr(b_hh), N.ptr(h0),
+                                                 out.data_ptr(), N.ptr(hprev), coef.data_ptr(), B, S, H, N.stream()), "oa_gru_scan_fwd_coef")
+        return out, hprev
     _launch(N.require().oa_rnn_scan_fwd(dt(gates_i), gates, gates_i.contiguous().data_ptr(), w_hh.contiguous().data_ptr(), N.ptr(b_hh),
                                         N.ptr(h0), out.data_ptr(), N.ptr(hprev), B, S, H, N.stream()), "oa_rnn_scan_fwd")
     return out, hprev
 
 
-def rnn_scan_bwd(gates_i, w_hh, b_hh, hprev, dout, gates: int):
-    """Returns (dgates_i [B,S,gates*H], dgates_h [B,S,gates*H], dh0 [B,H])."""
+def rnn_scan_bwd(gates_i, w_hh, b_hh, hprev, dout, gates: int, coef: Optional[torch.Tensor] = None):
+    """Returns (dgates_i [B,S,gates*H], dgates_h [B,S,gates*H], dh0 [B,H]); `coef` as the forward scan filled it."""
     B, S, GH = gates_i.shape
     H = GH // gates
     dgi = torch.empty_like(gates_i)
@@ -1072,6 +1083,10 @@ def rnn_scan_bwd(gates_i, w_hh, b_hh, hprev, dout, gates: int):
         dh0.copy_(carry)
         return dgi, dgh, dh0
     lib = N.require()
+    if coef is not None:
+        _launch(lib.oa_gru_scan_bwd_coef(dt(gates_i), coef.data_ptr(), w_hh.contiguous().data_ptr(), dout.contiguous().data_ptr(), dgi.data_ptr(),
+                                         dgh.data_ptr(), dh0.data_ptr(), B, S, H, N.stream()), "oa_gru_scan_bwd_coef")
+        return dgi, dgh, dh0
     n = lib.oa_rnn_scan_bwd_scratch_floats(gates, B, S, H)
     sc = torch.empty(n, dtype=torch.float32, device=gates_i.device) if n else None
     _launch(lib.oa_rnn_scan_bwd(dt(gates_i), gates, gates_i.contiguous().data_ptr(), w_hh.contiguous().data_ptr(), N.ptr(b_hh),

@@ -27,3 +27,23 @@ def test_scan(gates, dtype, tol, B, S, H):
         for a, e, nm in zip(got, ref, ("dgi", "dgh", "dh0")):
             assert (a.float().cpu() - e).abs().max().item() <= tol * max(1.0, e.abs().max().item()), nm
     torch.cuda.synchronize()
+
+
+# The coefficients that the forward scan leaves: the same gradients as from the scan that works them out again.
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, 2e-5), (torch.bfloat16, 4e-2)])
+@pytest.mark.parametrize("B,S,H", [(1, 1, 80), (3, 2, 96), (2, 33, 112), (150, 5, 128), (2, 64, 128), (2, 5, 72)])
+def test_forward_coefficients(dtype, tol, B, S, H):
+    g = torch.Generator().manual_seed(B * 1009 + S * 31 + H)
+    r = lambda *s, k=1.0: (k * torch.randn(*s, generator=g)).to(dtype)
+    gi, w, b, h0, do = r(B, S, 3 * H), r(3 * H, H, k=H ** -0.5), r(3 * H, k=0.1), r(B, H, k=0.5), r(B, S, H)
+    coef = K.rnn_coef(gi.cuda(), 3)
+    assert (coef is None) == (H % 16 != 0)
+    if coef is not None:
+        coef.fill_(float("nan"))
+    out, hp = K.rnn_scan_fwd(gi.cuda(), w.cuda(), b.cuda(), 3, h0=h0.cuda(), coef=coef)
+    got = K.rnn_scan_bwd(gi.cuda(), w.cuda(), b.cuda(), hp, do.cuda(), 3, coef=coef)
+    outr, hpr = K.rnn_scan_fwd(gi.float(), w.float(), b.float(), 3, h0=h0.float())
+    ref = K.rnn_scan_bwd(gi.float(), w.float(), b.float(), hpr, do.float(), 3)
+    assert (out.float().cpu() - outr).abs().max().item() <= tol
+    for a, e, nm in zip(got, ref, ("dgi", "dgh", "dh0")):
+        assert (a.float().cpu() - e).abs().max().item() <= tol * max(1.0, e.abs().max().item()), nm
