@@ -150,16 +150,8 @@ __device__ __forceinline__ bool wait_ge_sys(const unsigned long long* p, unsigne
 
 // Whole-warp wait: every lane waits (so the warp stays converged) and the outcome is made uniform.
 __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity) {
-#ifdef OA_WARP_WAIT_ONE_LANE
-  bool ok = true;
-  if ((threadIdx.x & 31) == 0) ok = mbar_wait(bar, parity);
-  ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-  if (ok && (threadIdx.x & 31) != 0) ok = mbar_try_wait(bar, parity);   // completes at once; gives each lane the acquire
-  return __all_sync(0xffffffffu, ok);
-#else
   bool ok = mbar_wait(bar, parity);
   return __all_sync(0xffffffffu, ok);
-#endif
 }
 
 __device__ __forceinline__ void report_error(int* status, int code) {
