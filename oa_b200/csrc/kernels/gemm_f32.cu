@@ -342,7 +342,7 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ B, f
 }
 
 // The same products over fewer than F_BRIEF_K columns of K with tiles for every SM: 4 x 4 outputs per thread over all of K, stored from
-// registers.  Fewer registers leave room for three blocks per SM, and of a few stages of arithmetic what counts is how many blocks
+// registers.  Fewer registers leave room for more blocks per SM, and of a few stages of arithmetic what counts is how many blocks
 // overlap their loads and stores.  Against the kernel above: 2048 x 512 x 128 11.9 / 12.9 us, 8192 x 384 x 64 17 / 24, 4096 x 1024 x 160
 // 40 / 48, 50000 x 32 x 32 10.5 / 17; 1024 x 1024 x 256 21.1 / 20.6 (18 with both operands row-contiguous), 512 x 512 x 512 20.5 / 13.2.
 constexpr int F_BRIEF_K = 192;
