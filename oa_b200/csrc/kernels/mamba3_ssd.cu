@@ -726,6 +726,9 @@ inline bool ssd_dims_ok(const SsdDims& d) {
   return d.B > 0 && d.L > 0 && d.H > 0 && d.P > 0 && d.N > 0 && d.A >= 0 && d.L % SQ == 0 && d.nC == d.L / SQ && d.N % 4 == 0 && d.P % 2 == 0 &&
          2 * d.A <= d.N;
 }
+// The kernels read and write two bf16 at once: rows and base on 4 bytes (null: an operand that is not there).
+inline bool ssd_pairs_ok(const void* p, long long ld) { return !p || (ld % 2 == 0 && (reinterpret_cast<uintptr_t>(p) & 3) == 0); }
+inline bool ssd_at16(const void* a, const void* b) { return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15) == 0; }
 inline int ssd_status() { return cudaGetLastError() == cudaSuccess ? OA_OK : OA_ERR_LAUNCH; }
 
 }  // namespace oa
@@ -739,6 +742,7 @@ int oa_ssd_prep_fwd(const void* x, long long ldx, const void* Bn, const void* Cn
                     void* gamma, void* scale, void* w, void* qk, int B, int L, int H, int P, int N, int A, void* stream) {
   SsdDims d{B, L, H, P, N, A, L / SQ};
   if (!ssd_dims_ok(d) || (A > 0 && !theta)) return OA_ERR_ARG;
+  if (!ssd_pairs_ok(x, ldx) || !ssd_at16(Bb, Cb)) return OA_ERR_ALIGN;
   SsdPrepFwd a{(const __nv_bfloat16*)x, ldx, (const float*)Bn, (const float*)Cn, (const float*)Bb, (const float*)Cb, (const float*)dt,
                (const float*)adt, (const float*)trap, (const float*)theta, (__nv_bfloat16*)Ct, (__nv_bfloat16*)Bt, (__nv_bfloat16*)Ce,
                (__nv_bfloat16*)X, (__nv_bfloat16*)Xw, (float*)cum, (float*)gamma, (float*)scale, (float*)w, (float*)qk, d};
@@ -782,6 +786,7 @@ int oa_ssd_out_fwd(const void* Y, const void* z, long long ldz, void* y, void* y
                    void* stream) {
   SsdDims d{B, L, H, P, 4, 0, L / SQ};
   if (!ssd_dims_ok(d) || (z && !yraw)) return OA_ERR_ARG;
+  if (!ssd_pairs_ok(z, ldz) || !ssd_pairs_ok(y, ldy) || !ssd_pairs_ok(yraw, ldy)) return OA_ERR_ALIGN;
   const long long total = (long long)B * L * H * (P / 2);
   ssd_out_fwd_kernel<<<(int)((total + 255) / 256 > 148 * 32 ? 148 * 32 : (total + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
       (const float*)Y, (const __nv_bfloat16*)z, ldz, (__nv_bfloat16*)y, (__nv_bfloat16*)yraw, ldy, d);
@@ -792,6 +797,7 @@ int oa_ssd_dy_prep(const void* dy, const void* yraw, long long ldy, const void* 
                    int B, int L, int H, int P, void* stream) {
   SsdDims d{B, L, H, P, 4, 0, L / SQ};
   if (!ssd_dims_ok(d) || (z && (!yraw || !dz))) return OA_ERR_ARG;
+  if (!ssd_pairs_ok(dy, ldy) || !ssd_pairs_ok(yraw, ldy) || !ssd_pairs_ok(z, ldz) || !ssd_pairs_ok(dz, lddz)) return OA_ERR_ALIGN;
   if (!z && P % 8 == 0 && ldy % 8 == 0 && ((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(dY)) & 15) == 0 &&
       (long long)B * L * H * (P / 8) < 0x7fffff00LL) {
     const long long n = (long long)B * L * H * (P / 8);
@@ -830,6 +836,7 @@ int oa_ssd_dx_out(const void* dX, const void* dXw, const void* X, const void* w,
                   int P, void* stream) {
   SsdDims d{B, L, H, P, 4, 0, L / SQ};
   if (!ssd_dims_ok(d)) return OA_ERR_ARG;
+  if (!ssd_pairs_ok(dx, lddx)) return OA_ERR_ALIGN;
   ssd_dx_out_kernel<<<B * H * d.nC, 256, 0, (cudaStream_t)stream>>>((const float*)dX, (const float*)dXw, (const __nv_bfloat16*)X,
                                                                     (const float*)w, (__nv_bfloat16*)dx, lddx, (float*)dw, d);
   return ssd_status();

@@ -122,12 +122,16 @@ def _f32(t: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
 
 def _use_ssd(proj: torch.Tensor, d: "Mamba3Dims", L: int) -> bool:
     """The chunked tensor-core scan serves bf16 training on CUDA when the sequence is a whole number of chunks; fp32
-    inputs, ragged lengths and decode prefill (which needs the recurrent state) use the sequential kernels.
-    OA_MAMBA3_SSD=0 forces the sequential kernels."""
+    inputs, ragged lengths, odd row widths and decode prefill (which needs the recurrent state) use the sequential kernels.
+    OA_MAMBA3_SSD=0 forces the sequential kernels, OA_MAMBA3_SSD_FUSED=0 the statement of the chunked form, which takes any row width."""
     if os.environ.get("OA_MAMBA3_SSD", "1") == "0" or not proj.is_cuda or proj.dtype != torch.bfloat16:
         return False
     from . import mamba3_ssd as SSD
-    return SSD.supported(d, L, SSD.CHUNK)
+    return SSD.supported(d, L, SSD.CHUNK) and (not _fused_ssd() or SSD.rows_in_pairs(proj, d))
+
+
+def _fused_ssd() -> bool:
+    return os.environ.get("OA_MAMBA3_SSD_FUSED", "1") != "0"
 
 
 class Saved:
@@ -161,7 +165,7 @@ def core_fwd(proj: torch.Tensor, dt_bias, Bb, Cb, D, d: Mamba3Dims, B: int, L: i
         s = Saved()
         s.proj, s.params, s.dims, s.B, s.L = proj, (dtb, Bb32, Cb32, D32), d, B, L
         s.pre, s.Hck, s.Tck = (Bn, Cn, rstd, dt, adt, trap, angle), None, None
-        if os.environ.get("OA_MAMBA3_SSD_FUSED", "1") != "0":
+        if _fused_ssd():
             y, sv = SSD.ssd_fwd_cuda(proj, Bn, Cn, dt, adt, trap, angle, Bb32, Cb32, D32, d, B, L, save)
             s.ssd = sv
             return y, s

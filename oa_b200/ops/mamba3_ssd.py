@@ -71,6 +71,11 @@ def supported(d: M3.Mamba3Dims, L: int, Q: int = 128) -> bool:
     return L % Q == 0 and d.headdim % 8 == 0 and d.d_state % 8 == 0 and d.d_state <= 128 and d.angles <= 128
 
 
+def rows_in_pairs(proj: torch.Tensor, d: M3.Mamba3Dims) -> bool:
+    """Whether the glue kernels may move the columns of the projected rows two bf16 at a time, as they do."""
+    return d.d_in_proj % 2 == 0 and proj.data_ptr() % 4 == 0
+
+
 def ssd_fwd(x, z, Bn, Cn, dt, adt, trap, angle, Bb, Cb, D, d: M3.Mamba3Dims, B: int, L: int, Q: int = 128, gemm_dtype=None):
     """x, z [B, L, H, P] (z None without the in-scan gate); Bn, Cn [B, L, N]; dt, adt, trap [B, L, H]; angle [B, L, A]
     (fp32).  Returns (y [B, L, H, P] fp32, saved)."""
@@ -262,6 +267,7 @@ def ssd_fwd_cuda(proj: torch.Tensor, Bn, Cn, dt, adt, trap, angle, Bb, Cb, D, d:
     G = B * H * nC
     o = d.offsets()
     es = proj.element_size()
+    Bb, Cb = (t if t.data_ptr() % 16 == 0 else t.clone() for t in (Bb, Cb))       # read four values at a time
     bf = lambda *s: torch.empty(s, dtype=torch.bfloat16, device=dev)
     f32 = lambda *s: torch.empty(s, dtype=torch.float32, device=dev)
     theta = None
@@ -324,6 +330,8 @@ def ssd_bwd_cuda(s: SsdSavedCuda, proj: torch.Tensor, dy: torch.Tensor, dproj: t
     f32 = lambda *sh: torch.empty(sh, dtype=torch.float32, device=dev)
     z32 = lambda *sh: torch.zeros(sh, dtype=torch.float32, device=dev)
     dy = dy.contiguous()
+    if dy.data_ptr() % 4:
+        dy = dy.clone()
     fused = s.M is None
     dY = bf(G, Q, P)
     K._launch(lib.oa_ssd_dy_prep(dy.data_ptr(), N.ptr(s.yraw), d.d_inner, proj.data_ptr() + o[0] * es if d.has_z else None, d.d_in_proj,
