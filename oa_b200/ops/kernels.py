@@ -326,7 +326,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
 
 def weight_grad(dy: torch.Tensor, x: torch.Tensor, *, out: torch.Tensor, accumulate: bool, bias_out: torch.Tensor, bias_accumulate: bool) -> None:
     """out (+)= dy^T x and bias_out (+)= the column sums of dy; in fp32 the same tiles give both."""
-    if dy.is_cuda and dy.dtype == torch.float32 and not _f32_tensor_terms and dy.stride(1) == 1 and x.stride(1) == 1 and out.stride(1) == 1 \
+    if dy.is_cuda and x.is_cuda and dy.dtype == x.dtype == torch.float32 and not _f32_tensor_terms and dy.stride(1) == 1 and x.stride(1) == 1 and out.stride(1) == 1 \
             and out.dtype == torch.float32 and bias_out.dtype == torch.float32 and bias_out.is_contiguous():
         K, M = dy.shape
         Nn = x.shape[1]
