@@ -388,12 +388,16 @@ rnn_reg_bwd_kernel(const float* __restrict__ coef, const float* __restrict__ zg,
   if (dh0 && p == 0) rst<T>(dh0 + (long long)b * H + i, carry);
 }
 
-// GRU layers of 65 to 128 units (a multiple of 16): four lanes own TWO units, which halves the warps, and with them the passes through
+// GRU layers of 80, 96, 112 and 128 units: four lanes own TWO units, which halves the warps, and with them the passes through
 // the activations that all lanes of a quad make together, and the shared-memory reads per product.  After a reduce-scatter over the
-// quad two lanes hold each unit.  A thread's weights are 192 registers.  A forward scan that a backward scan follows also writes
-// the coefficients (below: rnn_reg_coef_kernel), which are by-products of its step, instead of leaving a kernel to run the recurrent
-// products of all steps again.
-// 64 sequences of 128 steps, 128 units, fp32: forward 127 -> 88 us, backward 74 + 151 -> 86 us.
+// quad two lanes hold each unit.  A thread's weights are 192 registers.  Whole warps need multiples of 16 units; up to 64 units and at
+// 72, 88, 104 and 120 the kernels above stay.
+// 64 sequences of 128 steps, 128 units, fp32: forward 129 -> 85 us, backward with the coefficients of rnn_reg_coef_kernel 228 -> 162.
+// Forward at 80 units 109 -> 80, 96: 113 -> 81, 112: 124 -> 83, in bf16 125 -> 93, 129 -> 95, 140 -> 95; one sequence alike, 600 sequences
+// of 64 steps 273 -> 201 at 80 units.  The products are padded to 128 columns: instantiations by 16 measured 68 us at 80, 74 at 96.
+// A forward scan may also write those coefficients, by-products of its step (+ 2 us), instead of leaving the coefficient kernel to
+// run the recurrent products of all steps again: backward 162 -> 87.  They are five fp32 values per unit and step that live from the
+// forward to the backward pass, beside the 20 bytes (fp32) or 10 (bf16) that a layer keeps there anyway, so the caller bounds them.
 constexpr int GRU2_NM = 8;
 template <typename T>
 __device__ __forceinline__ void gru2_load(unsigned long long (&w)[2][3][GRU2_NM][2], const T* __restrict__ w_hh, int i0, int p, int H, bool by_row) {

@@ -30,6 +30,36 @@ def NextSeq() -> int:
     return n
 
 
+# Values that a forward pass may leave to save its backward pass work, but need not: at most this many bytes of them live per tape,
+# however many layers ask (about 0.15 % of a GPU's memory).
+KEEP_BYTES = 256 << 20
+
+
+class KeepAllowance:
+    """What is left of KEEP_BYTES: a node takes its share when it runs and gives it back when its backward pass has run."""
+
+    __slots__ = ("left",)
+
+    def __init__(self):
+        self.left = KEEP_BYTES
+
+    def Take(self, nbytes: int) -> bool:
+        if nbytes > self.left:
+            return False
+        self.left -= nbytes
+        return True
+
+    def Give(self, nbytes: int) -> None:
+        self.left += nbytes
+
+
+def Keeping() -> KeepAllowance:
+    """The allowance of this thread's innermost open tape."""
+    if getattr(_tls, "keep", None) is None:
+        _tls.keep = KeepAllowance()
+    return _tls.keep
+
+
 # A data-parallel wrapper overlaps its gradient reduction with the rest of the backward pass: it registers a hook that is
 # called (a) when a backward pass starts and (b) each time a leaf has received its LAST gradient contribution of the pass.
 _leaf_ready_hook = None
@@ -92,6 +122,7 @@ class OaGradientTape:
     def __init__(self):
         self._prev = IsEnabled()
         self._active = True
+        self._keep_outside, _tls.keep = getattr(_tls, "keep", None), KeepAllowance()
         SetEnabled(True)
 
     def __enter__(self):
@@ -104,6 +135,7 @@ class OaGradientTape:
     def Close(self) -> None:
         if self._active:
             SetEnabled(self._prev)
+            _tls.keep = self._keep_outside
             self._active = False
 
     def Backward(self, root, grad: Optional[torch.Tensor] = None) -> None:

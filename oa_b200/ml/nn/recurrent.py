@@ -25,13 +25,19 @@ def RecurrentScan(gates_i: OaMatrix, w_hh: OaMatrix, b_hh: Optional[OaMatrix], g
     tg, tw = F._c(gates_i.Tensor()), F._c(w_hh.Tensor())
     tb = b_hh.Tensor() if b_hh is not None else None
     need = AG.IsEnabled() and (gates_i.RequiresGrad() or w_hh.RequiresGrad())
-    coef = K.rnn_coef(tg, gates) if need else None
+    # Coefficients kept for the backward scan save it a pass over the recurrent products (148 sequences of 704 steps, 128 units: 1.00
+    # against 1.69 ms for both scans in fp32, 1.53 against 2.47 in bf16) and cost 20 bytes per unit and step (254 MiB there) until it has
+    # run, where without them they are scratch of one scan at a time: as far as the tape's allowance goes.
+    keeping = AG.Keeping()
+    coef = K.rnn_coef(tg, gates, keeping.Take) if need else None
     out_t, hprev = K.rnn_scan_fwd(tg, tw, tb, gates, save=need, coef=coef)
     out = OaMatrix(out_t)
 
     def back(g):
         F._ctx_add(name + "Bwd")
         dgi, dgh, _ = K.rnn_scan_bwd(tg, tw, tb, hprev, F._c(g), gates, coef=coef)
+        if coef is not None:
+            keeping.Give(coef.numel() * 4)
         B, S, GH = dgh.shape
         H = GH // gates
         dgh2, hp2 = dgh.reshape(B * S, GH), hprev.reshape(B * S, H)

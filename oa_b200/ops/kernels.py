@@ -1005,11 +1005,12 @@ def flash_bwd(q, k, v, o, dout, lse, batch: int, seq: int, heads: int, head_dim:
 
 
 # ---------------------------------------------------------------- recurrent scans
-def rnn_coef(gates_i: torch.Tensor, gates: int) -> Optional[torch.Tensor]:
-    """Room for the coefficients that a forward scan of this shape leaves for the backward one; None where it leaves none."""
+def rnn_coef(gates_i: torch.Tensor, gates: int, may_keep=lambda nbytes: True) -> Optional[torch.Tensor]:
+    """Room for the coefficients that a forward scan of this shape leaves for the backward one; None where it leaves none or where
+    `may_keep(bytes)` says no (the backward scan then works them out in scratch of its own)."""
     B, S, GH = gates_i.shape
     n = N.require().oa_gru_coef_floats(gates, B, S, GH // gates) if gates_i.is_cuda else 0
-    return torch.empty(n, dtype=torch.float32, device=gates_i.device) if n else None
+    return torch.empty(n, dtype=torch.float32, device=gates_i.device) if n and may_keep(4 * n) else None
 
 
 def rnn_scan_fwd(gates_i: torch.Tensor, w_hh: torch.Tensor, b_hh: Optional[torch.Tensor], gates: int, h0: Optional[torch.Tensor] = None,

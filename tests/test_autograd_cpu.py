@@ -232,3 +232,15 @@ def test_backward_root_must_be_scalar():
     with AG.OaGradientTape() as tape:
         with pytest.raises(ValueError):
             tape.Backward(F.Exp(a))
+
+
+def test_kept_values_are_bounded_per_tape():
+    with AG.OaGradientTape():
+        outer = AG.Keeping()
+        assert outer.Take(AG.KEEP_BYTES - 10) and not outer.Take(11) and outer.Take(10)
+        with AG.OaGradientTape():
+            assert AG.Keeping() is not outer and AG.Keeping().left == AG.KEEP_BYTES
+        assert AG.Keeping() is outer and outer.left == 0
+        outer.Give(10)
+        assert outer.Take(10)
+    assert AG.Keeping() is not outer

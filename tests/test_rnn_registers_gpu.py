@@ -47,3 +47,41 @@ def test_forward_coefficients(dtype, tol, B, S, H):
     assert (out.float().cpu() - outr).abs().max().item() <= tol
     for a, e, nm in zip(got, ref, ("dgi", "dgh", "dh0")):
         assert (a.float().cpu() - e).abs().max().item() <= tol * max(1.0, e.abs().max().item()), nm
+
+
+def test_coefficients_held_are_bounded(monkeypatch):
+    # four scans on one tape, room for the coefficients of two: the others' backward scans work theirs out again, with the same gradients
+    from oa_b200.core.matrix import OaMatrix
+    from oa_b200.ml import autograd as AG
+    from oa_b200.ml.nn.recurrent import RecurrentScan
+
+    B, S, H = 4, 96, 128
+    share = 4 * K.rnn_coef(torch.empty(B, S, 3 * H, device="cuda"), 3).numel()
+    monkeypatch.setattr(AG, "KEEP_BYTES", 2 * share + share // 2)
+    g = torch.Generator(device="cuda").manual_seed(5)
+    w, b = torch.randn(3 * H, H, device="cuda", generator=g) * H ** -0.5, torch.randn(3 * H, device="cuda", generator=g) * 0.1
+    x, do = torch.randn(B, S, 3 * H, device="cuda", generator=g), torch.randn(B, S, H, device="cuda", generator=g)
+
+    def scans():
+        xs = [OaMatrix(x.clone()) for _ in range(4)]
+        ws = [OaMatrix(w.clone()) for _ in range(4)]
+        for m in xs + ws:
+            m.SetRequiresGrad(True)
+        return xs, ws
+
+    for _ in range(2):                                          # the share comes back with the backward pass
+        xs, ws = scans()
+        with AG.OaGradientTape() as tape:
+            torch.cuda.synchronize()
+            before = torch.cuda.memory_allocated()
+            outs = [RecurrentScan(m, v, OaMatrix(b), 3, "GruScan") for m, v in zip(xs, ws)]
+            held = torch.cuda.memory_allocated() - before
+            assert held <= 4 * 2 * (4 * B * S * H) + 2 * share + 8 * 512        # outputs, previous states, two scans' coefficients
+            for o in outs:
+                tape.Backward(o, do)
+            assert AG.Keeping().left == AG.KEEP_BYTES
+    dx = [m.GradTensor() for m in xs]
+    dw = [m.GradTensor() for m in ws]
+    for i in (1, 2, 3):                                         # each within the 2e-5 of the tests above
+        assert float((dx[i] - dx[0]).abs().max()) <= 4e-5 * max(1.0, float(dx[0].abs().max()))
+        assert float((dw[i] - dw[0]).norm()) <= 4e-5 * float(dw[0].norm())
