@@ -159,18 +159,24 @@ __device__ __forceinline__ void report_error(int* status, int code) {
 }
 
 // ---------------------------------------------------------------- programmatic dependent launch
-// A kernel launched with launch_pdl() may start while its predecessor in the stream is still running: its CTAs become
+// A kernel launched with the programmatic flag may start while its predecessor in the stream is still running: its CTAs become
 // resident as SMs free up and run their prologue (barrier initialisation, TMEM allocation, descriptor prefetch) under
 // the predecessor's tail.  pdl_wait() returns once the predecessor has completed and its memory is visible; a kernel
-// launched this way touches no global memory before it.  pdl_launch_dependents(), executed by every CTA of the
+// launched this way touches no global memory before it, with one exception: a few-row product reads a weight that its caller
+// states to be at rest (gemm_skinny.cu).  pdl_launch_dependents(), executed by every CTA of the
 // predecessor, is what allows the early start; in a kernel that is launched the ordinary way both are no-ops.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-// Off unless OA_PDL=1: on the flagship step (591 launches replayed as one graph) both placements of the trigger that were
+// OA_PDL=0: no launch carries the flag; unset: short launches (below) and few-row products; 1: every launch that can.  Long kernels go
+// without it by default: on the flagship step (591 launches replayed as one graph) both placements of the trigger that were
 // tried, at the start and at the end of the long kernels, measured 0.1-0.5 ms per step SLOWER than ordinary launches.
-inline bool pdl_enabled() {
-  static const bool on = [] { const char* e = getenv("OA_PDL"); return e && e[0] == '1'; }();
-  return on;
+enum PdlMode { PDL_NONE, PDL_SHORT, PDL_ALL };
+inline PdlMode pdl_mode() {
+  static const PdlMode mode = [] {
+    const char* e = getenv("OA_PDL");
+    return !e ? PDL_SHORT : e[0] == '0' ? PDL_NONE : e[0] == '1' ? PDL_ALL : PDL_SHORT;
+  }();
+  return mode;
 }
 // Only for kernels that call pdl_wait() before their first global access.
 template <typename... KArgs, typename... Args>
@@ -189,7 +195,7 @@ inline cudaError_t launch_pdl_if(bool on, void (*kernel)(KArgs...), dim3 grid, d
 }
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
-  return launch_pdl_if(pdl_enabled(), kernel, grid, block, smem, st, static_cast<KArgs>(args)...);
+  return launch_pdl_if(pdl_mode() == PDL_ALL, kernel, grid, block, smem, st, static_cast<KArgs>(args)...);
 }
 // Kernels of a few microseconds, which follow one another in a decoding step or in the step of a small model: there the start of a
 // launch (1 to 2 us from its predecessor's last store to its own first load) is a good part of the time, and with the trigger at the
@@ -199,7 +205,7 @@ constexpr long long PDL_SHORT_BLOCKS = 1024;
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_short(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
   const bool few = (long long)grid.x * grid.y * grid.z <= PDL_SHORT_BLOCKS;
-  return launch_pdl_if(few || pdl_enabled(), kernel, grid, block, smem, st, static_cast<KArgs>(args)...);
+  return launch_pdl_if(pdl_mode() == PDL_ALL || (few && pdl_mode() == PDL_SHORT), kernel, grid, block, smem, st, static_cast<KArgs>(args)...);
 }
 
 // ---------------------------------------------------------------- proxies / fences

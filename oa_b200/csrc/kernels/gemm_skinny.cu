@@ -195,7 +195,7 @@ static int launch_skinny(const CUtensorMap& tw, const CUtensorMap& tx, const Ski
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 2;
+  cfg.numAttrs = pdl_mode() == PDL_NONE ? 1 : 2;
   return cudaLaunchKernelEx(&cfg, gemm_skinny_kernel<MT>, tw, tx, p) == cudaSuccess && cudaGetLastError() == cudaSuccess ? OA_OK : OA_ERR_LAUNCH;
 }
 

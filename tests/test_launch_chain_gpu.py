@@ -1,0 +1,52 @@
+"""Programmatic launches: which launches carry the flag under each value of OA_PDL, read from the edges of a captured graph."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+EDGES = """
+import ctypes
+import torch
+from oa_b200.ops import kernels as K
+x = torch.zeros(1024, device="cuda")
+a, w = torch.zeros(4, 512, device="cuda").bfloat16(), torch.zeros(512, 512, device="cuda").bfloat16()
+rows, gain = torch.zeros(8192, 1024, device="cuda").bfloat16(), torch.ones(1024, device="cuda").bfloat16()
+
+def step():
+    K.binary("add", x, x)
+    K.binary("add", x, x)
+    K.gemm(a, w)
+    K.rmsnorm_fwd(rows, gain, 1e-6)
+
+step()
+torch.cuda.synchronize()
+g = torch.cuda.CUDAGraph(keep_graph=True)
+with torch.cuda.graph(g):
+    step()
+n = ctypes.c_size_t(3)
+src, dst, data = (ctypes.c_void_p * 3)(), (ctypes.c_void_p * 3)(), (ctypes.c_uint8 * 24)()      # an edge: from port, to port, type, reserved
+err = ctypes.CDLL("libcudart.so.12").cudaGraphGetEdges_v2(ctypes.c_void_p(g.raw_cuda_graph()), src, dst, data, ctypes.byref(n))
+assert err == 0 and n.value == 3, (err, n.value)
+order = {s: (d, data[8 * i + 2]) for i, (s, d) in enumerate(zip(src, dst))}
+at = next(s for s in order if s not in [d for d, _ in order.values()])
+kinds = []
+while at in order:
+    at, kind = order[at]
+    kinds.append(kind)                    # 1: programmatic
+print("edges", *kinds)
+"""
+
+
+# two short launches, a product of few rows, and a launch of many blocks
+@pytest.mark.parametrize("value,want", [("0", "0 0 0"), (None, "1 1 0"), ("1", "1 1 1")])
+def test_oa_pdl(value, want):
+    env = {k: v for k, v in os.environ.items() if k != "OA_PDL"}
+    if value is not None:
+        env["OA_PDL"] = value
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", EDGES], capture_output=True, text=True, env=env, cwd=root, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+    assert r.stdout.split("edges ")[-1].strip() == want
