@@ -148,8 +148,9 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ B, float*
 // shared memory in short ones.  Before -> now: 2048 x 128 x 512 20.3 -> 13.1 us,
 // 512 x 512 x 512 20.5 -> 13.2, 128 x 128 x 4096 in slices 14.2 -> 11.6 to 13.3, 4096^3 with both operands row-contiguous 3.50 -> 2.72 ms,
 // with both K-contiguous 3.57 -> 3.4 (there the pairs of a register file's double width do not lie side by side).
-// The next kernel's launch is let in at the end, not at the start: blocks that were resident early sit where this kernel left
-// room, not one per SM, and products that followed one another took up to 1.5 times as long.
+// No early trigger for the next launch: its blocks would sit in pairs where this kernel has left room, not one per SM, and two blocks
+// of products share the multiply-add pipe.  A feed-forward of 2048 x 128 and 512 inner columns (two products) in a captured chain: 29.4 us
+// without a trigger, 38.7 with one before the epilogue (30.0 without the flag on the launches); a data and weight gradient 28.8 and 40.9.
 constexpr int F_THREADS = 256;
 template <int ROWS, int MN, int KW>   // a [ROWS x KW] tile: [k][row] when MN, else [row][k]
 struct F32Tile {
@@ -305,7 +306,6 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ B, f
     }
   }
   if (A_MN && sums) f32_store_sum(epi, a_sum, m0 + threadIdx.x, M, k_chunk > 0 ? b : 0);
-  pdl_launch_dependents();
   __syncthreads();                                    // the last stage has been read; the copies still counted are empty
   {
     float* mine = ring + group * (ROWS * FT);

@@ -40,13 +40,50 @@ print("edges", *kinds)
 """
 
 
-# two short launches, a product of few rows, and a launch of many blocks
-@pytest.mark.parametrize("value,want", [("0", "0 0 0"), (None, "1 1 0"), ("1", "1 1 1")])
-def test_oa_pdl(value, want):
+CHAIN = """
+import torch
+from oa_b200.ops import kernels as K
+x, w1, w2 = torch.randn(2048, 128, device="cuda"), torch.randn(512, 128, device="cuda") / 128 ** 0.5, torch.randn(128, 512, device="cuda") / 512 ** 0.5
+
+def step():
+    for _ in range(20):
+        K.gemm(K.gemm(x, w1), w2)
+
+step()
+torch.cuda.synchronize()
+g = torch.cuda.CUDAGraph()
+with torch.cuda.graph(g):
+    step()
+times = []
+for _ in range(15):
+    a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    g.replay()
+    a.record()
+    g.replay()
+    b.record()
+    torch.cuda.synchronize()
+    times.append(a.elapsed_time(b))
+print("ms", sorted(times)[7])
+"""
+
+
+def _run(code, value):
     env = {k: v for k, v in os.environ.items() if k != "OA_PDL"}
     if value is not None:
         env["OA_PDL"] = value
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-    r = subprocess.run([sys.executable, "-c", EDGES], capture_output=True, text=True, env=env, cwd=root, timeout=300)
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, env=env, cwd=root, timeout=300)
     assert r.returncode == 0, r.stderr[-2000:]
-    assert r.stdout.split("edges ")[-1].strip() == want
+    return r.stdout
+
+
+# two short launches, a product of few rows, and a launch of many blocks
+@pytest.mark.parametrize("value,want", [("0", "0 0 0"), (None, "1 1 0"), ("1", "1 1 1")])
+def test_oa_pdl(value, want):
+    assert _run(EDGES, value).split("edges ")[-1].strip() == want
+
+
+def test_chained_products():
+    # the products' blocks need an SM each: a launch that comes early must not put them in pairs, which took 1.3 times as long
+    ms = [float(_run(CHAIN, value).split("ms ")[-1]) for value in (None, "0")]
+    assert ms[0] <= 1.1 * ms[1], ms
