@@ -178,6 +178,7 @@ inline PdlMode pdl_mode() {
   }();
   return mode;
 }
+inline bool pdl_on(bool is_short) { return pdl_mode() == PDL_ALL || (is_short && pdl_mode() == PDL_SHORT); }
 // Only for kernels that call pdl_wait() before their first global access.
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl_if(bool on, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
@@ -195,7 +196,7 @@ inline cudaError_t launch_pdl_if(bool on, void (*kernel)(KArgs...), dim3 grid, d
 }
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
-  return launch_pdl_if(pdl_mode() == PDL_ALL, kernel, grid, block, smem, st, static_cast<KArgs>(args)...);
+  return launch_pdl_if(pdl_on(false), kernel, grid, block, smem, st, static_cast<KArgs>(args)...);
 }
 // Kernels of a few microseconds, which follow one another in a decoding step or in the step of a small model: there the start of a
 // launch (1 to 2 us from its predecessor's last store to its own first load) is a good part of the time, and with the trigger at the
@@ -205,7 +206,7 @@ constexpr long long PDL_SHORT_BLOCKS = 1024;
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_short(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
   const bool few = (long long)grid.x * grid.y * grid.z <= PDL_SHORT_BLOCKS;
-  return launch_pdl_if(pdl_mode() == PDL_ALL || (few && pdl_mode() == PDL_SHORT), kernel, grid, block, smem, st, static_cast<KArgs>(args)...);
+  return launch_pdl_if(pdl_on(few), kernel, grid, block, smem, st, static_cast<KArgs>(args)...);
 }
 
 // ---------------------------------------------------------------- proxies / fences

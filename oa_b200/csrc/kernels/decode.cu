@@ -412,7 +412,13 @@ static int launch_decode_stream(const void* q, long long q_stride, const void* k
   }
   const int n_bh = batch * heads, items = n_bh * splits;
   const int grid = items < 2 * 148 ? items : 2 * 148;
-  launch_short(decode_attn_stream_kernel<HD>, dim3(grid), dim3(160), smem, st, (const __nv_bfloat16*)q, q_stride, (const __nv_bfloat16*)kc,
+  // Early launch only while a CTA has one item and most SMs have two CTAs.  CTAs that become resident as the launch before them drains
+  // do not sit as a launch on a free chip places them: up to one per SM they come in pairs, and beyond 2 x 148 items the CTAs with an item
+  // more share SMs (1024 items are four or three per CTA).  Prompt of 100 and 24 steps at the 7B-class width, 32 heads, with / without
+  // the flag: 2 rows (64 items) 6.33 / 6.26 ms, 4 (128) 6.43 / 6.43, 6 (192) 6.71 / 6.76, 8 (256) 6.80 / 6.87, 10 (320) 6.85 / 6.81, 16
+  // (512) 7.52 / 7.42, 32 (1024) 9.24 / 8.78, 40 10.2 / 9.59; 2600 positions, 2 rows (256) 10.1 / 10.4, 5 (1120) 17.0 / 16.9.
+  const bool early = items > 148 && items <= 2 * 148;
+  launch_pdl_if(pdl_on(early), decode_attn_stream_kernel<HD>, dim3(grid), dim3(160), smem, st, (const __nv_bfloat16*)q, q_stride, (const __nv_bfloat16*)kc,
                (const __nv_bfloat16*)vc, (float*)partial, (__nv_bfloat16*)out, out_stride, heads, n_bh, splits, len, max_seq, sl2, pos_dev, status);
   if (splits > 1) launch_short(decode_merge_kernel<HD>, dim3(n_bh), dim3(HD), 0, st, (const float*)partial, (__nv_bfloat16*)out, out_stride, heads, splits);
   return cudaGetLastError() == cudaSuccess ? OA_OK : OA_ERR_LAUNCH;

@@ -11,25 +11,18 @@ EDGES = """
 import ctypes
 import torch
 from oa_b200.ops import kernels as K
-x = torch.zeros(1024, device="cuda")
-a, w = torch.zeros(4, 512, device="cuda").bfloat16(), torch.zeros(512, 512, device="cuda").bfloat16()
-rows, gain = torch.zeros(8192, 1024, device="cuda").bfloat16(), torch.ones(1024, device="cuda").bfloat16()
 
-def step():
-    K.binary("add", x, x)
-    K.binary("add", x, x)
-    K.gemm(a, w)
-    K.rmsnorm_fwd(rows, gain, 1e-6)
-
+%s
 step()
 torch.cuda.synchronize()
 g = torch.cuda.CUDAGraph(keep_graph=True)
 with torch.cuda.graph(g):
     step()
-n = ctypes.c_size_t(3)
-src, dst, data = (ctypes.c_void_p * 3)(), (ctypes.c_void_p * 3)(), (ctypes.c_uint8 * 24)()      # an edge: from port, to port, type, reserved
+m = LAUNCHES - 1
+n = ctypes.c_size_t(m)
+src, dst, data = (ctypes.c_void_p * m)(), (ctypes.c_void_p * m)(), (ctypes.c_uint8 * (8 * m))()      # an edge: from port, to port, type, reserved
 err = ctypes.CDLL("libcudart.so.12").cudaGraphGetEdges_v2(ctypes.c_void_p(g.raw_cuda_graph()), src, dst, data, ctypes.byref(n))
-assert err == 0 and n.value == 3, (err, n.value)
+assert err == 0 and n.value == m, (err, n.value)
 order = {s: (d, data[8 * i + 2]) for i, (s, d) in enumerate(zip(src, dst))}
 at = next(s for s in order if s not in [d for d, _ in order.values()])
 kinds = []
@@ -39,6 +32,30 @@ while at in order:
 print("edges", *kinds)
 """
 
+# two short launches, a product of few rows, and a launch of many blocks
+MIXED = """
+x = torch.zeros(1024, device="cuda")
+a, w = torch.zeros(4, 512, device="cuda").bfloat16(), torch.zeros(512, 512, device="cuda").bfloat16()
+rows, gain = torch.zeros(8192, 1024, device="cuda").bfloat16(), torch.ones(1024, device="cuda").bfloat16()
+LAUNCHES = 4
+
+def step():
+    K.binary("add", x, x)
+    K.binary("add", x, x)
+    K.gemm(a, w)
+    K.rmsnorm_fwd(rows, gain, 1e-6)
+"""
+
+# cache append, attention of BATCH x 4 heads over unsplit positions
+DECODE = """
+q = torch.zeros(BATCH, 3 * 256, device="cuda").bfloat16()
+k, v = (torch.zeros(BATCH, 4, 16, 64, device="cuda").bfloat16() for _ in range(2))
+LAUNCHES = 2
+
+def step():
+    K.rope_kv_append(q, k, v, 3, 1e4)
+    K.decode_attn(q[:, :256], k, v, 4)
+"""
 
 CHAIN = """
 import torch
@@ -77,13 +94,18 @@ def _run(code, value):
     return r.stdout
 
 
-# two short launches, a product of few rows, and a launch of many blocks
 @pytest.mark.parametrize("value,want", [("0", "0 0 0"), (None, "1 1 0"), ("1", "1 1 1")])
 def test_oa_pdl(value, want):
-    assert _run(EDGES, value).split("edges ")[-1].strip() == want
+    assert _run(EDGES % MIXED, value).split("edges ")[-1].strip() == want
 
 
 def test_chained_products():
     # the products' blocks need an SM each: a launch that comes early must not put them in pairs, which took 1.3 times as long
     ms = [float(_run(CHAIN, value).split("ms ")[-1]) for value in (None, "0")]
     assert ms[0] <= 1.1 * ms[1], ms
+
+
+# up to an SM each, two to an SM at most, more items than CTAs
+@pytest.mark.parametrize("batch,want", [(37, "0"), (38, "1"), (74, "1"), (75, "0")])
+def test_decode_attention(batch, want):
+    assert _run(EDGES % DECODE.replace("BATCH", str(batch)), None).split("edges ")[-1].strip() == want
