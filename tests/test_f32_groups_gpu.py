@@ -44,7 +44,9 @@ def test_attention_rows_off_16_bytes(hd, off):
 @pytest.mark.parametrize("rows,m,n", [(1, 4, 4), (37, 65, 12), (600, 70, 33), (2048, 128, 512), (2048, 512, 128), (500, 1000, 1400), (130, 700, 1500)])
 @pytest.mark.parametrize("accumulate", [False, True])
 @pytest.mark.parametrize("off", [0, 1])
-def test_weight_and_bias_gradient(rows, m, n, accumulate, off):
+def test_weight_and_bias_gradient(rows, m, n, accumulate, off, monkeypatch):
+    launch, names = K._launch, []
+    monkeypatch.setattr(K, "_launch", lambda rc, name, *a, **k: (names.append(name), launch(rc, name, *a, **k)))
     g = torch.Generator(device="cuda").manual_seed(rows + m + n)
     r = lambda *s: torch.randn(*s, device="cuda", generator=g)
     dy, x = r(rows, (m + 7) // 4 * 4)[:, off:off + m], r(rows, (n + 3) // 4 * 4)[:, :n]
@@ -53,6 +55,8 @@ def test_weight_and_bias_gradient(rows, m, n, accumulate, off):
     if accumulate:
         want_w, want_b = want_w + w.double(), want_b + b.double()
     K.weight_grad(dy, x, out=w, accumulate=accumulate, bias_out=b, bias_accumulate=accumulate)
+    # rows off 16 bytes take a product and a column sum of their own
+    assert (names == ["oa_gemm_f32_weight_grad"]) if off == 0 else ("oa_gemm_f32_weight_grad" not in names and "oa_col_sum" in names), names
     assert float((w.double() - want_w).norm() / want_w.norm()) <= 2e-6
     # a column sum of up to 2048 terms of unit variance: a few 2^-24 times the partial sums it runs through, at most sqrt(rows) each
     assert float((b.double() - want_b).abs().max()) <= 2.0 ** -24 * 16 * (rows + 1) ** 0.5
