@@ -122,7 +122,7 @@ class OaGradientTape:
     def __init__(self):
         self._prev = IsEnabled()
         self._active = True
-        self._keep_outside, _tls.keep = getattr(_tls, "keep", None), KeepAllowance()
+        self._keep_outside, _tls.keep = getattr(_tls, "keep", None), None       # made when it is first asked for
         SetEnabled(True)
 
     def __enter__(self):
