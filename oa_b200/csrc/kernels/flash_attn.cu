@@ -785,6 +785,7 @@ struct BwdKvCfg {
   static constexpr int TM_S = 0, TM_DP = NS * FA_BN, TM_DV = TM_DP + FA_BN, TM_DK = TM_DV + HD;
 };
 
+// Two probabilities exp2(s sl2 + nl), over the scores; two p (dp scale + nd), over the probabilities
 __device__ __forceinline__ void bwd_prob2(uint32_t& a, uint32_t& b, unsigned long long sl2, unsigned long long nl) {
   f2_to(f2_fma(f2_of(a, b), sl2, nl), a, b);
   a = __float_as_uint(fast_exp2(__uint_as_float(a))); b = __float_as_uint(fast_exp2(__uint_as_float(b)));
@@ -792,11 +793,7 @@ __device__ __forceinline__ void bwd_prob2(uint32_t& a, uint32_t& b, unsigned lon
 __device__ __forceinline__ void bwd_ds2(uint32_t& a, uint32_t& b, uint32_t d0, uint32_t d1, unsigned long long scale, unsigned long long nd) {
   f2_to(f2_mul(f2_of(a, b), f2_fma(f2_of(d0, d1), scale, nd)), a, b);
 }
-// exp2(s sl2 + nl); p (dp scale + nd); 32 values of a lane as bf16 over 16 columns
-__device__ __forceinline__ uint32_t bwd_prob(uint32_t s, float sl2, float nl) { return __float_as_uint(fast_exp2(fmaf(__uint_as_float(s), sl2, nl))); }
-__device__ __forceinline__ uint32_t bwd_ds(uint32_t p, uint32_t dp, float scale, float nd) {
-  return __float_as_uint(__uint_as_float(p) * fmaf(__uint_as_float(dp), scale, nd));
-}
+// 32 values of a lane as bf16 over 16 columns
 __device__ __forceinline__ void bwd_store16(uint32_t taddr, const uint32_t* v) {
   uint32_t w[16];
 #pragma unroll
