@@ -13,7 +13,7 @@
 // work per score; KS = 4 makes four times as many, shorter CTAs (which under the causal mask also skip more of the other side), lets
 // the next tile arrive through cp.async under this one, and is taken while KS = 1 would leave SMs idle (af_split).
 // 16 x 4 heads of 32 dimensions and 128 positions are 64 CTAs with KS = 1, one warp per scheduler: 29 us forward
-// and 83 us both gradients.  With KS = 4: 14 us, and 38 for both gradients (19, and 53, with eight
+// and 83 us both gradients.  With KS = 4: 14 us, and 38 for both gradients (16.9, and 53.3, with eight
 // dimensions per thread, whose dot products each took two shuffles).
 // Forward and dQ rows are queries (keys / values stream through shared memory), dK / dV rows are keys (queries and output gradients
 // stream through shared memory together with their log-sum-exp and delta = rowsum(dO * O)).

@@ -200,8 +200,12 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
 }
 // Kernels of a few microseconds, which follow one another in a decoding step or in the step of a small model: there the start of a
 // launch (1 to 2 us from its predecessor's last store to its own first load) is a good part of the time, and with the trigger at the
-// kernel's start it runs under the predecessor.  Up to PDL_SHORT_BLOCKS blocks, where all of them are resident at once or nearly so;
-// for grids of many waves the flag bought nothing (above).
+// kernel's start it runs under the predecessor.  Forty dependent launches in a graph, us each without / with the flag: additions of 148
+// blocks 1.59 / 1.38, 1024 2.36 / 1.94, 1184 2.61 / 2.05, 16384 30.2 / 29.7; SwiGLU, which triggers early, 148 1.79 / 1.33, 1024 2.87 / 2.51,
+// 4096 6.09 / 5.58; fp32 products of 256 columns 148 13.3 / 12.7, 1024 68.6 / 67.9.  So half a microsecond whatever the grid: up to
+// PDL_SHORT_BLOCKS, beyond which that is a few percent of a launch.  No watched case moved by more than 0.5 % with the line at any number
+// of blocks (layers of mixture of experts 2036 / 2028 us, Mamba-3 2143 / 2142, attention 907 / 910); with the line at 0 they took 2050, 2157, 908.
+// Kernels whose blocks need an SM to themselves trigger late or take the flag by a rule of their own (gemm_f32.cu, decode.cu).
 constexpr long long PDL_SHORT_BLOCKS = 1024;
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_short(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {

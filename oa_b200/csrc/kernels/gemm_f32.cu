@@ -6,10 +6,10 @@
 //   C[b][m,n] = v + residual (+ C)
 // The epilogue carries what the bf16 kernel's does, so that a Transformer layer in fp32 launches no pass of its own for the saved
 // pre-activation, the activation's gradient or the residual sum.
-// Two kernels of 256 threads and 64 x 64 (or 32 x 64) output tiles, the tiling class of the reference's GemmTiled
+// Three kernels of 256 threads and 64 x 64 (or 32 x 64) output tiles, the tiling class of the reference's GemmTiled
 // (Source/Private/Oa/Core/Shader/Compute/Blas/Gemm/GemmTiled.slang:1-110), with runtime strides so that NT / NN / TN products and
 // Bmm need no transposed copies: gemm_f32_tile_kernel where each operand has one contiguous direction and 16-byte rows (an
-// asynchronous ring of K tiles), gemm_f32_kernel for any other strides (the next K tile prefetched into registers).  Few tiles with a
+// asynchronous ring of K tiles), gemm_f32_brief_kernel for short reductions of such operands, gemm_f32_kernel for any other strides (the next K tile prefetched into registers).  Few tiles with a
 // long reduction: K is sliced over more blocks, and the kernel that adds the slices up carries the epilogue.
 #include <type_traits>
 

@@ -13,9 +13,9 @@
 //
 // What bounds it: the weights' bytes, at 5.6 TB/s in a long product (128-byte pieces of 128 rows), plus 4 to 6 us to start, to meet in
 // the cluster and to store.  The start is taken off where the caller knows that nothing in flight writes W (w_at_rest, a decoding
-// step replayed as a graph): a CTA fills its ring, 27 MB over the chip, under the kernels between two products.  With the launches
-// between them chained the same way (launch_short) a 7B-class two-block step with one row went from 268 to 233 us, 32 + 1 of
-// them with their prompt from 9.45 to 8.23 ms (32 rows, 48 steps: 21.65 to 21.04 ms).
+// step replayed as a graph): a CTA fills its ring, 27 MB over the chip, under the kernels between two products, which are chained the
+// same way (launch_short).  A prompt of 100 and 32 steps of two 7B-class blocks with one row: 8.84 ms with ordinary launches, 8.86 with
+// chained ones alone, 8.14 with the weights requested ahead as well; 256 and 48 steps with 32 rows: 21.0, 20.8 and 20.1 ms.
 // One row against 12288 x 4096 / 4096 x 4096 / 32000 x 4096: 31 / 18 / 66 us, with the tile kernel 38 / 22 / 69; a decoding step of
 // two 7B-class blocks and the head with 32 rows: 233 us of products, 336 us before (tile kernel on the transposed product, split-K
 // reduction, transposing copy and residual add as launches of their own).  Below 512 columns of K or 256 of N the tile kernel's

@@ -113,7 +113,7 @@ xent_kernel(const T* __restrict__ logits, const int* __restrict__ targets, float
 // to shared memory through cp.async; every thread reads back only the 16-byte vectors that it copied itself, so no barrier
 // stands between the copy and its use, and the gradient can be written over the logits.  What bounds it: one read and one
 // write of the logits; the CTAs of an SM (three at 64,000-byte rows) cover one another's reductions.  16384 x 32000 bf16:
-// 475 us with two reads, 410 us (5.1 TB/s) with one.
+// 475 us with two reads, 403 us (5.2 TB/s) with one (419 alone).
 __device__ __forceinline__ void xent_cp16(void* smem_dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_dst)), "l"(src) : "memory");
 }

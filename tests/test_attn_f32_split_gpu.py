@@ -1,4 +1,4 @@
-"""fp32 attention with eight and with 32 head dimensions per thread, at widths and lengths off the tile grid and on both sides of the rule."""
+"""fp32 attention with one and with four groups of threads to a row, at widths and lengths off the tile grid and on both sides of the rule."""
 import pytest
 import torch
 
@@ -27,8 +27,8 @@ def test_attention(hd, causal, batch, seq, heads):
         assert float((a.double() - e.detach()).norm() / torch.maximum(e.detach().norm(), do.double().norm())) <= 8e-6
 
 
-# With a CTA or more per SM the narrow form does more work per score: a full mask took 1.5 times a causal one, 32 dimensions per thread
-# take the same time for both.
+# With a CTA or more per SM a row shared by more threads does more work per score: there a full mask took 1.5 times a causal one, where the
+# form with one group of threads to a row takes the same time for both.
 def test_many_rows_take_the_wide_form():
     def us(causal):
         qkv = torch.randn(8 * 512, 3 * 256, device="cuda")
