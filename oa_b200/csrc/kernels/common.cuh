@@ -489,6 +489,25 @@ __device__ __forceinline__ float2 unpack_bf16x2(uint32_t v) {
   return __bfloat1622float2(b);
 }
 
+// Four 16-byte pieces per lane: lane l of a group of four ends with piece l of each of the group's lanes, in lane order (its own inverse).
+// Between a row to a lane and a store or load that covers eight rows' 64 bytes instead of 32 rows' 16: rows that lie apart cost
+// an access its time by the lines it touches.
+__device__ __forceinline__ void exchange4(uint4* v, int lane) {
+#pragma unroll
+  for (int bit = 1; bit <= 2; bit <<= 1) {
+    const bool up = lane & bit;
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      if (g & bit) continue;
+      uint4 &lo = v[g], &hi = v[g | bit];
+      uint4 x = up ? lo : hi;
+      x.x = __shfl_xor_sync(0xffffffffu, x.x, bit); x.y = __shfl_xor_sync(0xffffffffu, x.y, bit);
+      x.z = __shfl_xor_sync(0xffffffffu, x.z, bit); x.w = __shfl_xor_sync(0xffffffffu, x.w, bit);
+      if (up) lo = x; else hi = x;
+    }
+  }
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

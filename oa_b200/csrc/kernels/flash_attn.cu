@@ -9,12 +9,13 @@
 // head h at column h*head_dim), and O is written merged ([B*S, H*head_dim]), so there are no SplitHeads / MergeHeads
 // passes.
 //
-// Measured facts that shape the kernels: one tcgen05.mma costs about 50 cycles to issue from a thread (the N = 64
-// products are issue bound), an MUFU exponential occupies its pipe for 8 cycles per warp (1024 cycles per 128 x 128
-// tile), and a warp that waits for the tensor pipe between key blocks idles the SFU.  Hence: score tiles are copied
-// to registers and released at once so the next score product is issued under this block's exponentials, products are
-// issued by two or three warps, and every kernel but the single-tile forward is persistent (one CTA per SM walks its
-// work items in snake order, heaviest causal items first), so TMEM, barriers and the operand rings live across items.
+// Measured facts that shape the kernels (clocks of one tcgen05.mma in a row of them): both operands from shared memory 66 at N = 128, 50 at
+// N = 64; A from TMEM 64 and 33; two warps that issue at once share the pipe evenly; a group of eight is seen complete 330 clocks
+// after its last product.  An MUFU exponential occupies its pipe for 8 clocks per warp (1024 per 128 x 128 tile).  Hence: where the
+// columns allow it score tiles are copied to registers and released at once so the next score product is issued under this block's
+// exponentials; where they do not, the issuing order sees to it that a tile's products run under another's exponentials; descriptors are
+// made once; and every kernel but the single-tile forward is persistent (one CTA per SM walks its work items in snake order, heaviest
+// causal items first), so TMEM, barriers and the operand rings live across items.
 //
 // Backward is two kernels, both deterministic (single writer per output element, like the reference's
 // FlashCausalBwdQ / FlashCausalBwdKV): one accumulates dK, dV in TMEM over the query blocks of a key block, the other dQ
@@ -30,9 +31,73 @@ constexpr int FA_BN = 128;   // keys per tile
 constexpr float LOG2E = 1.4426950408889634f;
 constexpr int FA_THREADS = 320;   // single-tile forward: 8 softmax warps + MMA warp + TMA warp
 
+// The descriptor of an operand that starts `bytes` further (the address is in units of 16 bytes in the low bits): an issuing warp makes
+// its descriptors once and only adds to them between products.
+__device__ __forceinline__ uint64_t desc_at(uint64_t desc, uint32_t bytes) { return desc + (bytes >> 4); }
+__device__ __forceinline__ uint64_t desc_k(const void* smem) { return umma_smem_desc_sw128(smem_u32(smem), 16, 1024); }             // reduction contiguous
+__device__ __forceinline__ uint64_t desc_mn(const void* smem) { return umma_smem_desc_sw128(smem_u32(smem), FA_BN * 128, 1024); }   // 128 rows of the reduction
+
 // 64-thread named barrier shared by the two warps that own the same 32 query rows.
 __device__ __forceinline__ void pair_sync(int quad) {
   asm volatile("bar.sync %0, 64;" ::"r"(quad + 1) : "memory");
+}
+
+// Two exponentials 2^x on the multiply-add pipe: x = n + f with n the nearest integer (added and taken off at 1.5 * 2^23), 2^f by the
+// minimax polynomial of degree 5 on [-1/2, 1/2] (relative error 7.5e-8, 2.1e-7 with the rounding of its steps; ex2.approx states 2^-22 =
+// 2.4e-7), 2^n as an exponent field, which is zero at n = -127: below that, -inf included, the result is 0 as ex2.approx.ftz gives it.
+// NaN stays NaN; x up to 127.
+__device__ __forceinline__ unsigned long long f2_splat(float v) { return f2_of(__float_as_uint(v), __float_as_uint(v)); }
+__device__ __forceinline__ float max_nan(float a, float b) {
+  float d;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
+  return d;
+}
+__device__ __forceinline__ unsigned long long exp2_fma2(unsigned long long x) {
+  uint32_t a, b;
+  f2_to(x, a, b);
+  x = f2_of(__float_as_uint(max_nan(__uint_as_float(a), -127.f)), __float_as_uint(max_nan(__uint_as_float(b), -127.f)));
+  const unsigned long long t = f2_add(x, f2_splat(12582912.f));
+  const unsigned long long f = f2_fma(f2_add(t, f2_splat(-12582912.f)), f2_splat(-1.f), x);
+  unsigned long long r = f2_fma(f2_splat(0.00132764725f), f, f2_splat(0.00967554096f));
+  r = f2_fma(r, f, f2_splat(0.0555071309f));
+  r = f2_fma(r, f, f2_splat(0.240221202f));
+  r = f2_fma(r, f, f2_splat(0.693146944f));
+  r = f2_fma(r, f, f2_splat(1.00000012f));
+  f2_to(t, a, b);
+  return f2_mul(r, f2_of((a << 23) + 0x3f800000u, (b << 23) + 0x3f800000u));
+}
+__device__ __forceinline__ unsigned long long exp2_mufu2(unsigned long long x) {
+  uint32_t a, b;
+  f2_to(x, a, b);
+  return f2_of(__float_as_uint(fast_exp2(__uint_as_float(a))), __float_as_uint(fast_exp2(__uint_as_float(b))));
+}
+__device__ __forceinline__ uint32_t f2_bf16(unsigned long long v) {
+  uint32_t a, b;
+  f2_to(v, a, b);
+  return pack_bf16x2(__uint_as_float(a), __uint_as_float(b));
+}
+// How many of eight pairs of exponentials go to the multiply-add pipe: one in the forward pass, one and two in the backward pass, where
+// two warps of a scheduler reach their exponentials together.  The pipe relieves the special-function units and costs issue slots.  Zero /
+// one / two / three, forward: 8 x 2048 x 16 heads of 64 causal 121.9 / 113.7 / 119.0 / 126.7 us, 1 x 4096 x 16 full 103.7 / 106.7 / 114.0 / 119.9,
+// 2 x 3001 x 16 of 128 80.4 / 79.5 / - / 83.7.  Backward, one / two / three / four: 8 x 2048 x 16 of 64 341 / 330 / 336 / 349; of 128, one / two /
+// three: 1 x 4096 x 32 423 / 424 / 433.
+constexpr int FA_FMA_PAIRS = 1;
+
+// 32 fp32 columns of a warp's 32 rows (one row to a lane) as bf16, 64 bytes of eight rows to a store (the rows lie apart by a whole
+// projection).  `at`: the row of this warp's first lane; rows from `rows` on are not written.
+__device__ __forceinline__ void store_rows(__nv_bfloat16* at, long long stride, int rows, const uint32_t* a, float mul, int lane) {
+  uint4 v[4];
+#pragma unroll
+  for (int g = 0; g < 4; ++g) {
+    const float* f = reinterpret_cast<const float*>(a) + g * 8;
+    v[g] = make_uint4(pack_bf16x2(f[0] * mul, f[1] * mul), pack_bf16x2(f[2] * mul, f[3] * mul), pack_bf16x2(f[4] * mul, f[5] * mul), pack_bf16x2(f[6] * mul, f[7] * mul));
+  }
+  exchange4(v, lane);
+  const int r0 = lane & ~3;
+  at += (long long)r0 * stride + (lane & 3) * 8;
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (r0 + k < rows) *reinterpret_cast<uint4*>(at + k * stride) = v[k];
 }
 
 struct FlashParams {
@@ -323,18 +388,22 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 }
 
 // ===================================================================================== forward: two tiles per CTA
-// Two adjacent 128-query tiles of one (batch, head) share a CTA and the K / V rings but are otherwise independent pipelines
-// (softmax warps 0-3 + MMA warp 8 for tile 0, warps 4-7 + MMA warp 9 for tile 1), so their phases drift apart and the
-// exponentials of one tile cover the TMEM traffic, row maxima and barrier hand-offs of the other.  One thread owns one query
-// row (all 128 key columns: no partner exchange).  The score tile is copied to registers and RELEASED at once, so
-// Q K_{j+1}^T is issued while the exponentials of block j run; probabilities have their own TMEM columns:
-// S0 | S1 | P0 | P1 | O0 | O1 = 128 + 128 + 64 + 64 + 64 + 64.
-// The running maximum is updated lazily, as above.
+// Two adjacent 128-query tiles of one (batch, head) share a CTA and the K / V rings, softmax warps 0-3 for tile 0, warps 4-7 for
+// tile 1, and the exponentials of one tile cover the TMEM traffic, row maxima and barrier hand-offs of the other.  One thread owns one
+// query row (all 128 key columns: no partner exchange).  The running maximum is updated lazily, as above.
 // Two threads per row (sixteen softmax warps, maxima exchanged through shared memory) measured 127.7 instead of 121.7 us at head
-// dim 64 (8 x 2048 x 16) and 193 instead of 188 us at head dim 128 (4096 x 32): halving a row's share of the exponentials does not
-// shorten the chain scores -> exponentials -> P V -> next scores of a tile, which one partner tile covers only in part.
-// Head dim 128: O takes the columns of P, so P_t overwrites the first half of S_t (S0 | S1 | O0 | O1 = 4 x 128 columns).  Then
-// Q K_{j+1}^T is issued behind P V_j by the same thread, and it is the other tile's products and exponentials that fill the gap.
+// dim 64 (8 x 2048 x 16).
+// Head dim 64: the score tile is copied to registers and RELEASED at once, so Q K_{j+1}^T is issued while the exponentials of block j
+// run; probabilities have their own TMEM columns, S0 | S1 | P0 | P1 | O0 | O1 = 128 + 128 + 64 + 64 + 64 + 64, and each tile an issuing
+// warp (one warp for both: 125 us against 116, 8 x 2048 x 16 causal).  Bound by the exponentials, 2048 clocks of about 3,000 a pair of blocks.
+// Head dim 128: O takes the columns of P, so P_t overwrites the first half of S_t (S0 | S1 | O0 | O1 = 4 x 128 columns), and Q K_{j+1}^T
+// of a tile can only follow its P V_j.  What counts is that the tiles take turns: ONE warp issues P V and the next scores of one tile and
+// then those of the other, so that a tile's products run at the full rate under the other's exponentials.  With a warp for each tile the
+// products of both were in the pipe together and the exponentials of both after them: 4,870 clocks a pair of blocks, 3,510 in turns, of which the
+// products need 2,080 (and more while copies and operands share the 128 bytes a clock of shared memory).  P is handed over in halves of
+// the keys.  Measured 1 x 4096 x 32 / 2 x 3001 x 16 causal: 168 / 108 us before, 134 / 86 in turns, 130 / 84 with P in halves, 124 / 79.5 with
+// packed arithmetic and a part of the exponentials on the multiply-add pipe.  A wait more in the issuing warp, even for a
+// barrier that is complete, costs (141 / 90 us with the ring waits and arrivals made once per tile and not once for both).
 template <int HD_>
 struct FwdPairCfg {
   static constexpr int HD = HD_;
@@ -349,7 +418,8 @@ struct FwdPairCfg {
   static constexpr int SMEM_BYTES = OFF_BAR + 256;
   static constexpr int TMEM_COLS = 512;
   static constexpr int TM_S = 0, TM_P = ALIAS ? 0 : 256, P_STEP = ALIAS ? FA_BN : 64, TM_O = ALIAS ? 256 : 384;   // S: + 128 * tile, O: + HD * tile
-  static constexpr int THREADS = 352;                        // 8 softmax warps, 2 MMA warps, 1 TMA warp
+  static constexpr int MMA_WARPS = ALIAS ? 1 : 2, TMA_WARP = 8 + MMA_WARPS;   // after 8 softmax warps
+  static constexpr int THREADS = (TMA_WARP + 1) * 32;
 };
 
 __device__ __forceinline__ float fmax3(float a, float b, float c) {
@@ -372,16 +442,16 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::OFF_BAR);
   uint64_t* q_full = bars + 0;
-  uint64_t* q_empty = bars + 1;            // both MMA warps are done with the Q tiles of the item
+  uint64_t* q_empty = bars + 1;            // the MMA warps are done with the Q tiles of the item
   uint64_t* k_full = bars + 2;             // [NS]
   uint64_t* k_empty = k_full + NS;         // [NS]  one arrival per MMA warp
   uint64_t* v_full = k_empty + NS;         // [NS]
   uint64_t* v_empty = v_full + NS;         // [NS]  one arrival per MMA warp
   uint64_t* s_full = v_empty + NS;         // [2]   S_t holds Q_t K_j^T
   uint64_t* s_empty = s_full + 2;          // [2]   ... and is in registers (4 warps)
-  uint64_t* p_full = s_full + 4;           // [2]   P_t written (and O_t rescaled if needed) (4 warps)
-  uint64_t* o_done = s_full + 6;           // [2]   O_t += P_t V_j finished: P_t may be overwritten, O_t may be rescaled
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(s_full + 8);
+  uint64_t* p_full = s_full + 4;           // [2][2]  P_t written, by half of the keys (the first: O_t rescaled if needed) (4 warps)
+  uint64_t* o_done = s_full + 8;           // [2]   O_t += P_t V_j finished: P_t may be overwritten, O_t may be rescaled
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(s_full + 10);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nblk = (p.seq + FA_BM - 1) / FA_BM;
@@ -400,9 +470,9 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV);
     mbar_init(q_full, 1);
-    mbar_init(q_empty, 2);
-    for (int s = 0; s < NS; ++s) { mbar_init(&k_full[s], 1); mbar_init(&v_full[s], 1); mbar_init(&k_empty[s], 2); mbar_init(&v_empty[s], 2); }
-    for (int t = 0; t < 2; ++t) { mbar_init(&s_full[t], 1); mbar_init(&s_empty[t], 4); mbar_init(&p_full[t], 4); mbar_init(&o_done[t], 1); }
+    mbar_init(q_empty, Cfg::MMA_WARPS);
+    for (int s = 0; s < NS; ++s) { mbar_init(&k_full[s], 1); mbar_init(&v_full[s], 1); mbar_init(&k_empty[s], Cfg::MMA_WARPS); mbar_init(&v_empty[s], Cfg::MMA_WARPS); }
+    for (int t = 0; t < 2; ++t) { mbar_init(&s_full[t], 1); mbar_init(&s_empty[t], 4); mbar_init(&p_full[2 * t], 4); mbar_init(&p_full[2 * t + 1], 4); mbar_init(&o_done[t], 1); }
     mbar_fence_init();
   }
   if (warp == 8) { tmem_alloc<Cfg::TMEM_COLS>(tmem_slot); tmem_relinquish(); }
@@ -422,7 +492,7 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     nkv1 = (2 * pr + 1 < nblk) ? (p.causal ? (2 * pr + 2) : nblk) : 0;
   };
 
-  if (warp == 10) {
+  if (warp == Cfg::TMA_WARP) {
     // ------------- producer
     uint32_t blk = 0, itc = 0;   // K / V blocks and items loaded so far
     bool ok = true;
@@ -462,27 +532,97 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       }
       ++itc;
     }
-  } else if (warp == 8 || warp == 9) {
+  } else if (ALIAS && warp == 8) {
+    // ------------- MMA issuer of both tiles, in turn (warp-uniform waits, one lane issues)
+    constexpr uint32_t idesc_qk = umma_idesc_bf16(FA_BM, FA_BN, 0, 0);
+    constexpr uint32_t idesc_pv = umma_idesc_bf16(FA_BM, HD, 0, 1);
+    uint32_t base = 0, itc = 0, pc[2] = {0, 0};   // K / V blocks before this item, items, P V products of each tile so far
+    bool ok = true;
+    const uint64_t q_desc = desc_k(smem + Cfg::OFF_Q), k_desc = desc_k(smem + Cfg::OFF_K), v_desc = desc_mn(smem + Cfg::OFF_V);
+    // S_t = Q_t K^T of ring block `blk`; `first` / `last`: of the tiles that read it, `end`: nothing reads Q after it
+    auto issue_qk = [&](int t, uint32_t blk, bool first, bool last, bool end) -> bool {
+      const int st = blk % NS;
+      if (first && !warp_wait(&k_full[st], (blk / NS) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_FULL); return false; }
+      tc_fence_after();
+      if (elect_one()) {
+        const uint64_t qd = desc_at(q_desc, t * Cfg::Q_BYTES), kd = desc_at(k_desc, st * Cfg::KV_BYTES);
+#pragma unroll
+        for (int ks = 0; ks < HD / 16; ++ks) {
+          const uint32_t off = (ks >> 2) * (FA_BM * 128) + (ks & 3) * 32;
+          umma_f16(tmem_base + Cfg::TM_S + t * FA_BN, desc_at(qd, off), desc_at(kd, off), idesc_qk, ks > 0 ? 1u : 0u);
+        }
+        umma_commit(&s_full[t]);
+        if (last) umma_commit(&k_empty[st]);
+        if (end) umma_commit(q_empty);
+      }
+      __syncwarp();
+      return true;
+    };
+    for (int round = 0; round < n_rounds && ok; ++round) {
+      const int item = item_of(round);
+      if (item >= n_items) continue;
+      int pr, h, b, n[2];
+      decode(item, pr, h, b, n[0], n[1]);
+      const int n_it = max(n[0], n[1]);
+      if (!warp_wait(q_full, itc & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_FULL); break; }
+      // a block's tiles: both, or the one whose row of blocks is longer (tile 1, unless it is absent)
+      auto qk = [&](int t, int j) -> bool {
+        const bool last = j >= n[1 - t] || t == 1;
+        return issue_qk(t, base + j, t == 0 || j >= n[0], last, last && j + 1 == n_it);
+      };
+      if (n[0] > 0) ok = qk(0, 0);
+      if (ok && n[1] > 0) ok = qk(1, 0);
+      for (int j = 0; j < n_it && ok; ++j) {
+        const int st = (base + j) % NS;
+        if (!warp_wait(&v_full[st], ((base + j) / NS) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_FULL); ok = false; break; }
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          if (j >= n[t]) continue;
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            if (!warp_wait(&p_full[2 * t + half], pc[t] & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_SOFTMAX); ok = false; break; }
+            tc_fence_after();
+            if (elect_one()) {
+              const uint64_t vd = desc_at(v_desc, st * Cfg::KV_BYTES);
+              const uint32_t p_tm = tmem_base + Cfg::TM_P + t * Cfg::P_STEP, o_tm = tmem_base + Cfg::TM_O + t * HD;
+#pragma unroll
+              for (int ks = half * 4; ks < half * 4 + 4; ++ks)
+                umma_f16_ts(o_tm, p_tm + ks * 8, desc_at(vd, ks * 2048), idesc_pv, (j > 0 || ks > 0) ? 1u : 0u);
+              if (half == 1) {
+                if (t == 1 || j >= n[1]) umma_commit(&v_empty[st]);
+                if (j + 1 == n[t]) umma_commit(&o_done[t]);
+              }
+            }
+            __syncwarp();
+          }
+          if (!ok) break;
+          ++pc[t];
+          if (j + 1 < n[t]) { ok = qk(t, j + 1); if (!ok) break; }   // overwrites P_j: ordered after P_j V_j by the pipe
+        }
+      }
+      base += n_it;
+      ++itc;
+    }
+  } else if (!ALIAS && warp >= 8) {
     // ------------- MMA issuer of tile t (warp-uniform waits, lane 0 issues)
     const int t = warp - 8;
     constexpr uint32_t idesc_qk = umma_idesc_bf16(FA_BM, FA_BN, 0, 0);
     constexpr uint32_t idesc_pv = umma_idesc_bf16(FA_BM, HD, 0, 1);
-    const uint32_t q_addr = smem_u32(smem + Cfg::OFF_Q + t * Cfg::Q_BYTES);
+    const uint64_t qd = desc_k(smem + Cfg::OFF_Q + t * Cfg::Q_BYTES), k_desc = desc_k(smem + Cfg::OFF_K), v_desc = desc_mn(smem + Cfg::OFF_V);
     const uint32_t s_tm = tmem_base + Cfg::TM_S + t * FA_BN, p_tm = tmem_base + Cfg::TM_P + t * Cfg::P_STEP, o_tm = tmem_base + Cfg::TM_O + t * HD;
     uint32_t base = 0, itc = 0, sc = 0, pc = 0;   // K / V blocks before this item, items, S products and P V products of this tile so far
     bool ok = true;
     auto issue_qk = [&](uint32_t blk, bool last) -> bool {       // S_t = Q_t K^T of ring block `blk`
       const int st = blk % NS;
       if (!warp_wait(&k_full[st], (blk / NS) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_FULL); return false; }
-      if (!ALIAS && sc > 0 && !warp_wait(&s_empty[t], (sc - 1) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_TMEM_EMPTY); return false; }
+      if (sc > 0 && !warp_wait(&s_empty[t], (sc - 1) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_TMEM_EMPTY); return false; }
       tc_fence_after();
       if (elect_one()) {
-        const uint32_t k_addr = smem_u32(smem + Cfg::OFF_K + st * Cfg::KV_BYTES);
+        const uint64_t kd = desc_at(k_desc, st * Cfg::KV_BYTES);
 #pragma unroll
         for (int ks = 0; ks < HD / 16; ++ks) {
           const uint32_t off = (ks >> 2) * (FA_BM * 128) + (ks & 3) * 32;
-          umma_f16(s_tm, umma_smem_desc_sw128(q_addr + off, 16, 1024), umma_smem_desc_sw128(k_addr + off, 16, 1024),
-                   idesc_qk, ks > 0 ? 1u : 0u);
+          umma_f16(s_tm, desc_at(qd, off), desc_at(kd, off), idesc_qk, ks > 0 ? 1u : 0u);
         }
         umma_commit(&k_empty[st]);
         umma_commit(&s_full[t]);
@@ -502,22 +642,21 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       if (!warp_wait(q_full, itc & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_FULL); break; }
       if (n > 0) ok = issue_qk(base, n == 1);
       for (int j = 0; j < n && ok; ++j) {
-        if (!ALIAS && j + 1 < n) { ok = issue_qk(base + j + 1, j + 2 == n); if (!ok) break; }
+        if (j + 1 < n) { ok = issue_qk(base + j + 1, j + 2 == n); if (!ok) break; }
         const int st = (base + j) % NS;
         if (!warp_wait(&v_full[st], ((base + j) / NS) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_FULL); ok = false; break; }
-        if (!warp_wait(&p_full[t], pc & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_SOFTMAX); ok = false; break; }
+        if (!warp_wait(&p_full[2 * t], pc & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_SOFTMAX); ok = false; break; }
         tc_fence_after();
         if (elect_one()) {
-          const uint32_t v_addr = smem_u32(smem + Cfg::OFF_V + st * Cfg::KV_BYTES);
+          const uint64_t vd = desc_at(v_desc, st * Cfg::KV_BYTES);
 #pragma unroll
           for (int ks = 0; ks < FA_BN / 16; ++ks)
-            umma_f16_ts(o_tm, p_tm + ks * 8, umma_smem_desc_sw128(v_addr + ks * 2048, FA_BN * 128, 1024), idesc_pv, (j > 0 || ks > 0) ? 1u : 0u);
+            umma_f16_ts(o_tm, p_tm + ks * 8, desc_at(vd, ks * 2048), idesc_pv, (j > 0 || ks > 0) ? 1u : 0u);
           umma_commit(&v_empty[st]);
-          if (!ALIAS || j + 1 == n) umma_commit(&o_done[t]);
+          umma_commit(&o_done[t]);
         }
         __syncwarp();
         ++pc;
-        if (ALIAS && j + 1 < n) { ok = issue_qk(base + j + 1, j + 2 == n); if (!ok) break; }   // overwrites P_j: ordered after P_j V_j by the pipe
       }
       // blocks of this item that this tile does not use (the last one of the pair's shorter tile, or all of an absent tile):
       // the rings still expect one arrival per MMA warp, given once the block has landed
@@ -598,40 +737,54 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           ++pc;
           tc_fence_after();
         }
-        float l0 = 0.f, l1 = 0.f, l2 = 0.f, l3 = 0.f;
+        auto rescale = [&]() {                               // some row of this warp moved its maximum: rescale O
+          if (j == 0 || !__any_sync(0xffffffffu, grow)) return;
+#pragma unroll 1
+          for (int q = 0; q < HD / 32; ++q) {
+            uint32_t o[32];
+            tmem_ld32(o_addr + q * 32, o);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+            tmem_st32(o_addr + q * 32, o);
+          }
+        };
+        auto hand_over = [&](int half) {
+          tmem_st_wait();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&p_full[2 * t + half]);
+        };
+        unsigned long long l01 = 0, l23 = 0;
+        const unsigned long long sl22 = f2_splat(sl2), neg_m2 = f2_splat(neg_m);
 #pragma unroll
         for (int c = 0; c < FA_BN / 32; ++c) {
           uint32_t pk[16];
 #pragma unroll
           for (int i = 0; i < 32; i += 4) {
-            const float e0 = fast_exp2(fmaf(__uint_as_float(sv[c * 32 + i]), sl2, neg_m));
-            const float e1 = fast_exp2(fmaf(__uint_as_float(sv[c * 32 + i + 1]), sl2, neg_m));
-            const float e2 = fast_exp2(fmaf(__uint_as_float(sv[c * 32 + i + 2]), sl2, neg_m));
-            const float e3 = fast_exp2(fmaf(__uint_as_float(sv[c * 32 + i + 3]), sl2, neg_m));
-            l0 += e0; l1 += e1; l2 += e2; l3 += e3;
-            pk[i >> 1] = pack_bf16x2(e0, e1);
-            pk[(i >> 1) + 1] = pack_bf16x2(e2, e3);
+            const uint32_t* sc4 = sv + c * 32 + i;
+            const unsigned long long x01 = f2_fma(f2_of(sc4[0], sc4[1]), sl22, neg_m2), x23 = f2_fma(f2_of(sc4[2], sc4[3]), sl22, neg_m2);
+            const unsigned long long e01 = exp2_mufu2(x01), e23 = (i >> 2) % 4 < FA_FMA_PAIRS ? exp2_fma2(x23) : exp2_mufu2(x23);
+            l01 = f2_add(l01, e01);
+            l23 = f2_add(l23, e23);
+            pk[i >> 1] = f2_bf16(e01);
+            pk[(i >> 1) + 1] = f2_bf16(e23);
           }
           tmem_st16(p_addr + c * 16, pk);
-        }
-        l_run = l_run * alpha + ((l0 + l1) + (l2 + l3));
-        m_run = m_cand;
-        if (j > 0 && __any_sync(0xffffffffu, grow)) {
-          // some row of this warp moved its maximum: rescale O
-#pragma unroll
-          for (int c = 0; c < HD / 32; ++c) {
-            uint32_t o[32];
-            tmem_ld32(o_addr + c * 32, o);
-            tmem_ld_wait();
-#pragma unroll
-            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-            tmem_st32(o_addr + c * 32, o);
+          if (ALIAS && (c & 1)) {                        // the products of half of the keys start under the other half's exponentials
+            if (c == 1) rescale();
+            hand_over(c >> 1);
           }
         }
-        tmem_st_wait();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&p_full[t]);
+        if (!ALIAS) {
+          rescale();
+          hand_over(0);
+        }
+        uint32_t lw[4];
+        f2_to(l01, lw[0], lw[1]);
+        f2_to(l23, lw[2], lw[3]);
+        l_run = l_run * alpha + ((__uint_as_float(lw[0]) + __uint_as_float(lw[1])) + (__uint_as_float(lw[2]) + __uint_as_float(lw[3])));
+        m_run = m_cand;
       }
       if (!ok) break;
       ok = warp_wait(&o_done[t], pc & 1);
@@ -639,16 +792,19 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       ++pc;
       tc_fence_after();
       const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
-      __nv_bfloat16* op = p.o + (long long)(row0 + qi) * p.o_stride + h * HD;
+      const int q0 = qbt * FA_BM + quad * 32;
+      __nv_bfloat16* op = p.o + (long long)(row0 + q0) * p.o_stride + h * HD;
 #pragma unroll
       for (int c = 0; c < HD / 32; ++c) {
         uint32_t o[32];
         tmem_ld32(o_addr + c * 32, o);
         tmem_ld_wait();
-        if (qi < p.seq) {
+        if (ALIAS) store_rows(op + c * 32, p.o_stride, p.seq - q0, o, inv, lane);
+        else if (qi < p.seq) {
+          __nv_bfloat16* od = p.o + (long long)(row0 + qi) * p.o_stride + h * HD + c * 32;
 #pragma unroll
           for (int g = 0; g < 4; ++g)
-            *reinterpret_cast<uint4*>(op + c * 32 + g * 8) = make_uint4(
+            *reinterpret_cast<uint4*>(od + g * 8) = make_uint4(
                 pack_bf16x2(__uint_as_float(o[g * 8]) * inv, __uint_as_float(o[g * 8 + 1]) * inv),
                 pack_bf16x2(__uint_as_float(o[g * 8 + 2]) * inv, __uint_as_float(o[g * 8 + 3]) * inv),
                 pack_bf16x2(__uint_as_float(o[g * 8 + 4]) * inv, __uint_as_float(o[g * 8 + 5]) * inv),
@@ -676,17 +832,18 @@ static int launch_fwd2(const CUtensorMap& tq, const CUtensorMap& tk, const CUten
   return cudaGetLastError() == cudaSuccess ? OA_OK : OA_ERR_LAUNCH;
 }
 
-// Head dim 128: whether the pair kernel beats one tile per CTA.  Per key block it is the slower one (its P lies over S: 2.8 us for two
-// tiles, 1.1 us for one), and it puts two tiles where one SM each was free; it gains what a CTA costs to start and to drain, so it
-// wants enough items and short rows of key blocks.  Measured, single tile against pair: causal 32 x 256 x 16 heads 49 / 34 us,
-// 1 x 2048 x 32 59.5 / 50, 1 x 4096 x 32 178 / 175, 1 x 8192 x 16 312 / 332, and with few items 1 x 1024 x 8 13.8 / 25.8,
-// 1 x 4096 x 10 71 / 93, 2 x 2048 x 10 43 / 49; full 64 x 384 x 16 162 / 136, 4 x 1024 x 32 96 / 106, 1 x 4096 x 32 278 / 370.  The
-// lines lie where a sweep over 1 to 36 blocks and 150 to 1000 items changes sign (three blocks, 160 items: 15.9 / 18.3).
+// Head dim 128: whether the pair kernel beats one tile per CTA.  A pair of tiles takes 1.55 times as long as one, so it loses only where
+// pairs leave SMs free that single tiles would fill.  Full rows are a matter of whole waves: single tile against pair, us, at 8 key blocks
+// 60 / 148 / 200 / 300 pairs 17.1 / 22.0, 30.6 / 24.2, 41.6 / 38.5, 67.7 / 54.0; at 32 64 / 96 / 160 / 304 / 992 pairs 43 / 62, 79 / 63, 112 / 114,
+// 184 / 171, 508 / 378; at 64 96 / 192 / 448 141 / 115, 210 / 227, 480 / 444.  Causal rows even out over the SMs: 4 blocks 60 / 148 / 300 pairs
+// 19.7 / 20.5, 22.0 / 19.7, 39.6 / 28.2; 9 blocks 60 / 100 / 150 / 445 21.0 / 22.1, 24.2 / 22.0, 30.0 / 24.0, 69.1 / 50.5; 16 blocks 96 / 144 / 600 34.2 / 35.8,
+// 42.7 / 36.3, 127 / 88; 32 blocks 96 / 144 / 992 50 / 61, 67 / 63, 306 / 207.
 static bool flash_pair_hd128(int nblk, long long heads, long long batch, int causal, int sms) {
   if (heads > 65535 || batch > 65535) return true;       // beyond the single-tile kernel's grid
-  const long long items = (long long)((nblk + 1) / 2) * heads * batch;
-  if (!causal) return nblk == 1 ? items > sms : (nblk <= 3 ? items >= 2 * sms : nblk == 4 && items >= 4 * sms);
-  return nblk <= 8 && nblk != 3 ? items > sms : (nblk <= 32 && 2 * items >= 3 * sms);
+  const long long rows = heads * batch, items = (long long)((nblk + 1) / 2) * rows;
+  if (causal) return nblk <= 7 || (nblk <= 12 ? 3 * items >= 2 * sms : items >= sms);
+  const long long pair_rounds = (items + sms - 1) / sms, tile_waves = (nblk * rows + sms - 1) / sms;
+  return 2 * tile_waves > 3 * pair_rounds || (tile_waves > pair_rounds && nblk < 24);
 }
 
 template <int HD>
