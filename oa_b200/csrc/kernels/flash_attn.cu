@@ -82,6 +82,7 @@ __device__ __forceinline__ uint32_t f2_bf16(unsigned long long v) {
 // 2 x 3001 x 16 of 128 80.4 / 79.5 / - / 83.7.  Backward, one / two / three / four: 8 x 2048 x 16 of 64 341 / 330 / 336 / 349; of 128, one / two /
 // three: 1 x 4096 x 32 423 / 424 / 433.
 constexpr int FA_FMA_PAIRS = 1;
+template <int HD> constexpr int FA_BWD_FMA_PAIRS = HD == 64 ? 2 : 1;
 
 // 32 fp32 columns of a warp's 32 rows (one row to a lane) as bf16, 64 bytes of eight rows to a store (the rows lie apart by a whole
 // projection).  `at`: the row of this warp's first lane; rows from `rows` on are not written.
@@ -915,13 +916,20 @@ constexpr int FA_BWD_THREADS = 352;   // 8 softmax warps + 2 MMA issuer warps + 
 // probabilities (scores and dV), the other those that hang on dS (dP and dK, or dP and dQ); within a warp the products that reuse
 // tensor-memory columns are ordered by the pipe.  The bf16 results overwrite the columns they were computed from, each half of the
 // columns within its own 64, so neither half waits for the other before it stores, and the gradient products start on the first half.
-// Bound by the latency of that chain: at head dim 64 the exponentials take 1024 of about 2,900 clocks per tile, at head dim 128 the
-// products 2,200 of about 4,000, and a barrier that is already complete costs a warp 100 clocks or more while the pipes are busy.
-// Measured, dK/dV and dQ kernel, with one barrier for both phases (scores and dP issued together, both read before either was
-// computed on) -> this: 2 x 3001 x 16 heads of 128 194 and 129 -> 161 and 109 us, 1 x 4096 x 32 of 128 325 and 206 -> 268 and 182,
-// 8 x 2048 x 16 of 64 195 and 164 -> 191 and 160.  Slower: one issuing warp for all four products (172 us, 260 us at head dim 64),
-// sixteen softmax warps (300 us at head dim 64 with the two phases merged into one pass; every wait is made by twice the warps),
-// one lane waiting for its warp (261 us), partner warps of a scheduler taking turns at the exponentials (212 us).
+// At head dim 128 the columns leave room for one score tile, so the scores of tile i + 1 can only follow dV of tile i, and the next
+// exponentials wait for both: the issuer of dK and dP waits its turn until those scores are in the pipe (`turn`), and its products run under
+// the exponentials.  Left to themselves they ran beside dV and the scores, which took twice as long, and nothing under the exponentials.
+// The kernels are bound by that chain: at head dim 64 the exponentials take 1024 of about 2,400 clocks per tile, at head dim 128 the
+// products 2,080 of about 3,500, and a barrier that is already complete costs a warp 100 clocks or more while the pipes are busy.
+// dK, dV and dQ leave through store_rows; with 16-byte stores of a row to a lane the end of an item took 4,000 to 5,000 clocks, 15 to 20 %.
+// Measured, us of the whole backward pass: before / dK, dP in turn / rows by store_rows / part of the exponentials on the multiply-add pipe
+// 1 x 4096 x 32 heads of 128 468 / 448 / 430 / 423, 2 x 3001 x 16 of 128 282 / 270 / 254 / 247, 8 x 2048 x 16 of 64 369 / 369 / 344 / 330, 8 x 512 x 16
+// of 64 60 / 60 / 55 / 53.
+// dK/dV and dQ kernel, with one barrier for both phases (scores and dP issued together, both read before either was computed on) -> with
+// two: 2 x 3001 x 16 heads of 128 194 and 129 -> 161 and 109 us, 8 x 2048 x 16 of 64 195 and 164 -> 191 and 160.  Slower: one issuing warp for all
+// four products (172 us, 260 us at head dim 64), sixteen softmax warps (300 us at head dim 64 with the two phases merged into one pass;
+// every wait is made by twice the warps), one lane waiting for its warp (261 us), partner warps of a scheduler taking turns at the
+// exponentials (212 us), and the halves of a tile as pipelines of their own (128 478, 64 365: a product of 64 columns takes 50 clocks, one of 128 66).
 //
 // The dK/dV kernel works on the TRANSPOSED tile, S^T = K Q^T with keys on the TMEM lanes, because dV = P^T dO and
 // dK = dS^T Q need P^T / dS^T with keys as the M dimension.  Per-query statistics (log-sum-exp, delta) are then per
@@ -943,9 +951,10 @@ struct BwdKvCfg {
 };
 
 // Two probabilities exp2(s sl2 + nl), over the scores; two p (dp scale + nd), over the probabilities
+template <bool FMA = false>
 __device__ __forceinline__ void bwd_prob2(uint32_t& a, uint32_t& b, unsigned long long sl2, unsigned long long nl) {
-  f2_to(f2_fma(f2_of(a, b), sl2, nl), a, b);
-  a = __float_as_uint(fast_exp2(__uint_as_float(a))); b = __float_as_uint(fast_exp2(__uint_as_float(b)));
+  const unsigned long long x = f2_fma(f2_of(a, b), sl2, nl);
+  f2_to(FMA ? exp2_fma2(x) : exp2_mufu2(x), a, b);
 }
 __device__ __forceinline__ void bwd_ds2(uint32_t& a, uint32_t& b, uint32_t d0, uint32_t d1, unsigned long long scale, unsigned long long nd) {
   f2_to(f2_mul(f2_of(a, b), f2_fma(f2_of(d0, d1), scale, nd)), a, b);
@@ -980,7 +989,8 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   uint64_t* dp_full = bars + 20;   // dP^T
   uint64_t* ds_full = bars + 21;   // [2]  dS^T, by column half (4 warps each)
   uint64_t* fin_full = bars + 23;  // dV, dK of the item are complete (both issuers arrive)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 24);
+  uint64_t* turn = bars + 24;      // NS == 1: the next tile's scores are in the pipe, dK and dP may follow
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 25);
   float* stat = reinterpret_cast<float*>(smem + Cfg::OFF_STAT);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1011,6 +1021,7 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     for (int s = 0; s < 4; ++s) mbar_init(&p_full[s], 4);
     mbar_init(dp_full, 1);
     mbar_init(fin_full, 2);
+    mbar_init(turn, 1);
     mbar_fence_init();
   }
   if (warp == 8) { tmem_alloc<Cfg::TMEM_COLS>(tmem_slot); tmem_relinquish(); }
@@ -1084,7 +1095,7 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     // ------------- MMA issuer A: S^T = K Q^T and dV += P^T dO.  S^T of a tile goes over the P^T that dV read NS tiles ago.
     constexpr uint32_t idesc_s = umma_idesc_bf16(FA_BN, FA_BM, 0, 0);
     constexpr uint32_t idesc_g = umma_idesc_bf16(FA_BN, HD, 0, 1);   // [keys x HD] += X^T[keys x q] (TMEM) * Y[q x HD]
-    const uint32_t k_addr = smem_u32(smem + Cfg::OFF_K);
+    const uint64_t k_desc = desc_k(smem + Cfg::OFF_K), q_desc = desc_k(smem + Cfg::OFF_Q), do_desc = desc_mn(smem + Cfg::OFF_DO);
     uint32_t itc = 0, qc = 0;
     bool ok = true;
     auto issue_s = [&](uint32_t n, bool last) -> bool {
@@ -1092,12 +1103,12 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       if (!warp_wait(&q_full[st], (n / NST) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_FULL); return false; }
       tc_fence_after();
       if (elect_one()) {
-        const uint32_t q_addr = smem_u32(smem + Cfg::OFF_Q + st * Cfg::T_BYTES);
+        const uint64_t qd = desc_at(q_desc, st * Cfg::T_BYTES);
         const uint32_t s_tm = tmem_base + Cfg::TM_S + (n % NS) * FA_BN;
 #pragma unroll
         for (int ks = 0; ks < HD / 16; ++ks) {
           const uint32_t off = (ks >> 2) * (FA_BM * 128) + (ks & 3) * 32;
-          umma_f16(s_tm, umma_smem_desc_sw128(k_addr + off, 16, 1024), umma_smem_desc_sw128(q_addr + off, 16, 1024), idesc_s, ks > 0 ? 1u : 0u);
+          umma_f16(s_tm, desc_at(k_desc, off), desc_at(qd, off), idesc_s, ks > 0 ? 1u : 0u);
         }
         umma_commit(&s_full[n % NS]);
         if (last) umma_commit(kv_empty);
@@ -1118,7 +1129,7 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         if (NS == 2 && it + 1 < n_it) { ok = issue_s(qc + 1, it + 2 == n_it); if (!ok) break; }
         const int st = qc % NST;
         if (!warp_wait(&do_full[st], (qc / NST) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_FULL); ok = false; break; }
-        const uint32_t b_addr = smem_u32(smem + Cfg::OFF_DO + st * Cfg::T_BYTES);
+        const uint64_t bd = desc_at(do_desc, st * Cfg::T_BYTES);
         const uint32_t a_addr = tmem_base + Cfg::TM_S + (qc % NS) * FA_BN;
         for (int half = 0; half < 2; ++half) {
           // an item's first product replaces the accumulator: wait until both halves' warps have read the previous item's
@@ -1128,7 +1139,7 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           if (elect_one()) {
 #pragma unroll
             for (int ks = 0; ks < 4; ++ks)    // reduction over the 64 queries of this half
-              umma_f16_ts(tmem_base + Cfg::TM_DV, a_addr + half * 64 + ks * 8, umma_smem_desc_sw128(b_addr + (half * 4 + ks) * 2048, FA_BM * 128, 1024),
+              umma_f16_ts(tmem_base + Cfg::TM_DV, a_addr + half * 64 + ks * 8, desc_at(bd, (half * 4 + ks) * 2048),
                           idesc_g, (it > 0 || half > 0 || ks > 0) ? 1u : 0u);
             if (half == 1) {
               umma_commit(&do_empty[st]);
@@ -1138,7 +1149,10 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           __syncwarp();
         }
         if (!ok) break;
-        if (NS == 1 && it + 1 < n_it) ok = issue_s(qc + 1, it + 2 == n_it);
+        if (NS == 1) {
+          if (it + 1 < n_it) ok = issue_s(qc + 1, it + 2 == n_it);
+          if (lane == 0) mbar_arrive(turn);
+        }
       }
       ++itc;
     }
@@ -1146,7 +1160,7 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     // ------------- MMA issuer B: dP^T = V dO^T and dK += dS^T Q.  dP^T of a tile goes over the dS^T that dK has read.
     constexpr uint32_t idesc_s = umma_idesc_bf16(FA_BN, FA_BM, 0, 0);
     constexpr uint32_t idesc_g = umma_idesc_bf16(FA_BN, HD, 0, 1);
-    const uint32_t v_addr = smem_u32(smem + Cfg::OFF_V);
+    const uint64_t v_desc = desc_k(smem + Cfg::OFF_V), do_desc = desc_k(smem + Cfg::OFF_DO), q_desc = desc_mn(smem + Cfg::OFF_Q);
     const uint32_t dp_tm = tmem_base + Cfg::TM_DP;
     uint32_t itc = 0, qc = 0;
     bool ok = true;
@@ -1155,11 +1169,11 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       if (!warp_wait(&do_full[st], (n / NST) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_FULL); return false; }
       tc_fence_after();
       if (elect_one()) {
-        const uint32_t do_addr = smem_u32(smem + Cfg::OFF_DO + st * Cfg::T_BYTES);
+        const uint64_t dd = desc_at(do_desc, st * Cfg::T_BYTES);
 #pragma unroll
         for (int ks = 0; ks < HD / 16; ++ks) {
           const uint32_t off = (ks >> 2) * (FA_BM * 128) + (ks & 3) * 32;
-          umma_f16(dp_tm, umma_smem_desc_sw128(v_addr + off, 16, 1024), umma_smem_desc_sw128(do_addr + off, 16, 1024), idesc_s, ks > 0 ? 1u : 0u);
+          umma_f16(dp_tm, desc_at(v_desc, off), desc_at(dd, off), idesc_s, ks > 0 ? 1u : 0u);
         }
         umma_commit(dp_full);
         umma_commit(&do_empty[st]);
@@ -1179,7 +1193,8 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       for (int it = 0; it < n_it && ok; ++it, ++qc) {
         const int st = qc % NST;
         if (!warp_wait(&q_full[st], (qc / NST) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_FULL); ok = false; break; }
-        const uint32_t b_addr = smem_u32(smem + Cfg::OFF_Q + st * Cfg::T_BYTES);
+        const uint64_t bd = desc_at(q_desc, st * Cfg::T_BYTES);
+        if (NS == 1 && !warp_wait(turn, qc & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_EMPTY); ok = false; break; }
         for (int half = 0; half < 2; ++half) {
           if (it == 0 && half == 0) ok = warp_wait(&ds_full[1], qc & 1);   // as for dV
           if (!ok || !warp_wait(&ds_full[half], qc & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_SOFTMAX); ok = false; break; }
@@ -1187,7 +1202,7 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           if (elect_one()) {
 #pragma unroll
             for (int ks = 0; ks < 4; ++ks)
-              umma_f16_ts(tmem_base + Cfg::TM_DK, dp_tm + half * 64 + ks * 8, umma_smem_desc_sw128(b_addr + (half * 4 + ks) * 2048, FA_BM * 128, 1024),
+              umma_f16_ts(tmem_base + Cfg::TM_DK, dp_tm + half * 64 + ks * 8, desc_at(bd, (half * 4 + ks) * 2048),
                           idesc_g, (it > 0 || half > 0 || ks > 0) ? 1u : 0u);
             if (half == 1) {
               umma_commit(&q_empty[st]);
@@ -1240,7 +1255,8 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             const ulonglong2 nl = nl4[c * 8 + (i >> 2)];
             uint32_t* sc = s + c * 32 + i;
             bwd_prob2(sc[0], sc[1], sl22, nl.x);
-            bwd_prob2(sc[2], sc[3], sl22, nl.y);
+            if ((i >> 2) % 4 < FA_BWD_FMA_PAIRS<HD>) bwd_prob2<true>(sc[2], sc[3], sl22, nl.y);
+            else bwd_prob2(sc[2], sc[3], sl22, nl.y);
           }
           if (diag) {
 #pragma unroll
@@ -1280,27 +1296,17 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       if (!ok) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_TMEM_FULL); break; }
       ++itc;
       tc_fence_after();
-      const int kj = jb * FA_BN + r;   // accumulator rows are keys
+      const int k0 = jb * FA_BN + quad * 32;   // accumulator rows are keys
 #pragma unroll 1
       for (int which = 0; which < 2; ++which) {
-        __nv_bfloat16* base = (which == 0 ? p.dv : p.dk) + (long long)(row0 + kj) * p.dkv_stride + h * HD;
-        const uint32_t tcol = which == 0 ? Cfg::TM_DV : Cfg::TM_DK;
-#pragma unroll 1
-        for (int cc = 0; cc < HD / 64; ++cc) {
-          const int c = half * (HD / 64) + cc;
-          uint32_t a[32];
-          tmem_ld32(t_lane + tcol + c * 32, a);
-          tmem_ld_wait();
-          if (kj < p.seq) {
+        __nv_bfloat16* base = (which == 0 ? p.dv : p.dk) + (long long)(row0 + k0) * p.dkv_stride + h * HD + half * (HD / 2);
+        const uint32_t tcol = t_lane + (which == 0 ? Cfg::TM_DV : Cfg::TM_DK) + half * (HD / 2);
+        uint32_t a[HD / 2];
 #pragma unroll
-            for (int g = 0; g < 4; ++g)
-              *reinterpret_cast<uint4*>(base + c * 32 + g * 8) = make_uint4(
-                  pack_bf16x2(__uint_as_float(a[g * 8]), __uint_as_float(a[g * 8 + 1])),
-                  pack_bf16x2(__uint_as_float(a[g * 8 + 2]), __uint_as_float(a[g * 8 + 3])),
-                  pack_bf16x2(__uint_as_float(a[g * 8 + 4]), __uint_as_float(a[g * 8 + 5])),
-                  pack_bf16x2(__uint_as_float(a[g * 8 + 6]), __uint_as_float(a[g * 8 + 7])));
-          }
-        }
+        for (int c = 0; c < HD / 64; ++c) tmem_ld32(tcol + c * 32, a + c * 32);
+        tmem_ld_wait();
+#pragma unroll
+        for (int c = 0; c < HD / 64; ++c) store_rows(base + c * 32, p.dkv_stride, p.seq - k0, a + c * 32, 1.f, lane);
       }
       tc_fence_before();   // dV / dK are read before this warp's next p_full / ds_full arrivals let the next item's products overwrite them
     }
@@ -1428,7 +1434,7 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   } else if (warp == 8) {
     // ------------- MMA issuer A: S = Q K_j^T
     constexpr uint32_t idesc_s = umma_idesc_bf16(FA_BM, FA_BN, 0, 0);
-    const uint32_t q_addr = smem_u32(smem + Cfg::OFF_Q);
+    const uint64_t q_desc = desc_k(smem + Cfg::OFF_Q), k_desc = desc_k(smem + Cfg::OFF_K);
     uint32_t itc = 0, kc = 0;
     bool ok = true;
     for (int round = 0; round < n_rounds && ok; ++round) {
@@ -1444,12 +1450,11 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         if (kc > 1 && !warp_wait(&s_empty[kc & 1], ((kc >> 1) - 1) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_TMEM_EMPTY); ok = false; break; }
         tc_fence_after();
         if (elect_one()) {
-          const uint32_t k_addr = smem_u32(smem + Cfg::OFF_K + st * Cfg::T_BYTES);
+          const uint64_t kd = desc_at(k_desc, st * Cfg::T_BYTES);
 #pragma unroll
           for (int ks = 0; ks < HD / 16; ++ks) {
             const uint32_t off = (ks >> 2) * (FA_BM * 128) + (ks & 3) * 32;
-            umma_f16(tmem_base + Cfg::TM_S + (kc & 1) * FA_BN, umma_smem_desc_sw128(q_addr + off, 16, 1024),
-                     umma_smem_desc_sw128(k_addr + off, 16, 1024), idesc_s, ks > 0 ? 1u : 0u);
+            umma_f16(tmem_base + Cfg::TM_S + (kc & 1) * FA_BN, desc_at(q_desc, off), desc_at(kd, off), idesc_s, ks > 0 ? 1u : 0u);
           }
           umma_commit(&s_full[kc & 1]);
           if (j + 1 == n_kv) umma_commit(q_empty);
@@ -1462,7 +1467,7 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     // ------------- MMA issuer B: dP = dO V_j^T and dQ += dS K_j (dS from TMEM, over dP)
     constexpr uint32_t idesc_s = umma_idesc_bf16(FA_BM, FA_BN, 0, 0);
     constexpr uint32_t idesc_q = umma_idesc_bf16(FA_BM, HD, 0, 1);   // dQ[q x HD] += dS[q x keys] * K[keys x HD]
-    const uint32_t do_addr = smem_u32(smem + Cfg::OFF_DO);
+    const uint64_t do_desc = desc_k(smem + Cfg::OFF_DO), v_desc = desc_k(smem + Cfg::OFF_V), k_desc = desc_mn(smem + Cfg::OFF_K);
     const uint32_t dp_tm = tmem_base + Cfg::TM_DP;
     uint32_t itc = 0, kc = 0;
     bool ok = true;
@@ -1471,11 +1476,11 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       if (!warp_wait(&v_full[st], (n / NV) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_FULL); return false; }
       tc_fence_after();
       if (elect_one()) {
-        const uint32_t v_addr = smem_u32(smem + Cfg::OFF_V + st * Cfg::T_BYTES);
+        const uint64_t vd = desc_at(v_desc, st * Cfg::T_BYTES);
 #pragma unroll
         for (int ks = 0; ks < HD / 16; ++ks) {
           const uint32_t off = (ks >> 2) * (FA_BM * 128) + (ks & 3) * 32;
-          umma_f16(dp_tm, umma_smem_desc_sw128(do_addr + off, 16, 1024), umma_smem_desc_sw128(v_addr + off, 16, 1024), idesc_s, ks > 0 ? 1u : 0u);
+          umma_f16(dp_tm, desc_at(do_desc, off), desc_at(vd, off), idesc_s, ks > 0 ? 1u : 0u);
         }
         umma_commit(dp_full);
         umma_commit(&v_empty[st]);
@@ -1495,7 +1500,7 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       for (int j = 0; j < n_kv && ok; ++j, ++kc) {
         const int st = kc % NK;
         if (!warp_wait(&k_full[st], (kc / NK) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_FULL); ok = false; break; }
-        const uint32_t k_addr = smem_u32(smem + Cfg::OFF_K + st * Cfg::T_BYTES);
+        const uint64_t kd = desc_at(k_desc, st * Cfg::T_BYTES);
         for (int half = 0; half < 2; ++half) {
           // an item's first product replaces the accumulator: wait until both halves' warps have read the previous item's
           if (j == 0 && half == 0) ok = warp_wait(&ds_full[1], kc & 1);
@@ -1504,7 +1509,7 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           if (elect_one()) {
 #pragma unroll
             for (int ks = 0; ks < 4; ++ks)
-              umma_f16_ts(tmem_base + Cfg::TM_DQ, dp_tm + half * 64 + ks * 8, umma_smem_desc_sw128(k_addr + (half * 4 + ks) * 2048, FA_BN * 128, 1024),
+              umma_f16_ts(tmem_base + Cfg::TM_DQ, dp_tm + half * 64 + ks * 8, desc_at(kd, (half * 4 + ks) * 2048),
                           idesc_q, (j > 0 || half > 0 || ks > 0) ? 1u : 0u);
             if (half == 1) {
               umma_commit(&k_empty[st]);
@@ -1555,7 +1560,11 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         const int k0 = j * FA_BN;
         const bool need_mask = (p.causal && j == ib) || (k0 + FA_BN > p.seq) || !q_ok;
 #pragma unroll
-        for (int i = 0; i < 64; i += 2) bwd_prob2(s[i], s[i + 1], sl22, nlse2);
+        for (int i = 0; i < 64; i += 4) {
+          bwd_prob2(s[i], s[i + 1], sl22, nlse2);
+          if ((i >> 2) % 4 < FA_BWD_FMA_PAIRS<HD>) bwd_prob2<true>(s[i + 2], s[i + 3], sl22, nlse2);
+          else bwd_prob2(s[i + 2], s[i + 3], sl22, nlse2);
+        }
         if (need_mask) {
           const int lim = q_ok ? (min(p.causal ? qi : 0x7fffffff, p.seq - 1) - (k0 + half * 64)) : -1;
 #pragma unroll
@@ -1584,23 +1593,14 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       if (!ok) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_TMEM_FULL); break; }
       ++itc;
       tc_fence_after();
-      __nv_bfloat16* base = p.dq + (long long)(row0 + qi) * p.dq_stride + h * HD;
-#pragma unroll 1
-      for (int cc = 0; cc < HD / 64; ++cc) {
-        const int c = half * (HD / 64) + cc;
-        uint32_t a[32];
-        tmem_ld32(t_lane + Cfg::TM_DQ + c * 32, a);
-        tmem_ld_wait();
-        if (q_ok) {
+      const int q0 = ib * FA_BM + quad * 32;
+      __nv_bfloat16* base = p.dq + (long long)(row0 + q0) * p.dq_stride + h * HD + half * (HD / 2);
+      uint32_t a[HD / 2];
 #pragma unroll
-          for (int g = 0; g < 4; ++g)
-            *reinterpret_cast<uint4*>(base + c * 32 + g * 8) = make_uint4(
-                pack_bf16x2(__uint_as_float(a[g * 8]), __uint_as_float(a[g * 8 + 1])),
-                pack_bf16x2(__uint_as_float(a[g * 8 + 2]), __uint_as_float(a[g * 8 + 3])),
-                pack_bf16x2(__uint_as_float(a[g * 8 + 4]), __uint_as_float(a[g * 8 + 5])),
-                pack_bf16x2(__uint_as_float(a[g * 8 + 6]), __uint_as_float(a[g * 8 + 7])));
-        }
-      }
+      for (int c = 0; c < HD / 64; ++c) tmem_ld32(t_lane + Cfg::TM_DQ + half * (HD / 2) + c * 32, a + c * 32);
+      tmem_ld_wait();
+#pragma unroll
+      for (int c = 0; c < HD / 64; ++c) store_rows(base + c * 32, p.dq_stride, p.seq - q0, a + c * 32, 1.f, lane);
       tc_fence_before();   // dQ is read before this warp's next ds_full arrival lets the next item's products overwrite it
     }
   }

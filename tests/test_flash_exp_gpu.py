@@ -64,3 +64,31 @@ def test_invalid_scores_show(hd, bad):
         q, k, v = (t.double() for t in _split(x, hd, 1))
         ref = torch.softmax(q @ k.t() / hd ** 0.5, -1) @ v
         assert torch.equal(torch.isnan(o), torch.isnan(ref)), (pos, bad)
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("batch,seq", [(2, 1), (2, 30), (2, 33), (3, 127), (2, 131), (2, 258), (1, 515)])
+def test_backward_writes_its_rows_only(hd, causal, batch, seq):
+    """Rows of one sequence end beside the next one's: gradients against 64 bits, and nothing beyond the last row."""
+    heads = 2
+    D = heads * hd
+    g = torch.Generator(device="cuda").manual_seed(seq)
+    qkv = torch.randn(batch * seq, 3 * D, device="cuda", generator=g).bfloat16()
+    do = torch.randn(batch * seq, D, device="cuda", generator=g).bfloat16()
+    o, lse = K.flash_fwd(*_split(qkv, hd, heads), batch, seq, heads, hd, causal=causal)
+    room = torch.full((batch * seq + 8, 3 * D), 7.0, device="cuda", dtype=torch.bfloat16)
+    K.flash_bwd(*_split(qkv, hd, heads), o, do, lse, batch, seq, heads, hd, causal=causal, dqkv=room[:batch * seq])
+    x = qkv.double().requires_grad_(True)
+    q, k, v = (t.reshape(batch, seq, heads, hd).transpose(1, 2) for t in _split(x, hd, heads))
+    s = q @ k.transpose(-1, -2) / hd ** 0.5
+    if causal:
+        s = s.masked_fill(~torch.ones(seq, seq, dtype=torch.bool, device="cuda").tril(), float("-inf"))
+    ref, = torch.autograd.grad((torch.softmax(s, -1) @ v).transpose(1, 2).reshape(batch * seq, D), x, do.double())
+    # probabilities, their gradients, the output of the forward pass and the results are rounded to bf16: in the norm up to 2^-9 each
+    for i in range(3):
+        e, r = room[:batch * seq, i * D:(i + 1) * D].double() - ref[:, i * D:(i + 1) * D], ref[:, i * D:(i + 1) * D]
+        assert float(e.norm()) <= 2.0 ** -7 * float(r.norm()) + 1e-2 * (seq == 1)
+    assert bool((room[batch * seq:] == 7.0).all())
+    torch.cuda.synchronize()
+    K.check_status()
