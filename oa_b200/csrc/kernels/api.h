@@ -251,6 +251,7 @@ int oa_upsample_nearest(int dtype, const void* in, void* out, long long planes, 
 int oa_kv_append(const void* k_src, const void* v_src, long long src_stride, void* k_cache, void* v_cache, int batch,
                  int s_new, int heads, int head_dim, int pos0, int max_seq, const int* pos_dev, void* stream);
 // Rotate-half embedding of q and k of one new token per sequence (x rows q | k | v) in place, and the append of k and v.
+int oa_decode_begin(const void* table, const int* ids, void* x, int* pos, int n_ids, int dim, int vocab, void* stream);
 int oa_rope_kv_append(void* x, long long row_stride, int batch, int heads, int head_dim, int pos, float theta,
                       const int* pos_dev, void* k_cache, void* v_cache, int max_seq, void* stream);
 int oa_decode_attn(const void* q, long long q_stride, const void* k_cache, const void* v_cache, void* out, long long out_stride,

@@ -1113,6 +1113,13 @@ def kv_append(k_src: torch.Tensor, v_src: torch.Tensor, k_cache: torch.Tensor, v
                                      heads, hd, pos0, max_seq, N.ptr(pos_dev), N.stream()), "oa_kv_append")
 
 
+def decode_begin(table: torch.Tensor, ids: torch.Tensor, x: torch.Tensor, pos: torch.Tensor) -> None:
+    """x [n, dim] = table[ids] and pos += 1 in one launch (bf16; ids int32 on the same device)."""
+    assert table.is_contiguous() and x.is_contiguous() and ids.is_contiguous() and ids.dtype == torch.int32 and pos.dtype == torch.int32
+    _launch(N.require().oa_decode_begin(table.data_ptr(), ids.data_ptr(), x.data_ptr(), pos.data_ptr(), ids.numel(), table.shape[1], table.shape[0],
+                                        N.stream()), "oa_decode_begin")
+
+
 def rope_kv_append(qkv: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, pos: int, theta: float,
                    pos_dev: Optional[torch.Tensor] = None) -> None:
     """One new token per sequence: RoPE on q and k of the packed rows [batch, 3 * heads * head_dim] in place, then k and v into the caches

@@ -38,8 +38,8 @@ class OaKvCache:
 
 class _GraphedStep:
     """One decode step captured in a CUDA graph.  The position lives on the device (`pos`, int32 [1]): RoPE, the cache
-    append and the attention length read it inside their kernels and the graph's last node adds one, so replaying needs no
-    host-side parameter.  `ids` is the static input, the captured function's result the static output."""
+    append and the attention length read it inside their kernels and the captured function or what runs before it adds one, so
+    replaying needs no host-side parameter.  `ids` is the static input, the captured function's result the static output."""
 
     def __init__(self, device, batch: int):
         self.pos = torch.zeros(1, dtype=torch.int32, device=device)
@@ -47,12 +47,18 @@ class _GraphedStep:
         self.graph: Optional[torch.cuda.CUDAGraph] = None
         self.out = None
 
-    def run(self, ids: torch.Tensor, fn, weights=lambda: ()):
-        """`weights()`: tensors that the step reads and never writes."""
-        self.ids.copy_(ids.reshape(self.ids.shape))
+    def run(self, ids: torch.Tensor, fn, weights=lambda: (), begin=None):
+        """`weights()`: tensors that the step reads and never writes.  `begin(ids)`: work on the caller's ids that runs before the
+        graph, which then leaves the position alone."""
+        if begin is None or ids.dtype != torch.int32 or ids.device != self.ids.device or not ids.is_contiguous():
+            self.ids.copy_(ids.reshape(self.ids.shape))
+            ids = self.ids
+        if begin is not None:
+            begin(ids)
         if self.graph is None:
             fn(self.ids)                              # eager once: lazily created buffers (workspaces) exist before the capture
-            self.pos.sub_(1)
+            if begin is None:
+                self.pos.sub_(1)
             torch.cuda.synchronize()
             g = torch.cuda.CUDAGraph()
             # a replay begins after everything before it on the stream, so whatever changed the weights has finished by then
@@ -71,6 +77,9 @@ class OaGptDecoder:
         self.Cache = OaKvCache(c.NLayers, batch, c.NHeads, max_seq, c.DModel // c.NHeads, w.dtype, w.device)
         self._graphed = _GraphedStep(w.device, batch) if use_graph and w.is_cuda and w.dtype == torch.bfloat16 else None
         self._pos_dev: Optional[torch.Tensor] = None      # set while a graphed step records / replays
+        if self._graphed is not None:
+            self._graphed.pos.fill_(-1)                   # of the newest token: a step begins by adding one
+            self._step_x = torch.zeros((batch, c.DModel), dtype=w.dtype, device=w.device)
 
     # ---- one block on new tokens
     def _block(self, i: int, x: OaMatrix, batch: int, s_new: int) -> OaMatrix:
@@ -108,14 +117,17 @@ class OaGptDecoder:
             return F.Linear(F.SiluMul(F.Linear(hh, f.Gate.Weight.Data), F.Linear(hh, f.Up.Weight.Data)), f.Down.Weight.Data, None, residual=x)
         return f.Forward(x)
 
-    def _forward(self, ids: torch.Tensor) -> torch.Tensor:
-        """ids [B, s_new] int32 -> logits of the last new position [B, vocab]; the cache grows by s_new."""
+    def _forward(self, ids: torch.Tensor, x: Optional[torch.Tensor] = None) -> torch.Tensor:
+        """ids [B, s_new] int32 -> logits of the last new position [B, vocab]; the cache grows by s_new.  `x`: the rows of the ids,
+        fetched already."""
         m = self.Model
         batch, s_new = ids.shape
         if self.Cache.Length + s_new > self.Cache.MaxSeq:
             raise ValueError("KV cache is full")
         with AG.OaGradNo():
-            if m.PosEmbed is not None:
+            if x is not None:
+                x = OaMatrix(x)
+            elif m.PosEmbed is not None:
                 pos = m.PosEmbed.Weight.Tensor()[self.Cache.Length:self.Cache.Length + s_new]
                 x = F.Embedding(m.Embed.Weight.Data, OaMatrix(ids.contiguous()), OaMatrix(pos.contiguous()), s_new)
             else:
@@ -130,16 +142,15 @@ class OaGptDecoder:
         self.Cache.Reset()
         out = self._forward(prompt)
         if self._graphed is not None:
-            self._graphed.pos.fill_(self.Cache.Length)
+            self._graphed.pos.fill_(self.Cache.Length - 1)
         return out
 
     def _graph_body(self, ids: torch.Tensor) -> torch.Tensor:
         self._pos_dev = self._graphed.pos
         try:
             length = self.Cache.Length
-            out = self._forward(ids)
+            out = self._forward(ids, self._step_x)
             self.Cache.Length = length                  # the host-side length advances once per Step, not per recording
-            self._graphed.pos.add_(1)
             return out
         finally:
             self._pos_dev = None
@@ -152,7 +163,8 @@ class OaGptDecoder:
             return self._forward(ids.reshape(-1, 1))
         if self.Cache.Length + 1 > self.Cache.MaxSeq:
             raise ValueError("KV cache is full")
-        out = g.run(ids, self._graph_body, lambda: [p.Data.Tensor() for p in self.Model.AllParameterPtrs()])
+        out = g.run(ids, self._graph_body, lambda: [p.Data.Tensor() for p in self.Model.AllParameterPtrs()],
+                    lambda new: K.decode_begin(self.Model.Embed.Weight.Tensor(), new, self._step_x, self._graphed.pos))
         self.Cache.Length += 1
         return out
 
