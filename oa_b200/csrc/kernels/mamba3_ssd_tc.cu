@@ -8,9 +8,10 @@
 //   ssd_chunk_bwd   recomputes M, then dM = dY X^T and every product of the backward pass that needs only this chunk:
 //                   dX = M^T dY + w (B~ dH^T), dC~ = dG B~ + e^cum (dY Hin) + dqk B~, dB~ = dG^T C~ + (w X) dH + dqk C~, and the row
 //                   and column sums that carry d cum, d scale, d gamma, d w.  dC~ and dB~ leave once, in fp32.
-// What bounds them: the bytes of the operands and, backward, the serial chain of a chunk (loads, scores, mask, products, stores)
-// on one CTA per SM.  2 x 4096 tokens x 48 heads: forward 76 us, backward 344 us; the batched products and elementwise kernels
-// they replace took 0.42 and 1.0 ms.
+// What bounds them: the bytes of the operands and, backward, the serial chain of a chunk (scores, mask, products, stores) on one CTA
+// per SM.  2 x 4096 tokens x 48 heads: forward 77 -> 72 us, backward 337 -> 280 us since a row's results leave as 64 bytes at a time (16 bytes
+// of a row to a lane touch 32 lines a store, and a chunk has 8,000 of them) and the next C~ and B~ arrive under the epilogue; the batched
+// products and elementwise kernels they replace took 0.42 and 1.0 ms.
 #include "common.cuh"
 #include "api.h"
 
@@ -160,10 +161,17 @@ ssd_chunk_fwd_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_const
       tc_fence_after();
       const long long row = (long long)b * p.L + (long long)c * CQ + t;
       const float e = __expf(ct);
-      __nv_bfloat16* yo = p.y + row * p.ldy + h * CP;
+      const long long row4 = row - (lane & 3);           // rows of this lane's group of four: accesses cover 64 bytes of eight rows
+      const int col4 = h * CP + (lane & 3) * 8;
 #pragma unroll 1
       for (int q = 0; q < 2; ++q) {
         uint32_t u[32], v[32];
+        uint4 zv[4], o[4], gated[4];
+        if (p.z) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) zv[k] = *reinterpret_cast<const uint4*>(p.z + (row4 + k) * p.ldz + col4 + q * 32);
+          exchange4(zv, lane);
+        }
         tmem_ld32(tm + t_lane + 128 + q * 32, u);
         tmem_ld32(tm + t_lane + 192 + q * 32, v);
         tmem_ld_wait();
@@ -172,19 +180,25 @@ ssd_chunk_fwd_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_const
           float r[8];
 #pragma unroll
           for (int j = 0; j < 8; ++j) r[j] = fmaf(e, __uint_as_float(v[8 * i + j]), __uint_as_float(u[8 * i + j]));
-          uint4 o = make_uint4(pack_bf16x2(r[0], r[1]), pack_bf16x2(r[2], r[3]), pack_bf16x2(r[4], r[5]), pack_bf16x2(r[6], r[7]));
+          o[i] = make_uint4(pack_bf16x2(r[0], r[1]), pack_bf16x2(r[2], r[3]), pack_bf16x2(r[4], r[5]), pack_bf16x2(r[6], r[7]));
           if (p.z) {
-            *reinterpret_cast<uint4*>(p.yraw + row * p.ldy + h * CP + q * 32 + i * 8) = o;
-            const uint4 zp = *reinterpret_cast<const uint4*>(p.z + row * p.ldz + h * CP + q * 32 + i * 8);
-            const uint32_t zs[4] = {zp.x, zp.y, zp.z, zp.w};
+            const uint32_t zs[4] = {zv[i].x, zv[i].y, zv[i].z, zv[i].w};
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
               const float2 zf = unpack_bf16x2(zs[j]);
               r[2 * j] *= silu_f(zf.x); r[2 * j + 1] *= silu_f(zf.y);
             }
-            o = make_uint4(pack_bf16x2(r[0], r[1]), pack_bf16x2(r[2], r[3]), pack_bf16x2(r[4], r[5]), pack_bf16x2(r[6], r[7]));
+            gated[i] = make_uint4(pack_bf16x2(r[0], r[1]), pack_bf16x2(r[2], r[3]), pack_bf16x2(r[4], r[5]), pack_bf16x2(r[6], r[7]));
           }
-          *reinterpret_cast<uint4*>(yo + q * 32 + i * 8) = o;
+        }
+        exchange4(o, lane);
+        __nv_bfloat16* raw_out = p.z ? p.yraw : p.y;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) *reinterpret_cast<uint4*>(raw_out + (row4 + k) * p.ldy + col4 + q * 32) = o[k];
+        if (p.z) {
+          exchange4(gated, lane);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) *reinterpret_cast<uint4*>(p.y + (row4 + k) * p.ldy + col4 + q * 32) = gated[k];
         }
       }
     } else if (lane == 0) {
@@ -209,8 +223,9 @@ struct SsdChunkBwd {
 };
 
 struct ChunkBwdSmem {
-  static constexpr int OFF_C = 0, OFF_B = 2 * HALF, OFF_X = 4 * HALF, OFF_XW = 5 * HALF, OFF_DY = 6 * HALF, OFF_H = 7 * HALF, OFF_DH = 8 * HALF;
-  static constexpr int OFF_M = 9 * HALF, OFF_DG = 11 * HALF;       // bf16 M and dG in the swizzle of the operands
+  // Two regions of 64 KB change roles from chunk to chunk: one holds C~ | B~, the other M | dG (bf16, in the swizzle of the operands).  The
+  // next chunk's C~ and B~ land where M and dG were as soon as the products have read those, under this chunk's epilogue.
+  static constexpr int OFF_R0 = 0, OFF_X = 4 * HALF, OFF_XW = 5 * HALF, OFF_DY = 6 * HALF, OFF_H = 7 * HALF, OFF_DH = 8 * HALF, OFF_R1 = 9 * HALF;
   static constexpr int OFF_F = 13 * HALF;
   static constexpr int BYTES = OFF_F + (3 + 4 + 2 + 2) * CQ * 4 + 1024;
   static_assert(BYTES <= 227 * 1024, "shared memory");
@@ -237,7 +252,7 @@ ssd_chunk_bwd_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_const
                      const __grid_constant__ CUtensorMap tmDH, const SsdChunkBwd p) {
   using S = ChunkBwdSmem;
   extern __shared__ uint8_t raw[];
-  __shared__ uint64_t cb_full, ops_full, s_full, m_full, fin_full, cb_free, ops_free;
+  __shared__ uint64_t cb_full, ops_full, s_full, m_full, fin_full, acc_free, ops_free;
   __shared__ uint32_t tmem_slot;
   uint8_t* sm = raw + ((1024u - (smem_u32(raw) & 1023u)) & 1023u);
   float* s_cum = reinterpret_cast<float*>(sm + S::OFF_F);
@@ -251,7 +266,7 @@ ssd_chunk_bwd_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_const
     tma_prefetch_desc(&tmC); tma_prefetch_desc(&tmB); tma_prefetch_desc(&tmX); tma_prefetch_desc(&tmXw);
     tma_prefetch_desc(&tmDY); tma_prefetch_desc(&tmH); tma_prefetch_desc(&tmDH);
     mbar_init(&cb_full, 1); mbar_init(&ops_full, 1); mbar_init(&s_full, 1); mbar_init(&m_full, 8); mbar_init(&fin_full, 1);
-    mbar_init(&cb_free, 8); mbar_init(&ops_free, 1);
+    mbar_init(&acc_free, 8); mbar_init(&ops_free, 1);
     mbar_fence_init();
   }
   if (warp == 8) { tmem_alloc<512>(&tmem_slot); tmem_relinquish(); }
@@ -263,15 +278,21 @@ ssd_chunk_bwd_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_const
   constexpr uint32_t TM_A = 0, TM_B = 128, TM_CE = 256, TM_XW = 384, TM_X = 448;
 
   if (warp == 8) {
-    const uint32_t c_a = smem_u32(sm + S::OFF_C), b_a = smem_u32(sm + S::OFF_B), x_a = smem_u32(sm + S::OFF_X), xw_a = smem_u32(sm + S::OFF_XW),
-                   dy_a = smem_u32(sm + S::OFF_DY), h_a = smem_u32(sm + S::OFF_H), dh_a = smem_u32(sm + S::OFF_DH), m_a = smem_u32(sm + S::OFF_M),
-                   dg_a = smem_u32(sm + S::OFF_DG);
+    const uint32_t x_a = smem_u32(sm + S::OFF_X), xw_a = smem_u32(sm + S::OFF_XW), dy_a = smem_u32(sm + S::OFF_DY), h_a = smem_u32(sm + S::OFF_H),
+                   dh_a = smem_u32(sm + S::OFF_DH);
     uint32_t n = 0;
     bool ok = true;
     for (int g = blockIdx.x; g < p.G && ok; g += gridDim.x, ++n) {
-      // operands that only the products read are free when the previous chunk's products are done; C~ and B~ when its epilogue is
+      uint8_t* cb = sm + ((n & 1) ? S::OFF_R1 : S::OFF_R0);
+      const uint32_t c_a = smem_u32(cb), b_a = c_a + 2 * HALF, m_a = smem_u32(sm + ((n & 1) ? S::OFF_R0 : S::OFF_R1)), dg_a = m_a + 2 * HALF;
+      // the previous chunk's products have read their operands, M and dG
       ok = warp_wait(&ops_free, (n & 1) ^ 1);
       if (ok && elect_one()) {
+        mbar_expect_tx(&cb_full, 4 * HALF);
+        for (int x = 0; x < 2; ++x) {
+          tma_load_2d(cb + x * HALF, &tmC, &cb_full, x * 64, g * CQ);
+          tma_load_2d(cb + (2 + x) * HALF, &tmB, &cb_full, x * 64, g * CQ);
+        }
         mbar_expect_tx(&ops_full, 5 * HALF);
         tma_load_2d(sm + S::OFF_DY, &tmDY, &ops_full, 0, g * CQ);
         tma_load_2d(sm + S::OFF_X, &tmX, &ops_full, 0, g * CQ);
@@ -282,16 +303,8 @@ ssd_chunk_bwd_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_const
         }
       }
       __syncwarp();
-      ok = ok && warp_wait(&cb_free, (n & 1) ^ 1);
-      if (ok && elect_one()) {
-        mbar_expect_tx(&cb_full, 4 * HALF);
-        for (int x = 0; x < 2; ++x) {
-          tma_load_2d(sm + S::OFF_C + x * HALF, &tmC, &cb_full, x * 64, g * CQ);
-          tma_load_2d(sm + S::OFF_B + x * HALF, &tmB, &cb_full, x * 64, g * CQ);
-        }
-      }
-      __syncwarp();
-      ok = ok && warp_wait(&ops_full, n & 1) && warp_wait(&cb_full, n & 1);
+      // the accumulators are free when the previous chunk's epilogue has read them
+      ok = ok && warp_wait(&cb_full, n & 1) && warp_wait(&ops_full, n & 1) && warp_wait(&acc_free, (n & 1) ^ 1);
       if (!ok) break;
       tc_fence_after();
       if (elect_one()) {
@@ -347,8 +360,11 @@ ssd_chunk_bwd_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_const
       if (half == 0) { s_cum[t] = ct; s_scale[t] = p.scale[gi]; }
       asm volatile("bar.sync 1, 256;" ::: "memory");   // also: the previous chunk's sums have been read
       // a wait that runs out is not left early: the worker warps meet at barriers, so they all finish the loop (without waiting again)
-      ok = ok && warp_wait(&s_full, n & 1);
+      // C~ and B~ are waited for here: the barrier of the next chunk's may complete once this chunk's products are done
+      ok = ok && warp_wait(&s_full, n & 1) && warp_wait(&cb_full, n & 1);
       tc_fence_after();
+      const uint8_t* cb = sm + ((n & 1) ? S::OFF_R1 : S::OFF_R0);
+      const uint32_t m_a = smem_u32(sm + ((n & 1) ? S::OFF_R0 : S::OFF_R1));
       float rsum = 0.f;
 #pragma unroll 1
       for (int q = 0; q < 2; ++q) {
@@ -391,8 +407,8 @@ ssd_chunk_bwd_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_const
         const uint32_t off = half * HALF + t * 128 + q * 64;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          st_shared_v4(smem_u32(sm + S::OFF_M) + ((off + i * 16) ^ sw), make_uint4(m[4 * i], m[4 * i + 1], m[4 * i + 2], m[4 * i + 3]));
-          st_shared_v4(smem_u32(sm + S::OFF_DG) + ((off + i * 16) ^ sw), make_uint4(dg[4 * i], dg[4 * i + 1], dg[4 * i + 2], dg[4 * i + 3]));
+          st_shared_v4(m_a + ((off + i * 16) ^ sw), make_uint4(m[4 * i], m[4 * i + 1], m[4 * i + 2], m[4 * i + 3]));
+          st_shared_v4(m_a + 2 * HALF + ((off + i * 16) ^ sw), make_uint4(dg[4 * i], dg[4 * i + 1], dg[4 * i + 2], dg[4 * i + 3]));
         }
       }
       s_row[half * CQ + t] = rsum;
@@ -408,12 +424,13 @@ ssd_chunk_bwd_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_const
         p.col_mm[gi] = cg * s_scale[t];
       }
       const float dqk = s_dqk[t], e = __expf(ct);
-      ok = ok && warp_wait(&cb_full, n & 1) && warp_wait(&fin_full, n & 1);
+      ok = ok && warp_wait(&fin_full, n & 1);
       tc_fence_after();
       // dC~ (row t) and dB~ (row t as a key); this thread's half of the state columns
       float dce = 0.f;
-      float* dc_out = p.dC + gi * CN + half * 64;
-      float* db_out = p.dB + gi * CN + half * 64;
+      const long long g4 = gi - (lane & 3);             // first row of this lane's group of four: stores cover 64 bytes of eight rows
+      float* dc_out = p.dC + g4 * CN + half * 64 + (lane & 3) * 4;
+      float* db_out = p.dB + g4 * CN + half * 64 + (lane & 3) * 4;
 #pragma unroll 1
       for (int q = 0; q < 4; ++q) {
         uint32_t a[16], ce[16], d2[16];
@@ -422,27 +439,36 @@ ssd_chunk_bwd_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_const
         tmem_ld16(tm + t_lane + TM_B + half * 64 + q * 16, d2);
         tmem_ld_wait();
         const uint32_t off = half * HALF + t * 128 + q * 32;
+        uint4 oc[4], ob[4];
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-          const uint4 cp = *reinterpret_cast<const uint4*>(sm + S::OFF_C + ((off + i * 16) ^ sw));
-          const uint4 bp = *reinterpret_cast<const uint4*>(sm + S::OFF_B + ((off + i * 16) ^ sw));
+          const uint4 cp = *reinterpret_cast<const uint4*>(cb + ((off + i * 16) ^ sw));
+          const uint4 bp = *reinterpret_cast<const uint4*>(cb + 2 * HALF + ((off + i * 16) ^ sw));
           const uint32_t cw[4] = {cp.x, cp.y, cp.z, cp.w}, bw[4] = {bp.x, bp.y, bp.z, bp.w};
-          float oc[8], ob[8];
+          float fc[8], fb[8];
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             const float2 cv = unpack_bf16x2(cw[j]), bv = unpack_bf16x2(bw[j]);
             const int k = i * 8 + 2 * j;
             const float c0 = __uint_as_float(ce[k]), c1 = __uint_as_float(ce[k + 1]);
             dce += c0 * cv.x + c1 * cv.y;
-            oc[2 * j] = __uint_as_float(a[k]) + c0 * e + dqk * bv.x;
-            oc[2 * j + 1] = __uint_as_float(a[k + 1]) + c1 * e + dqk * bv.y;
-            ob[2 * j] = __uint_as_float(d2[k]) + dqk * cv.x;
-            ob[2 * j + 1] = __uint_as_float(d2[k + 1]) + dqk * cv.y;
+            fc[2 * j] = __uint_as_float(a[k]) + c0 * e + dqk * bv.x;
+            fc[2 * j + 1] = __uint_as_float(a[k + 1]) + c1 * e + dqk * bv.y;
+            fb[2 * j] = __uint_as_float(d2[k]) + dqk * cv.x;
+            fb[2 * j + 1] = __uint_as_float(d2[k + 1]) + dqk * cv.y;
           }
-          float4* o = reinterpret_cast<float4*>(dc_out + q * 16 + i * 8);
-          o[0] = make_float4(oc[0], oc[1], oc[2], oc[3]); o[1] = make_float4(oc[4], oc[5], oc[6], oc[7]);
-          o = reinterpret_cast<float4*>(db_out + q * 16 + i * 8);
-          o[0] = make_float4(ob[0], ob[1], ob[2], ob[3]); o[1] = make_float4(ob[4], ob[5], ob[6], ob[7]);
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            oc[2 * i + j] = make_uint4(__float_as_uint(fc[4 * j]), __float_as_uint(fc[4 * j + 1]), __float_as_uint(fc[4 * j + 2]), __float_as_uint(fc[4 * j + 3]));
+            ob[2 * i + j] = make_uint4(__float_as_uint(fb[4 * j]), __float_as_uint(fb[4 * j + 1]), __float_as_uint(fb[4 * j + 2]), __float_as_uint(fb[4 * j + 3]));
+          }
+        }
+        exchange4(oc, lane);
+        exchange4(ob, lane);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          *reinterpret_cast<uint4*>(dc_out + k * CN + q * 16) = oc[k];
+          *reinterpret_cast<uint4*>(db_out + k * CN + q * 16) = ob[k];
         }
       }
       // dx and dw: this thread's 32 of the head's 64 columns
@@ -456,13 +482,15 @@ ssd_chunk_bwd_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_const
         tmem_ld_wait();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&cb_free);        // C~, B~ and the accumulators may be replaced
-        const uint4* xp = reinterpret_cast<const uint4*>(p.X + gi * CP + half * 32);
-        uint4* o = reinterpret_cast<uint4*>(p.dx + row * p.lddx + h * CP + half * 32);
+        if (lane == 0) mbar_arrive(&acc_free);        // C~, B~ and the accumulators may be replaced
+        const uint4* xp = reinterpret_cast<const uint4*>(p.X + g4 * CP + half * 32) + (lane & 3);
+        uint4 xv[4], o[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) xv[k] = xp[k * (CP / 8)];
+        exchange4(xv, lane);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const uint4 xv = xp[i];
-          const uint32_t xs[4] = {xv.x, xv.y, xv.z, xv.w};
+          const uint32_t xs[4] = {xv[i].x, xv[i].y, xv[i].z, xv[i].w};
           uint32_t r[4];
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
@@ -473,6 +501,10 @@ ssd_chunk_bwd_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_const
           }
           o[i] = make_uint4(r[0], r[1], r[2], r[3]);
         }
+        exchange4(o, lane);
+        __nv_bfloat16* dxo = p.dx + (row - (lane & 3)) * p.lddx + h * CP + half * 32 + (lane & 3) * 8;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) *reinterpret_cast<uint4*>(dxo + k * p.lddx) = o[k];
       }
       // both halves of a token meet: the half 1 threads leave their sums in shared memory
       if (half == 1) { s_fin[t] = dce; s_fin[CQ + t] = dwv; }
