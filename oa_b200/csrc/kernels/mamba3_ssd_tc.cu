@@ -10,7 +10,9 @@
 //                   and column sums that carry d cum, d scale, d gamma, d w.  dC~ and dB~ leave once, in fp32.
 // What bounds them: the bytes of the operands and, backward, the serial chain of a chunk (scores, mask, products, stores) on one CTA
 // per SM.  2 x 4096 tokens x 48 heads: forward 77 -> 72 us, backward 337 -> 280 us since a row's results leave as 64 bytes at a time (16 bytes
-// of a row to a lane touch 32 lines a store, and a chunk has 8,000 of them) and the next C~ and B~ arrive under the epilogue; the batched
+// of a row to a lane touch 32 lines a store, and a chunk has 8,000 of them) and the next C~ and B~ arrive under the epilogue, 187 us
+// with the mask in packed arithmetic, its blocks below the diagonal without a choice per element (the scheduler of the last 32 tokens, which
+// meets every block of columns, took 7,800 of a chunk's 24,600 clocks for it), and a token's scalars and X requested ahead; the batched
 // products and elementwise kernels they replace took 0.42 and 1.0 ms.
 #include "common.cuh"
 #include "api.h"
@@ -255,8 +257,8 @@ ssd_chunk_bwd_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_const
   __shared__ uint64_t cb_full, ops_full, s_full, m_full, fin_full, acc_free, ops_free;
   __shared__ uint32_t tmem_slot;
   uint8_t* sm = raw + ((1024u - (smem_u32(raw) & 1023u)) & 1023u);
-  float* s_cum = reinterpret_cast<float*>(sm + S::OFF_F);
-  float* s_scale = s_cum + CQ;
+  float* s_ncum = reinterpret_cast<float*>(sm + S::OFF_F);
+  float* s_scale = s_ncum + CQ;
   float* s_dqk = s_scale + CQ;
   float* s_col = s_dqk + CQ;                        // [4 row quadrants][128]
   float* s_row = s_col + 4 * CQ;                    // [2 column halves][128]
@@ -352,12 +354,21 @@ ssd_chunk_bwd_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_const
     const uint32_t sw = (uint32_t)(t & 7) << 4;      // 128-byte swizzle of the thread's row
     uint32_t n = 0;
     bool ok = true;
+    // the scalars of a token, requested a chunk ahead
+    float n_cum = 0.f, n_gam = 0.f, n_qk = 0.f, n_scale = 0.f, n_w = 0.f, n_d = 0.f;
+    auto request = [&](int g) {
+      if (g >= p.G) return;
+      const long long gi = (long long)g * CQ + t;
+      n_cum = p.cum[gi]; n_gam = p.gamma[gi]; n_qk = p.qk[gi]; n_scale = p.scale[gi]; n_w = p.w[gi];
+      n_d = p.D ? p.D[(g / p.nC) % p.H] : 0.f;
+    };
+    request(blockIdx.x);
     for (int g = blockIdx.x; g < p.G; g += gridDim.x, ++n) {
       const long long gi = (long long)g * CQ + t;
       const int c = g % p.nC, bh = g / p.nC, h = bh % p.H, b = bh / p.H;
-      const float ct = p.cum[gi], gam = p.gamma[gi];
-      const float dval = (p.D ? p.D[h] : 0.f) + gam * p.qk[gi];
-      if (half == 0) { s_cum[t] = ct; s_scale[t] = p.scale[gi]; }
+      const float ct = n_cum, gam = n_gam, wv = n_w;
+      const float dval = n_d + gam * n_qk;
+      if (half == 0) { s_ncum[t] = -ct; s_scale[t] = n_scale; }
       asm volatile("bar.sync 1, 256;" ::: "memory");   // also: the previous chunk's sums have been read
       // a wait that runs out is not left early: the worker warps meet at barriers, so they all finish the loop (without waiting again)
       // C~ and B~ are waited for here: the barrier of the next chunk's may complete once this chunk's products are done
@@ -379,28 +390,68 @@ ssd_chunk_bwd_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_const
           tmem_ld32(tm + t_lane + TM_A + qc * 32, gv);
           tmem_ld32(tm + t_lane + TM_B + qc * 32, dv);
           tmem_ld_wait();
-          const float4 *cs4 = reinterpret_cast<const float4*>(s_cum + qc * 32), *sc4 = reinterpret_cast<const float4*>(s_scale + qc * 32);
-          const int lim = qc == quad ? lane : 32;
+          const ulonglong2 *nc2 = reinterpret_cast<const ulonglong2*>(s_ncum + qc * 32), *sc2 = reinterpret_cast<const ulonglong2*>(s_scale + qc * 32);
+          const unsigned long long ct2 = f2_of(__float_as_uint(ct), __float_as_uint(ct)), l2e = f2_of(0x3fb8aa3bu, 0x3fb8aa3bu);   // log2 e
           float ge[32];
+          // two columns: decay e, then e scale, G and dM times it, G dM e
+          auto pair = [&](int k, unsigned long long nc, unsigned long long sc, unsigned long long& ge2, uint32_t* mv, uint32_t* g2) {
+            uint32_t x0, x1;
+            f2_to(f2_mul(f2_add(ct2, nc), l2e), x0, x1);
+            const unsigned long long e = f2_of(__float_as_uint(fast_exp2(__uint_as_float(x0))), __float_as_uint(fast_exp2(__uint_as_float(x1))));
+            const unsigned long long es = f2_mul(e, sc), gg = f2_of(gv[k], gv[k + 1]), dm = f2_of(dv[k], dv[k + 1]);
+            f2_to(f2_mul(gg, es), mv[0], mv[1]);
+            f2_to(f2_mul(dm, es), g2[0], g2[1]);
+            ge2 = f2_mul(f2_mul(dm, gg), e);
+          };
+          if (qc < quad) {                            // every column is an earlier token
+            unsigned long long rs = 0;
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const float4 cs = cs4[i], sc = sc4[i];
-            const float csv[4] = {cs.x, cs.y, cs.z, cs.w}, scv[4] = {sc.x, sc.y, sc.z, sc.w};
-            float mv[4], gvv[4];
+            for (int i = 0; i < 8; ++i) {
+              const ulonglong2 nc = nc2[i], sc = sc2[i];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const int k = 4 * i + j;
-              const float e = k < lim ? __expf(ct - csv[j]) : 0.f;
-              const float gg = __uint_as_float(gv[k]), dm = __uint_as_float(dv[k]);
-              const float es = e * scv[j];
-              mv[j] = k < lim ? gg * es : (k == lim ? dval : 0.f);    // chosen, not multiplied by 0: a later token may hold an infinity
-              gvv[j] = k < lim ? dm * es : 0.f;
-              ge[k] = k < lim ? dm * gg * e : 0.f;
-              rsum += ge[k] * scv[j];
-              if (k == lim) { p.diag[gi] = dm; s_dqk[t] = dm * gam; }
+              for (int j = 0; j < 2; ++j) {
+                const int k = 4 * i + 2 * j;
+                uint32_t mv[2], g2[2], u0, u1;
+                unsigned long long ge2;
+                pair(k, j ? nc.y : nc.x, j ? sc.y : sc.x, ge2, mv, g2);
+                m[k >> 1] = pack_bf16x2(__uint_as_float(mv[0]), __uint_as_float(mv[1]));
+                dg[k >> 1] = pack_bf16x2(__uint_as_float(g2[0]), __uint_as_float(g2[1]));
+                rs = f2_fma(ge2, j ? sc.y : sc.x, rs);
+                f2_to(ge2, u0, u1);
+                ge[k] = __uint_as_float(u0); ge[k + 1] = __uint_as_float(u1);
+              }
             }
-            m[2 * i] = pack_bf16x2(mv[0], mv[1]); m[2 * i + 1] = pack_bf16x2(mv[2], mv[3]);
-            dg[2 * i] = pack_bf16x2(gvv[0], gvv[1]); dg[2 * i + 1] = pack_bf16x2(gvv[2], gvv[3]);
+            uint32_t r0, r1;
+            f2_to(rs, r0, r1);
+            rsum += __uint_as_float(r0) + __uint_as_float(r1);
+          } else {                                    // the block on the diagonal: columns below `lane`, itself, and none
+            float dmd = 0.f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const ulonglong2 nc = nc2[i], sc = sc2[i];
+              const float4 scf = reinterpret_cast<const float4*>(sc2)[i];
+              const float scv[4] = {scf.x, scf.y, scf.z, scf.w};
+#pragma unroll
+              for (int j = 0; j < 2; ++j) {
+                const int k = 4 * i + 2 * j;
+                uint32_t mv[2], g2[2], u[2];
+                unsigned long long ge2;
+                pair(k, j ? nc.y : nc.x, j ? sc.y : sc.x, ge2, mv, g2);
+                f2_to(ge2, u[0], u[1]);
+#pragma unroll
+                for (int z = 0; z < 2; ++z) {         // chosen, not multiplied by 0: a later token may hold an infinity
+                  mv[z] = k + z < lane ? mv[z] : (k + z == lane ? __float_as_uint(dval) : 0u);
+                  g2[z] = k + z < lane ? g2[z] : 0u;
+                  ge[k + z] = k + z < lane ? __uint_as_float(u[z]) : 0.f;
+                  rsum += ge[k + z] * scv[2 * j + z];
+                  dmd = k + z == lane ? __uint_as_float(dv[k + z]) : dmd;
+                }
+                m[k >> 1] = pack_bf16x2(__uint_as_float(mv[0]), __uint_as_float(mv[1]));
+                dg[k >> 1] = pack_bf16x2(__uint_as_float(g2[0]), __uint_as_float(g2[1]));
+              }
+            }
+            p.diag[gi] = dmd;
+            s_dqk[t] = dmd * gam;
           }
           s_col[quad * CQ + qc * 32 + lane] = lane_transpose_sum(ge, lane);
         }
@@ -424,11 +475,16 @@ ssd_chunk_bwd_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_const
         p.col_mm[gi] = cg * s_scale[t];
       }
       const float dqk = s_dqk[t], e = __expf(ct);
+      const long long g4 = gi - (lane & 3);             // first row of this lane's group of four: accesses cover 64 bytes of eight rows
+      const uint4* xp = reinterpret_cast<const uint4*>(p.X + g4 * CP + half * 32) + (lane & 3);
+      uint4 xv[4], o[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) xv[k] = xp[k * (CP / 8)];
+      request(g + gridDim.x);
       ok = ok && warp_wait(&fin_full, n & 1);
       tc_fence_after();
       // dC~ (row t) and dB~ (row t as a key); this thread's half of the state columns
       float dce = 0.f;
-      const long long g4 = gi - (lane & 3);             // first row of this lane's group of four: stores cover 64 bytes of eight rows
       float* dc_out = p.dC + g4 * CN + half * 64 + (lane & 3) * 4;
       float* db_out = p.dB + g4 * CN + half * 64 + (lane & 3) * 4;
 #pragma unroll 1
@@ -473,7 +529,6 @@ ssd_chunk_bwd_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_const
       }
       // dx and dw: this thread's 32 of the head's 64 columns
       float dwv = 0.f;
-      const float wv = p.w[gi];
       const long long row = (long long)b * p.L + (long long)c * CQ + t;
       {
         uint32_t u[32], v[32];
@@ -483,10 +538,6 @@ ssd_chunk_bwd_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_const
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&acc_free);        // C~, B~ and the accumulators may be replaced
-        const uint4* xp = reinterpret_cast<const uint4*>(p.X + g4 * CP + half * 32) + (lane & 3);
-        uint4 xv[4], o[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) xv[k] = xp[k * (CP / 8)];
         exchange4(xv, lane);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
