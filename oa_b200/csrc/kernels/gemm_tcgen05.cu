@@ -193,6 +193,39 @@ __device__ __forceinline__ void tma_store_piece(TmaStoreCtx* ts, const CUtensorM
   tma_store_packed(ts, m, w, col0);
 }
 
+// 32 fp32 columns of a warp's 32 rows, one row to a lane, stored (or added to what is there) as 64 bytes of eight rows at a time: 16 bytes of
+// a row to a lane make a store touch 32 lines.  `o`: this lane's row at the first column; `cols`: how many of the columns exist (a
+// multiple of 4); the whole warp calls it, rows from M on are left out.  Weight gradients (us, before -> with it): 3072 x 1024 of 16384
+// rows 86.5 -> 84.2, 1024 x 1024 of 16384 40.0 -> 38.0, fp32 accumulated 41.2 -> 38.0, 3000 x 1000 of 4096 accumulated 55.5 -> 44.7.  The single-CTA
+// kernel's batched products of 64 x 128 x 128 gain nothing (65.5 -> 68.3) and keep the direct stores.
+__device__ __forceinline__ void store_f32_rows(float* o, size_t ld, int row, int M, int cols, const float* v, bool add) {
+  const int lane = threadIdx.x & 31, in4 = lane & 3, r0 = row - in4;
+  o += in4 * 4;
+  o -= in4 * ld;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    uint4 x[4];
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      const float* f = v + h * 16 + g * 4;
+      x[g] = make_uint4(__float_as_uint(f[0]), __float_as_uint(f[1]), __float_as_uint(f[2]), __float_as_uint(f[3]));
+    }
+    exchange4(x, lane);
+    if (h * 16 + in4 * 4 >= cols) continue;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (r0 + k >= M) continue;
+      float4* d = reinterpret_cast<float4*>(o + k * ld + h * 16);
+      float4 y = make_float4(__uint_as_float(x[k].x), __uint_as_float(x[k].y), __uint_as_float(x[k].z), __uint_as_float(x[k].w));
+      if (add) {
+        const float4 c = *d;
+        y.x += c.x; y.y += c.y; y.z += c.z; y.w += c.w;
+      }
+      *d = y;
+    }
+  }
+}
+
 template <int BN>
 __device__ __forceinline__ void epilogue_chunk(const GemmParams& p, const uint32_t* r, int row, int col0, int split, int bi,
                                                const uint4* pre = nullptr, TmaStoreCtx* ts = nullptr) {
@@ -1008,19 +1041,11 @@ gemm_pair_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
             if (lane == 0) mbar_arrive_cluster(smem_u32(&tempty[acc]) & kPeerBitMask);
           }
           const int col0 = col_base + c * 32;
-          if (row < p.M) {
+          if (row - lane < p.M && col0 < p.N) {
+            float v[32];
 #pragma unroll
-            for (int g = 0; g < 8; ++g) {
-              if (col0 + g * 4 < p.N) {
-                float4 x = make_float4(__uint_as_float(r[g * 4]) * p.alpha, __uint_as_float(r[g * 4 + 1]) * p.alpha,
-                                       __uint_as_float(r[g * 4 + 2]) * p.alpha, __uint_as_float(r[g * 4 + 3]) * p.alpha);
-                if (add) {
-                  const float4 o = *reinterpret_cast<const float4*>(wrow + col0 + g * 4);
-                  x.x += o.x; x.y += o.y; x.z += o.z; x.w += o.w;
-                }
-                *reinterpret_cast<float4*>(wrow + col0 + g * 4) = x;
-              }
-            }
+            for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * p.alpha;
+            store_f32_rows(wrow + col0, LEAN == 5 ? p.N : p.ldc, row, p.M, p.N - col0, v, add);
           }
         }
         acc ^= 1;
