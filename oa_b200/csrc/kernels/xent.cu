@@ -113,10 +113,12 @@ xent_kernel(const T* __restrict__ logits, const int* __restrict__ targets, float
 // to shared memory through cp.async; every thread reads back only the 16-byte vectors that it copied itself, so no barrier
 // stands between the copy and its use, and the gradient can be written over the logits.  The row arrives in four groups of copies, and a
 // thread takes the exponentials of a group against a maximum of its own while the others are on their way.  What bounds it: one read and
-// one write of the logits; the CTAs of an SM (three at 64,000-byte rows) cover one another's reductions, and the exponentials, two to
-// a logit, take 230 us of 16384 x 32000 by themselves.  16384 x 32000 bf16: 475 us with two reads, 403 us with one and the maximum found
-// before the exponentials, 382 us (5.5 TB/s) like this; 8192 x 50264 331 -> 314, 32768 x 8192 205 -> 180, 4096 x 32000 110 -> 104, 500 x 32000
-// 22.8 -> 20.9, 4096 x 16384 fp32 83.4 -> 83.9.
+// one write of the logits, beside the exponentials (two to a logit, 230 us of 16384 x 32000 by themselves) and the instructions around
+// them, of which few are left: with a subtraction, a product and the other steps one element at a time they were 177 per 8 logits and
+// the issue slots 82 % taken.  The CTAs of an SM (three at 64,000-byte rows) cover one another's reductions.  16384 x 32000 bf16: 475 us with two
+// reads, 403 us with one and the maximum found before the exponentials, 382 us with the groups, 361 us (5.8 TB/s) with packed
+// multiply-adds throughout; 8192 x 50264 331 -> 314 -> 295, 32768 x 8192 205 -> 180 -> 172, 4096 x 32000 110 -> 104 -> 99, 4096 x 16384 fp32 83.4 -> 83.9 -> 84.5.
+// A quarter of the exponentials on the multiply-add pipe made it slower (382 -> 406).
 __device__ __forceinline__ void xent_cp16(void* smem_dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_dst)), "l"(src) : "memory");
 }
@@ -158,24 +160,80 @@ __device__ __forceinline__ void xent_vec_grad(const T* src, T* dst, float lse, f
   XIO<T>::store(dst, v);
 }
 
-// s += sum exp(v - m) of one vector, m raised to its largest element first
+// The vector's elements as fp32 pairs
+__device__ __forceinline__ void xent_pairs(const float* p, unsigned long long* v) {
+  const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(p);
+  v[0] = x.x; v[1] = x.y;
+}
+__device__ __forceinline__ void xent_pairs(const __nv_bfloat16* p, unsigned long long* v) {
+  const uint4 x = *reinterpret_cast<const uint4*>(p);
+  v[0] = f2_bf16x2(x.x); v[1] = f2_bf16x2(x.y); v[2] = f2_bf16x2(x.z); v[3] = f2_bf16x2(x.w);
+}
+__device__ __forceinline__ unsigned long long xent_splat(float v) { return f2_of(__float_as_uint(v), __float_as_uint(v)); }
+// 2^(v log2(e) + b), b = -m log2(e): one multiply-add where a subtraction and a product stood.  The product may overflow downwards (masks of
+// the type's lowest value give 2^-inf = 0) as long as b is far from it: rows whose maximum lies below XENT_FLOOR go the other way.
+__device__ __forceinline__ unsigned long long xent_exp2(unsigned long long v, unsigned long long b) {
+  uint32_t x0, x1;
+  f2_to(f2_fma(v, xent_splat(XENT_LOG2E), b), x0, x1);
+  return f2_of(__float_as_uint(fast_exp2(__uint_as_float(x0))), __float_as_uint(fast_exp2(__uint_as_float(x1))));
+}
+constexpr float XENT_FLOOR = -1e30f;
+
+// s += sum exp(v - m) of one vector, m (and b) raised to its largest element first
 template <typename T>
-__device__ __forceinline__ void xent_vec_add(const T* p, float& m, float& s) {
-  constexpr int V = XIO<T>::VEC;
+__device__ __forceinline__ void xent_vec_add(const T* p, float& m, unsigned long long& b, unsigned long long& s) {
+  constexpr int NP = XIO<T>::VEC / 2;
   const float mx = xent_vec_max<T>(p);
-  if (mx > m) { s *= __expf(m - mx); m = mx; }
-  float v[V];
-  XIO<T>::load(p, v);
-  const unsigned long long nm = f2_of(__float_as_uint(-m), __float_as_uint(-m)), l2 = f2_of(__float_as_uint(XENT_LOG2E), __float_as_uint(XENT_LOG2E));
-  float t = 0.f, u = 0.f;
-#pragma unroll
-  for (int j = 0; j < V; j += 2) {
-    uint32_t a, b;
-    f2_to(f2_mul(f2_add(f2_of(__float_as_uint(v[j]), __float_as_uint(v[j + 1])), nm), l2), a, b);
-    t += fast_exp2(__uint_as_float(a));
-    u += fast_exp2(__uint_as_float(b));
+  if (mx > m) {
+    s = f2_mul(s, xent_splat(fast_exp2((m - mx) * XENT_LOG2E)));
+    m = mx;
+    b = xent_splat(-mx * XENT_LOG2E);
   }
-  s += t + u;
+  unsigned long long v[NP];
+  xent_pairs(p, v);
+#pragma unroll
+  for (int j = 0; j < NP; ++j) s = f2_add(s, xent_exp2(v[j], b));
+}
+
+__device__ __forceinline__ void xent_store_pairs(float* p, const unsigned long long* v) { *reinterpret_cast<ulonglong2*>(p) = make_ulonglong2(v[0], v[1]); }
+__device__ __forceinline__ void xent_store_pairs(__nv_bfloat16* p, const unsigned long long* v) {
+  uint32_t w[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    uint32_t a, b;
+    f2_to(v[j], a, b);
+    w[j] = pack_bf16x2(__uint_as_float(a), __uint_as_float(b));
+  }
+  *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// Sum of exp(v - m) over a row in shared memory whose maximum lies below XENT_FLOOR (every logit masked by a finite value): m and the
+// sum, found one after the other.  The block calls it together.
+template <typename T, int THREADS>
+__device__ __noinline__ float2 xent_low_row(const T* srow, const T* p, int nvec, int vocab, float* red) {
+  constexpr int V = XIO<T>::VEC, W = THREADS / 32;
+  const int tid = threadIdx.x;
+  float m = -INFINITY, s = 0.f;
+  for (int i = tid; i < nvec; i += THREADS) m = fmaxf(m, xent_vec_max<T>(srow + i * V));
+  for (int c = nvec * V + tid; c < vocab; c += THREADS) m = fmaxf(m, XIO<T>::ld1(p + c));
+  m = warp_max(m);
+  __syncthreads();
+  if ((tid & 31) == 0) red[tid >> 5] = m;
+  __syncthreads();
+  for (int w = 0; w < W; ++w) m = fmaxf(m, red[w]);
+  for (int i = tid; i < nvec; i += THREADS) {
+    float v[V];
+    XIO<T>::load(srow + i * V, v);
+    for (int j = 0; j < V; ++j) s += __expf(v[j] - m);
+  }
+  for (int c = nvec * V + tid; c < vocab; c += THREADS) s += __expf(XIO<T>::ld1(p + c) - m);
+  s = warp_sum(s);
+  __syncthreads();
+  if ((tid & 31) == 0) red[tid >> 5] = s;
+  __syncthreads();
+  s = 0.f;
+  for (int w = 0; w < W; ++w) s += red[w];
+  return make_float2(m, s);
 }
 
 template <typename T, int THREADS>
@@ -193,6 +251,7 @@ xent_smem_kernel(const T* __restrict__ logits, const int* __restrict__ targets, 
 #pragma unroll
   for (int g = 0; g < 4; ++g) {
     const int end = min(nvec, (g + 1) * piece);
+#pragma unroll 2
     for (int i = g * piece + tid; i < end; i += THREADS) xent_cp16(srow + i * V, p + i * V);
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
@@ -200,12 +259,13 @@ xent_smem_kernel(const T* __restrict__ logits, const int* __restrict__ targets, 
   const bool ignored = (tgt == ignore_index);
   const bool oor = !ignored && (tgt < 0 || tgt >= vocab);
   const float tgt_logit = (tid == 0 && !ignored && !oor) ? XIO<T>::ld1(p + tgt) : 0.f;   // before any thread overwrites the row
-  float m = -FLT_MAX, s = 0.f;                           // finite: a masked logit (-inf) adds exp(-inf) = 0 whatever came before it
+  float m = XENT_FLOOR, s = 0.f;                         // finite: a masked logit (-inf) adds exp(-inf) = 0 whatever came before it
   for (int c = nvec * V + tid; c < vocab; c += THREADS) {
     const float v = XIO<T>::ld1(p + c);
     if (v > m) { s *= __expf(m - v); m = v; }
     s += __expf(v - m);
   }
+  unsigned long long b2 = xent_splat(-m * XENT_LOG2E), s2 = f2_of(__float_as_uint(s), 0u);
 #pragma unroll
   for (int g = 0; g < 4; ++g) {
     if (g == 0) asm volatile("cp.async.wait_group 3;" ::: "memory");
@@ -213,7 +273,13 @@ xent_smem_kernel(const T* __restrict__ logits, const int* __restrict__ targets, 
     else if (g == 2) asm volatile("cp.async.wait_group 1;" ::: "memory");
     else asm volatile("cp.async.wait_group 0;" ::: "memory");
     const int end = min(nvec, (g + 1) * piece);
-    for (int i = g * piece + tid; i < end; i += THREADS) xent_vec_add<T>(srow + i * V, m, s);
+#pragma unroll 2
+    for (int i = g * piece + tid; i < end; i += THREADS) xent_vec_add<T>(srow + i * V, m, b2, s2);
+  }
+  {
+    uint32_t a, b;
+    f2_to(s2, a, b);
+    s = __uint_as_float(a) + __uint_as_float(b);
   }
   const float mw = warp_max(m);
   s = warp_sum(s * __expf(m - mw));
@@ -225,12 +291,30 @@ xent_smem_kernel(const T* __restrict__ logits, const int* __restrict__ targets, 
   s = 0.f;
 #pragma unroll
   for (int w = 0; w < W; ++w) s += red_s[w] * __expf(red_m[w] - m);
+  const bool low = s == 0.f;                             // the same in every thread
+  if (low) {
+    const float2 ms = xent_low_row<T, THREADS>(srow, p, nvec, vocab, red_m);
+    m = ms.x; s = ms.y;
+  }
   const float lse = m + logf(s);
   if (tid == 0) row_loss[row] = ignored ? 0.f : (oor ? __int_as_float(0x7fc00000) : lse - tgt_logit);
   if (!dlogits) return;
   T* d = dlogits + row * ld;
   const float gs = ignored ? 0.f : grad_scale;
-  for (int i = tid; i < nvec; i += THREADS) xent_vec_grad<T>(srow + i * V, d + i * V, lse, gs, tgt - i * V);
+  const unsigned long long nl = xent_splat(-lse * XENT_LOG2E), gs2 = xent_splat(gs);
+  const int hit = tgt >= 0 ? tgt / V : -1;               // the vector that holds the target, or none
+#pragma unroll 2
+  for (int i = tid; i < nvec; i += THREADS) {
+    if (low || i == hit) {
+      xent_vec_grad<T>(srow + i * V, d + i * V, lse, gs, tgt - i * V);
+      continue;
+    }
+    unsigned long long v[V / 2];
+    xent_pairs(srow + i * V, v);
+#pragma unroll
+    for (int j = 0; j < V / 2; ++j) v[j] = f2_mul(xent_exp2(v[j], nl), gs2);
+    xent_store_pairs(d + i * V, v);
+  }
   for (int c = nvec * V + tid; c < vocab; c += THREADS) {
     const float g = (__expf(XIO<T>::ld1(p + c) - lse) - (c == tgt ? 1.f : 0.f)) * gs;
     if constexpr (sizeof(T) == 4) d[c] = g; else d[c] = __float2bfloat16_rn(g);
@@ -326,7 +410,15 @@ __global__ void mean_f32_kernel(const float* __restrict__ x, float* __restrict__
   __shared__ float red[32];
   pdl_wait();
   float s = 0.f;
-  for (long long i = threadIdx.x; i < n; i += blockDim.x) s += x[i];
+  long long i = threadIdx.x;
+  for (; i + 7LL * blockDim.x < n; i += 8LL * blockDim.x) {      // eight loads on their way together
+    float v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = x[i + (long long)u * blockDim.x];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) s += v[u];
+  }
+  for (; i < n; i += blockDim.x) s += x[i];
   s = warp_sum(s);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
   __syncthreads();

@@ -31,7 +31,10 @@ def test_row(vocab, kind, dtype):
     lse = torch.logsumexp(r, 1)
     ref = lse - r.gather(1, t.long()[:, None])[:, 0]
     grad = (torch.exp(r - lse[:, None]) - torch.nn.functional.one_hot(t.long(), vocab)) * 0.5
-    if kind == "masked":                                   # in fp32 log(vocab) is lost beside the lowest value
+    if kind == "masked":                                   # in fp32 log(vocab) is lost beside the lowest value: every entry counts as 1
+        other = torch.ones(vocab, dtype=torch.bool, device="cuda")
+        other[t[4].long()] = False
+        assert float(loss[4]) == 0.0 and bool((d[4][other] == 0.5).all()) and float(d[4, t[4].long()]) == 0.0
         ref, grad, loss, d = ref[:4], grad[:4], loss[:4], d[:4]
     # exponentials to 2^-22 and sums of as many terms in fp32; the gradient is rounded to its type
     assert float(((loss.double() - ref).abs() / ref.abs().clamp_min(1.0)).max()) <= 2e-6
