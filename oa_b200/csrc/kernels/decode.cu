@@ -371,28 +371,53 @@ rope_kv_append_kernel(__nv_bfloat16* x, long long row_stride, int heads, int hd,
 // position moved on by one.  As nodes of the graph these are a copy of the ids, a gather and an addition of one number, three links of
 // the step's chain; prompt of 100 and 32 steps of two 7B-class blocks with one row 8.15 -> 8.05 ms, 256 and 48 steps with 32 rows 19.92 -> 19.65.
 __global__ void __launch_bounds__(256)
-decode_begin_kernel(const uint4* __restrict__ table, const int* __restrict__ ids, uint4* __restrict__ x, int* pos, int n_ids, int vecs, int vocab) {
+decode_begin_kernel(const uint4* __restrict__ table, const int* __restrict__ ids, uint4* __restrict__ x, int* pos, int vecs, int vocab,
+                    const uint4* __restrict__ norm_w, uint4* __restrict__ x_w, float* __restrict__ squares) {
+  __shared__ float red[8];
   pdl_launch_dependents();
   pdl_wait();
   const uint32_t nan2 = pack_bf16x2(__int_as_float(0x7fc00000), __int_as_float(0x7fc00000));
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < (long long)n_ids * vecs; i += (long long)gridDim.x * blockDim.x) {
-    const int id = ids[i / vecs];
-    x[i] = id >= 0 && id < vocab ? table[(long long)id * vecs + i % vecs] : make_uint4(nan2, nan2, nan2, nan2);
+  const int row = blockIdx.x, id = ids[row];
+  float ss = 0.f;
+  for (int i = threadIdx.x; i < vecs; i += blockDim.x) {
+    const uint4 v = id >= 0 && id < vocab ? table[(long long)id * vecs + i] : make_uint4(nan2, nan2, nan2, nan2);
+    x[(long long)row * vecs + i] = v;
+    if (!norm_w) continue;
+    const uint4 w = norm_w[i];
+    const uint32_t vs[4] = {v.x, v.y, v.z, v.w}, ws[4] = {w.x, w.y, w.z, w.w};
+    uint32_t o[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float2 a = unpack_bf16x2(vs[k]), b = unpack_bf16x2(ws[k]);
+      ss += a.x * a.x + a.y * a.y;
+      o[k] = pack_bf16x2(a.x * b.x, a.y * b.y);
+    }
+    x_w[(long long)row * vecs + i] = make_uint4(o[0], o[1], o[2], o[3]);
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) *pos += 1;
+  if (row == 0 && threadIdx.x == 0) *pos += 1;
+  if (!norm_w) return;
+  ss = warp_sum(ss);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int k = 1; k < 8; ++k) ss += red[k];
+    squares[row] = ss;
+  }
 }
 
 }  // namespace oa
 
 using namespace oa;
 
-// x [n_ids, dim] = table[ids] (bf16; an id outside [0, vocab) gives a row of NaN), *pos += 1.
-extern "C" int oa_decode_begin(const void* table, const int* ids, void* x, int* pos, int n_ids, int dim, int vocab, void* stream) {
-  if (dim % 8 || ((reinterpret_cast<uintptr_t>(table) | reinterpret_cast<uintptr_t>(x)) & 15)) return OA_ERR_ALIGN;
-  if (n_ids <= 0 || dim <= 0) return OA_ERR_ARG;
-  const long long blocks = ((long long)n_ids * (dim / 8) + 255) / 256;
-  launch_short(decode_begin_kernel, dim3((unsigned)(blocks < 148 * 8 ? blocks : 148 * 8)), dim3(256), 0, (cudaStream_t)stream, (const uint4*)table, ids, (uint4*)x,
-               pos, n_ids, dim / 8, vocab);
+// x [n_ids, dim] = table[ids] (bf16; an id outside [0, vocab) gives a row of NaN), *pos += 1.  With norm_w [dim] also x_w = x * norm_w and
+// squares [n_ids], the sums of the rows' squares.
+extern "C" int oa_decode_begin(const void* table, const int* ids, void* x, int* pos, int n_ids, int dim, int vocab, const void* norm_w, void* x_w,
+                               float* squares, void* stream) {
+  if (dim % 8 || ((reinterpret_cast<uintptr_t>(table) | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(norm_w) | reinterpret_cast<uintptr_t>(x_w)) & 15))
+    return OA_ERR_ALIGN;
+  if (n_ids <= 0 || dim <= 0 || (norm_w && (!x_w || !squares))) return OA_ERR_ARG;
+  launch_short(decode_begin_kernel, dim3((unsigned)n_ids), dim3(256), 0, (cudaStream_t)stream, (const uint4*)table, ids, (uint4*)x, pos, dim / 8, vocab,
+               (const uint4*)norm_w, (uint4*)x_w, squares);
   return cudaGetLastError() == cudaSuccess ? OA_OK : OA_ERR_LAUNCH;
 }
 

@@ -1113,11 +1113,40 @@ def kv_append(k_src: torch.Tensor, v_src: torch.Tensor, k_cache: torch.Tensor, v
                                      heads, hd, pos0, max_seq, N.ptr(pos_dev), N.stream()), "oa_kv_append")
 
 
-def decode_begin(table: torch.Tensor, ids: torch.Tensor, x: torch.Tensor, pos: torch.Tensor) -> None:
-    """x [n, dim] = table[ids] and pos += 1 in one launch (bf16; ids int32 on the same device)."""
+def decode_begin(table: torch.Tensor, ids: torch.Tensor, x: torch.Tensor, pos: torch.Tensor, norm_w: Optional[torch.Tensor] = None,
+                 x_w: Optional[torch.Tensor] = None, squares: Optional[torch.Tensor] = None) -> None:
+    """x [n, dim] = table[ids] and pos += 1 in one launch (bf16; ids int32 on the same device).  With norm_w [dim] also x_w = x * norm_w and
+    squares [n] fp32, the sums of the rows' squares: what few_rows_step takes for an RMS norm in front of it."""
     assert table.is_contiguous() and x.is_contiguous() and ids.is_contiguous() and ids.dtype == torch.int32 and pos.dtype == torch.int32
     _launch(N.require().oa_decode_begin(table.data_ptr(), ids.data_ptr(), x.data_ptr(), pos.data_ptr(), ids.numel(), table.shape[1], table.shape[0],
-                                        N.stream()), "oa_decode_begin")
+                                        N.ptr(norm_w), N.ptr(x_w), N.ptr(squares), N.stream()), "oa_decode_begin")
+
+
+def few_rows_step(x: torch.Tensor, w: torch.Tensor, *, bias: Optional[torch.Tensor] = None, residual: Optional[torch.Tensor] = None,
+                  norm_w: Optional[torch.Tensor] = None, squares: Optional[torch.Tensor] = None, eps: float = 0.0, gated: bool = False):
+    """One product of a decoding step on the few-row kernel, bf16, with the RMS norms around it.
+
+    `squares` [n, M] fp32: x is rows times a norm's weight, and the result is scaled by that norm's factor, rsqrt(sum(squares) / K + eps).
+    `gated`: w holds gates and values, and the result is silu(gate) * value.  `norm_w`: returns (out, out * norm_w, squares of out)
+    for the norm behind.  None for shapes that the kernel leaves to others; nothing was done then."""
+    M, Kd = x.shape
+    Nn = w.shape[0]
+    cols = Nn // 2 if gated else Nn
+    assert x.dtype == w.dtype == torch.bfloat16 and x.stride(1) == 1 and w.stride(1) == 1 and w.shape[1] == Kd
+    assert residual is None or (residual.shape == (M, cols) and residual.stride(1) == 1)
+    lib = N.require()
+    out = torch.empty((M, cols), dtype=x.dtype, device=x.device)
+    out_w = torch.empty_like(out) if norm_w is not None else None
+    sq = torch.empty((lib.oa_few_rows_tiles(Nn), M), dtype=torch.float32, device=x.device) if norm_w is not None else None
+    at_rest = w.untyped_storage().data_ptr() in getattr(_weights_at_rest, "storages", ())
+    rc = lib.oa_few_rows_step(x.data_ptr(), w.data_ptr(), out.data_ptr(), M, Nn, Kd, x.stride(0), w.stride(0), out.stride(0), N.ptr(bias), N.ptr(residual),
+                              residual.stride(0) if residual is not None else 0, cols if gated else 0, N.ptr(norm_w), N.ptr(out_w), N.ptr(sq),
+                              N.ptr(squares), squares.shape[0] if squares is not None else 0, float(eps), int(at_rest),
+                              status_word(x.device).data_ptr(), N.stream())
+    if rc in (C["OA_ERR_UNSUPPORTED"], C["OA_ERR_ALIGN"]):
+        return None
+    _launch(rc, f"oa_few_rows_step M={M} N={Nn} K={Kd}", outputs=(out,))
+    return out if norm_w is None else (out, out_w, sq)
 
 
 def rope_kv_append(qkv: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, pos: int, theta: float,

@@ -22,6 +22,12 @@ def test_rows_and_position(n, dim, vocab):
     ref = K.embedding_fwd(table, ids)
     assert torch.equal(x.view(torch.int16), ref.view(torch.int16)) and bool(x[n // 2].isnan().all())
     assert pos.item() == 42
+    # with the norm behind it
+    w, xw, sq = torch.randn(dim, device="cuda").bfloat16(), torch.zeros_like(x), torch.zeros(1, n, device="cuda")
+    K.decode_begin(table, ids, x, pos, w, xw, sq)
+    ok = ids < vocab
+    assert torch.equal(xw[ok], (ref[ok].float() * w.float()).bfloat16()) and pos.item() == 43
+    assert torch.allclose(sq[0][ok].double(), (ref[ok].double() ** 2).sum(1), rtol=1e-5) and bool(sq[0][~ok].isnan().all())
 
 
 def test_ids_of_any_kind_continue_the_same_text():
