@@ -557,6 +557,11 @@ def _rows(t: torch.Tensor):
     return t if t.dim() == 2 else t.reshape(-1, t.shape[-1])
 
 
+def _folds(pending: Optional[torch.Tensor]) -> bool:
+    """Whether a kernel may read a pending gradient in 16-byte pieces while it writes the sum."""
+    return pending is not None and pending.is_contiguous() and pending.data_ptr() % 16 == 0
+
+
 def _as(t: torch.Tensor, shape) -> torch.Tensor:
     return t if t.shape == shape else t.reshape(shape)
 
@@ -888,16 +893,21 @@ def LayerNorm(x: OaMatrix, w: OaMatrix, b: Optional[OaMatrix], eps: float = 1e-5
     y, mean, rstd = K.layernorm_fwd(x2, tw, b.Tensor() if b is not None else None, eps)
     out = _w(_as(y, tx.shape))
 
-    def back(g):
+    def back(g, pending=None):
+        # `pending`: what x has already collected through the residual stream; the kernel adds it while it writes dx
         ws = w.GradSink() if (w.IsLeaf() and w.RequiresGrad()) else None
         bs = b.GradSink() if (b is not None and b.IsLeaf() and b.RequiresGrad()) else None
         if (ws is None) != (bs is None) or (ws and bs and ws[1] != bs[1]):
             ws = bs = None  # mixed states: fall back to returned gradients
-        dx, dw, db = K.layernorm_bwd(x2, tw, _rows(g), mean, rstd, dw_out=ws[0] if ws else None,
+        dres = _rows(pending) if _folds(pending) else None
+        dx, dw, db = K.layernorm_bwd(x2, tw, _rows(g), mean, rstd, dres=dres, dw_out=ws[0] if ws else None,
                                      db_out=bs[0] if bs else None, accumulate=bool(ws and ws[1]), want_bias=b is not None)
-        return (_as(dx, tx.shape), None if ws else dw, None if bs else db)
+        dx = _as(dx, tx.shape)
+        if pending is not None and dres is None:
+            dx = K.binary("add", pending, dx)
+        return (dx, None if ws else dw, None if bs else db)
 
-    return AG.attach("LayerNorm", out, [x, w, b], back)
+    return AG.attach("LayerNorm", out, [x, w, b], back, fold=0)
 
 
 # ======================================================================= gated activations

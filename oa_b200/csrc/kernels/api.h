@@ -128,7 +128,7 @@ int oa_rmsnorm_bwd(int dtype, const void* x, const void* w, const void* dy, cons
 int oa_layernorm_fwd(int dtype, const void* x, const void* w, const void* b, void* y, float* mean, float* rstd,
                      long long rows, int cols, float eps, void* stream);
 int oa_layernorm_bwd(int dtype, const void* x, const void* w, const void* dy, const float* mean, const float* rstd,
-                     void* dx, void* dw, void* db, int dw_dtype, long long rows, int cols, float* scratch,
+                     void* dx, void* dw, void* db, int dw_dtype, long long rows, int cols, const void* dres, float* scratch,
                      int accumulate_dw, void* stream);
 
 // ---- loss (xent.cu)

@@ -770,7 +770,7 @@ def layernorm_fwd(x, w, b, eps):
     return y, mean, rstd
 
 
-def layernorm_bwd(x, w, dy, mean, rstd, *, dw_out=None, db_out=None, accumulate=False, want_bias=True):
+def layernorm_bwd(x, w, dy, mean, rstd, *, dres=None, dw_out=None, db_out=None, accumulate=False, want_bias=True):
     rows, cols = x.shape
     dx = torch.empty_like(x)
     dw = dw_out if dw_out is not None else torch.empty(cols, dtype=w.dtype, device=x.device)
@@ -779,7 +779,8 @@ def layernorm_bwd(x, w, dy, mean, rstd, *, dw_out=None, db_out=None, accumulate=
         xf, df, wf = x.float(), dy.float(), w.float()
         xh = (xf - mean[:, None]) * rstd[:, None]
         g = df * wf
-        dx.copy_(rstd[:, None] * (g - g.mean(-1, keepdim=True) - xh * (g * xh).mean(-1, keepdim=True)))
+        v = rstd[:, None] * (g - g.mean(-1, keepdim=True) - xh * (g * xh).mean(-1, keepdim=True))
+        dx.copy_(v + dres.float() if dres is not None else v)
         s = (df * xh).sum(0)
         dw.copy_(s + dw.float() if accumulate else s)
         if db is not None:
@@ -788,8 +789,8 @@ def layernorm_bwd(x, w, dy, mean, rstd, *, dw_out=None, db_out=None, accumulate=
         return dx, dw, db
     sc = scratch(x.device, _norm_bwd_scratch_bytes(rows, cols), "norm")
     _launch(N.require().oa_layernorm_bwd(dt(x), x.data_ptr(), w.data_ptr(), dy.data_ptr(), mean.data_ptr(), rstd.data_ptr(),
-                                         dx.data_ptr(), dw.data_ptr(), N.ptr(db), dt(dw), rows, cols, sc.data_ptr(),
-                                         int(accumulate), N.stream()), "oa_layernorm_bwd", 3)
+                                         dx.data_ptr(), dw.data_ptr(), N.ptr(db), dt(dw), rows, cols, N.ptr(dres), sc.data_ptr(),
+                                         int(accumulate), N.stream()), "oa_layernorm_bwd", 2)
     return dx, dw, db
 
 
