@@ -13,8 +13,13 @@
 // work per score; KS = 4 makes four times as many, shorter CTAs (which under the causal mask also skip more of the other side), lets
 // the next tile arrive through cp.async under this one, and is taken while KS = 1 would leave SMs idle (af_split).
 // 16 x 4 heads of 32 dimensions and 128 positions are 64 CTAs with KS = 1, one warp per scheduler: 29 us forward
-// and 83 us both gradients.  With KS = 4: 14 us, and 38 for both gradients (16.9, and 53.3, with eight
-// dimensions per thread, whose dot products each took two shuffles).
+// and 83 us both gradients.  With KS = 4: 12.6 us, and 31 for both gradients (eight dimensions per thread, whose dot products each took
+// two shuffles, were 2.5 and 15 us slower).
+// What bounds it: eight to twelve warps per SM, whose reads of shared memory and dot products wait for one another.  So the two gradients
+// run side by side: the CTAs of dQ, which needs nothing of dK and dV, start as soon as those of dK and dV are all under way, fill the room
+// that these leave, and end after them.  A row's own dimensions come in 16-byte pieces where the operands allow it, and under the causal
+// mask the longest CTAs start first.  Both gradients one after the other / side by side, us: 16 x 128 of 4 x 32 causal 37.8 / 31.2, 2 x 1024
+// of 4 x 64 full 469 / 320, 8 x 256 of 4 x 128 causal 254 / 201, 16 x 512 of 4 x 32 causal 270 / 255, 3 x 77 of 5 x 40 21.7 / 13.4.
 // Forward and dQ rows are queries (keys / values stream through shared memory), dK / dV rows are keys (queries and output gradients
 // stream through shared memory together with their log-sum-exp and delta = rowsum(dO * O)).
 #include "common.cuh"
@@ -57,6 +62,18 @@ __device__ __forceinline__ void af_load_tile(float* sm, const float* __restrict_
 __device__ __forceinline__ void af_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void af_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// A thread's 32 dimensions of its own row, zeros beyond hd and for rows that are not there
+__device__ __forceinline__ void af_own(float* dst, const float* __restrict__ row, int left, bool ok, bool vec) {
+  if (!ok) left = 0;
+  if (vec) {
+#pragma unroll
+    for (int t = 0; t < AF_W; t += 4) *reinterpret_cast<float4*>(dst + t) = t < left ? *reinterpret_cast<const float4*>(row + t) : make_float4(0.f, 0.f, 0.f, 0.f);
+  } else {
+#pragma unroll
+    for (int t = 0; t < AF_W; ++t) dst[t] = t < left ? row[t] : 0.f;
+  }
+}
 
 // sum over the DS threads that share a row's dot products (neighbouring lanes)
 template <int DS>
@@ -149,15 +166,15 @@ attn_f32_fwd_kernel(const float* __restrict__ q, const float* __restrict__ k, co
   __shared__ __align__(16) float sK[Cfg::BUFS * Cfg::TILE], sV[Cfg::BUFS * Cfg::TILE];
   pdl_wait();
   const int h = blockIdx.y, b = blockIdx.z;
-  const int i0 = blockIdx.x * Cfg::ROWS;
+  const int i0 = (gridDim.x - 1 - blockIdx.x) * Cfg::ROWS;       // under the causal mask the longest first
   const int i = i0 + threadIdx.x / Cfg::TPR, seg = threadIdx.x % DS, ks = threadIdx.x % Cfg::TPR / DS;
   const long long row0 = (long long)b * seq;
   const bool row_ok = i < seq;
   float qr[AF_W], acc[AF_W];
+  af_own(qr, q + (row0 + i) * rs + h * hd + seg * AF_W, hd - seg * AF_W, row_ok, vec);
 #pragma unroll
   for (int t = 0; t < AF_W; ++t) {
-    const int d = seg * AF_W + t;
-    qr[t] = (row_ok && d < hd) ? q[(row0 + i) * rs + h * hd + d] * scale : 0.f;
+    qr[t] *= scale;
     acc[t] = 0.f;
   }
   float m = -INFINITY, l = 0.f;
@@ -212,7 +229,8 @@ attn_f32_fwd_kernel(const float* __restrict__ q, const float* __restrict__ k, co
   if (seg == 0 && ks == 0 && lse) lse[((long long)b * heads + h) * seq + i] = m + logf(l);
 }
 
-// dQ: rows are queries; K and V stream through shared memory.
+// dQ: rows are queries; K and V stream through shared memory.  Launched behind the kernel below, which allows this one's start only once
+// everything before both has ended; so there is nothing to wait for before the end, where whatever follows must find both kernels done.
 template <int DS, int KS>
 __global__ void __launch_bounds__(AF_THREADS)
 attn_f32_bwd_q_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
@@ -222,21 +240,21 @@ attn_f32_bwd_q_kernel(const float* __restrict__ q, const float* __restrict__ k, 
   using Cfg = AfCfg<DS, KS>;
   constexpr int NJ = AF_TILE / KS;
   __shared__ __align__(16) float sK[Cfg::BUFS * Cfg::TILE], sV[Cfg::BUFS * Cfg::TILE];
-  pdl_wait();
   const int h = blockIdx.y, b = blockIdx.z;
-  const int i0 = blockIdx.x * Cfg::ROWS;
+  const int i0 = (gridDim.x - 1 - blockIdx.x) * Cfg::ROWS;       // under the causal mask the longest first
   const int i = i0 + threadIdx.x / Cfg::TPR, seg = threadIdx.x % DS, ks = threadIdx.x % Cfg::TPR / DS;
   const long long row0 = (long long)b * seq;
   const bool row_ok = i < seq;
   float qr[AF_W], dor[AF_W], acc[AF_W];
   float delta = 0.f;
+  const int left = hd - seg * AF_W;
+  af_own(acc, o + (row0 + i) * os + h * hd + seg * AF_W, left, row_ok, vec);
+  af_own(dor, dout + (row0 + i) * os + h * hd + seg * AF_W, left, row_ok, vec);
+  af_own(qr, q + (row0 + i) * rs + h * hd + seg * AF_W, left, row_ok, vec);
 #pragma unroll
   for (int t = 0; t < AF_W; ++t) {
-    const int d = seg * AF_W + t;
-    const bool ok = row_ok && d < hd;
-    qr[t] = ok ? q[(row0 + i) * rs + h * hd + d] * scale : 0.f;
-    dor[t] = ok ? dout[(row0 + i) * os + h * hd + d] : 0.f;
-    if (ok) delta = fmaf(dor[t], o[(row0 + i) * os + h * hd + d], delta);
+    qr[t] *= scale;
+    if (t < left) delta = fmaf(dor[t], acc[t], delta);
     acc[t] = 0.f;
   }
   delta = af_reduce<DS>(delta);
@@ -256,6 +274,7 @@ attn_f32_bwd_q_kernel(const float* __restrict__ q, const float* __restrict__ k, 
     }
   });
   af_scatter_sum<DS, KS>(acc, ks);
+  pdl_wait();                                                    // this grid ends after the other gradients'
   if (!row_ok) return;
 #pragma unroll
   for (int t = 0; t < AF_W / KS; ++t) {
@@ -276,18 +295,18 @@ attn_f32_bwd_kv_kernel(const float* __restrict__ q, const float* __restrict__ k,
   __shared__ __align__(16) float sQ[Cfg::BUFS * Cfg::TILE], sDO[Cfg::BUFS * Cfg::TILE];
   __shared__ float sL[2][AF_TILE], sDelta[2][AF_TILE];
   pdl_wait();
+  pdl_launch_dependents();
   const int h = blockIdx.y, b = blockIdx.z;
   const int j0 = blockIdx.x * Cfg::ROWS;
   const int j = j0 + threadIdx.x / Cfg::TPR, seg = threadIdx.x % DS, ks = threadIdx.x % Cfg::TPR / DS;
   const long long row0 = (long long)b * seq;
   const bool row_ok = j < seq;
   float kr[AF_W], vr[AF_W], acck[AF_W], accv[AF_W];
+  af_own(kr, k + (row0 + j) * rs + h * hd + seg * AF_W, hd - seg * AF_W, row_ok, vec);
+  af_own(vr, v + (row0 + j) * rs + h * hd + seg * AF_W, hd - seg * AF_W, row_ok, vec);
 #pragma unroll
   for (int t = 0; t < AF_W; ++t) {
-    const int d = seg * AF_W + t;
-    const bool ok = row_ok && d < hd;
-    kr[t] = ok ? k[(row0 + j) * rs + h * hd + d] * scale : 0.f;
-    vr[t] = ok ? v[(row0 + j) * rs + h * hd + d] : 0.f;
+    kr[t] *= scale;
     acck[t] = 0.f; accv[t] = 0.f;
   }
   // delta and log-sum-exp of the 32 queries of a tile: 4 threads per query, shuffle-combined.  Tiles alternate between two slots, so
@@ -402,9 +421,9 @@ extern "C" int oa_attn_f32_bwd(const float* q, const float* k, const float* v, c
   dim3 grid((seq + rows - 1) / rows, heads, batch);
   const int vec = af_vec(head_dim, row_stride, o_row_stride, q, k, v, o, dout);
 #define AF_BWD(D, S)                                                                                                                        \
-  launch_short(attn_f32_bwd_q_kernel<D, S>, grid, dim3(AF_THREADS), 0, st, q, k, v, o, dout, lse, dq, heads, seq, head_dim, row_stride,       \
-               o_row_stride, d_row_stride, scale, causal, vec);                                                                             \
   launch_short(attn_f32_bwd_kv_kernel<D, S>, grid, dim3(AF_THREADS), 0, st, q, k, v, o, dout, lse, dk, dv, heads, seq, head_dim, row_stride,  \
+               o_row_stride, d_row_stride, scale, causal, vec);                                                                             \
+  launch_short(attn_f32_bwd_q_kernel<D, S>, grid, dim3(AF_THREADS), 0, st, q, k, v, o, dout, lse, dq, heads, seq, head_dim, row_stride,       \
                o_row_stride, d_row_stride, scale, causal, vec)
   if (split == -4) { AF_BWD(1, 4); }
   else if (split == -8) { AF_BWD(2, 4); }
