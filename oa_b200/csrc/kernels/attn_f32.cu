@@ -371,14 +371,18 @@ attn_f32_bwd_kv_kernel(const float* __restrict__ q, const float* __restrict__ k,
 using namespace oa;
 
 // DS, or -4 DS for KS = 4, which is taken up to `limit` CTAs of the KS = 1 form: one per SM, or somewhat more where the causal mask lets the
-// shorter CTAs skip work, and wherever a sequence would leave most rows of a wide CTA empty.  KS = 1 against 4 (4 heads), forward, full mask,
-// 48 x 128 of 32 dimensions (192 CTAs) 33.8 / 33.5 us, 28 x 128 of 64 (224) 38.4 / 40.7; causal 16 x 512 of 32 (256) 107 / 98, 36 x 128 of 64 (288)
-// 38.7 / 39.4.  Backward, full, 48 x 128 of 32 (192) 123 / 103, 28 x 128 of 64 (224) 119 / 131, 14 x 128 of 64 (112) 79 / 76, but 2 x 1024 of 64 (128)
-// 470 / 489; causal 36 x 128 of 64 (288) 117 / 114.  100 x 16 of 64 (400 CTAs) 13.3 / 8.2 and 50.9 / 28.2.
-static inline int af_split(int hd, int batch, int heads, int seq, int limit) {
+// shorter CTAs skip work, and wherever a sequence would leave most rows of a wide CTA empty; in the backward pass of a full mask (`pair`) not where
+// the KS = 1 forms of both kernels fill the chip together, up to 148 CTAs each at two to an SM, from where KS = 4 needs a second wave.  KS = 1
+// against 4 (4 heads, us), forward, full mask, 14 x 128 of 64 dimensions (112 CTAs) 32.2 / 22.4, 48 x 128 of 32 (192) 29.8 / 31.0, 28 x 128 of 64 (224)
+// 34.4 / 37.7; causal 16 x 512 of 32 (256) 104 / 93, 36 x 128 of 64 (288) 35.2 / 35.6.  Backward, full, 18 x 128 of 32 (72) 43.6 / 35.0, 10 x 128 of 64 (80)
+// 47.2 / 39.7, 20 x 128 of 32 (80) 47.4 / 50.9, 5 x 512 of 32 (80) 143 / 176, 14 x 128 of 64 (112) 50 / 58, 2 x 1024 of 64 (128) 319 / 400, 40 x 128 of 32
+// (160) 91.5 / 83.7, 48 x 128 of 32 (192) 92 / 94; causal 16 x 512 of 32 (256) 261 / 255, 64 x 128 of 32 (256) 108 / 86, 36 x 128 of 64 (288) 99 / 100.
+// 100 x 16 of 64 (400) 11.6 / 6.8 and 40 / 20.
+static inline int af_split(int hd, int batch, int heads, int seq, int limit, bool pair = false) {
   const int wide = hd <= 32 ? 1 : (hd <= 64 ? 2 : 4);
   const long long ctas = (long long)((seq + AF_THREADS / wide - 1) / (AF_THREADS / wide)) * heads * batch;
-  return hd <= 64 && (seq <= AF_TILE || ctas <= limit) ? -4 * wide : wide;
+  const bool together = pair && ctas > (wide == 1 ? 74 : 80) && ctas <= 148;
+  return hd <= 64 && (seq <= AF_TILE || (ctas <= limit && !together)) ? -4 * wide : wide;
 }
 
 // Whether every row of the streamed operands can be read in 16-byte pieces.
@@ -417,7 +421,7 @@ extern "C" int oa_attn_f32_bwd(const float* q, const float* k, const float* v, c
   if (batch <= 0 || heads <= 0 || seq <= 0) return OA_OK;
   if (heads > 65535 || batch > 65535) return OA_ERR_ARG;
   cudaStream_t st = (cudaStream_t)stream;
-  const int split = af_split(head_dim, batch, heads, seq, causal ? 300 : (seq > 128 ? 96 : 192)), rows = AF_THREADS / (split < 0 ? -split : split);
+  const int split = af_split(head_dim, batch, heads, seq, causal ? 300 : (seq > 128 ? 96 : 192), !causal), rows = AF_THREADS / (split < 0 ? -split : split);
   dim3 grid((seq + rows - 1) / rows, heads, batch);
   const int vec = af_vec(head_dim, row_stride, o_row_stride, q, k, v, o, dout);
 #define AF_BWD(D, S)                                                                                                                        \
