@@ -119,6 +119,9 @@ xent_kernel(const T* __restrict__ logits, const int* __restrict__ targets, float
 // reads, 403 us with one and the maximum found before the exponentials, 382 us with the groups, 361 us (5.8 TB/s) with packed
 // multiply-adds throughout; 8192 x 50264 331 -> 314 -> 295, 32768 x 8192 205 -> 180 -> 172, 4096 x 32000 110 -> 104 -> 99, 4096 x 16384 fp32 83.4 -> 83.9 -> 84.5.
 // A quarter of the exponentials on the multiply-add pipe made it slower (382 -> 406).
+// Errors against 64 bits, standard deviation 2, subtraction first and probabilities from the rounded log-sum-exp / now: fp32 gradients over
+// 4096 columns 3.3e-7 / 1.3e-7, over 32000 3.8e-7 / 1.7e-7; losses 4.6e-7 / 4.2e-7; the same time (357 / 354 us for 16384 x 32000 bf16) as with a
+// product of m and log2(e) rounded into every term, whose gradients were at 5.5e-7 and wrong far from zero.
 __device__ __forceinline__ void xent_cp16(void* smem_dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_dst)), "l"(src) : "memory");
 }
@@ -170,29 +173,49 @@ __device__ __forceinline__ void xent_pairs(const __nv_bfloat16* p, unsigned long
   v[0] = f2_bf16x2(x.x); v[1] = f2_bf16x2(x.y); v[2] = f2_bf16x2(x.z); v[3] = f2_bf16x2(x.w);
 }
 __device__ __forceinline__ unsigned long long xent_splat(float v) { return f2_of(__float_as_uint(v), __float_as_uint(v)); }
-// 2^(v log2(e) + b), b = -m log2(e): one multiply-add where a subtraction and a product stood.  The product may overflow downwards (masks of
-// the type's lowest value give 2^-inf = 0) as long as b is far from it: rows whose maximum lies below XENT_FLOOR go the other way.
+// 2^(v log2(e) + b): one multiply-add where a subtraction and a product stood.  b is the whole number beside -m log2(e): a row's terms pass
+// from one maximum to another, and from threads to the row, by powers of two, and nothing is lost on the way.  A probability is a term over
+// the sum of terms, whatever b is; the loss, which needs the sum as it counts from m, is given what lies between (xent_rest).
+// Rows whose maximum lies beyond XENT_WIDE either way are worked out apart (xent_wide_row), by subtraction: far out, the product is
+// rounded to more than a whole number.
 __device__ __forceinline__ unsigned long long xent_exp2(unsigned long long v, unsigned long long b) {
   uint32_t x0, x1;
   f2_to(f2_fma(v, xent_splat(XENT_LOG2E), b), x0, x1);
   return f2_of(__float_as_uint(fast_exp2(__uint_as_float(x0))), __float_as_uint(fast_exp2(__uint_as_float(x1))));
 }
-constexpr float XENT_FLOOR = -1e30f;
+constexpr float XENT_WIDE = 1048576.f;
+// By adding 1.5 * 2^23 and taking it off: whole numbers up to 2^22
+__device__ __forceinline__ float xent_base(float m) { return fmaf(-m, XENT_LOG2E, 12582912.f) - 12582912.f; }
+// 2^(-m log2(e) - b), b within 1/2 of the exponent's first part: the Taylor series of the exponential up to x^7 (x^8 / 8! is 5e-9)
+__device__ __forceinline__ float xent_rest(float m, float b) {
+  const float x = fmaf(-m, XENT_LOG2E, -b) * 0.693147181f;
+  float r = fmaf(x, 1.f / 5040.f, 1.f / 720.f);
+  r = fmaf(x, r, 1.f / 120.f);
+  r = fmaf(x, r, 1.f / 24.f);
+  r = fmaf(x, r, 1.f / 6.f);
+  r = fmaf(x, r, 0.5f);
+  r = fmaf(x, r, 1.f);
+  return fmaf(x, r, 1.f);
+}
+
+// The running maximum raised to mx: terms added so far count from the new b on
+__device__ __forceinline__ void xent_raise(float mx, float& m, float& b, unsigned long long& s) {
+  const float nb = xent_base(mx);
+  s = f2_mul(s, xent_splat(fast_exp2(nb - b)));
+  m = mx;
+  b = nb;
+}
 
 // s += sum exp(v - m) of one vector, m (and b) raised to its largest element first
 template <typename T>
-__device__ __forceinline__ void xent_vec_add(const T* p, float& m, unsigned long long& b, unsigned long long& s) {
+__device__ __forceinline__ void xent_vec_add(const T* p, float& m, float& b, unsigned long long& s) {
   constexpr int NP = XIO<T>::VEC / 2;
   const float mx = xent_vec_max<T>(p);
-  if (mx > m) {
-    s = f2_mul(s, xent_splat(fast_exp2((m - mx) * XENT_LOG2E)));
-    m = mx;
-    b = xent_splat(-mx * XENT_LOG2E);
-  }
+  if (mx > m) xent_raise(mx, m, b, s);
   unsigned long long v[NP];
   xent_pairs(p, v);
 #pragma unroll
-  for (int j = 0; j < NP; ++j) s = f2_add(s, xent_exp2(v[j], b));
+  for (int j = 0; j < NP; ++j) s = f2_add(s, xent_exp2(v[j], xent_splat(b)));
 }
 
 __device__ __forceinline__ void xent_store_pairs(float* p, const unsigned long long* v) { *reinterpret_cast<ulonglong2*>(p) = make_ulonglong2(v[0], v[1]); }
@@ -207,10 +230,10 @@ __device__ __forceinline__ void xent_store_pairs(__nv_bfloat16* p, const unsigne
   *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-// Sum of exp(v - m) over a row in shared memory whose maximum lies below XENT_FLOOR (every logit masked by a finite value): m and the
-// sum, found one after the other.  The block calls it together.
+// Sum of exp(v - m) over a row in shared memory whose maximum lies beyond XENT_WIDE (every logit masked by a finite value, or one far above
+// what a model gives): m and the sum, found one after the other.  The block calls it together.
 template <typename T, int THREADS>
-__device__ __noinline__ float2 xent_low_row(const T* srow, const T* p, int nvec, int vocab, float* red) {
+__device__ __noinline__ float2 xent_wide_row(const T* srow, const T* p, int nvec, int vocab, float* red) {
   constexpr int V = XIO<T>::VEC, W = THREADS / 32;
   const int tid = threadIdx.x;
   float m = -INFINITY, s = 0.f;
@@ -259,13 +282,14 @@ xent_smem_kernel(const T* __restrict__ logits, const int* __restrict__ targets, 
   const bool ignored = (tgt == ignore_index);
   const bool oor = !ignored && (tgt < 0 || tgt >= vocab);
   const float tgt_logit = (tid == 0 && !ignored && !oor) ? XIO<T>::ld1(p + tgt) : 0.f;   // before any thread overwrites the row
-  float m = XENT_FLOOR, s = 0.f;                         // finite: a masked logit (-inf) adds exp(-inf) = 0 whatever came before it
+  // finite: a masked logit (-inf, or any value below) adds 0 whatever came before it
+  float m = -XENT_WIDE, b = xent_base(m);
+  unsigned long long s2 = 0;
   for (int c = nvec * V + tid; c < vocab; c += THREADS) {
     const float v = XIO<T>::ld1(p + c);
-    if (v > m) { s *= __expf(m - v); m = v; }
-    s += __expf(v - m);
+    if (v > m) xent_raise(v, m, b, s2);
+    s2 = f2_add(s2, f2_of(__float_as_uint(fast_exp2(fmaf(v, XENT_LOG2E, b))), 0u));
   }
-  unsigned long long b2 = xent_splat(-m * XENT_LOG2E), s2 = f2_of(__float_as_uint(s), 0u);
 #pragma unroll
   for (int g = 0; g < 4; ++g) {
     if (g == 0) asm volatile("cp.async.wait_group 3;" ::: "memory");
@@ -274,49 +298,62 @@ xent_smem_kernel(const T* __restrict__ logits, const int* __restrict__ targets, 
     else asm volatile("cp.async.wait_group 0;" ::: "memory");
     const int end = min(nvec, (g + 1) * piece);
 #pragma unroll 2
-    for (int i = g * piece + tid; i < end; i += THREADS) xent_vec_add<T>(srow + i * V, m, b2, s2);
+    for (int i = g * piece + tid; i < end; i += THREADS) xent_vec_add<T>(srow + i * V, m, b, s2);
   }
-  {
-    uint32_t a, b;
-    f2_to(s2, a, b);
-    s = __uint_as_float(a) + __uint_as_float(b);
-  }
-  const float mw = warp_max(m);
-  s = warp_sum(s * __expf(m - mw));
+  uint32_t s_lo, s_hi;
+  f2_to(s2, s_lo, s_hi);
+  const float mw = warp_max(m), bw = xent_base(mw);
+  float s = warp_sum((__uint_as_float(s_lo) + __uint_as_float(s_hi)) * fast_exp2(bw - b));
   if ((tid & 31) == 0) { red_m[tid >> 5] = mw; red_s[tid >> 5] = s; }
   __syncthreads();
   m = red_m[0];
 #pragma unroll
   for (int w = 1; w < W; ++w) m = fmaxf(m, red_m[w]);
+  b = xent_base(m);
   s = 0.f;
 #pragma unroll
-  for (int w = 0; w < W; ++w) s += red_s[w] * __expf(red_m[w] - m);
-  const bool low = s == 0.f;                             // the same in every thread
-  if (low) {
-    const float2 ms = xent_low_row<T, THREADS>(srow, p, nvec, vocab, red_m);
-    m = ms.x; s = ms.y;
+  for (int w = 0; w < W; ++w) s += red_s[w] * fast_exp2(b - xent_base(red_m[w]));
+  const bool wide = !(fabsf(m) < XENT_WIDE);             // the same in every thread; whatever s is then
+  float lse = 0.f;
+  if (wide) {
+    const float2 ms = xent_wide_row<T, THREADS>(srow, p, nvec, vocab, red_m);
+    lse = ms.x + logf(ms.y);
   }
-  const float lse = m + logf(s);
-  if (tid == 0) row_loss[row] = ignored ? 0.f : (oor ? __int_as_float(0x7fc00000) : lse - tgt_logit);
+  if (tid == 0)
+    row_loss[row] = ignored ? 0.f : oor ? __int_as_float(0x7fc00000) : wide ? lse - tgt_logit : (m - tgt_logit) + logf(s * xent_rest(m, b));
   if (!dlogits) return;
   T* d = dlogits + row * ld;
   const float gs = ignored ? 0.f : grad_scale;
-  const unsigned long long nl = xent_splat(-lse * XENT_LOG2E), gs2 = xent_splat(gs);
+  // probabilities: terms counted from the sum's own power of two, 2^e <= s < 2^(e + 1), over s 2^-e
+  const int e = (__float_as_int(s) >> 23) - 127;
+  const float sn = s * __int_as_float((127 - e) << 23), inv = 1.f / sn;
+  b -= (float)e;
+  const unsigned long long b2 = xent_splat(b), gs2 = xent_splat(gs * inv);
   const int hit = tgt >= 0 ? tgt / V : -1;               // the vector that holds the target, or none
 #pragma unroll 2
   for (int i = tid; i < nvec; i += THREADS) {
-    if (low || i == hit) {
+    if (wide) {
       xent_vec_grad<T>(srow + i * V, d + i * V, lse, gs, tgt - i * V);
       continue;
     }
     unsigned long long v[V / 2];
     xent_pairs(srow + i * V, v);
 #pragma unroll
-    for (int j = 0; j < V / 2; ++j) v[j] = f2_mul(xent_exp2(v[j], nl), gs2);
+    for (int j = 0; j < V / 2; ++j) v[j] = xent_exp2(v[j], b2);
+    if (i == hit) {
+#pragma unroll
+      for (int j = 0; j < V / 2; ++j) {
+        const int k = tgt - i * V - 2 * j;
+        v[j] = f2_add(v[j], f2_of(__float_as_uint(k == 0 ? -sn : 0.f), __float_as_uint(k == 1 ? -sn : 0.f)));
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < V / 2; ++j) v[j] = f2_mul(v[j], gs2);
     xent_store_pairs(d + i * V, v);
   }
   for (int c = nvec * V + tid; c < vocab; c += THREADS) {
-    const float g = (__expf(XIO<T>::ld1(p + c) - lse) - (c == tgt ? 1.f : 0.f)) * gs;
+    const float v = XIO<T>::ld1(p + c), pr = wide ? __expf(v - lse) : fast_exp2(fmaf(v, XENT_LOG2E, b)) * inv;
+    const float g = (pr - (c == tgt ? 1.f : 0.f)) * gs;
     if constexpr (sizeof(T) == 4) d[c] = g; else d[c] = __float2bfloat16_rn(g);
   }
 }
