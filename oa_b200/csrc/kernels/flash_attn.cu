@@ -919,6 +919,9 @@ constexpr int FA_BWD_THREADS = 352;   // 8 softmax warps + 2 MMA issuer warps + 
 // At head dim 128 the columns leave room for one score tile, so the scores of tile i + 1 can only follow dV of tile i, and the next
 // exponentials wait for both: the issuer of dK and dP waits its turn until those scores are in the pipe (`turn`), and its products run under
 // the exponentials.  Left to themselves they ran beside dV and the scores, which took twice as long, and nothing under the exponentials.
+// A turn is given once per tile but an item's last, which has no scores behind it.  That the giver cannot be two turns ahead, when the barrier's
+// parity would read as none, follows from the ring: turn i + 1 is given behind the scores of tile i + 2, whose Q takes the place that dK of tile
+// i has left, and across items from the end of an item, which waits for the last dK.
 // The kernels are bound by that chain: at head dim 64 the exponentials take 1024 of about 2,400 clocks per tile, at head dim 128 the
 // products 2,080 of about 3,500, and a barrier that is already complete costs a warp 100 clocks or more while the pipes are busy.
 // dK, dV and dQ leave through store_rows; with 16-byte stores of a row to a lane the end of an item took 4,000 to 5,000 clocks, 15 to 20 %.
@@ -989,7 +992,7 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   uint64_t* dp_full = bars + 20;   // dP^T
   uint64_t* ds_full = bars + 21;   // [2]  dS^T, by column half (4 warps each)
   uint64_t* fin_full = bars + 23;  // dV, dK of the item are complete (both issuers arrive)
-  uint64_t* turn = bars + 24;      // NS == 1: the next tile's scores are in the pipe, dK and dP may follow
+  uint64_t* turn = bars + 24;      // NS == 1: the next tile's scores are in the pipe, dK and dP may follow (not for an item's last tile)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 25);
   float* stat = reinterpret_cast<float*>(smem + Cfg::OFF_STAT);
 
@@ -1149,8 +1152,8 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           __syncwarp();
         }
         if (!ok) break;
-        if (NS == 1) {
-          if (it + 1 < n_it) ok = issue_s(qc + 1, it + 2 == n_it);
+        if (NS == 1 && it + 1 < n_it) {
+          ok = issue_s(qc + 1, it + 2 == n_it);
           if (lane == 0) mbar_arrive(turn);
         }
       }
@@ -1162,7 +1165,7 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     constexpr uint32_t idesc_g = umma_idesc_bf16(FA_BN, HD, 0, 1);
     const uint64_t v_desc = desc_k(smem + Cfg::OFF_V), do_desc = desc_k(smem + Cfg::OFF_DO), q_desc = desc_mn(smem + Cfg::OFF_Q);
     const uint32_t dp_tm = tmem_base + Cfg::TM_DP;
-    uint32_t itc = 0, qc = 0;
+    uint32_t itc = 0, qc = 0, turns = 0;
     bool ok = true;
     auto issue_dp = [&](uint32_t n, bool last) -> bool {
       const int st = n % NST;
@@ -1194,7 +1197,10 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         const int st = qc % NST;
         if (!warp_wait(&q_full[st], (qc / NST) & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_FULL); ok = false; break; }
         const uint64_t bd = desc_at(q_desc, st * Cfg::T_BYTES);
-        if (NS == 1 && !warp_wait(turn, qc & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_EMPTY); ok = false; break; }
+        if (NS == 1 && it + 1 < n_it) {
+          if (!warp_wait(turn, turns & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_EMPTY); ok = false; break; }
+          ++turns;
+        }
         for (int half = 0; half < 2; ++half) {
           if (it == 0 && half == 0) ok = warp_wait(&ds_full[1], qc & 1);   // as for dV
           if (!ok || !warp_wait(&ds_full[half], qc & 1)) { if (lane == 0) report_error(p.status, OA_KERR_WAIT_SOFTMAX); ok = false; break; }
