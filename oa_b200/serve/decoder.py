@@ -57,17 +57,25 @@ class _GraphedStep:
         if begin is not None:
             begin(ids)
         if self.graph is None:
-            fn(self.ids)                              # eager once: lazily created buffers (workspaces) exist before the capture
-            if begin is None:
-                self.pos.sub_(1)
-            torch.cuda.synchronize()
-            g = torch.cuda.CUDAGraph()
-            # a replay begins after everything before it on the stream, so whatever changed the weights has finished by then
-            with torch.cuda.graph(g, capture_error_mode="thread_local"), K.weights_at_rest(weights()):
-                self.out = fn(self.ids)
-            self.graph = g
+            try:
+                self._record(fn, weights, begin is None)
+            except BaseException:
+                if begin is not None:
+                    self.pos.sub_(1)                  # no step was made: the next one begins where this one did
+                raise
         self.graph.replay()
         return self.out
+
+    def _record(self, fn, weights, counts: bool):
+        fn(self.ids)                                  # eager once: lazily created buffers (workspaces) exist before the capture
+        if counts:
+            self.pos.sub_(1)
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        # a replay begins after everything before it on the stream, so whatever changed the weights has finished by then
+        with torch.cuda.graph(g, capture_error_mode="thread_local"), K.weights_at_rest(weights()):
+            self.out = fn(self.ids)
+        self.graph = g
 
 
 class OaGptDecoder:
