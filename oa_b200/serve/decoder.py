@@ -100,8 +100,8 @@ class OaGptDecoder:
         """Whether every block is RMS norms, packed projections without biases and a gated feed-forward: the step then runs as products
         of a few rows that also do the norms' work (False once one of them has turned out not to fit)."""
         m = self.Model
-        if not isinstance(m.LnFinal, OaRmsNorm) or m.PosEmbed is not None:
-            return False
+        if not m.Blocks or not isinstance(m.LnFinal, OaRmsNorm) or m.PosEmbed is not None:
+            return False                              # without blocks there is no norm for the rows to begin with
         for b in m.Blocks:
             a = b.Attention
             if b.Moe is not None or b.FfnKind == "gelu" or not isinstance(b.LnAttn, OaRmsNorm) or a.RopeTheta <= 0:
