@@ -1129,11 +1129,13 @@ def few_rows_step(x: torch.Tensor, w: torch.Tensor, *, bias: Optional[torch.Tens
 
     `squares` [n, M] fp32: x is rows times a norm's weight, and the result is scaled by that norm's factor, rsqrt(sum(squares) / K + eps).
     `gated`: w holds gates and values, and the result is silu(gate) * value.  `norm_w`: returns (out, out * norm_w, squares of out)
-    for the norm behind.  None for shapes that the kernel leaves to others; nothing was done then."""
+    for the norm behind.  None for shapes, and weights in an order, that the kernel leaves to others; nothing was done then."""
     M, Kd = x.shape
     Nn = w.shape[0]
     cols = Nn // 2 if gated else Nn
-    assert x.dtype == w.dtype == torch.bfloat16 and x.stride(1) == 1 and w.stride(1) == 1 and w.shape[1] == Kd
+    assert x.dtype == w.dtype == torch.bfloat16 and x.stride(1) == 1 and w.shape[1] == Kd
+    if w.stride(1) != 1:
+        return None
     assert residual is None or (residual.shape == (M, cols) and residual.stride(1) == 1)
     lib = N.require()
     out = torch.empty((M, cols), dtype=x.dtype, device=x.device)
