@@ -21,19 +21,16 @@ def test_norm_behind_and_in_front(m, n, k):
     g = torch.Generator(device="cuda").manual_seed(m + n)
     r = lambda *s: torch.randn(*s, device="cuda", generator=g)
     x, w, res, nw = r(m, k).bfloat16(), (r(n, k) / k ** 0.5).bfloat16(), (3 * r(m, n)).bfloat16(), (1 + 0.2 * r(n)).bfloat16()
-    got = K.few_rows_step(x, w, residual=res, norm_w=nw)
-    if got is None:                                         # left to the tile kernels
-        assert K.few_rows_step(x, w) is None
-        return
-    out, out_w, sq = got
+    out, out_w, sq = K.few_rows_step(x, w, residual=res, norm_w=nw)      # all of these are the few-row kernel's
     y = x.double() @ w.double().t() + res.double()
     assert _rel(out, y) <= TOL
     assert torch.equal(out_w, (out.float() * nw.float()).bfloat16())
     assert _rel(sq.sum(0), (out.double() ** 2).sum(1)) <= 1e-5
     # the product behind: as if it had been given the normed rows
     w2, bias = (r(512, n) / n ** 0.5).bfloat16(), r(512).bfloat16()
-    if K.few_rows_step(out_w[:, :n], w2) is not None:
-        got2 = K.few_rows_step(out_w, w2, squares=sq, eps=1e-5, bias=bias)
+    got2 = K.few_rows_step(out_w, w2, squares=sq, eps=1e-5, bias=bias)
+    assert (got2 is None) == (n < 512)                       # reductions too short for it
+    if got2 is not None:
         o = out.double()
         normed = o * torch.rsqrt((o * o).mean(1, keepdim=True) + 1e-5) * nw.double()
         assert _rel(got2, normed @ w2.double().t() + bias.double()) <= TOL
@@ -48,10 +45,15 @@ def test_gated(m, f, k):
     r = lambda *s: torch.randn(*s, device="cuda", generator=g)
     x, w, sq = r(m, k).bfloat16(), (r(2 * f, k) / k ** 0.5).bfloat16(), r(3, m).abs()
     got = K.few_rows_step(x, w, squares=sq, eps=1e-6, gated=True)
-    if got is None:
-        assert K.few_rows_step(x, w) is None
-        return
     z = x.double() @ w.double().t() * torch.rsqrt(sq.double().sum(0) / k + 1e-6)[:, None]
     assert got.shape == (m, f) and _rel(got, torch.nn.functional.silu(z[:, :f]) * z[:, f:]) <= TOL
     torch.cuda.synchronize()
     K.check_status()
+
+
+# short reductions, few columns, many rows, wide and shallow weights for many rows (on 148 SMs), weights in another order
+@pytest.mark.parametrize("m,n,k", [(1, 512, 504), (1, 248, 512), (65, 512, 512), (64, 12288, 512), (33, 40960, 2048)])
+def test_left_to_others(m, n, k):
+    x, w = torch.randn(m, k, device="cuda").bfloat16(), torch.randn(n, k, device="cuda").bfloat16()
+    assert K.few_rows_step(x, w) is None
+    assert K.few_rows_step(x, torch.randn(k, 1024, device="cuda").bfloat16().t()) is None
