@@ -7,19 +7,20 @@
 // product is streamed through shared memory 32 rows at a time with an online softmax, so there is no
 // sequence-length cap and global memory is read in whole rows.
 //
-// Work split (all three kernels): a CTA of 128 threads owns 128 / (DS KS) rows of one (batch, head).  A row is shared by DS threads that
+// Work split (forward and both gradients): a CTA of 128 threads owns 128 / (DS KS) rows of one (batch, head).  A row is shared by DS threads that
 // keep 32 head dimensions each in registers (their partial dot products meet in shuffles) and by KS groups of those that take every
 // KS-th row of the other side, with a running maximum and sums of their own that meet once, at the end.  KS = 1 does the least
 // work per score; KS = 4 makes four times as many, shorter CTAs (which under the causal mask also skip more of the other side), lets
 // the next tile arrive through cp.async under this one, and is taken while KS = 1 would leave SMs idle (af_split).
 // 16 x 4 heads of 32 dimensions and 128 positions are 64 CTAs with KS = 1, one warp per scheduler: 29 us forward
-// and 83 us both gradients.  With KS = 4: 12.6 us, and 31 for both gradients (eight dimensions per thread, whose dot products each took
+// and 83 us both gradients.  With KS = 4: 12.6 us, and 25.7 for both gradients (eight dimensions per thread, whose dot products each took
 // two shuffles, were 2.5 and 15 us slower).
-// What bounds it: eight to twelve warps per SM, whose reads of shared memory and dot products wait for one another.  So the two gradients
-// run side by side: the CTAs of dQ, which needs nothing of dK and dV, start as soon as those of dK and dV are all under way, fill the room
-// that these leave, and end after them.  A row's own dimensions come in 16-byte pieces where the operands allow it, and under the causal
-// mask the longest CTAs start first.  Both gradients one after the other / side by side, us: 16 x 128 of 4 x 32 causal 37.8 / 31.2, 2 x 1024
-// of 4 x 64 full 469 / 320, 8 x 256 of 4 x 128 causal 254 / 201, 16 x 512 of 4 x 32 causal 270 / 255, 3 x 77 of 5 x 40 21.7 / 13.4.
+// What bounds it: eight to twelve warps per SM, whose reads of shared memory and dot products wait for one another.  So the two gradients,
+// neither of which needs the other, share one launch: the blocks of dQ fill the room that those of dK and dV leave.  A row's own dimensions
+// come in 16-byte pieces where the operands allow it, and under the causal mask the longest blocks of each kind start first.  Both gradients
+// as two launches one after the other / as one, us: 16 x 128 of 4 x 32 causal 37.8 / 25.7, 16 x 512 of 4 x 32 causal 270 / 224, 8 x 256 of 4 x 128
+// causal 254 / 179, 2 x 1024 of 4 x 64 full 469 / 358.  (As two launches of which the second began without a wait they took 31, 255, 201 and
+// 319; but what a kernel reads that does not wait for those before it, nothing promises.)
 // Forward and dQ rows are queries (keys / values stream through shared memory), dK / dV rows are keys (queries and output gradients
 // stream through shared memory together with their log-sum-exp and delta = rowsum(dO * O)).
 #include "common.cuh"
@@ -128,7 +129,7 @@ struct AfCfg {
   static constexpr int BUFS = ASYNC ? 2 : 1, TILE = AF_TILE * DS * AF_SEG;
 };
 
-// The two streamed matrices of all three kernels, tile by tile: body(j0, x tile, y tile) for j0 in [lo, hi) in steps of 32.
+// The two streamed matrices of each pass, tile by tile: body(j0, x tile, y tile) for j0 in [lo, hi) in steps of 32.
 template <int DS, int KS, typename Body>
 __device__ __forceinline__ void af_stream(float* sx, float* sy, const float* __restrict__ x, long long xs, const float* __restrict__ y, long long ys,
                                           long long row0, int lo, int hi, int limit, int col0, int hd, bool vec, Body body) {
@@ -229,18 +230,15 @@ attn_f32_fwd_kernel(const float* __restrict__ q, const float* __restrict__ k, co
   if (seg == 0 && ks == 0 && lse) lse[((long long)b * heads + h) * seq + i] = m + logf(l);
 }
 
-// dQ: rows are queries; K and V stream through shared memory.  Launched behind the kernel below, which allows this one's start only once
-// everything before both has ended; so there is nothing to wait for before the end, where whatever follows must find both kernels done.
+// dQ: rows are queries; K and V stream through shared memory.
 template <int DS, int KS>
-__global__ void __launch_bounds__(AF_THREADS)
-attn_f32_bwd_q_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
-                      const float* __restrict__ o, const float* __restrict__ dout, const float* __restrict__ lse,
-                      float* __restrict__ dq, int heads, int seq, int hd, long long rs, long long os, long long ds_, float scale,
-                      int causal, int vec) {
+__device__ __forceinline__ void af_bwd_q(float* sK, float* sV, int b, const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
+                                         const float* __restrict__ o, const float* __restrict__ dout, const float* __restrict__ lse,
+                                         float* __restrict__ dq, int heads, int seq, int hd, long long rs, long long os, long long ds_, float scale,
+                                         int causal, int vec) {
   using Cfg = AfCfg<DS, KS>;
   constexpr int NJ = AF_TILE / KS;
-  __shared__ __align__(16) float sK[Cfg::BUFS * Cfg::TILE], sV[Cfg::BUFS * Cfg::TILE];
-  const int h = blockIdx.y, b = blockIdx.z;
+  const int h = blockIdx.y;
   const int i0 = (gridDim.x - 1 - blockIdx.x) * Cfg::ROWS;       // under the causal mask the longest first
   const int i = i0 + threadIdx.x / Cfg::TPR, seg = threadIdx.x % DS, ks = threadIdx.x % Cfg::TPR / DS;
   const long long row0 = (long long)b * seq;
@@ -274,7 +272,6 @@ attn_f32_bwd_q_kernel(const float* __restrict__ q, const float* __restrict__ k, 
     }
   });
   af_scatter_sum<DS, KS>(acc, ks);
-  pdl_wait();                                                    // this grid ends after the other gradients'
   if (!row_ok) return;
 #pragma unroll
   for (int t = 0; t < AF_W / KS; ++t) {
@@ -285,18 +282,14 @@ attn_f32_bwd_q_kernel(const float* __restrict__ q, const float* __restrict__ k, 
 
 // dK, dV: rows are keys; Q and dO stream through shared memory with the queries' log-sum-exp and delta.
 template <int DS, int KS>
-__global__ void __launch_bounds__(AF_THREADS)
-attn_f32_bwd_kv_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
-                       const float* __restrict__ o, const float* __restrict__ dout, const float* __restrict__ lse,
-                       float* __restrict__ dk, float* __restrict__ dv, int heads, int seq, int hd, long long rs, long long os,
-                       long long ds_, float scale, int causal, int vec) {
+__device__ __forceinline__ void af_bwd_kv(float* sQ, float* sDO, int b, const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
+                                          const float* __restrict__ o, const float* __restrict__ dout, const float* __restrict__ lse,
+                                          float* __restrict__ dk, float* __restrict__ dv, int heads, int seq, int hd, long long rs, long long os,
+                                          long long ds_, float scale, int causal, int vec) {
   using Cfg = AfCfg<DS, KS>;
   constexpr int NI = AF_TILE / KS;
-  __shared__ __align__(16) float sQ[Cfg::BUFS * Cfg::TILE], sDO[Cfg::BUFS * Cfg::TILE];
   __shared__ float sL[2][AF_TILE], sDelta[2][AF_TILE];
-  pdl_wait();
-  pdl_launch_dependents();
-  const int h = blockIdx.y, b = blockIdx.z;
+  const int h = blockIdx.y;
   const int j0 = blockIdx.x * Cfg::ROWS;
   const int j = j0 + threadIdx.x / Cfg::TPR, seg = threadIdx.x % DS, ks = threadIdx.x % Cfg::TPR / DS;
   const long long row0 = (long long)b * seq;
@@ -366,23 +359,56 @@ attn_f32_bwd_kv_kernel(const float* __restrict__ q, const float* __restrict__ k,
   }
 }
 
+// Both gradients in one launch: the first half of the grid takes dK and dV, the second dQ.  (The halves of a sequence beside one another
+// put two of a kind on some SMs: 2 x 1024 of 4 x 64, full mask, 380 us for 358.)
+template <int DS, int KS>
+__global__ void __launch_bounds__(AF_THREADS)
+attn_f32_bwd_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
+                    const float* __restrict__ o, const float* __restrict__ dout, const float* __restrict__ lse, float* __restrict__ dq,
+                    float* __restrict__ dk, float* __restrict__ dv, int heads, int seq, int hd, long long rs, long long os,
+                    long long ds_, float scale, int causal, int vec) {
+  using Cfg = AfCfg<DS, KS>;
+  __shared__ __align__(16) float sx[Cfg::BUFS * Cfg::TILE], sy[Cfg::BUFS * Cfg::TILE];
+  pdl_wait();
+  const int batch = gridDim.z >> 1, b = blockIdx.z;
+  if (b < batch) af_bwd_kv<DS, KS>(sx, sy, b, q, k, v, o, dout, lse, dk, dv, heads, seq, hd, rs, os, ds_, scale, causal, vec);
+  else af_bwd_q<DS, KS>(sx, sy, b - batch, q, k, v, o, dout, lse, dq, heads, seq, hd, rs, os, ds_, scale, causal, vec);
+}
+
+// One gradient to a launch
+template <int DS, int KS, bool KV>
+__global__ void __launch_bounds__(AF_THREADS)
+attn_f32_bwd_part_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
+                         const float* __restrict__ o, const float* __restrict__ dout, const float* __restrict__ lse, float* __restrict__ dq,
+                         float* __restrict__ dk, float* __restrict__ dv, int heads, int seq, int hd, long long rs, long long os,
+                         long long ds_, float scale, int causal, int vec) {
+  using Cfg = AfCfg<DS, KS>;
+  __shared__ __align__(16) float sx[Cfg::BUFS * Cfg::TILE], sy[Cfg::BUFS * Cfg::TILE];
+  pdl_wait();
+  if (KV) af_bwd_kv<DS, KS>(sx, sy, blockIdx.z, q, k, v, o, dout, lse, dk, dv, heads, seq, hd, rs, os, ds_, scale, causal, vec);
+  else af_bwd_q<DS, KS>(sx, sy, blockIdx.z, q, k, v, o, dout, lse, dq, heads, seq, hd, rs, os, ds_, scale, causal, vec);
+}
+
 }  // namespace oa
 
 using namespace oa;
 
+// CTAs of the KS = 1 form
+static inline long long af_ctas(int hd, int batch, int heads, int seq) {
+  const int rows = AF_THREADS / (hd <= 32 ? 1 : (hd <= 64 ? 2 : 4));
+  return (long long)((seq + rows - 1) / rows) * heads * batch;
+}
+
 // DS, or -4 DS for KS = 4, which is taken up to `limit` CTAs of the KS = 1 form: one per SM, or somewhat more where the causal mask lets the
-// shorter CTAs skip work, and wherever a sequence would leave most rows of a wide CTA empty; in the backward pass of a full mask (`pair`) not where
-// the KS = 1 forms of both kernels fill the chip together, up to 148 CTAs each at two to an SM, from where KS = 4 needs a second wave.  KS = 1
-// against 4 (4 heads, us), forward, full mask, 14 x 128 of 64 dimensions (112 CTAs) 32.2 / 22.4, 48 x 128 of 32 (192) 29.8 / 31.0, 28 x 128 of 64 (224)
-// 34.4 / 37.7; causal 16 x 512 of 32 (256) 104 / 93, 36 x 128 of 64 (288) 35.2 / 35.6.  Backward, full, 18 x 128 of 32 (72) 43.6 / 35.0, 10 x 128 of 64 (80)
-// 47.2 / 39.7, 20 x 128 of 32 (80) 47.4 / 50.9, 5 x 512 of 32 (80) 143 / 176, 14 x 128 of 64 (112) 50 / 58, 2 x 1024 of 64 (128) 319 / 400, 40 x 128 of 32
-// (160) 91.5 / 83.7, 48 x 128 of 32 (192) 92 / 94; causal 16 x 512 of 32 (256) 261 / 255, 64 x 128 of 32 (256) 108 / 86, 36 x 128 of 64 (288) 99 / 100.
-// 100 x 16 of 64 (400) 11.6 / 6.8 and 40 / 20.
-static inline int af_split(int hd, int batch, int heads, int seq, int limit, bool pair = false) {
+// shorter CTAs skip work, and wherever a sequence would leave most rows of a wide CTA empty.  KS = 1 against 4 (4 heads, us), forward, full mask,
+// 14 x 128 of 64 dimensions (112 CTAs) 32.2 / 22.4, 48 x 128 of 32 (192) 29.8 / 31.0, 28 x 128 of 64 (224) 34.4 / 37.7; causal 16 x 512 of 32 (256) 104 / 93,
+// 36 x 128 of 64 (288) 35.2 / 35.6.  Backward, where a launch has twice the CTAs, full, 18 x 128 of 32 (72) 38.0 / 33.2, 24 x 128 of 32 (96) 49.9 / 45.6,
+// 3 x 1024 of 32 (96) 296 / 306, 3 x 512 of 64 (96) 185 / 179, 28 x 128 of 32 (112) 50.2 / 54.8, 14 x 128 of 64 (112) 55.5 / 61.2, 2 x 1024 of 64 (128) 359 / 480,
+// 48 x 128 of 32 (192) 73 / 86; causal 16 x 512 of 32 (256) 237 / 224, 64 x 128 of 32 (256) 93 / 77, 36 x 128 of 64 (288) 104 / 96, 48 x 128 of 64 (384) 129 / 125, but
+// 5 x 512 of 64 (160) 178 / 169, 8 x 512 of 64 (256) 247 / 254, 2 x 2048 of 64 (256) 856 / 914.
+static inline int af_split(int hd, int batch, int heads, int seq, int limit) {
   const int wide = hd <= 32 ? 1 : (hd <= 64 ? 2 : 4);
-  const long long ctas = (long long)((seq + AF_THREADS / wide - 1) / (AF_THREADS / wide)) * heads * batch;
-  const bool together = pair && ctas > (wide == 1 ? 74 : 80) && ctas <= 148;
-  return hd <= 64 && (seq <= AF_TILE || (ctas <= limit && !together)) ? -4 * wide : wide;
+  return hd <= 64 && (seq <= AF_TILE || af_ctas(hd, batch, heads, seq) <= limit) ? -4 * wide : wide;
 }
 
 // Whether every row of the streamed operands can be read in 16-byte pieces.
@@ -421,19 +447,30 @@ extern "C" int oa_attn_f32_bwd(const float* q, const float* k, const float* v, c
   if (batch <= 0 || heads <= 0 || seq <= 0) return OA_OK;
   if (heads > 65535 || batch > 65535) return OA_ERR_ARG;
   cudaStream_t st = (cudaStream_t)stream;
-  const int split = af_split(head_dim, batch, heads, seq, causal ? 300 : (seq > 128 ? 96 : 192), !causal), rows = AF_THREADS / (split < 0 ? -split : split);
-  dim3 grid((seq + rows - 1) / rows, heads, batch);
+  const int limit = !causal ? 96 : (head_dim > 32 && seq > 128 ? 240 : 300);
+  const int split = af_split(head_dim, batch, heads, seq, limit), rows = AF_THREADS / (split < 0 ? -split : split);
   const int vec = af_vec(head_dim, row_stride, o_row_stride, q, k, v, o, dout);
-#define AF_BWD(D, S)                                                                                                                        \
-  launch_short(attn_f32_bwd_kv_kernel<D, S>, grid, dim3(AF_THREADS), 0, st, q, k, v, o, dout, lse, dk, dv, heads, seq, head_dim, row_stride,  \
-               o_row_stride, d_row_stride, scale, causal, vec);                                                                             \
-  launch_short(attn_f32_bwd_q_kernel<D, S>, grid, dim3(AF_THREADS), 0, st, q, k, v, o, dout, lse, dq, heads, seq, head_dim, row_stride,       \
-               o_row_stride, d_row_stride, scale, causal, vec)
-  if (split == -4) { AF_BWD(1, 4); }
-  else if (split == -8) { AF_BWD(2, 4); }
-  else if (split == 1) { AF_BWD(1, 1); }
-  else if (split == 2) { AF_BWD(2, 1); }
-  else { AF_BWD(4, 1); }
+  // The registers of dK and dV leave room for two CTAs on an SM, those of dQ alone for three.  With a full mask and several waves that outweighs
+  // what the two kinds gain beside one another.  One launch / two, 4 heads of 64: 16 x 512 (512 CTAs) 691 / 661 us, 8 x 1024 1333 / 1233, 24 x 512 1018 / 904,
+  // but 12 x 512 (384) 506 / 524, 5 x 512 265 / 330; causal 24 x 512 629 / 631, 16 x 512 430 / 452; of 128, full, 16 x 512 1676 / 1732; of 32 433 / 536 for 24 x 512.
+  const bool apart = split == 2 && !causal && af_ctas(head_dim, batch, heads, seq) > 400;
+  const int most = apart ? 65535 : 32767;                // sequences in a grid, which holds each once or twice
+  for (int b0 = 0; b0 < batch; b0 += most) {
+    const int nb = batch - b0 < most ? batch - b0 : most;
+    const dim3 grid((seq + rows - 1) / rows, heads, apart ? nb : 2 * nb);
+    const long long at = (long long)b0 * seq, qa = at * row_stride, oa = at * o_row_stride, da = at * d_row_stride;
+#define AF_BWD(...)                                                                                                                          \
+  launch_short(__VA_ARGS__, grid, dim3(AF_THREADS), 0, st, q + qa, k + qa, v + qa, o + oa, dout + oa, lse + at * heads, dq + da, dk + da, dv + da, \
+               heads, seq, head_dim, row_stride, o_row_stride, d_row_stride, scale, causal, vec)
+    if (apart) {
+      AF_BWD((attn_f32_bwd_part_kernel<2, 1, true>));
+      AF_BWD((attn_f32_bwd_part_kernel<2, 1, false>));
+    } else if (split == -4) AF_BWD((attn_f32_bwd_kernel<1, 4>));
+    else if (split == -8) AF_BWD((attn_f32_bwd_kernel<2, 4>));
+    else if (split == 1) AF_BWD((attn_f32_bwd_kernel<1, 1>));
+    else if (split == 2) AF_BWD((attn_f32_bwd_kernel<2, 1>));
+    else AF_BWD((attn_f32_bwd_kernel<4, 1>));
+  }
 #undef AF_BWD
   return cudaGetLastError() == cudaSuccess ? OA_OK : OA_ERR_LAUNCH;
 }

@@ -1001,7 +1001,7 @@ def flash_bwd(q, k, v, o, dout, lse, batch: int, seq: int, heads: int, head_dim:
         return dq, dk, dv
     _launch(lib.oa_attn_f32_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), dout.data_ptr(), lse.data_ptr(),
                                 dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), batch, heads, seq, head_dim, q.stride(0),
-                                o.stride(0), dq.stride(0), float(scale), int(causal), N.stream()), "oa_attn_f32_bwd", 2)
+                                o.stride(0), dq.stride(0), float(scale), int(causal), N.stream()), "oa_attn_f32_bwd")
     return dq, dk, dv
 
 

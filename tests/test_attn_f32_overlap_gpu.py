@@ -1,4 +1,4 @@
-"""fp32 attention gradients whose two kernels run side by side: what comes before is read, what follows finds both done, eagerly and in a graph."""
+"""fp32 attention gradients beside their neighbours in a stream: what comes before is read, what follows finds both done, eagerly and in a graph."""
 import pytest
 import torch
 
@@ -7,8 +7,10 @@ from oa_b200.ops import kernels as K
 pytestmark = pytest.mark.gpu
 
 
-# blocks for a part of the chip, on both sides of a full mask's line and for several waves, the last tile ragged, every split of a row
-@pytest.mark.parametrize("batch,seq,heads,hd", [(1, 33, 1, 32), (16, 128, 4, 32), (18, 128, 4, 32), (19, 128, 4, 32), (40, 128, 4, 64), (2, 515, 4, 64), (3, 200, 2, 128), (64, 160, 4, 20)])
+# blocks for a part of the chip, on both sides of a full mask's lines and for several waves (both gradients in one launch, and in two), the last tile
+# ragged, every split of a row, more sequences than a grid holds twice
+@pytest.mark.parametrize("batch,seq,heads,hd", [(1, 33, 1, 32), (16, 128, 4, 32), (18, 128, 4, 32), (19, 128, 4, 32), (40, 128, 4, 64), (2, 515, 4, 64), (3, 200, 2, 128), (64, 160, 4, 20), (34, 130, 4, 64),
+                                               (33000, 2, 1, 4)])
 @pytest.mark.parametrize("causal", [False, True])
 def test_neighbours_in_the_stream(batch, seq, heads, hd, causal):
     D, rows = heads * hd, batch * seq
