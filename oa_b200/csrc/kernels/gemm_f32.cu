@@ -22,7 +22,7 @@
 namespace oa {
 
 constexpr int FT = 64, FK = 16;   // output tile width (and height of the plain kernel), columns of K per stage of the plain kernel
-constexpr int F_SMS = 148;
+int num_sms();
 
 struct F32Epi {
   const float *bias, *residual, *aux_in;
@@ -779,8 +779,8 @@ static bool gemm_f32_tiles(const float* A, const float* B, float* C, int M, int 
   const long long wide = (N + FT - 1) / FT, tiles = wide * ((M + 63) / 64) * z, tiles32 = wide * ((M + 31) / 32) * z;
   // Beyond one wave two blocks on an SM share it better than one after the other: 2048 x 384 x 128 11.3 us in the brief kernel, 12.3 in the
   // wide one, 2048 x 384 x 192 14.5 to 16.0 against 13.3 with two blocks.
-  const bool one_wave = tiles <= F_SMS;
-  const int rows = one_wave && (cluster || tiles32 <= F_SMS) ? 32 : 64;
+  const bool one_wave = tiles <= num_sms();
+  const int rows = one_wave && (cluster || tiles32 <= num_sms()) ? 32 : 64;
   const bool brief = !one_wave && (k_chunk > 0 ? k_chunk : K) < F_BRIEF_K;
   const dim3 grid((unsigned)wide, (M + rows - 1) / rows, z);
   if (grid.y > 65535) return false;
@@ -850,7 +850,7 @@ static int f32_cluster(int M, int N, int K, int batch, int* k_chunk) {
   int unused = 0;
   const long long tiles64 = (long long)((N + FT - 1) / FT) * ((M + FT - 1) / FT);
   const int chunk = ((K + s - 1) / s + 3) / 4 * 4;
-  const int most = !filled ? 128 : tiles64 * f32_splits(M, N, K, batch, &unused) > F_SMS ? 768 : s >= 4 ? 256 : 0;
+  const int most = !filled ? 128 : tiles64 * f32_splits(M, N, K, batch, &unused) > num_sms() ? 768 : s >= 4 ? 256 : 0;
   if (chunk > most) return 1;
   *k_chunk = chunk;
   return s;
