@@ -778,8 +778,10 @@ static bool gemm_f32_tiles(const float* A, const float* B, float* C, int M, int 
   const int z = k_chunk > 0 ? slices : batch;
   const long long wide = (N + FT - 1) / FT, tiles = wide * ((M + 63) / 64) * z, tiles32 = wide * ((M + 31) / 32) * z;
   // Beyond one wave two blocks on an SM share it better than one after the other: 2048 x 384 x 128 11.3 us in the brief kernel, 12.3 in the
-  // wide one, 2048 x 384 x 192 14.5 to 16.0 against 13.3 with two blocks.
-  const bool one_wave = tiles <= num_sms();
+  // wide one, 2048 x 384 x 192 14.5 to 16.0 against 13.3 with two blocks.  Up to eight columns of K one of the wide kernel's groups has all the
+  // work and the others' sums are only added up: 20 x 48 x 8 2.77 us wide, 2.07 brief (the same sums), 2048 x 128 x 4 3.49 / 2.95; with A
+  // row-contiguous 2.65 / 2.62 and, 64 x 64, 2.70 / 2.79.
+  const bool one_wave = tiles <= num_sms() && (K > 8 || !a_k);
   const int rows = one_wave && (cluster || tiles32 <= num_sms()) ? 32 : 64;
   const bool brief = !one_wave && (k_chunk > 0 ? k_chunk : K) < F_BRIEF_K;
   const dim3 grid((unsigned)wide, (M + rows - 1) / rows, z);

@@ -13,9 +13,10 @@ def _rel(got, want):
     return float((got.double() - want).norm() / want.norm())
 
 
-# 32-row tiles for exactly the chip and one more, 64-row tiles likewise; clusters of eight, four and two, with slices off four columns; the sizes around each line
+# 32-row tiles for exactly the chip and one more, 64-row tiles likewise; clusters of eight, four and two, with slices off four columns; the sizes around each line; eight
+# columns of K and nine
 SHAPES = [(1, 1, 4), (148 * 32, 64, 40), (148 * 32 + 1, 60, 40), (148 * 64, 64, 33), (148 * 64 + 1, 64, 33), (130, 130, 300),
-          (128, 128, 513), (100, 190, 1021), (65, 385, 1024), (512, 128, 1537), (512, 130, 3000), (64, 1024, 700), (33, 2048, 1536)]
+          (20, 48, 8), (20, 48, 9), (2048, 130, 5), (128, 128, 513), (100, 190, 1021), (65, 385, 1024), (512, 128, 1537), (512, 130, 3000), (64, 1024, 700), (33, 2048, 1536)]
 
 
 @pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, False), (True, True)])
