@@ -40,12 +40,15 @@ int oa_gemm_bf16(const void* A, const void* B, void* out, int M, int N, int K, i
                  int b_mn, const void* bias, const void* residual, int ldr, void* aux_out, const void* aux_in,
                  int ldaux, int act, int out_f32, int accumulate, float alpha, void* workspace,
                  size_t workspace_bytes, int force_bn, int* status, void* stream);
-// y = act(alpha x W^T + bias) + residual for at most 64 rows of x; OA_ERR_UNSUPPORTED where oa_gemm_bf16 takes a tile kernel.
-// w_at_rest: nothing still in flight on the stream writes W.
+// Sums of squares by tile that oa_few_rows_step leaves for N columns.
 int oa_few_rows_tiles(int N);
+// One product of a decoding step with the RMS norms around it: x W^T scaled by the factor of the norm in front (squares_in), + bias + residual,
+// and for the norm behind also times norm_w with the rows' sums of squares; or, gated, silu(gate) * value.  OA_ERR_UNSUPPORTED as below.
 int oa_few_rows_step(const void* x, const void* w, void* out, int M, int N, int K, int ldx, int ldw, int ldc, const void* bias, const void* residual,
                      int ldr, int gated, const void* norm_w, void* out_w, float* squares_out, const float* squares_in, int n_squares, float eps,
                      int w_at_rest, int* status, void* stream);
+// y = act(alpha x W^T + bias) + residual for at most 64 rows of x; OA_ERR_UNSUPPORTED where oa_gemm_bf16 takes a tile kernel.
+// w_at_rest: nothing still in flight on the stream writes W.
 int oa_gemm_bf16_few_rows(const void* x, const void* w, void* out, int M, int N, int K, int ldx, int ldw, int ldc,
                           const void* bias, const void* residual, int ldr, int act, int out_f32, float alpha, int w_at_rest,
                           int* status, void* stream);
@@ -254,9 +257,11 @@ int oa_upsample_nearest(int dtype, const void* in, void* out, long long planes, 
 // ---- KV-cache serving (decode.cu)
 int oa_kv_append(const void* k_src, const void* v_src, long long src_stride, void* k_cache, void* v_cache, int batch,
                  int s_new, int heads, int head_dim, int pos0, int max_seq, const int* pos_dev, void* stream);
-// Rotate-half embedding of q and k of one new token per sequence (x rows q | k | v) in place, and the append of k and v.
+// What comes before a replayed step: rows of the table by id, the position moved on by one, and for a norm behind the rows times its weight and
+// their sums of squares.
 int oa_decode_begin(const void* table, const int* ids, void* x, int* pos, int n_ids, int dim, int vocab, const void* norm_w, void* x_w,
                     float* squares, void* stream);
+// Rotate-half embedding of q and k of one new token per sequence (x rows q | k | v) in place, and the append of k and v.
 int oa_rope_kv_append(void* x, long long row_stride, int batch, int heads, int head_dim, int pos, float theta,
                       const int* pos_dev, void* k_cache, void* v_cache, int max_seq, void* stream);
 int oa_decode_attn(const void* q, long long q_stride, const void* k_cache, const void* v_cache, void* out, long long out_stride,

@@ -43,8 +43,8 @@ __device__ __forceinline__ void pair_sync(int quad) {
 }
 
 // Two exponentials 2^x on the multiply-add pipe: x = n + f with n the nearest integer (added and taken off at 1.5 * 2^23), 2^f by the
-// minimax polynomial of degree 5 on [-1/2, 1/2] (relative error 7.5e-8, 2.1e-7 with the rounding of its steps; ex2.approx states 2^-22 =
-// 2.4e-7), 2^n as an exponent field, which is zero at n = -127: below that, -inf included, the result is 0 as ex2.approx.ftz gives it.
+// minimax polynomial of degree 5 on [-1/2, 1/2] (Remez exchange on the relative error: 7.5e-8, with coefficients rounded to fp32 1.55e-7,
+// 2.1e-7 with the rounding of its steps; ex2.approx states 2^-22 = 2.4e-7), 2^n as an exponent field, which is zero at n = -127: below that, -inf included, the result is 0 as ex2.approx.ftz gives it.
 // NaN stays NaN; x up to 127.
 __device__ __forceinline__ unsigned long long f2_splat(float v) { return f2_of(__float_as_uint(v), __float_as_uint(v)); }
 __device__ __forceinline__ float max_nan(float a, float b) {
@@ -800,6 +800,8 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         uint32_t o[32];
         tmem_ld32(o_addr + c * 32, o);
         tmem_ld_wait();
+        // At head dim 64 a row's 16 bytes to a lane are the faster: 8 x 2048 x 16 causal 109.0 us (115.6 through store_rows), 1 x 4096 x 16 full
+        // 103.2 (114.3), 32 x 256 x 16 23.0 (24.1), 64 x 128 x 16 full 21.2 (22.8)
         if (ALIAS) store_rows(op + c * 32, p.o_stride, p.seq - q0, o, inv, lane);
         else if (qi < p.seq) {
           __nv_bfloat16* od = p.o + (long long)(row0 + qi) * p.o_stride + h * HD + c * 32;
