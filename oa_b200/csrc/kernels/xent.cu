@@ -111,17 +111,18 @@ xent_kernel(const T* __restrict__ logits, const int* __restrict__ targets, float
 
 // The same with the row kept on the chip, so that the logits are read once.  Rows of up to XENT_SMEM_MAX bytes: the row goes
 // to shared memory through cp.async; every thread reads back only the 16-byte vectors that it copied itself, so no barrier
-// stands between the copy and its use, and the gradient can be written over the logits.  The row arrives in four groups of copies, and a
-// thread takes the exponentials of a group against a maximum of its own while the others are on their way.  What bounds it: one read and
-// one write of the logits, beside the exponentials (two to a logit, 230 us of 16384 x 32000 by themselves) and the instructions around
-// them, of which few are left: with a subtraction, a product and the other steps one element at a time they were 177 per 8 logits and
-// the issue slots 82 % taken.  The CTAs of an SM (three at 64,000-byte rows) cover one another's reductions.  16384 x 32000 bf16: 475 us with two
-// reads, 403 us with one and the maximum found before the exponentials, 382 us with the groups, 361 us (5.8 TB/s) with packed
-// multiply-adds throughout; 8192 x 50264 331 -> 314 -> 295, 32768 x 8192 205 -> 180 -> 172, 4096 x 32000 110 -> 104 -> 99, 4096 x 16384 fp32 83.4 -> 83.9 -> 84.5.
+// stands between the copy and its use, and the gradient can be written over the logits.  A thread takes the exponentials of its vectors
+// against a maximum of its own, in one pass.  What bounds it: one read and one write of the logits, beside the exponentials (two to a logit,
+// 230 us of 16384 x 32000 by themselves) and the instructions around them, of which few are left: with a subtraction, a product and the other
+// steps one element at a time they were 177 per 8 logits and the issue slots 82 % taken.  The CTAs of an SM (three at 64,000-byte rows) cover
+// one another's waits; with the copy in four groups, each worked on as it landed, rows took longer (the figures below), short ones and fp32 most.
+// us, two passes over the row on the chip one element at a time / one pass, packed, in four groups / now: 16384 x 32000 bf16 401 / 357 / 332 (6.3 TB/s;
+// 475 with two reads of the logits), 8192 x 50264 338 / 302 / 300, 32768 x 8192 209 / 175 / 165, 16384 x 4096 65 / 60 / 52, 500 x 32000 19.6 / 18.6 / 16.5; fp32
+// 4096 x 16384 83.3 / 83.9 / 82.5, 8192 x 2048 24.7 / 26.8 / 22.7, 2048 x 5000 14.6 / 16.5 / 14.5.
 // A quarter of the exponentials on the multiply-add pipe made it slower (382 -> 406).
 // Errors against 64 bits, standard deviation 2, subtraction first and probabilities from the rounded log-sum-exp / now: fp32 gradients over
-// 4096 columns 3.3e-7 / 1.3e-7, over 32000 3.8e-7 / 1.7e-7; losses 4.6e-7 / 4.2e-7; the same time (357 / 354 us for 16384 x 32000 bf16) as with a
-// product of m and log2(e) rounded into every term, whose gradients were at 5.5e-7 and wrong far from zero.
+// 4096 columns 3.3e-7 / 1.3e-7, over 32000 3.8e-7 / 1.7e-7; losses 4.6e-7 / 4.2e-7.  With a product of m and log2(e) rounded into every term the
+// gradients were at 5.5e-7, and wrong far from zero.
 __device__ __forceinline__ void xent_cp16(void* smem_dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_dst)), "l"(src) : "memory");
 }
@@ -270,14 +271,8 @@ xent_smem_kernel(const T* __restrict__ logits, const int* __restrict__ targets, 
   const long long row = blockIdx.x;
   const T* p = logits + row * ld;
   const int tid = threadIdx.x, nvec = vocab / V;
-  const int piece = (nvec + 4 * THREADS - 1) / (4 * THREADS) * THREADS;     // vectors per copy group
-#pragma unroll
-  for (int g = 0; g < 4; ++g) {
-    const int end = min(nvec, (g + 1) * piece);
-#pragma unroll 2
-    for (int i = g * piece + tid; i < end; i += THREADS) xent_cp16(srow + i * V, p + i * V);
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  }
+  for (int i = tid; i < nvec; i += THREADS) xent_cp16(srow + i * V, p + i * V);
+  asm volatile("cp.async.commit_group;" ::: "memory");
   const int tgt = targets[row];
   const bool ignored = (tgt == ignore_index);
   const bool oor = !ignored && (tgt < 0 || tgt >= vocab);
@@ -290,16 +285,9 @@ xent_smem_kernel(const T* __restrict__ logits, const int* __restrict__ targets, 
     if (v > m) xent_raise(v, m, b, s2);
     s2 = f2_add(s2, f2_of(__float_as_uint(fast_exp2(fmaf(v, XENT_LOG2E, b))), 0u));
   }
-#pragma unroll
-  for (int g = 0; g < 4; ++g) {
-    if (g == 0) asm volatile("cp.async.wait_group 3;" ::: "memory");
-    else if (g == 1) asm volatile("cp.async.wait_group 2;" ::: "memory");
-    else if (g == 2) asm volatile("cp.async.wait_group 1;" ::: "memory");
-    else asm volatile("cp.async.wait_group 0;" ::: "memory");
-    const int end = min(nvec, (g + 1) * piece);
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
 #pragma unroll 2
-    for (int i = g * piece + tid; i < end; i += THREADS) xent_vec_add<T>(srow + i * V, m, b, s2);
-  }
+  for (int i = tid; i < nvec; i += THREADS) xent_vec_add<T>(srow + i * V, m, b, s2);
   uint32_t s_lo, s_hi;
   f2_to(s2, s_lo, s_hi);
   const float mw = warp_max(m), bw = xent_base(mw);

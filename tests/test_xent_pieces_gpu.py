@@ -1,4 +1,4 @@
-"""Cross-entropy with the row in shared memory: it arrives in four pieces that are worked on as they land, with a running maximum per thread."""
+"""Cross-entropy with the row in shared memory, with a running maximum per thread."""
 import pytest
 import torch
 
@@ -8,7 +8,7 @@ pytestmark = pytest.mark.gpu
 LOWEST = float(torch.finfo(torch.bfloat16).min)
 
 
-# a row that fills no piece, pieces of one vector per thread and of several, an odd number of vectors, a remainder off the vectors
+# one vector per thread and several, an odd number of vectors, a remainder off the vectors
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("vocab", [4104, 4112, 8192, 16392, 20003, 32008])
 @pytest.mark.parametrize("kind", ["random", "rising", "falling", "masked"])
